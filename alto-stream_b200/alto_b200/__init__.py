@@ -37,8 +37,8 @@ OK, ERR_INVALID, ERR_CUDA, ERR_NOMEM, ERR_NOT_SPD, ERR_UNSUPPORTED, ERR_TIMEOUT 
 F32, BF16, F64 = 0, 1, 2
 AUTO, ATOMIC, STAGED, STREAM, SORTED, DETERMINISTIC = range(6)
 FEED_BULK = 0x100  # OR with ATOMIC / SORTED: line streamed through shared memory by bulk copy
-FEED_DENSE = 0x200  # OR with SORTED (3 modes): the walk compiled for five blocks per SM
-FEED_FIXED_TARGET = 0x400  # OR with SORTED (3 modes): as FEED_DENSE, compiled once per target mode
+FEED_DENSE = 0x200  # OR with SORTED (3 modes): accepted, the one row-sorted walk runs
+FEED_FIXED_TARGET = 0x400  # OR with SORTED (3 modes): accepted, the one row-sorted walk runs
 UNCONSTRAINED, NONNEG, LASSO = range(3)
 CPSTREAM, SPCPSTREAM = range(2)  # streaming models (alto_stream_set_model)
 FIT_REFERENCE, FIT_EXACT = 0, 1

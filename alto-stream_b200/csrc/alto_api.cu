@@ -295,7 +295,7 @@ alto_status alto_tensor_device_bytes(const alto_tensor* t, uint64_t* bytes) {
   }
   uint64_t b = t->line.bytes + t->perm.bytes + t->tile_iv.bytes + t->prtn_iv.bytes + t->scratch.bytes +
                t->scan_scratch.bytes + t->err.bytes;
-  for (int m = 0; m < ALTO_MAX_MODES; ++m) b += t->sorted[m].line.bytes + t->sorted[m].tile_iv.bytes;
+  for (int m = 0; m < ALTO_MAX_MODES; ++m) b += t->sorted[m].line.bytes + t->sorted[m].extra.bytes + t->sorted[m].tile_iv.bytes;
   *bytes = b;
   return ALTO_OK;
 }
@@ -363,7 +363,7 @@ alto_status alto_mttkrp_variant_run(alto_tensor* t, int mode, const void* const*
     return ALTO_ERR_INVALID;
   }
   return run_mttkrp_feed(t, mode, factors, fdtype, rank, out, accumulate, v,
-                         v == ALTO_MTTKRP_AUTO ? -1 : (fixed ? 3 : dense ? 2 : bulk), (cudaStream_t)stream);
+                         v == ALTO_MTTKRP_AUTO ? -1 : bulk, (cudaStream_t)stream);
 }
 
 alto_status alto_mttkrp_autotune(alto_tensor* t, const void* const* factors, alto_dtype fdtype,

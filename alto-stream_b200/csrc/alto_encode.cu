@@ -900,18 +900,25 @@ __global__ void gather_line_kernel(const uint4* __restrict__ line, int words,
   }
 }
 
-// Gather line records in the given order, writing them with the rows
-// decoded (3-mode lines): {row 0, row 1, row 2, value}.
-__global__ void gather_decode3_kernel(const void* __restrict__ line, LineDecode dec,
-                                      const uint32_t* __restrict__ order, uint32_t nnz,
-                                      uint4* __restrict__ out) {
+// Gather line records in the given order (order NULL: as they are), writing
+// them decoded (kDecoded) for target mode `mode` of N.
+template <int N>
+__global__ void gather_decode_kernel(const void* __restrict__ line, LineDecode dec, int mode,
+                                     const uint32_t* __restrict__ order, uint32_t nnz, uint4* __restrict__ out,
+                                     void* __restrict__ extra) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += gridDim.x * blockDim.x) {
     uint64_t lo, hi;
     float v;
-    rec_read(line, dec.hi_words, order[i], lo, hi, v);
-    out[i] = make_uint4((uint32_t)line_field(lo, hi, dec.pos[0], dec.mask[0]),
-                        (uint32_t)line_field(lo, hi, dec.pos[1], dec.mask[1]),
-                        (uint32_t)line_field(lo, hi, dec.pos[2], dec.mask[2]), __float_as_uint(v));
+    rec_read(line, dec.hi_words, order ? order[i] : i, lo, hi, v);
+    uint32_t r[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      const int m = j == N - 1 ? mode : (j < mode ? j : j + 1);
+      r[j] = (uint32_t)line_field(lo, hi, dec.pos[m], dec.mask[m]);
+    }
+    out[i] = make_uint4(r[0], r[1], r[2], N == 3 ? __float_as_uint(v) : r[N > 3 ? 3 : 0]);
+    if (N == 4) static_cast<float*>(extra)[i] = v;
+    if (N == 5) static_cast<uint2*>(extra)[i] = make_uint2(r[N - 1], __float_as_uint(v));
   }
 }
 
@@ -984,9 +991,10 @@ alto_status build_sorted_line(alto_tensor* t, int mode, cudaStream_t st) {
   SortedLine& s = t->sorted[mode];
   const uint64_t nnz = t->nnz;
   const int hw = t->dec.hi_words;
-  // 3-mode copies store the rows decoded (same 16 bytes per record)
-  s.hw = t->nmodes == 3 ? kDecoded3 : hw;
+  s.hw = decoded_modes(t->nmodes) ? kDecoded : hw;
   ALTO_TRY(tensor_ensure(t, s.line, (nnz + kLinePad) * rec_bytes(s.hw)));
+  if (s.hw == kDecoded && t->nmodes > 3)
+    ALTO_TRY(tensor_ensure(t, s.extra, (nnz + kLinePad) * decoded_extra_bytes(t->nmodes)));
   const size_t cap = std::max<uint64_t>(nnz, 1);
   size_t off = 0;
   size_t o_r0 = off; off = align_up(off + cap * 8, 256);
@@ -1008,9 +1016,13 @@ alto_status build_sorted_line(alto_tensor* t, int mode, cudaStream_t st) {
     uint64_t* nohi[2] = {nullptr, nullptr};
     ALTO_TRY(radix_sort_pairs(rk, nohi, pm, n32, t->mode_bits[mode], sort_scratch,
                               t->err.as<int>() + kSortErrorWord, st, &cur));
-    if (s.hw == kDecoded3)
-      gather_decode3_kernel<<<grid_for(nnz, 256), 256, 0, st>>>(t->line.p, t->dec, pm[cur], n32,
-                                                                 s.line.as<uint4>());
+    const unsigned gg = grid_for(nnz, 256);
+    if (s.hw == kDecoded && t->nmodes == 3)
+      gather_decode_kernel<3><<<gg, 256, 0, st>>>(t->line.p, t->dec, mode, pm[cur], n32, s.line.as<uint4>(), s.extra.p);
+    else if (s.hw == kDecoded && t->nmodes == 4)
+      gather_decode_kernel<4><<<gg, 256, 0, st>>>(t->line.p, t->dec, mode, pm[cur], n32, s.line.as<uint4>(), s.extra.p);
+    else if (s.hw == kDecoded)
+      gather_decode_kernel<5><<<gg, 256, 0, st>>>(t->line.p, t->dec, mode, pm[cur], n32, s.line.as<uint4>(), s.extra.p);
     else
       gather_line_kernel<<<grid_for(nnz, 256), 256, 0, st>>>(t->line.as<uint4>(), rec_bytes(hw) / 16,
                                                              pm[cur], n32, s.line.as<uint4>());
@@ -1020,7 +1032,7 @@ alto_status build_sorted_line(alto_tensor* t, int mode, cudaStream_t st) {
   ALTO_TRY(tensor_ensure(t, s.tile_iv, (size_t)std::max<uint32_t>(t->ntiles, 1) * t->nmodes * 2 * 4));
   // (tile intervals are read only by shared-memory staging, which never
   // walks a sorted copy; the decoded copies carry none)
-  if (t->ntiles && s.hw != kDecoded3) {
+  if (t->ntiles && s.hw != kDecoded) {
     tile_interval_kernel<<<t->ntiles, 256, 0, st>>>(s.line.p, t->dec, n32, t->tile_nnz,
                                                     s.tile_iv.as<uint32_t>());
     ALTO_LAUNCHED();

@@ -13,7 +13,8 @@ struct FactorSet {
 };
 
 struct MttkrpArgs {
-  const void* line;  // line records (LineRec16 / LineRec32)
+  const void* line;   // line records (LineRec16 / LineRec32, or kDecoded's first array)
+  const void* extra;  // kDecoded: the records' second array
   // DETERMINISTIC: per lane-group sub-range, its first and last run (slots
   // 2s and 2s+1: output row and R partial sums)
   uint32_t* det_rows;
@@ -29,6 +30,7 @@ struct MttkrpArgs {
   uint32_t chunk_tiles;
   LineDecode dec;
   FactorSet fac;
+  FactorSet in;  // the input modes' factors in mode order (kDecoded walks)
   float* out;
 };
 

@@ -173,11 +173,21 @@ struct __align__(16) LineRec32 {
   uint32_t pad[3];
 };
 
-// Record format code 3: a 3-mode record with the rows stored decoded,
-// {row of mode 0, row of mode 1, row of mode 2, value} (16 bytes); used for
-// the row-sorted copies of 3-mode lines, where the kernels then skip the
-// bit-field decode.
-constexpr int kDecoded3 = 3;
+// Record format code 3, of the row-sorted copies of 3- to 5-mode lines: the
+// rows stored decoded, those of the input modes (every mode but the sorted
+// one) first, in mode order, then the sorted mode's row, then the value; 16
+// bytes per record in a first array and the rest in a second one:
+//   3 modes {in 0, in 1, row, value}
+//   4 modes {in 0, in 1, in 2, row}        {value}
+//   5 modes {in 0, in 1, in 2, in 3}       {row, value}
+// The walks then need no bit-field decode and no selection of the target
+// among the modes: on the 5-mode tensor these were two thirds of the walk's
+// instructions, which is what bounded it (64 warp instructions per nonzero at
+// rank 64, issue slots 70% busy, DRAM 4%).
+constexpr int kDecoded = 3;
+__host__ __device__ __forceinline__ bool decoded_modes(int nmodes) { return nmodes >= 3 && nmodes <= 5; }
+// Bytes per record of the second array.
+__host__ __device__ __forceinline__ int decoded_extra_bytes(int nmodes) { return (nmodes - 3) * 4; }
 
 __host__ __device__ __forceinline__ int rec_bytes(int hi_words) { return hi_words == 2 ? 32 : 16; }
 
@@ -234,7 +244,8 @@ namespace alto {
 // A copy of the line ordered by one mode's row (see build_sorted_line).
 struct SortedLine {
   DevBuf line, tile_iv;
-  int hw = 0;  // record format: the line's hi_words, or kDecoded3
+  DevBuf extra;  // kDecoded: the records' second array
+  int hw = 0;    // record format: the line's hi_words, or kDecoded
   uint32_t ntiles = 0;
   uint64_t for_nnz = 0;
   bool ready = false;
@@ -244,8 +255,7 @@ struct SortedLine {
 struct TuneEntry {
   int mode, rank, fdtype;
   alto_mttkrp_variant variant;
-  int feed;  // 0 direct, 1 line streamed through shared memory by bulk copy, 2 direct at five blocks per SM,
-             // 3 as 2 with the target mode fixed at compile time
+  int feed;  // 0 direct, 1 line streamed through shared memory by bulk copy (ATOMIC)
 };
 }  // namespace alto
 

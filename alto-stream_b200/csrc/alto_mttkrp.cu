@@ -22,10 +22,12 @@
 //     the single-row output of the stream mode is its degenerate case); or
 //   * to global memory with 16-byte vector atomics (red.global.add.v4.f32),
 //     the reference's atomic variant (ATOMIC); or
-//   * (SORTED) the same kernel walks a per-mode copy of the line ordered by
-//     the output row (ALTO order among equal rows), so every run of a row is
+//   * (SORTED) the walk runs over a per-mode copy of the line ordered by the
+//     output row (ALTO order among equal rows), so every run of a row is
 //     contiguous, reduces in registers, and is written once per warp chunk --
-//     the reference's op_sched traversal, materialised.
+//     the reference's op_sched traversal, materialised.  The copies of 3- to
+//     5-mode lines hold their rows decoded and have a walk of their own
+//     (walk_kernel).
 // ALTO_MTTKRP_AUTO uses the autotuned choice when alto_mttkrp_autotune has
 // measured one, else a rule on the tile intervals and the mode's reuse.
 #include <algorithm>
@@ -75,12 +77,9 @@ __device__ __forceinline__ uint32_t field32(uint32_t w0, uint32_t w1, uint32_t w
   return v & mask;
 }
 
-// Row of mode m of a record held as words w (HW = kDecoded3: stored
-// decoded; else the field of the mode-contiguous key).
-template <int HW>
+// Row of mode m of a record held as words w (the field of the
+// mode-contiguous key).
 __device__ __forceinline__ uint32_t rec_row(const uint32_t (&w)[4], const LineDecode& dec, int m) {
-  // (selects, not w[m]: a runtime index would move w to local memory)
-  if (HW == kDecoded3) return m == 0 ? w[0] : (m == 1 ? w[1] : w[2]);
   return field32(w[0], w[1], w[2], w[3], dec.pos[m], (uint32_t)dec.mask[m]);
 }
 
@@ -208,16 +207,12 @@ struct OpenRun {
   float acc[V];
 };
 
-// TGT >= 0 (decoded 3-mode records only) fixes the target mode at compile
-// time: the target and input rows are then fixed words of the record and the
-// input factors fixed arguments, with no per-nonzero selects or mode checks.
-template <int R, typename FT, int HW, int NM, bool SMEM, bool DET = false, bool CARRY = false, int TGT = -1>
+template <int R, typename FT, int HW, int NM, bool SMEM, bool DET = false, bool CARRY = false>
 __device__ __forceinline__ void warp_range(const MttkrpArgs& a, const void* line, uint32_t ws, uint32_t we,
                                            bool staged, float* smem, uint32_t iv_start, uint32_t sr_base = 0,
                                            OpenRun<LaneWidth<R>::V>* carry = nullptr) {
-  static_assert(TGT < 0 || (HW == kDecoded3 && NM == 3), "a compile-time target needs decoded 3-mode records");
   using LW = LaneWidth<R>;
-  const int target = TGT >= 0 ? TGT : a.target;
+  const int target = a.target;
   constexpr int V = LW::V, G = LW::G, NPW = LW::NPW;
   // nonzeros per step: 2 for 3 modes (4 measured faster for DET only), 1
   // beyond (two measured 30% slower on the rank-64 5-mode tensor: its four
@@ -258,8 +253,8 @@ __device__ __forceinline__ void warp_range(const MttkrpArgs& a, const void* line
 #pragma unroll
       for (int j = 0; j < NM - 1; ++j) {
         const int m = j < target ? j : j + 1;
-        if ((TGT >= 0 || m < a.dec.nmodes) && valid[u]) {
-          const uint32_t r = rec_row<HW>(w[u], a.dec, m);
+        if (m < a.dec.nmodes && valid[u]) {
+          const uint32_t r = rec_row(w[u], a.dec, m);
           load_row<FT, V, G>(a.fac.f[m], (size_t)r * R, sub, f[u][j]);
         }
       }
@@ -269,7 +264,7 @@ __device__ __forceinline__ void warp_range(const MttkrpArgs& a, const void* line
     bool ok[U];
 #pragma unroll
     for (int u = 0; u < U; ++u) {
-      rows[u] = rec_row<HW>(w[u], a.dec, target);
+      rows[u] = rec_row(w[u], a.dec, target);
       vals[u] = v[u];
       ok[u] = valid[u];
     }
@@ -357,7 +352,7 @@ __device__ __forceinline__ void warp_range(const MttkrpArgs& a, const void* line
     bool ok0[1];
     const uint32_t at = gs > 0 ? gs - 1 : 0;
     load_keys<HW, 1, SMEM>(line, at, at + 1, w0, v0, ok0);
-    const uint32_t r0 = rec_row<HW>(w0[0], a.dec, a.target);
+    const uint32_t r0 = rec_row(w0[0], a.dec, a.target);
     det_slot<R, V, G>(a, slot0, r0, sub, acc, true);
     det_slot<R, V, G>(a, slot0 + 1, r0, sub, acc, true);
   } else if (nrun == 0) {
@@ -368,8 +363,8 @@ __device__ __forceinline__ void warp_range(const MttkrpArgs& a, const void* line
   }
 }
 
-template <int R, typename FT, int HW, bool STAGE, int NM, bool DET = false, int MINB = 3, int TGT = -1>
-__global__ void __launch_bounds__(kMttkrpThreads, MINB)
+template <int R, typename FT, int HW, bool STAGE, int NM, bool DET = false>
+__global__ void __launch_bounds__(kMttkrpThreads, 3)
     mttkrp_tile_kernel(const MttkrpArgs a) {
   extern __shared__ float4 smem4[];
   float* smem = reinterpret_cast<float*>(smem4);
@@ -396,7 +391,7 @@ __global__ void __launch_bounds__(kMttkrpThreads, MINB)
         const uint32_t chunk = (te - ts + kMttkrpWarps - 1) / kMttkrpWarps;
         const uint32_t ws = min(ts + warp * chunk, te);
         const uint32_t we = min(ws + chunk, te);
-        warp_range<R, FT, HW, NM, false, false, true, TGT>(a, a.line, ws, we, false, smem, 0, 0, &run);
+        warp_range<R, FT, HW, NM, false, false, true>(a, a.line, ws, we, false, smem, 0, 0, &run);
       }
       if (run.row != kNoRow)
         flush_row<R, LW::V, LW::G>(false, smem, 0, a.out, run.row, (threadIdx.x & 31) % LW::G, run.acc);
@@ -436,6 +431,327 @@ __global__ void __launch_bounds__(kMttkrpThreads, MINB)
       __syncthreads();
     }
   }
+}
+
+// ------------------------------------------------ the row-sorted walk
+//
+// SORTED and DETERMINISTIC on 3- to 5-mode tensors: the walk over a kDecoded
+// copy.  As warp_range, a warp's range is split into NPW contiguous
+// sub-ranges, one per lane group of G = R / V lanes; each lane holds V floats
+// of every row.  The walk is bound by issue slots, not by a bandwidth (5
+// modes at rank 64: 64 warp instructions per nonzero with a decoded key and
+// four floats a lane), so a step does as little as possible besides its row
+// loads: the rows come decoded, target last (no decode, no selection among
+// the modes), the loads past the end of a sub-range are clamped to the last
+// record instead of being predicated, and V is as wide as the registers
+// allow, which divides the per-nonzero overhead by the nonzeros in flight.
+
+template <int NIN>
+struct DecRec {
+  uint32_t in[NIN];
+  uint32_t row;
+  float v;
+};
+
+template <int NIN>
+__device__ __forceinline__ DecRec<NIN> load_dec(const void* line, const void* extra, uint32_t i) {
+  const uint4 q = __ldg(static_cast<const uint4*>(line) + i);
+  DecRec<NIN> r;
+  r.in[0] = q.x;
+  r.in[1] = q.y;
+  if constexpr (NIN == 2) {
+    r.row = q.z;
+    r.v = __uint_as_float(q.w);
+  } else if constexpr (NIN == 3) {
+    r.in[2] = q.z;
+    r.row = q.w;
+    r.v = __ldg(static_cast<const float*>(extra) + i);
+  } else {
+    r.in[2] = q.z;
+    r.in[3] = q.w;
+    const uint2 e = __ldg(static_cast<const uint2*>(extra) + i);
+    r.row = e.x;
+    r.v = __uint_as_float(e.y);
+  }
+  return r;
+}
+
+// How a lane group of the walk covers a row of R factors: V floats a lane in
+// pieces of P floats (one load each: 16 bytes, or 8 for four bfloat16), piece
+// p of lane `sub` at column p P G + P sub, so one load of the group's lanes
+// reads P G consecutive factors.
+template <int R, typename FT, int V>
+struct WalkMap {
+  static constexpr int G = R / V;
+  static constexpr int NPW = 32 / G;
+  static constexpr int P = sizeof(FT) == 4 ? 4 : (V < 8 ? V : 8);
+  __device__ static int col(int q, int sub) {  // column of this lane's float4 q (q < V / 4)
+    constexpr int H = P / 4;                   // float4s per piece
+    return (q / H) * P * G + P * sub + (q % H) * 4;
+  }
+};
+
+template <int R, typename FT, int V>
+__device__ __forceinline__ void walk_row(const void* base, uint32_t row, int sub, float (&x)[V]) {
+  using WM = WalkMap<R, FT, V>;
+  const char* p = static_cast<const char*>(base) + (size_t)row * (R * sizeof(FT)) + (WM::P * sub) * sizeof(FT);
+  if constexpr (sizeof(FT) == 4) {
+#pragma unroll
+    for (int q = 0; q < V / 4; ++q) {
+      const float4 f = __ldg(reinterpret_cast<const float4*>(p + (size_t)q * WM::P * WM::G * sizeof(FT)));
+      x[4 * q] = f.x;
+      x[4 * q + 1] = f.y;
+      x[4 * q + 2] = f.z;
+      x[4 * q + 3] = f.w;
+    }
+  } else if constexpr (V >= 8) {
+#pragma unroll
+    for (int q = 0; q < V / 8; ++q) {
+      const uint4 u = __ldg(reinterpret_cast<const uint4*>(p + (size_t)q * WM::P * WM::G * sizeof(FT)));
+      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        x[8 * q + 2 * h] = __uint_as_float(w[h] << 16);
+        x[8 * q + 2 * h + 1] = __uint_as_float(w[h] & 0xffff0000u);
+      }
+    }
+  } else {
+    const float4 f = load4<FT>(p, 0);
+    x[0] = f.x;
+    x[1] = f.y;
+    x[2] = f.z;
+    x[3] = f.w;
+  }
+}
+
+template <int R, typename FT, int V>
+__device__ __forceinline__ void walk_flush(float* out, uint32_t row, int sub, const float (&acc)[V]) {
+  float* o = out + (size_t)row * R;
+#pragma unroll
+  for (int q = 0; q < V / 4; ++q)
+    atomicAdd(reinterpret_cast<float4*>(o + WalkMap<R, FT, V>::col(q, sub)),
+              make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]));
+}
+
+// The row pieces of U nonzeros in flight.
+template <int NIN, int V, int U>
+struct WalkStage {
+  float f[U][NIN][V];
+  uint32_t row[U];
+  float v[U];
+};
+
+// Sub-range [gs, ge) of a lane group, `steps` steps of U nonzeros (the same
+// for every group of the warp).  D steps are in the air: the rows of step
+// k + D - 1 are requested, and the records of step k + 2 D - 1, before step k
+// is summed.  DET: as warp_range's, slots of sub-range `slot0 / 2`; else the
+// open run is taken from and left in `run`.
+template <int R, typename FT, int NIN, int V, int U, int D, bool DET>
+__device__ __forceinline__ void walk_range(const MttkrpArgs& a, uint32_t gs, uint32_t ge, uint32_t steps, int sub,
+                                           OpenRun<V>& run, uint32_t slot0) {
+  const void* base[NIN];
+#pragma unroll
+  for (int j = 0; j < NIN; ++j) base[j] = a.in.f[j];
+  const void* line = a.line;
+  const void* extra = a.extra;
+  const uint32_t last = a.nnz - 1;
+  uint32_t nrun = 0;
+  DecRec<NIN> rec[D][U];
+  WalkStage<NIN, V, U> st[D];
+  auto fetch = [&](DecRec<NIN>(&r)[U], uint32_t at) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) r[u] = load_dec<NIN>(line, extra, min(at + u, last));
+  };
+  auto issue = [&](WalkStage<NIN, V, U>& s, const DecRec<NIN>(&r)[U]) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+#pragma unroll
+      for (int j = 0; j < NIN; ++j) walk_row<R, FT, V>(base[j], r[u].in[j], sub, s.f[u][j]);
+      s.row[u] = r[u].row;
+      s.v[u] = r[u].v;
+    }
+  };
+  auto sum = [&](const WalkStage<NIN, V, U>& s, uint32_t at) {
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (at + u >= ge) continue;
+      float2 p[V / 2];  // packed FP32x2, the last factor fused into the sum
+#pragma unroll
+      for (int h = 0; h < V / 2; ++h) {
+        p[h] = __fmul2_rn(make_float2(s.v[u], s.v[u]), make_float2(s.f[u][0][2 * h], s.f[u][0][2 * h + 1]));
+#pragma unroll
+        for (int j = 1; j < NIN - 1; ++j)
+          p[h] = __fmul2_rn(p[h], make_float2(s.f[u][j][2 * h], s.f[u][j][2 * h + 1]));
+      }
+      if (s.row[u] != run.row) {
+        if (run.row != kNoRow) {
+          if constexpr (!DET) {
+            walk_flush<R, FT, V>(a.out, run.row, sub, run.acc);
+          } else {
+            if (nrun++ == 0)
+              det_slot<R, V, WalkMap<R, FT, V>::G>(a, slot0, run.row, sub, run.acc, false);
+            else
+              det_plain<R, V, WalkMap<R, FT, V>::G>(a.out, run.row, sub, run.acc);
+          }
+        }
+        run.row = s.row[u];
+#pragma unroll
+        for (int h = 0; h < V / 2; ++h) {
+          const float2 x = __fmul2_rn(p[h], make_float2(s.f[u][NIN - 1][2 * h], s.f[u][NIN - 1][2 * h + 1]));
+          run.acc[2 * h] = x.x;
+          run.acc[2 * h + 1] = x.y;
+        }
+      } else {
+#pragma unroll
+        for (int h = 0; h < V / 2; ++h) {
+          const float2 x = __ffma2_rn(p[h], make_float2(s.f[u][NIN - 1][2 * h], s.f[u][NIN - 1][2 * h + 1]),
+                                      make_float2(run.acc[2 * h], run.acc[2 * h + 1]));
+          run.acc[2 * h] = x.x;
+          run.acc[2 * h + 1] = x.y;
+        }
+      }
+    }
+  };
+#pragma unroll
+  for (int d = 0; d < D; ++d) fetch(rec[d], gs + d * U);
+#pragma unroll
+  for (int d = 0; d < D - 1; ++d) {
+    issue(st[d], rec[d]);
+    fetch(rec[d], gs + (d + D) * U);
+  }
+  uint32_t i = gs;
+  for (uint32_t k = 0; k < steps; k += D, i += D * U) {
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+      constexpr int kAhead = D - 1;
+      issue(st[(d + kAhead) % D], rec[(d + kAhead) % D]);
+      fetch(rec[(d + kAhead) % D], i + (d + kAhead + D) * U);
+      sum(st[d], i + d * U);
+    }
+  }
+  if constexpr (DET) {
+    constexpr int G = WalkMap<R, FT, V>::G;
+    if (run.row == kNoRow) {
+      // empty sub-range: both slots carry the row of the entry before it (the
+      // last run of an earlier sub-range) with zeros, keeping slot rows sorted
+      const uint32_t r0 = load_dec<NIN>(line, extra, gs > 0 ? min(gs - 1, last) : 0).row;
+      det_slot<R, V, G>(a, slot0, r0, sub, run.acc, true);
+      det_slot<R, V, G>(a, slot0 + 1, r0, sub, run.acc, true);
+    } else if (nrun == 0) {
+      det_slot<R, V, G>(a, slot0, run.row, sub, run.acc, false);
+      det_slot<R, V, G>(a, slot0 + 1, run.row, sub, run.acc, true);
+    } else {
+      det_slot<R, V, G>(a, slot0 + 1, run.row, sub, run.acc, false);
+    }
+  }
+}
+
+// The widths of the walk: V floats a lane, U nonzeros a step, D steps in the
+// air, MINB blocks an SM (the register budget), by rank, input modes and
+// factor type.  Eight floats a lane halve the instructions per nonzero but
+// also the lanes per nonzero, so there are twice as many lane groups, with
+// runs half as long and twice the updates: measured better at rank 64 (5 modes,
+// 12M nonzeros: float32 631 us against 645, bfloat16 494 against 541) and worse
+// at rank 16 and 32 (power-law 3-mode, 40M nonzeros, rank 32: 936 us against
+// 809; uniform 1000^3, 1M nonzeros, rank 16: 27.6 against 21.5).  3 modes in
+// float32 wait for their rows (two loads a nonzero, the longest stall by far),
+// so a long walk keeps two steps in the air at three blocks an SM (40M
+// nonzeros: 769 us; one step at five blocks 802); a short one has its rows in
+// L2 and wants the blocks (5M: 124 us against 119; 20,000: 2.9 against 2.4),
+// and with more rows per nonzero two steps spill (2.1 ms against 0.63).
+template <int R, typename FT, int NIN, bool DET, bool DEEP = false>
+struct WalkCfg {
+  static constexpr int V = R >= 64 ? 8 : 4;
+  static constexpr int U = NIN == 2 && V == 4 ? 2 : 1;
+  static constexpr int D = DEEP ? 2 : 1;
+  static constexpr int MINB = DEEP ? 3 : NIN == 2 && V == 4 && !DET ? 5 : 4;
+};
+// Whether two steps in the air pay: 3 modes in float32 whose walk is long and
+// gathers from more than the L2 holds.
+template <int R, typename FT, int NIN>
+constexpr bool kCanBeDeep = NIN == 2 && R < 64 && sizeof(FT) == 4;
+constexpr uint32_t kDeepNnz = 8u << 20;
+
+// This lane's group's part of warp `warp`'s share of tile `tile`.
+template <int NPW, int G, int U>
+struct TilePart {
+  uint32_t gs, ge, steps;
+  __device__ TilePart(const MttkrpArgs& a, uint32_t tile, int warp, int grp) {
+    const uint32_t ts = tile * a.tile_nnz;
+    const uint32_t te = min(ts + a.tile_nnz, a.nnz);
+    const uint32_t chunk = (te - ts + kMttkrpWarps - 1) / kMttkrpWarps;
+    const uint32_t ws = min(ts + warp * chunk, te);
+    const uint32_t we = min(ws + chunk, te);
+    const uint32_t sublen = (we - ws + NPW - 1) / NPW;
+    gs = min(ws + grp * sublen, we);
+    ge = min(gs + sublen, we);
+    steps = (sublen + U - 1) / U;
+  }
+};
+
+// The lane groups' open runs at the end of a chunk: when a whole warp ends on
+// one row (a hot row, or a mode of few rows) its groups are summed first, in
+// group order, and the row is updated once instead of once per group.  Groups
+// of G lanes; lanes past the last group hold zeros.
+template <int V>
+__device__ __forceinline__ bool merge_groups(uint32_t row, float (&acc)[V], int G, int npw, int lane) {
+  const uint32_t row0 = __shfl_sync(0xffffffffu, row, 0);
+  if (!__all_sync(0xffffffffu, row == row0 || lane >= G * npw)) return false;
+  for (int g = 1; g < npw; ++g)
+#pragma unroll
+    for (int q = 0; q < V; ++q) {
+      const float x = __shfl_sync(0xffffffffu, acc[q], (g * G + lane) & 31);
+      if (lane < G) acc[q] += x;
+    }
+  return true;
+}
+
+template <int R, typename FT, int NIN, bool DEEP>
+__global__ void __launch_bounds__(kMttkrpThreads, WalkCfg<R, FT, NIN, false, DEEP>::MINB)
+    walk_kernel(const MttkrpArgs a) {
+  using C = WalkCfg<R, FT, NIN, false, DEEP>;
+  using WM = WalkMap<R, FT, C::V>;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int grp = lane / WM::G, sub = lane % WM::G;
+  // chunks of consecutive tiles, the open run carried through them (as in
+  // mttkrp_tile_kernel)
+  const uint32_t ct = a.chunk_tiles ? a.chunk_tiles : 1;
+  const uint32_t nchunks = (a.ntiles + ct - 1) / ct;
+  for (uint32_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
+    OpenRun<C::V> run;
+    run.row = kNoRow;
+#pragma unroll
+    for (int q = 0; q < C::V; ++q) run.acc[q] = 0.f;
+    const uint32_t t_end = min(c * ct + ct, a.ntiles);
+    for (uint32_t tile = c * ct; tile < t_end; ++tile) {
+      const TilePart<WM::NPW, WM::G, C::U> p(a, tile, warp, grp);
+      walk_range<R, FT, NIN, C::V, C::U, C::D, false>(a, p.gs, p.ge, p.steps, sub, run, 0);
+    }
+    const bool one = WM::NPW > 1 && merge_groups<C::V>(run.row, run.acc, WM::G, WM::NPW, lane);
+    if (run.row != kNoRow && !(one && grp)) walk_flush<R, FT, C::V>(a.out, run.row, sub, run.acc);
+  }
+}
+
+// One tile of the deterministic walk.
+template <int R, int NIN>
+__device__ __forceinline__ void det_walk_tile(const MttkrpArgs& a, uint32_t tile) {
+  using C = WalkCfg<R, float, NIN, true>;
+  using WM = WalkMap<R, float, C::V>;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int grp = lane / WM::G, sub = lane % WM::G;
+  const TilePart<WM::NPW, WM::G, C::U> p(a, tile, warp, grp);
+  OpenRun<C::V> run;
+  run.row = kNoRow;
+#pragma unroll
+  for (int q = 0; q < C::V; ++q) run.acc[q] = 0.f;
+  walk_range<R, float, NIN, C::V, C::U, C::D, true>(a, p.gs, p.ge, p.steps, sub, run,
+                                              2 * ((tile * kMttkrpWarps + warp) * WM::NPW + grp));
+}
+
+template <int R, int NIN>
+__global__ void __launch_bounds__(kMttkrpThreads, WalkCfg<R, float, NIN, true>::MINB)
+    det_walk_kernel(const MttkrpArgs a) {
+  for (uint32_t tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) det_walk_tile<R, NIN>(a, tile);
 }
 
 // ------------------------------------------------ deterministic fix-up
@@ -657,8 +973,8 @@ __global__ void __launch_bounds__(256) det_zero_group_kernel(Strided<DetItem> it
   }
 }
 
-template <int R, int HW, int NM>
-__global__ void __launch_bounds__(kMttkrpThreads, 3)
+template <int R, int NIN>
+__global__ void __launch_bounds__(kMttkrpThreads, WalkCfg<R, float, NIN, true>::MINB)
     det_tile_group_kernel(Strided<DetItem> items, const uint32_t* __restrict__ tile_off) {
   // the item's arguments staged in shared memory: the walk reads them per
   // nonzero (as a launch of its own reads them from the parameter bank)
@@ -666,7 +982,6 @@ __global__ void __launch_bounds__(kMttkrpThreads, 3)
   __shared__ int s_item;
   const int K = *items.count;
   const uint32_t total = K > 0 ? tile_off[K] : 0;
-  const int warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) s_item = -1;
   for (uint32_t v = blockIdx.x; v < total; v += gridDim.x) {
     const int s = item_of(tile_off, K, v);
@@ -682,15 +997,7 @@ __global__ void __launch_bounds__(kMttkrpThreads, 3)
       if (threadIdx.x == 0) s_item = s;
     }
     __syncthreads();
-    const MttkrpArgs& a = sa;
-    const uint32_t tile = v - tile_off[s];
-    const uint32_t ts = tile * a.tile_nnz;
-    const uint32_t te = min(ts + a.tile_nnz, a.nnz);
-    const uint32_t chunk = (te - ts + kMttkrpWarps - 1) / kMttkrpWarps;
-    const uint32_t ws = min(ts + warp * chunk, te);
-    const uint32_t we = min(ws + chunk, te);
-    warp_range<R, float, HW, NM, false, true>(a, a.line, ws, we, false, nullptr, 0,
-                                              (tile * kMttkrpWarps + warp) * LaneWidth<R>::NPW);
+    det_walk_tile<R, NIN>(sa, v - tile_off[s]);
   }
 }
 
@@ -839,45 +1146,168 @@ __global__ void __launch_bounds__(kMttkrpThreads, 3)
   }
 }
 
-// Any rank: one warp per nonzero, lanes stride the rank, scalar atomics.
-template <typename FT, int HW>
-__global__ void __launch_bounds__(kMttkrpThreads)
-    mttkrp_generic_kernel(const MttkrpArgs a, int rank) {
-  const int lane = threadIdx.x & 31;
-  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t i = gw; i < a.nnz; i += nw) {
-    uint32_t rows[ALTO_MAX_MODES];
-    float v;
-    if (HW == kDecoded3) {
-      const uint4 q = static_cast<const uint4*>(a.line)[i];
-      rows[0] = q.x;
-      rows[1] = q.y;
-      rows[2] = q.z;
-#pragma unroll
-      for (int m = 3; m < ALTO_MAX_MODES; ++m) rows[m] = 0;
-      v = __uint_as_float(q.w);
+// ------------------------------------------------ any rank, any alignment
+//
+// The walk at a rank (or alignment) the specialised kernels do not take: a
+// lane group of G = ceil(R / V) lanes per nonzero -- any G up to 32, so 32 / G
+// groups share a warp -- each lane holding V = 4 factors in V / VW loads of VW
+// factors, VW the widest of 4, 2, 1 that divides the rank and that every
+// pointer is aligned for.  Sub-ranges, runs and chunks are the specialised
+// walk's (one vector atomic per run and lane); ranks above 128 take one
+// column window of 128 per blockIdx.y.  Bound by issue slots and, where runs
+// are short, by atomics.  A warp per nonzero with a scalar atomic per
+// factor, its form before, took 802 us per mode on a ragged 4-mode tensor of 3M
+// nonzeros at rank 10, at any of the line orders.
+
+template <typename FT, int VW>
+__device__ __forceinline__ void any_piece(const char* p, float* x) {
+  if constexpr (VW == 4) {
+    const float4 f = load4<FT>(p, 0);
+    x[0] = f.x;
+    x[1] = f.y;
+    x[2] = f.z;
+    x[3] = f.w;
+  } else if constexpr (sizeof(FT) == 4) {
+    if constexpr (VW == 2) {
+      const float2 f = __ldg(reinterpret_cast<const float2*>(p));
+      x[0] = f.x;
+      x[1] = f.y;
     } else {
-      uint64_t lo, hi;
-      rec_read(a.line, HW, i, lo, hi, v);
-#pragma unroll
-      for (int m = 0; m < ALTO_MAX_MODES; ++m)
-        rows[m] = m < a.dec.nmodes ? (uint32_t)line_field(lo, hi, a.dec.pos[m], a.dec.mask[m]) : 0;
+      x[0] = __ldg(reinterpret_cast<const float*>(p));
     }
-    for (int r = lane; r < rank; r += 32) {
-      float x = v;
+  } else if constexpr (VW == 2) {
+    const uint32_t u = __ldg(reinterpret_cast<const uint32_t*>(p));
+    x[0] = __uint_as_float(u << 16);
+    x[1] = __uint_as_float(u & 0xffff0000u);
+  } else {
+    x[0] = __uint_as_float((uint32_t)__ldg(reinterpret_cast<const unsigned short*>(p)) << 16);
+  }
+}
+
+template <int VW>
+__device__ __forceinline__ void any_flush(float* o, const float* x) {
+  if constexpr (VW == 4)
+    atomicAdd(reinterpret_cast<float4*>(o), make_float4(x[0], x[1], x[2], x[3]));
+  else if constexpr (VW == 2)
+    atomicAdd(reinterpret_cast<float2*>(o), make_float2(x[0], x[1]));
+  else
+    atomicAdd(o, x[0]);
+}
+
+// A record of either kind: DEC reads a kDecoded copy of NIN + 1 modes, else
+// the line (any record format; NIN is the input-mode count, or the most there
+// can be, then a.dec.nmodes - 1 of them are read).
+template <int NIN, bool DEC>
+__device__ __forceinline__ DecRec<NIN> any_rec(const MttkrpArgs& a, uint32_t i) {
+  if constexpr (DEC) {
+    return load_dec<NIN>(a.line, a.extra, i);
+  } else {
+    uint64_t lo, hi;
+    DecRec<NIN> r;
+    rec_read(a.line, a.dec.hi_words, i, lo, hi, r.v);
 #pragma unroll
-      for (int m = 0; m < ALTO_MAX_MODES; ++m) {
-        if (m < a.dec.nmodes && m != a.target) {
-          const size_t off = (size_t)rows[m] * rank + r;
-          if (sizeof(FT) == 4)
-            x *= __ldg(static_cast<const float*>(a.fac.f[m]) + off);
-          else
-            x *= __bfloat162float(static_cast<const __nv_bfloat16*>(a.fac.f[m])[off]);
+    for (int j = 0; j < NIN; ++j) {
+      const int m = j < a.target ? j : j + 1;
+      r.in[j] = m < a.dec.nmodes ? (uint32_t)line_field(lo, hi, a.dec.pos[m], a.dec.mask[m]) : 0;
+    }
+    r.row = (uint32_t)line_field(lo, hi, a.dec.pos[a.target], a.dec.mask[a.target]);
+    return r;
+  }
+}
+
+template <typename FT, int VW, int NIN, bool DEC>
+__global__ void __launch_bounds__(kMttkrpThreads, 4) any_walk_kernel(const MttkrpArgs a, int rank) {
+  constexpr int V = 4, Q = V / VW;
+  constexpr int U = NIN <= 3 ? 2 : 1;
+  const int c0 = blockIdx.y * 32 * V;  // this window's first column
+  const int cols = min(rank - c0, 32 * V);
+  const int G = (cols + V - 1) / V, NPW = 32 / G;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int grp = lane / G, sub = lane % G;
+  const bool idle = grp >= NPW;
+  // this lane's pieces: columns (q G + sub) VW of the window (a piece past
+  // the last column reads the last one and is not written)
+  int col[Q];
+  bool mine[Q];
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    const int c = (q * G + sub) * VW;
+    mine[q] = c < cols && !idle;
+    col[q] = c0 + min(c, cols - VW);
+  }
+  const uint32_t last = a.nnz - 1;
+  const uint32_t ct = a.chunk_tiles ? a.chunk_tiles : 1;
+  const uint32_t nchunks = (a.ntiles + ct - 1) / ct;
+  const char* base[NIN];
+#pragma unroll
+  for (int j = 0; j < NIN; ++j) base[j] = static_cast<const char*>(a.in.f[j]);
+  const size_t row_bytes = (size_t)rank * sizeof(FT);
+  for (uint32_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
+    uint32_t cur = kNoRow;
+    float acc[V];
+#pragma unroll
+    for (int q = 0; q < V; ++q) acc[q] = 0.f;
+    auto flush = [&]() {
+      float* o = a.out + (size_t)cur * rank;
+#pragma unroll
+      for (int q = 0; q < Q; ++q)
+        if (mine[q]) any_flush<VW>(o + col[q], acc + q * VW);
+    };
+    const uint32_t t_end = min(c * ct + ct, a.ntiles);
+    for (uint32_t tile = c * ct; tile < t_end; ++tile) {
+      const uint32_t ts = tile * a.tile_nnz;
+      const uint32_t te = min(ts + a.tile_nnz, a.nnz);
+      const uint32_t chunk = (te - ts + kMttkrpWarps - 1) / kMttkrpWarps;
+      const uint32_t ws = min(ts + warp * chunk, te);
+      const uint32_t we = min(ws + chunk, te);
+      const uint32_t sublen = (we - ws + NPW - 1) / NPW;
+      const uint32_t gs = min(ws + grp * sublen, we);
+      const uint32_t ge = idle ? gs : min(gs + sublen, we);
+      DecRec<NIN> rec[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) rec[u] = any_rec<NIN, DEC>(a, min(gs + u, last));
+      for (uint32_t i = gs, k = 0; k < sublen; k += U, i += U) {
+        float f[U][NIN][V];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+          for (int j = 0; j < NIN; ++j) {
+            if (NIN > 4 && j + 1 >= a.dec.nmodes) continue;
+            const char* p = base[j] + rec[u].in[j] * row_bytes;
+#pragma unroll
+            for (int q = 0; q < Q; ++q) any_piece<FT, VW>(p + col[q] * sizeof(FT), &f[u][j][q * VW]);
+          }
+        uint32_t rows[U];
+        float vals[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          rows[u] = rec[u].row;
+          vals[u] = rec[u].v;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) rec[u] = any_rec<NIN, DEC>(a, min(i + U + u, last));
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          if (i + u >= ge) continue;
+          if (rows[u] != cur) {
+            if (cur != kNoRow) flush();
+            cur = rows[u];
+#pragma unroll
+            for (int q = 0; q < V; ++q) acc[q] = 0.f;
+          }
+#pragma unroll
+          for (int q = 0; q < V; ++q) {
+            float x = vals[u];
+#pragma unroll
+            for (int j = 0; j < NIN; ++j)
+              if (NIN <= 4 || j + 1 < a.dec.nmodes) x *= f[u][j][q];
+            acc[q] += x;
+          }
         }
       }
-      atomicAdd(a.out + (size_t)rows[a.target] * rank + r, x);
     }
+    const bool one = NPW > 1 && merge_groups<V>(cur, acc, G, NPW, lane);
+    if (cur != kNoRow && !(one && grp)) flush();
   }
 }
 
@@ -904,7 +1334,20 @@ static uint32_t chunk_tiles_for(uint32_t ntiles, unsigned grid) {
   return c;
 }
 
-template <int R, typename FT, int HW, bool STAGE, int NM, int MINB = 3, int TGT = -1>
+// The tiles of a walk that has no use for their intervals: sized so that
+// `grid` blocks get the same number of equal tiles (the tensor's own tiles leave
+// a last wave that is nearly empty: 489 tiles of 2048 on 444 blocks at 1M
+// nonzeros), at most kWalkTile nonzeros each, in multiples of `unit` (one step
+// of every lane group of a block).
+constexpr uint32_t kWalkTile = 4096;
+static void even_tiles(MttkrpArgs* a, unsigned grid, uint32_t unit) {
+  const uint64_t rounds = std::max<uint64_t>(((uint64_t)a->nnz + (uint64_t)grid * kWalkTile - 1) / ((uint64_t)grid * kWalkTile), 1);
+  const uint64_t per = (a->nnz + grid * rounds - 1) / (grid * rounds);
+  a->tile_nnz = (uint32_t)std::max<uint64_t>((per + unit - 1) / unit * unit, unit);
+  a->ntiles = (uint32_t)(((uint64_t)a->nnz + a->tile_nnz - 1) / a->tile_nnz);
+}
+
+template <int R, typename FT, int HW, bool STAGE, int NM>
 static alto_status launch_tile(const MttkrpArgs& a, cudaStream_t st) {
   MttkrpArgs b = a;
   b.stage_rows = STAGE ? kStageBytes / (R * 4) : 0;
@@ -912,19 +1355,19 @@ static alto_status launch_tile(const MttkrpArgs& a, cudaStream_t st) {
   static int blocks_per_sm = 0;
   if (!blocks_per_sm) {
     if (STAGE)
-      ALTO_TRY_CUDA(cudaFuncSetAttribute(mttkrp_tile_kernel<R, FT, HW, STAGE, NM, false, MINB, TGT>,
+      ALTO_TRY_CUDA(cudaFuncSetAttribute(mttkrp_tile_kernel<R, FT, HW, STAGE, NM, false>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, kStageBytes));
     else  // no shared memory: all of the unified L1 / shared storage as L1 (factor rows hit it)
-      ALTO_TRY_CUDA(cudaFuncSetAttribute(mttkrp_tile_kernel<R, FT, HW, STAGE, NM, false, MINB, TGT>,
+      ALTO_TRY_CUDA(cudaFuncSetAttribute(mttkrp_tile_kernel<R, FT, HW, STAGE, NM, false>,
                                          cudaFuncAttributePreferredSharedMemoryCarveout, 0));
     ALTO_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &blocks_per_sm, mttkrp_tile_kernel<R, FT, HW, STAGE, NM, false, MINB, TGT>, kMttkrpThreads, smem));
+        &blocks_per_sm, mttkrp_tile_kernel<R, FT, HW, STAGE, NM, false>, kMttkrpThreads, smem));
     if (blocks_per_sm < 1) blocks_per_sm = 1;
   }
   unsigned grid = std::min<unsigned>(a.ntiles, (unsigned)(num_sms() * blocks_per_sm));
   if (!grid) return ALTO_OK;
   b.chunk_tiles = chunk_tiles_for(a.ntiles, grid);
-  mttkrp_tile_kernel<R, FT, HW, STAGE, NM, false, MINB, TGT><<<grid, kMttkrpThreads, smem, st>>>(b);
+  mttkrp_tile_kernel<R, FT, HW, STAGE, NM, false><<<grid, kMttkrpThreads, smem, st>>>(b);
   ALTO_LAUNCHED();
   return ALTO_OK;
 }
@@ -948,21 +1391,68 @@ static alto_status launch_tma(const MttkrpArgs& a, int* err, cudaStream_t st) {
   return ALTO_OK;
 }
 
-// Deterministic MTTKRP: the tile kernel in DET mode (float32 factors, the
-// specialised ranks) followed by the two fix-up kernels.
-template <int R, int HW, int NM>
-static alto_status launch_det_nm(const MttkrpArgs& a, const DetLong& dl, cudaStream_t st) {
+template <int R, typename FT, int NIN, bool DEEP = false>
+static alto_status launch_walk(const MttkrpArgs& a, cudaStream_t st) {
+  if constexpr (kCanBeDeep<R, FT, NIN> && !DEEP)
+    if (a.nnz >= kDeepNnz) return launch_walk<R, FT, NIN, true>(a, st);
   static int blocks_per_sm = 0;
   if (!blocks_per_sm) {
-    ALTO_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &blocks_per_sm, mttkrp_tile_kernel<R, float, HW, false, NM, true>, kMttkrpThreads, 0));
+    // no shared memory: all of the unified L1 / shared storage as L1 (factor rows hit it)
+    ALTO_TRY_CUDA(cudaFuncSetAttribute(walk_kernel<R, FT, NIN, DEEP>, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                       0));
+    ALTO_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, walk_kernel<R, FT, NIN, DEEP>,
+                                                                kMttkrpThreads, 0));
     if (blocks_per_sm < 1) blocks_per_sm = 1;
   }
-  const unsigned grid = std::min<unsigned>(a.ntiles, (unsigned)(num_sms() * blocks_per_sm));
-  if (!grid) return ALTO_OK;
-  mttkrp_tile_kernel<R, float, HW, false, NM, true><<<grid, kMttkrpThreads, 0, st>>>(a);
+  if (!a.nnz) return ALTO_OK;
+  MttkrpArgs b = a;
+  using C = WalkCfg<R, FT, NIN, false, DEEP>;
+  const unsigned full = (unsigned)(num_sms() * blocks_per_sm);
+  even_tiles(&b, full, kMttkrpWarps * WalkMap<R, FT, C::V>::NPW * C::U);
+  const unsigned grid = std::min<unsigned>(b.ntiles, full);
+  b.chunk_tiles = chunk_tiles_for(b.ntiles, grid);
+  walk_kernel<R, FT, NIN, DEEP><<<grid, kMttkrpThreads, 0, st>>>(b);
   ALTO_LAUNCHED();
-  const uint32_t nslots = a.ntiles * kMttkrpWarps * LaneWidth<R>::NPW * 2;
+  return ALTO_OK;
+}
+
+template <typename FT, int VW, int NIN, bool DEC>
+static alto_status launch_any(const MttkrpArgs& a, int rank, cudaStream_t st) {
+  const unsigned windows = (unsigned)((rank + 127) / 128);
+  if (!a.nnz) return ALTO_OK;
+  MttkrpArgs b = a;
+  even_tiles(&b, (unsigned)num_sms() * 4, 128);
+  const unsigned grid = std::min<unsigned>(b.ntiles, (unsigned)num_sms() * 4);
+  b.chunk_tiles = chunk_tiles_for(b.ntiles, grid);
+  any_walk_kernel<FT, VW, NIN, DEC><<<dim3(grid, windows), kMttkrpThreads, 0, st>>>(b, rank);
+  ALTO_LAUNCHED();
+  return ALTO_OK;
+}
+
+template <typename FT, int VW>
+static alto_status launch_any_modes(const MttkrpArgs& a, int rank, bool decoded, cudaStream_t st) {
+  switch (a.dec.nmodes) {
+    case 3: return decoded ? launch_any<FT, VW, 2, true>(a, rank, st) : launch_any<FT, VW, 2, false>(a, rank, st);
+    case 4: return decoded ? launch_any<FT, VW, 3, true>(a, rank, st) : launch_any<FT, VW, 3, false>(a, rank, st);
+    case 5: return decoded ? launch_any<FT, VW, 4, true>(a, rank, st) : launch_any<FT, VW, 4, false>(a, rank, st);
+    default: return launch_any<FT, VW, ALTO_MAX_MODES - 1, false>(a, rank, st);
+  }
+}
+
+// The widest load (4, 2 or 1 factors) that divides the rank and that the
+// factors and the output are aligned for.
+template <typename FT>
+static alto_status launch_any_width(const MttkrpArgs& a, int rank, bool decoded, cudaStream_t st) {
+  uintptr_t bits = reinterpret_cast<uintptr_t>(a.out) | ((uintptr_t)rank * 4);
+  for (int j = 0; j + 1 < a.dec.nmodes; ++j)
+    bits |= (reinterpret_cast<uintptr_t>(a.in.f[j]) | ((uintptr_t)rank * sizeof(FT))) * (4 / sizeof(FT));
+  if (bits % 16 == 0) return launch_any_modes<FT, 4>(a, rank, decoded, st);
+  if (bits % 8 == 0) return launch_any_modes<FT, 2>(a, rank, decoded, st);
+  return launch_any_modes<FT, 1>(a, rank, decoded, st);
+}
+
+// The fix-up kernels of a deterministic MTTKRP whose walk left nslots slots.
+static alto_status launch_det_fix(const MttkrpArgs& a, uint32_t nslots, int R, const DetLong& dl, cudaStream_t st) {
   const unsigned g1 = std::min<unsigned>((nslots + 7) / 8, (unsigned)num_sms() * 16);
   det_fix_short_kernel<<<g1, 256, 0, st>>>(a.det_rows, a.det_vals, nslots, R, a.out, dl);
   ALTO_LAUNCHED();
@@ -973,40 +1463,84 @@ static alto_status launch_det_nm(const MttkrpArgs& a, const DetLong& dl, cudaStr
   return ALTO_OK;
 }
 
-template <int R, int HW>
-static alto_status launch_det(const MttkrpArgs& a, const DetLong& dl, cudaStream_t st) {
-  if constexpr (HW == kDecoded3) return launch_det_nm<R, HW, 3>(a, dl, st);
-  switch (a.dec.nmodes) {
-    case 3: return launch_det_nm<R, HW, 3>(a, dl, st);
-    case 4: return launch_det_nm<R, HW, 4>(a, dl, st);
-    case 5: return launch_det_nm<R, HW, 5>(a, dl, st);
-    default: return launch_det_nm<R, HW, ALTO_MAX_MODES>(a, dl, st);
+// Deterministic MTTKRP (float32 factors, the specialised ranks): the walk of
+// the row-sorted copy, then the fix-up kernels.
+template <int R, int NIN>
+static alto_status launch_det_walk(const DetItem& it, cudaStream_t st) {
+  static int blocks_per_sm = 0;
+  if (!blocks_per_sm) {
+    ALTO_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, det_walk_kernel<R, NIN>,
+                                                                kMttkrpThreads, 0));
+    if (blocks_per_sm < 1) blocks_per_sm = 1;
   }
+  const unsigned grid = std::min<unsigned>(it.a.ntiles, (unsigned)(num_sms() * blocks_per_sm));
+  if (!grid) return ALTO_OK;
+  det_walk_kernel<R, NIN><<<grid, kMttkrpThreads, 0, st>>>(it.a);
+  ALTO_LAUNCHED();
+  return launch_det_fix(it.a, it.nslots, R, it.dl, st);
 }
 
-template <int HW>
-static alto_status launch_det_rank(const MttkrpArgs& a, int rank, const DetLong& dl,
-                                   cudaStream_t st) {
+// As launch_det_walk on lines that are not decoded (2 modes, or more than 5).
+template <int R, int HW>
+static alto_status launch_det_line(const DetItem& it, cudaStream_t st) {
+  static int blocks_per_sm = 0;
+  if (!blocks_per_sm) {
+    ALTO_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &blocks_per_sm, mttkrp_tile_kernel<R, float, HW, false, ALTO_MAX_MODES, true>, kMttkrpThreads, 0));
+    if (blocks_per_sm < 1) blocks_per_sm = 1;
+  }
+  const unsigned grid = std::min<unsigned>(it.a.ntiles, (unsigned)(num_sms() * blocks_per_sm));
+  if (!grid) return ALTO_OK;
+  mttkrp_tile_kernel<R, float, HW, false, ALTO_MAX_MODES, true><<<grid, kMttkrpThreads, 0, st>>>(it.a);
+  ALTO_LAUNCHED();
+  return launch_det_fix(it.a, it.nslots, R, it.dl, st);
+}
+
+template <int R>
+static alto_status launch_det(const DetItem& it, cudaStream_t st) {
+  if (it.hw == kDecoded) {
+    switch (it.a.dec.nmodes) {
+      case 3: return launch_det_walk<R, 2>(it, st);
+      case 4: return launch_det_walk<R, 3>(it, st);
+      default: return launch_det_walk<R, 4>(it, st);
+    }
+  }
+  if (it.hw == 0) return launch_det_line<R, 0>(it, st);
+  if (it.hw == 1) return launch_det_line<R, 1>(it, st);
+  return launch_det_line<R, 2>(it, st);
+}
+
+static alto_status launch_det_rank(const DetItem& it, int rank, cudaStream_t st) {
   switch (rank) {
-    case 8: return launch_det<8, HW>(a, dl, st);
-    case 16: return launch_det<16, HW>(a, dl, st);
-    case 32: return launch_det<32, HW>(a, dl, st);
-    case 64: return launch_det<64, HW>(a, dl, st);
-    case 128: return launch_det<128, HW>(a, dl, st);
+    case 8: return launch_det<8>(it, st);
+    case 16: return launch_det<16>(it, st);
+    case 32: return launch_det<32>(it, st);
+    case 64: return launch_det<64>(it, st);
+    case 128: return launch_det<128>(it, st);
     default: break;
   }
   set_error("the deterministic MTTKRP takes rank 8, 16, 32, 64 or 128 (got %d)", rank);
   return ALTO_ERR_UNSUPPORTED;
 }
 
-// Lane groups per warp of the specialised kernels at this rank.
-static uint32_t groups_per_warp(int rank) {
+template <int R>
+static uint32_t det_groups(int nmodes, int hw) {
+  if (hw != kDecoded) return LaneWidth<R>::NPW;
+  switch (nmodes) {
+    case 3: return WalkMap<R, float, WalkCfg<R, float, 2, true>::V>::NPW;
+    case 4: return WalkMap<R, float, WalkCfg<R, float, 3, true>::V>::NPW;
+    default: return WalkMap<R, float, WalkCfg<R, float, 4, true>::V>::NPW;
+  }
+}
+
+// Lane groups per warp of the deterministic walk.
+static uint32_t groups_per_warp(int rank, int nmodes, int hw) {
   switch (rank) {
-    case 8: return LaneWidth<8>::NPW;
-    case 16: return LaneWidth<16>::NPW;
-    case 32: return LaneWidth<32>::NPW;
-    case 64: return LaneWidth<64>::NPW;
-    default: return LaneWidth<128>::NPW;
+    case 8: return det_groups<8>(nmodes, hw);
+    case 16: return det_groups<16>(nmodes, hw);
+    case 32: return det_groups<32>(nmodes, hw);
+    case 64: return det_groups<64>(nmodes, hw);
+    default: return det_groups<128>(nmodes, hw);
   }
 }
 
@@ -1014,20 +1548,9 @@ bool deterministic_supported(int rank, alto_dtype fdtype) {
   return fdtype == ALTO_F32 && (rank == 8 || rank == 16 || rank == 32 || rank == 64 || rank == 128);
 }
 
+// The ALTO line (or a copy that keeps its record format).
 template <int R, typename FT, int HW>
-static alto_status launch_modes(const MttkrpArgs& a, bool stage, bool bulk_feed, int dense, int* err,
-                                cudaStream_t st) {
-  if constexpr (HW == kDecoded3) {  // sorted 3-mode copies: no staging
-    if (dense == 2 && !bulk_feed) {  // the target mode fixed at compile time
-      switch (a.target) {
-        case 0: return launch_tile<R, FT, HW, false, 3, 5, 0>(a, st);
-        case 1: return launch_tile<R, FT, HW, false, 3, 5, 1>(a, st);
-        default: return launch_tile<R, FT, HW, false, 3, 5, 2>(a, st);
-      }
-    }
-    if (dense && !bulk_feed) return launch_tile<R, FT, HW, false, 3, 5>(a, st);
-    return bulk_feed ? launch_tma<R, FT, HW, 3>(a, err, st) : launch_tile<R, FT, HW, false, 3>(a, st);
-  } else {
+static alto_status launch_modes(const MttkrpArgs& a, bool stage, bool bulk_feed, int* err, cudaStream_t st) {
 #define NM_CASE(NN)                                                                   \
   case NN:                                                                            \
     if (stage) return launch_tile<R, FT, HW, true, NN>(a, st);                        \
@@ -1041,31 +1564,41 @@ static alto_status launch_modes(const MttkrpArgs& a, bool stage, bool bulk_feed,
                    : launch_tile<R, FT, HW, false, ALTO_MAX_MODES>(a, st);
   }
 #undef NM_CASE
-  }
 }
 
-template <typename FT, int HW>
-static alto_status launch_rank(const MttkrpArgs& a, int rank, bool stage, bool bulk_feed, int dense,
-                               bool aligned, int* err, cudaStream_t st) {
+// hw: the record format of the line walked.  The specialised ranks need
+// 16-byte aligned rows (8 for bfloat16); any other call takes the any-rank walk.
+template <int R, typename FT>
+static alto_status launch_specialised(const MttkrpArgs& a, int hw, bool stage, bool bulk_feed, int* err,
+                                      cudaStream_t st) {
+  if (hw == kDecoded) {
+    switch (a.dec.nmodes) {
+      case 3: return launch_walk<R, FT, 2>(a, st);
+      case 4: return launch_walk<R, FT, 3>(a, st);
+      default: return launch_walk<R, FT, 4>(a, st);
+    }
+  }
+  if (hw == 0) return launch_modes<R, FT, 0>(a, stage, bulk_feed, err, st);
+  if (hw == 1) return launch_modes<R, FT, 1>(a, stage, bulk_feed, err, st);
+  return launch_modes<R, FT, 2>(a, stage, bulk_feed, err, st);
+}
+
+template <typename FT>
+static alto_status launch_rank(const MttkrpArgs& a, int rank, int hw, bool stage, bool bulk_feed, uintptr_t misalign,
+                               int* err, cudaStream_t st) {
+  // (the decoded walk reads bfloat16 rows in 16-byte pieces)
+  const bool aligned = misalign % 16 == 0 || (sizeof(FT) == 2 && hw != kDecoded && misalign % 8 == 0);
   if (aligned) {
-#define RANK_CASE(RR) \
-  case RR:            \
-    return launch_modes<RR, FT, HW>(a, stage, bulk_feed, dense, err, st);
     switch (rank) {
-      RANK_CASE(8)
-      RANK_CASE(16)
-      RANK_CASE(32)
-      RANK_CASE(64)
-      RANK_CASE(128)
+      case 8: return launch_specialised<8, FT>(a, hw, stage, bulk_feed, err, st);
+      case 16: return launch_specialised<16, FT>(a, hw, stage, bulk_feed, err, st);
+      case 32: return launch_specialised<32, FT>(a, hw, stage, bulk_feed, err, st);
+      case 64: return launch_specialised<64, FT>(a, hw, stage, bulk_feed, err, st);
+      case 128: return launch_specialised<128, FT>(a, hw, stage, bulk_feed, err, st);
       default: break;
     }
-#undef RANK_CASE
   }
-  unsigned grid = (unsigned)std::min<uint64_t>((a.nnz + 7) / 8, (uint64_t)num_sms() * 16);
-  if (!grid) return ALTO_OK;
-  mttkrp_generic_kernel<FT, HW><<<grid, kMttkrpThreads, 0, st>>>(a, rank);
-  ALTO_LAUNCHED();
-  return ALTO_OK;
+  return launch_any_width<FT>(a, rank, hw == kDecoded, st);
 }
 
 // Fraction of the mode's tiles whose output interval fits the staging buffer
@@ -1099,17 +1632,47 @@ alto_mttkrp_variant choose_variant(const alto_tensor* t, int mode, int rank, alt
   return ALTO_MTTKRP_ATOMIC;
 }
 
+// The arguments of a walk of mode `mode` into `out`: of the line, or of the
+// mode's row-sorted copy (built if it is not there); *hw its record format.
+static alto_status fill_args(alto_tensor* t, int mode, const void* const* factors, float* out, bool sorted,
+                             MttkrpArgs* args, int* hw, cudaStream_t st) {
+  MttkrpArgs& a = *args;
+  a.line = t->line.p;
+  a.extra = nullptr;
+  a.tile_iv = t->tile_iv.as<uint32_t>();
+  a.ntiles = t->nnz ? t->ntiles : 0;
+  *hw = t->dec.hi_words;
+  if (sorted && t->nnz) {
+    if (!t->sorted[mode].ready || t->sorted[mode].for_nnz != t->nnz) ALTO_TRY(build_sorted_line(t, mode, st));
+    const SortedLine& s = t->sorted[mode];
+    a.line = s.line.p;
+    a.extra = s.extra.p;
+    a.tile_iv = s.tile_iv.as<uint32_t>();
+    a.ntiles = s.ntiles;
+    *hw = s.hw;
+  }
+  a.nnz = (uint32_t)t->nnz;
+  a.tile_nnz = t->tile_nnz;
+  a.target = mode;
+  a.dec = t->dec;
+  a.out = out;
+  int j = 0;
+  for (int m = 0; m < t->nmodes; ++m) {
+    a.fac.f[m] = factors[m];
+    if (m != mode) a.in.f[j++] = factors[m];
+  }
+  return ALTO_OK;
+}
+
 alto_status run_mttkrp(alto_tensor* t, int mode, const void* const* factors, alto_dtype fdtype,
                        int rank, float* out, int accumulate, alto_mttkrp_variant variant,
                        cudaStream_t st) {
   return run_mttkrp_feed(t, mode, factors, fdtype, rank, out, accumulate, variant, -1, st);
 }
 
-// feed: 1 streams the line through shared memory by bulk copy, 0 loads it
-// directly, 2 loads it directly with five blocks per SM (decoded 3-mode
-// copies: at most 48 registers a thread; six, at 40, measured slower), 3 as
-// 2 with the target mode fixed at compile time, -1 uses the autotuned choice
-// (direct when untuned).
+// feed: 1 streams the line through shared memory by bulk copy (a line that is
+// not decoded), 0 loads it directly, -1 uses the autotuned choice (direct
+// when untuned).
 alto_status run_mttkrp_feed(alto_tensor* t, int mode, const void* const* factors, alto_dtype fdtype,
                             int rank, float* out, int accumulate, alto_mttkrp_variant variant, int feed,
                             cudaStream_t st) {
@@ -1129,52 +1692,25 @@ alto_status run_mttkrp_feed(alto_tensor* t, int mode, const void* const* factors
   if (det) {
     DetItem it;
     ALTO_TRY(det_prepare(t, mode, factors, rank, out, &it, st));
-    if (it.hw == 0) return launch_det_rank<0>(it.a, rank, it.dl, st);
-    if (it.hw == 1) return launch_det_rank<1>(it.a, rank, it.dl, st);
-    if (it.hw == kDecoded3) return launch_det_rank<kDecoded3>(it.a, rank, it.dl, st);
-    return launch_det_rank<2>(it.a, rank, it.dl, st);
+    return launch_det_rank(it, rank, st);
   }
   MttkrpArgs a{};
-  a.line = t->line.p;
-  a.tile_iv = t->tile_iv.as<uint32_t>();
-  a.ntiles = t->ntiles;
   int hw = t->dec.hi_words;  // record format of the line walked
-  if (variant == ALTO_MTTKRP_SORTED) {
-    if (!t->sorted[mode].ready || t->sorted[mode].for_nnz != t->nnz)
-      ALTO_TRY(build_sorted_line(t, mode, st));
-    const SortedLine& s = t->sorted[mode];
-    a.line = s.line.p;
-    a.tile_iv = s.tile_iv.as<uint32_t>();
-    a.ntiles = s.ntiles;
-    hw = s.hw;
-  }
-  a.nnz = (uint32_t)t->nnz;
-  a.tile_nnz = t->tile_nnz;
-  a.target = mode;
-  a.dec = t->dec;
-  a.out = out;
-  bool aligned = (reinterpret_cast<uintptr_t>(out) % 16) == 0;
-  const int esz = fdtype == ALTO_BF16 ? 2 : 4;
-  for (int m = 0; m < t->nmodes; ++m) {
-    a.fac.f[m] = factors[m];
-    if (m != mode && (reinterpret_cast<uintptr_t>(factors[m]) % (4 * esz)) != 0) aligned = false;
-  }
+  ALTO_TRY(fill_args(t, mode, factors, out, variant == ALTO_MTTKRP_SORTED, &a, &hw, st));
+  // the low address bits of the output and the input factors
+  uintptr_t misalign = reinterpret_cast<uintptr_t>(out);
+  uintptr_t fac_bits = 0;
+  for (int m = 0; m < t->nmodes; ++m)
+    if (m != mode) fac_bits |= reinterpret_cast<uintptr_t>(factors[m]);
   const bool stage = variant == ALTO_MTTKRP_STAGED || variant == ALTO_MTTKRP_STREAM;
   ALTO_TRY(ensure_error_words(t, st));
   int* err = t->err.as<int>();
   const bool bulk = feed == 1;
-  const int dense = feed == 2 ? 1 : feed == 3 ? 2 : 0;
   if (fdtype == ALTO_BF16) {
-    if (hw == 0) return launch_rank<__nv_bfloat16, 0>(a, rank, stage, bulk, 0, aligned, err, st);
-    if (hw == 1) return launch_rank<__nv_bfloat16, 1>(a, rank, stage, bulk, 0, aligned, err, st);
-    if (hw == kDecoded3)
-      return launch_rank<__nv_bfloat16, kDecoded3>(a, rank, false, bulk, dense, aligned, err, st);
-    return launch_rank<__nv_bfloat16, 2>(a, rank, stage, bulk, 0, aligned, err, st);
+    if (misalign % 16) fac_bits |= 1;  // (float4 updates of the output)
+    return launch_rank<__nv_bfloat16>(a, rank, hw, stage, bulk, fac_bits % 16, err, st);
   }
-  if (hw == 0) return launch_rank<float, 0>(a, rank, stage, bulk, 0, aligned, err, st);
-  if (hw == 1) return launch_rank<float, 1>(a, rank, stage, bulk, 0, aligned, err, st);
-  if (hw == kDecoded3) return launch_rank<float, kDecoded3>(a, rank, false, bulk, dense, aligned, err, st);
-  return launch_rank<float, 2>(a, rank, stage, bulk, 0, aligned, err, st);
+  return launch_rank<float>(a, rank, hw, stage, bulk, (misalign | fac_bits) % 16, err, st);
 }
 
 alto_status det_prepare(alto_tensor* t, int mode, const void* const* factors, int rank, float* out, DetItem* item,
@@ -1184,34 +1720,17 @@ alto_status det_prepare(alto_tensor* t, int mode, const void* const* factors, in
     return ALTO_ERR_UNSUPPORTED;
   }
   MttkrpArgs a{};
-  a.line = t->line.p;
-  a.tile_iv = t->tile_iv.as<uint32_t>();
-  a.ntiles = t->nnz ? t->ntiles : 0;
   int hw = t->dec.hi_words;
-  // (a mode of length 1 is already in row order in the ALTO line)
-  if (t->dims[mode] > 1 && t->nnz) {
-    if (!t->sorted[mode].ready || t->sorted[mode].for_nnz != t->nnz) ALTO_TRY(build_sorted_line(t, mode, st));
-    const SortedLine& s = t->sorted[mode];
-    a.line = s.line.p;
-    a.tile_iv = s.tile_iv.as<uint32_t>();
-    a.ntiles = s.ntiles;
-    hw = s.hw;
-  }
-  a.nnz = (uint32_t)t->nnz;
-  a.tile_nnz = t->tile_nnz;
-  a.target = mode;
-  a.dec = t->dec;
-  a.out = out;
+  // (a mode of length 1 is already in row order in a line that is not decoded)
+  ALTO_TRY(fill_args(t, mode, factors, out, t->dims[mode] > 1 || decoded_modes(t->nmodes), &a, &hw, st));
   bool aligned = (reinterpret_cast<uintptr_t>(out) % 16) == 0;
-  for (int m = 0; m < t->nmodes; ++m) {
-    a.fac.f[m] = factors[m];
+  for (int m = 0; m < t->nmodes; ++m)
     if (m != mode && (reinterpret_cast<uintptr_t>(factors[m]) % 16) != 0) aligned = false;
-  }
   if (!aligned) {
     set_error("the deterministic MTTKRP needs 16-byte aligned factors and output");
     return ALTO_ERR_UNSUPPORTED;
   }
-  const uint64_t nslots = (uint64_t)a.ntiles * kMttkrpWarps * groups_per_warp(rank) * 2;
+  const uint64_t nslots = (uint64_t)a.ntiles * kMttkrpWarps * groups_per_warp(rank, t->nmodes, hw) * 2;
   ALTO_TRY(tensor_ensure(t, t->det_rows, std::max<uint64_t>(nslots, 1) * 4));
   ALTO_TRY(tensor_ensure(t, t->det_vals, std::max<uint64_t>(nslots, 1) * rank * 4));
   // long chains: each has more than kShortChain slots; segments:
@@ -1237,18 +1756,18 @@ alto_status det_prepare(alto_tensor* t, int mode, const void* const* factors, in
   return ALTO_OK;
 }
 
-template <int R, int HW, int NM>
+template <int R, int NIN>
 static alto_status det_group_nm(Strided<DetItem> items, const uint32_t* tile_off, cudaStream_t st) {
   static int blocks_per_sm = 0;
   if (!blocks_per_sm) {
-    ALTO_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, det_tile_group_kernel<R, HW, NM>,
+    ALTO_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, det_tile_group_kernel<R, NIN>,
                                                                 kMttkrpThreads, 0));
     if (blocks_per_sm < 1) blocks_per_sm = 1;
   }
   const unsigned sm = (unsigned)num_sms();
   det_zero_group_kernel<<<sm * 4, 256, 0, st>>>(items);
   ALTO_LAUNCHED();
-  det_tile_group_kernel<R, HW, NM><<<sm * blocks_per_sm, kMttkrpThreads, 0, st>>>(items, tile_off);
+  det_tile_group_kernel<R, NIN><<<sm * blocks_per_sm, kMttkrpThreads, 0, st>>>(items, tile_off);
   ALTO_LAUNCHED();
   det_short_group_kernel<<<sm * 16, 256, 0, st>>>(items, R);
   ALTO_LAUNCHED();
@@ -1262,13 +1781,9 @@ static alto_status det_group_nm(Strided<DetItem> items, const uint32_t* tile_off
 template <int R>
 static alto_status det_group_rank(Strided<DetItem> items, const uint32_t* tile_off, int hw, int nmodes,
                                   cudaStream_t st) {
-  if (hw == kDecoded3 && nmodes == 3) return det_group_nm<R, kDecoded3, 3>(items, tile_off, st);
-#define DG_CASE(H, NN) \
-  if (hw == H && nmodes == NN) return det_group_nm<R, H, NN>(items, tile_off, st);
-  DG_CASE(0, 3) DG_CASE(0, 4) DG_CASE(0, 5)
-  DG_CASE(1, 3) DG_CASE(1, 4) DG_CASE(1, 5)
-  DG_CASE(2, 3) DG_CASE(2, 4) DG_CASE(2, 5)
-#undef DG_CASE
+  if (hw == kDecoded && nmodes == 3) return det_group_nm<R, 2>(items, tile_off, st);
+  if (hw == kDecoded && nmodes == 4) return det_group_nm<R, 3>(items, tile_off, st);
+  if (hw == kDecoded && nmodes == 5) return det_group_nm<R, 4>(items, tile_off, st);
   set_error("grouped MTTKRP: record format %d with %d modes is not supported", hw, nmodes);
   return ALTO_ERR_UNSUPPORTED;
 }
@@ -1309,8 +1824,7 @@ alto_status autotune(alto_tensor* t, const void* const* factors, alto_dtype fdty
       int feed;
     };
     const Cand cands[] = {{ALTO_MTTKRP_ATOMIC, 0}, {ALTO_MTTKRP_ATOMIC, 1}, {ALTO_MTTKRP_STAGED, 0},
-                          {ALTO_MTTKRP_SORTED, 0}, {ALTO_MTTKRP_SORTED, 1}, {ALTO_MTTKRP_SORTED, 2},
-                          {ALTO_MTTKRP_SORTED, 3}};
+                          {ALTO_MTTKRP_SORTED, 0}};
     alto_mttkrp_variant best = ALTO_MTTKRP_ATOMIC;
     int best_feed = 0;
     float best_ms = 1e30f;
@@ -1318,7 +1832,6 @@ alto_status autotune(alto_tensor* t, const void* const* factors, alto_dtype fdty
       const alto_mttkrp_variant v = c.v;
       if (v == ALTO_MTTKRP_STAGED && stageable_fraction(t, m, rank) == 0.0) continue;
       if (v == ALTO_MTTKRP_SORTED && t->nnz / std::max<uint64_t>(t->dims[m], 1) < 2) continue;
-      if (c.feed >= 2 && t->nmodes != 3) continue;  // (decoded 3-mode copies only)
       status = run_mttkrp_feed(t, m, factors, fdtype, rank, out.as<float>(), 0, v, c.feed, st);  // warm / build
       if (status != ALTO_OK) break;
       cudaEventRecord(e0, st);

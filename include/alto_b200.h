@@ -59,15 +59,14 @@ typedef enum {
 
 /* OR-ed into the variant given to alto_mttkrp_variant_run (ATOMIC or
  * SORTED): stream the line through shared memory with bulk copies
- * (cp.async.bulk, double buffered) instead of loading it directly. */
+ * (cp.async.bulk, double buffered) instead of loading it directly.  The
+ * row-sorted copies of 3- to 5-mode tensors have one walk, which loads them
+ * directly: on those SORTED runs it with or without this flag. */
 #define ALTO_MTTKRP_FEED_BULK 0x100
-/* OR-ed into SORTED on a 3-mode tensor: the row-sorted walk compiled for
- * five resident blocks per SM (at most 48 registers a thread) instead of
- * four (the autotuner tries it). */
+/* OR-ed into SORTED on a 3-mode tensor: accepted for callers that chose among
+ * the earlier walks of the row-sorted copy; the one walk there is now fixes
+ * the target mode in the copy and is at least as fast as each of them. */
 #define ALTO_MTTKRP_FEED_DENSE 0x200
-/* OR-ed into SORTED on a 3-mode tensor: the five-blocks walk compiled once
- * per target mode, so the rows of the decoded records need no per-nonzero
- * mode selection (the autotuner tries it). */
 #define ALTO_MTTKRP_FEED_FIXED_TARGET 0x400
 
 /* Constraint of the CP-stream factor solves (src/constraints.cpp:39-66; the

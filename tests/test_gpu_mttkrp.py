@@ -203,6 +203,50 @@ def test_autotune_records_a_choice_per_mode():
         assert rel_err(t.mttkrp(m, Fd, R).cpu().numpy(), ref) <= TOL
 
 
+# ------------------------------------------------- row-sorted and any-rank walks
+
+@pytest.mark.parametrize("R", [1, 3, 6, 10, 12, 24, 33, 64, 100, 130, 260])
+@pytest.mark.parametrize("nmodes", [2, 3, 4, 5, 6])
+def test_walks_of_every_rank_and_mode_count(nmodes, R):
+    """The row-sorted and the any-rank walk at ranks around their lane splits
+    (one lane, a lane group that does not divide the warp, several column
+    windows) and with factors and output at odd addresses: the same bound as
+    the specialised kernels.  The last run's length leaves partial steps."""
+    import torch
+
+    dims = np.array([37, 53, 41, 29, 31, 23][:nmodes], np.uint64)
+    cidx, vals = synth.uniform_coo(dims, 1501 if nmodes == 2 else 9973, seed=R)
+    t = A.create_alto(dims, cidx, vals)
+    enc = O.build(dims, cidx, vals.astype(np.float32).astype(np.float64))
+    rng = np.random.default_rng(R)
+    F = [rng.uniform(-1.0, 1.0, (int(d), R)) for d in dims]
+    for dtype in (torch.float32, torch.bfloat16):
+        for shift in (0, 1, 2):
+            Fd = []
+            for f in F:
+                room = torch.zeros(f.size + shift, dtype=dtype, device="cuda")
+                room[shift:] = torch.tensor(f.ravel(), dtype=torch.float32, device="cuda").to(dtype)
+                Fd.append(room[shift:].view(f.shape))
+            Fo = seen_by_gpu(Fd)
+            for m in range(nmodes):
+                fs = [f.copy() for f in Fo]
+                fs[m][:] = 0
+                ref = O.mttkrp(enc, m, fs, R)[m]
+                room = torch.full((int(dims[m]) * R + shift,), np.nan, device="cuda")
+                out = room[shift:].view(int(dims[m]), R)
+                for v in (A.SORTED, A.ATOMIC, A.AUTO):
+                    t.mttkrp(m, Fd, R, out=out, variant=v)
+                    got = out.cpu().numpy()
+                    assert rel_err(got, ref) <= TOL, (dtype, shift, m, v, rel_err(got, ref))
+                    assert shift == 0 or bool(torch.isnan(room[:shift]).all())  # nothing written before it
+
+
+def test_decoded_copies_of_keys_above_96_bits():
+    dims = np.array([700000, 650000, 800000, 600000, 900000], np.uint64)
+    cidx, vals = synth.uniform_coo(dims, 30000, seed=3)
+    check_modes(dims, cidx, vals, 8, variants=(A.SORTED, A.ATOMIC, A.SORTED | A.FEED_BULK))
+
+
 # ------------------------------------------------- deterministic variant
 
 def check_deterministic(dims, cidx, vals, R, seed=0, stream_mode=-1):
