@@ -23,8 +23,17 @@
 
 namespace alto {
 
-constexpr int kGramThreads = 256;
-constexpr int kGramRows = 32;
+// d += a b on the float64 tensor cores, one 8 x 8 x 4 step of a warp: lane l
+// gives a = A[l / 4][l % 4] and b = B[l % 4][l / 4] and holds D[l / 4][2 (l % 4)]
+// and the element to its right.  Float64 products and sums, as __fma_rn; the
+// tensor cores' float64 rate is that of the FMA units (37 TFLOP/s measured for
+// both), but an instruction is 256 multiply-adds for two operand registers a
+// lane, where the FMA form reads shared memory for every few.
+__device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
 
 static int g_sms = 0;
 static int sms() {
@@ -41,279 +50,297 @@ template <typename T>
 __device__ __forceinline__ double ld(const T* p, size_t i) {
   return (double)p[i];
 }
-template <>
-__device__ __forceinline__ double ld<__nv_bfloat16>(const __nv_bfloat16* p, size_t i) {
-  return (double)__bfloat162float(p[i]);
+
+// ------------------------------------------------------------ Grams
+//
+// G = U^T U and, in the same pass, C = P^T U with the change statistics, as
+// float64 tensor-core products over the rows.  A fragment of four rows by
+// eight columns -- lane l holds (row l % 4, column l / 4), converted from the
+// float32 element it loads -- is at once the A operand of the output tiles of
+// its columns as rows and the B operand of those of its columns as columns, so
+// a warp reads each element once, with no shared memory, and a step of four
+// rows is T (T + 1) / 2 + T^2 products for 2 T loads (T = ceil(R / 8); G only
+// on and above the diagonal tiles).  Bound by the float64 rate from rank 32
+// (120,000 rows at rank 32: 11 us), by HBM below.  The form before staged the
+// rows in shared memory and read two doubles for every multiply-add (73 us
+// there; 93 us for 20,000 rows at rank 64).
+//
+// Up to rank 32 every warp of a block holds all tiles and takes its own rows;
+// above, the block's eight warps share the rows and warp w holds the tiles of
+// tile rows w, w + 8, ... (the accumulators of rank 64 are eight warps' registers).
+
+constexpr int kGramThreads = 128;      // T <= 4
+constexpr int kGramThreadsWide = 256;  // T > 4
+constexpr int kGramBlocksPerSm = 2;
+
+__host__ __device__ constexpr int gram_tiles(int R) { return (R + 7) / 8; }
+// Output tiles, 64 doubles each, of one pass: G's on and above the diagonal,
+// then C's.  Lane l of a tile's warp owns elements 2 l and 2 l + 1:
+// (l / 4, 2 (l % 4)) and its right neighbour.
+__host__ __device__ constexpr int gram_out_tiles(int T, bool cross) { return T * (T + 1) / 2 + (cross ? T * T : 0); }
+__host__ __device__ constexpr int gram_tile_of(int T, int a, int b) { return a * T - a * (a - 1) / 2 + (b - a); }
+// Doubles of one block's partial result (with the three statistics).
+__host__ __device__ constexpr int gram_partial_len(int R, bool cross) {
+  return gram_out_tiles(gram_tiles(R), cross) * 64 + (cross ? 3 : 0);
 }
 
-// Partial A^T B over a block's row range; PPT (a, b) pairs per thread.
-template <int PPT, typename TA, typename TB>
-__global__ void __launch_bounds__(kGramThreads)
-    gram_partial_kernel(const TA* __restrict__ A, const TB* __restrict__ B, uint64_t I, int R,
-                        uint64_t rows_per_block, double* __restrict__ partials) {
-  extern __shared__ double sm[];
-  double* sa = sm;
-  double* sb = sm + kGramRows * R;
-  double acc[PPT];
-#pragma unroll
-  for (int k = 0; k < PPT; ++k) acc[k] = 0.0;
-  const uint64_t r0 = (uint64_t)blockIdx.x * rows_per_block;
-  const uint64_t r1 = min(r0 + rows_per_block, I);
-  const int RR = R * R;
-  for (uint64_t t0 = r0; t0 < r1; t0 += kGramRows) {
-    const int nr = (int)min((uint64_t)kGramRows, r1 - t0);
-    for (int q = threadIdx.x; q < nr * R; q += kGramThreads) {
-      sa[q] = ld(A, t0 * R + q);
-      sb[q] = ld(B, t0 * R + q);
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < PPT; ++k) {
-      const int p = threadIdx.x + k * kGramThreads;
-      if (p < RR) {
-        const int a = p / R, b = p % R;
-        double s = 0.0;
-        for (int r = 0; r < nr; ++r) s += sa[r * R + a] * sb[r * R + b];
-        acc[k] += s;
-      }
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int k = 0; k < PPT; ++k) {
-    const int p = threadIdx.x + k * kGramThreads;
-    if (p < RR) partials[(size_t)blockIdx.x * RR + p] = acc[k];
-  }
+__device__ __forceinline__ void change_stats(double p, double u, double (&q)[3]) {
+  const double d = p - u;
+  q[0] = __fma_rn(p, u, q[0]);
+  q[1] = __fma_rn(d, d, q[1]);
+  q[2] = __fma_rn(u, u, q[2]);
 }
 
-// out[p] = sum over blocks b of partials[b][p] in a fixed order: block x
-// takes 32 consecutive p (one per lane, coalesced), warp w sums blocks
-// w, w+8, w+16, ... and the 8 warp sums are added in warp order.  Launch with
-// reduce_grid(n) blocks of kReduceThreads threads.
-constexpr int kReduceThreads = 256;
-__host__ __device__ inline unsigned reduce_grid(int n) { return (unsigned)((n + 31) / 32); }
-
-__global__ void __launch_bounds__(kReduceThreads)
-    reduce_partials_kernel(const double* __restrict__ partials, int nblocks, int n, double* __restrict__ out) {
-  __shared__ double s[kReduceThreads / 32][32];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int p = blockIdx.x * 32 + lane;
-  double acc = 0.0;
-  if (p < n)
-    for (int b = w; b < nblocks; b += kReduceThreads / 32) acc += partials[(size_t)b * n + p];
-  s[w][lane] = acc;
-  __syncthreads();
-  if (w == 0 && p < n) {
-    double t = s[0][lane];
-    for (int k = 1; k < kReduceThreads / 32; ++k) t += s[k][lane];
-    out[p] = t;
-  }
-}
-
-template <typename TA, typename TB>
-static alto_status gram_launch(const TA* A, const TB* B, uint64_t I, int R, double* out,
-                               DevBuf& scratch, cudaStream_t st) {
-  const int RR = R * R;
-  const int ppt = (RR + kGramThreads - 1) / kGramThreads;
-  uint64_t nb = std::min<uint64_t>((I + 255) / 256, (uint64_t)sms() * 2);
-  if (nb < 1) nb = 1;
-  const uint64_t rpb = (I + nb - 1) / nb;
-  nb = I ? (I + rpb - 1) / rpb : 1;
-  ALTO_TRY(scratch.ensure(nb * RR * sizeof(double)));
-  const size_t smem = 2 * kGramRows * R * sizeof(double);
-  double* part = scratch.as<double>();
-  if (I == 0) {
-    ALTO_TRY_CUDA(cudaMemsetAsync(out, 0, RR * sizeof(double), st));
-    return ALTO_OK;
-  }
-  // (the shared-memory limit is raised once per kernel, outside any capture)
-#define GRAM_CASE(P)                                                                             \
-  case P:                                                                                        \
-    if (smem > 48 * 1024) {                                                                      \
-      static size_t raised = 0;                                                                  \
-      if (smem > raised) {                                                                       \
-        ALTO_TRY_CUDA(cudaFuncSetAttribute(gram_partial_kernel<P, TA, TB>,                      \
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-        raised = smem;                                                                           \
-      }                                                                                          \
-    }                                                                                            \
-    gram_partial_kernel<P, TA, TB><<<(unsigned)nb, kGramThreads, smem, st>>>(A, B, I, R, rpb, part); \
-    break;
-  switch (ppt <= 1 ? 1 : ppt <= 2 ? 2 : ppt <= 4 ? 4 : ppt <= 8 ? 8 : ppt <= 16 ? 16 : 64) {
-    GRAM_CASE(1)
-    GRAM_CASE(2)
-    GRAM_CASE(4)
-    GRAM_CASE(8)
-    GRAM_CASE(16)
-    GRAM_CASE(64)
-  }
-#undef GRAM_CASE
-  ALTO_LAUNCHED();
-  reduce_partials_kernel<<<reduce_grid(RR), kReduceThreads, 0, st>>>(part, (int)nb, RR, out);
-  ALTO_LAUNCHED();
-  return ALTO_OK;
-}
-
-// One pass over P and U (float32, I x R): per-block partials of U^T U,
-// P^T U and {sum p u, sum (p - u)^2, sum u^2} (the CP-stream Gram, cross
-// Gram and change statistics of a freshly updated factor), layout
-// [block][2 R^2 + 3].  The rows are staged kGramRows at a time in two
-// alternating shared-memory buffers (one barrier per chunk).  For ranks 23
-// to 32 the next chunk's loads are issued into registers before the
-// current chunk's products, so their latency overlaps the arithmetic
-// (measured 17% faster at rank 32; at ranks up to 16 the extra registers
-// cost more occupancy than the overlap gains, and larger ranks' accumulators
-// fill the registers).  Dynamic shared memory: 4 kGramRows R doubles.
-template <int PPT>
-constexpr int gram_stage_regs() {  // ceil(kGramRows R / threads) for the largest R of PPT
-  return PPT <= 1 ? 2 : PPT <= 2 ? 3 : PPT <= 4 ? 4 : PPT <= 16 ? 8 : 16;
-}
-
-template <int PPT>
-__device__ __forceinline__ void gram_cross_partial_body(const float* __restrict__ P, const float* __restrict__ U,
-                                                        uint64_t I, int R, uint64_t rows_per_block,
-                                                        double* __restrict__ partials, uint32_t block) {
-  constexpr int L = gram_stage_regs<PPT>();
-  constexpr bool kPipe = PPT == 4;
-  extern __shared__ double sm[];
-  double g[PPT], c[PPT];
+// The block's three statistics: warp butterflies, then warps in order.
+__device__ __forceinline__ void store_stats(double (&q)[3], double* __restrict__ out) {
+  __shared__ double wq[3][8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
-  for (int k = 0; k < PPT; ++k) g[k] = c[k] = 0.0;
-  double q0 = 0.0, q1 = 0.0, q2 = 0.0;
-  const uint64_t r0 = (uint64_t)block * rows_per_block;
-  const uint64_t r1 = min(r0 + rows_per_block, I);
-  const int RR = R * R;
-  float pre_p[kPipe ? L : 1], pre_u[kPipe ? L : 1];
-  auto fetch = [&](uint64_t t0) {  // chunk at row t0 into registers
-    const int n = (int)min((uint64_t)kGramRows, r1 - t0) * R;
-#pragma unroll
-    for (int l = 0; l < (kPipe ? L : 1); ++l) {
-      const int q = threadIdx.x + l * kGramThreads;
-      pre_p[l] = q < n ? P[t0 * R + q] : 0.f;
-      pre_u[l] = q < n ? U[t0 * R + q] : 0.f;
-    }
-  };
-  if (kPipe && r0 < r1) fetch(r0);
-  int buf = 0;
-  for (uint64_t t0 = r0; t0 < r1; t0 += kGramRows) {
-    const int nr = (int)min((uint64_t)kGramRows, r1 - t0);
-    double* sp = sm + (size_t)buf * 2 * kGramRows * R;
-    double* su = sp + kGramRows * R;
-    if constexpr (kPipe) {
-#pragma unroll
-      for (int l = 0; l < L; ++l) {
-        const int q = threadIdx.x + l * kGramThreads;
-        if (q < nr * R) {
-          const double pv = (double)pre_p[l], uv = (double)pre_u[l];
-          sp[q] = pv;
-          su[q] = uv;
-          q0 += pv * uv;
-          q1 += (pv - uv) * (pv - uv);
-          q2 += uv * uv;
-        }
-      }
-    } else {
-      for (int q = threadIdx.x; q < nr * R; q += kGramThreads) {
-        const double pv = (double)P[t0 * R + q], uv = (double)U[t0 * R + q];
-        sp[q] = pv;
-        su[q] = uv;
-        q0 += pv * uv;
-        q1 += (pv - uv) * (pv - uv);
-        q2 += uv * uv;
-      }
-    }
-    __syncthreads();
-    if (kPipe && t0 + kGramRows < r1) fetch(t0 + kGramRows);
-#pragma unroll
-    for (int k = 0; k < PPT; ++k) {
-      const int p = threadIdx.x + k * kGramThreads;
-      if (p < RR) {
-        const int a = p / R, b = p % R;
-        double sg = 0.0, sc = 0.0;
-        for (int r = 0; r < nr; ++r) {
-          const double ub = su[r * R + b];
-          sg += su[r * R + a] * ub;
-          sc += sp[r * R + a] * ub;
-        }
-        g[k] += sg;
-        c[k] += sc;
-      }
-    }
-    buf ^= 1;
-  }
-  double* out = partials + (size_t)block * (2 * RR + 3);
-#pragma unroll
-  for (int k = 0; k < PPT; ++k) {
-    const int p = threadIdx.x + k * kGramThreads;
-    if (p < RR) {
-      out[p] = g[k];
-      out[RR + p] = c[k];
-    }
-  }
-  // the three statistics: warp butterflies, then warps in order
-  __shared__ double wq[3][kGramThreads / 32];
-  for (int o = 16; o; o >>= 1) {
-    q0 += __shfl_xor_sync(0xffffffffu, q0, o);
-    q1 += __shfl_xor_sync(0xffffffffu, q1, o);
-    q2 += __shfl_xor_sync(0xffffffffu, q2, o);
-  }
-  if ((threadIdx.x & 31) == 0) {
-    wq[0][threadIdx.x >> 5] = q0;
-    wq[1][threadIdx.x >> 5] = q1;
-    wq[2][threadIdx.x >> 5] = q2;
+  for (int k = 0; k < 3; ++k) {
+    for (int o = 16; o; o >>= 1) q[k] += __shfl_xor_sync(0xffffffffu, q[k], o);
+    if (lane == 0) wq[k][warp] = q[k];
   }
   __syncthreads();
   if (threadIdx.x < 3) {
     double t = 0.0;
-    for (int w = 0; w < kGramThreads / 32; ++w) t += wq[threadIdx.x][w];
-    out[2 * RR + threadIdx.x] = t;
+    for (int w = 0; w < nw; ++w) t += wq[threadIdx.x][w];
+    out[threadIdx.x] = t;
   }
   __syncthreads();
 }
 
-template <int PPT>
-__global__ void __launch_bounds__(kGramThreads)
-    gram_cross_partial_kernel(const float* __restrict__ P, const float* __restrict__ U, uint64_t I, int R,
-                              uint64_t rows_per_block, double* __restrict__ partials) {
-  gram_cross_partial_body<PPT>(P, U, I, R, rows_per_block, partials, blockIdx.x);
+// Partial sums over rows [r0, r1), T <= 4 column tiles.
+template <int T, bool CROSS>
+__device__ __forceinline__ void gram_narrow(const float* __restrict__ P, const float* __restrict__ U, uint64_t r0,
+                                            uint64_t r1, int R, double* __restrict__ out) {
+  constexpr int NG = T * (T + 1) / 2, NT = gram_out_tiles(T, CROSS), NW = kGramThreads / 32;
+  constexpr int S = T == 1 ? 8 : T == 2 ? 4 : 2;  // steps of four rows whose loads are issued together
+  __shared__ double red[NT * 64];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int kr = lane & 3, kc = lane >> 2;
+  double acc[NT][2];
+#pragma unroll
+  for (int t = 0; t < NT; ++t) acc[t][0] = acc[t][1] = 0.0;
+  double q[3] = {0.0, 0.0, 0.0};
+  float fu[S][T], fp[CROSS ? S : 1][T];
+  auto fetch = [&](uint64_t k0) {
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      const uint64_t row = k0 + (uint64_t)s * 4 * NW + kr;
+#pragma unroll
+      for (int c = 0; c < T; ++c) {
+        const int col = c * 8 + kc;
+        const bool ok = row < r1 && col < R;
+        fu[s][c] = ok ? U[row * R + col] : 0.f;
+        if (CROSS) fp[s][c] = ok ? P[row * R + col] : 0.f;
+      }
+    }
+  };
+  const uint64_t first = r0 + warp * 4;
+  if (first < r1) fetch(first);
+  for (uint64_t k0 = first; k0 < r1; k0 += (uint64_t)S * 4 * NW) {
+    float cu[S][T], cp[CROSS ? S : 1][T];
+#pragma unroll
+    for (int s = 0; s < S; ++s)
+#pragma unroll
+      for (int c = 0; c < T; ++c) {
+        cu[s][c] = fu[s][c];
+        if (CROSS) cp[s][c] = fp[s][c];
+      }
+    if (k0 + (uint64_t)S * 4 * NW < r1) fetch(k0 + (uint64_t)S * 4 * NW);
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      double u[T], p[T];
+#pragma unroll
+      for (int c = 0; c < T; ++c) {
+        u[c] = (double)cu[s][c];
+        if (CROSS) {
+          p[c] = (double)cp[s][c];
+          change_stats(p[c], u[c], q);
+        }
+      }
+#pragma unroll
+      for (int a = 0; a < T; ++a)
+#pragma unroll
+        for (int b = a; b < T; ++b) dmma_8x8x4(acc[gram_tile_of(T, a, b)], u[a], u[b]);
+      if (CROSS)
+#pragma unroll
+        for (int a = 0; a < T; ++a)
+#pragma unroll
+          for (int b = 0; b < T; ++b) dmma_8x8x4(acc[NG + a * T + b], p[a], u[b]);
+    }
+  }
+  // the warps' sums in warp order
+  for (int w = 0; w < NW; ++w) {
+    if (warp == w)
+#pragma unroll
+      for (int t = 0; t < NT; ++t)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          double& r = red[t * 64 + 2 * lane + e];
+          r = w == 0 ? acc[t][e] : r + acc[t][e];
+        }
+    __syncthreads();
+  }
+  for (int p = threadIdx.x; p < NT * 64; p += kGramThreads) out[p] = red[p];
+  if (CROSS) store_stats(q, out + NT * 64);
+  __syncthreads();
 }
 
-// reduce_partials_kernel with the result split over three outputs:
-// [0, n1) -> o1, [n1, 2 n1) -> o2, the rest -> o3.
-__device__ __forceinline__ void reduce_split_body(const double* __restrict__ partials, int nblocks, int n1, int n,
-                                                  double* __restrict__ o1, double* __restrict__ o2,
-                                                  double* __restrict__ o3, uint32_t block) {
+// The same for more than four column tiles (T at run time).
+template <bool CROSS>
+__device__ __forceinline__ void gram_wide(const float* __restrict__ P, const float* __restrict__ U, uint64_t r0,
+                                          uint64_t r1, int R, double* __restrict__ out) {
+  const int T = gram_tiles(R), NG = T * (T + 1) / 2;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int kr = lane & 3, kc = lane >> 2;
+  double q[3] = {0.0, 0.0, 0.0};
+  for (int a = warp; a < T; a += 8)
+    for (int cb = 0; cb < T; cb += 8) {
+      double g[8][2], c[CROSS ? 8 : 1][2];
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        g[b][0] = g[b][1] = 0.0;
+        if (CROSS) c[b][0] = c[b][1] = 0.0;
+      }
+      float fb[8], fa = 0.f, pa = 0.f;
+      auto fetch = [&](uint64_t k0) {
+        const uint64_t row = k0 + kr;
+        const bool in = row < r1;
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+          const int col = (cb + b) * 8 + kc;
+          fb[b] = in && col < R ? U[row * R + col] : 0.f;
+        }
+        const int col = a * 8 + kc;
+        fa = in && col < R ? U[row * R + col] : 0.f;
+        if (CROSS) pa = in && col < R ? P[row * R + col] : 0.f;
+      };
+      if (r0 < r1) fetch(r0);
+      for (uint64_t k0 = r0; k0 < r1; k0 += 4) {
+        double ub[8];
+#pragma unroll
+        for (int b = 0; b < 8; ++b) ub[b] = (double)fb[b];
+        const double ua = (double)fa, pv = (double)pa;
+        if (k0 + 4 < r1) fetch(k0 + 4);
+        if (CROSS && cb == 0) change_stats(pv, ua, q);
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+          if (cb + b >= a) dmma_8x8x4(g[b], ua, ub[b]);
+          if (CROSS) dmma_8x8x4(c[b], pv, ub[b]);
+        }
+      }
+#pragma unroll
+      for (int b = 0; b < 8; ++b) {
+        if (cb + b >= T) continue;
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          if (cb + b >= a) out[gram_tile_of(T, a, cb + b) * 64 + 2 * lane + e] = g[b][e];
+          if (CROSS) out[(NG + a * T + cb + b) * 64 + 2 * lane + e] = c[b][e];
+        }
+      }
+    }
+  if (CROSS) store_stats(q, out + gram_out_tiles(T, true) * 64);
+  __syncthreads();
+}
+
+// TT: 1 to 4 column tiles, or 0 for more.
+template <int TT, bool CROSS>
+__device__ __forceinline__ void gram_block(const float* __restrict__ P, const float* __restrict__ U, uint64_t I, int R,
+                                           uint64_t rows_per_block, double* __restrict__ partials, uint32_t block) {
+  const uint64_t r0 = (uint64_t)block * rows_per_block;
+  const uint64_t r1 = min(r0 + rows_per_block, I);
+  double* out = partials + (size_t)block * gram_partial_len(R, CROSS);
+  if constexpr (TT == 0)
+    gram_wide<CROSS>(P, U, r0, r1, R, out);
+  else
+    gram_narrow<TT, CROSS>(P, U, r0, r1, R, out);
+}
+
+template <int TT>
+struct GramLaunch {
+  static constexpr int kThreads = TT ? kGramThreads : kGramThreadsWide;
+  static constexpr int kMinBlocks = TT == 0 || TT == 4 ? 2 : 3;
+};
+
+template <int TT, bool CROSS>
+__global__ void __launch_bounds__(GramLaunch<TT>::kThreads, GramLaunch<TT>::kMinBlocks)
+    gram_kernel(const float* __restrict__ P, const float* __restrict__ U, uint64_t I, int R, uint64_t rows_per_block,
+                double* __restrict__ partials) {
+  gram_block<TT, CROSS>(P, U, I, R, rows_per_block, partials, blockIdx.x);
+}
+
+// sum over blocks b of partials[b][p] for 32 consecutive p (one per lane), in a
+// fixed order: warp w sums blocks w, w + nw, ... and the warp sums are added in
+// warp order.  Every thread of warp 0 gets its p's sum.
+constexpr int kReduceThreads = 512;
+__host__ __device__ inline unsigned reduce_grid(int n) { return (unsigned)((n + 31) / 32); }
+
+__device__ __forceinline__ double reduce_column(const double* __restrict__ partials, int nblocks, int n, int p) {
   __shared__ double s[kReduceThreads / 32][32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int p = block * 32 + lane;
   double acc = 0.0;
   if (p < n)
+#pragma unroll 4
     for (int b = w; b < nblocks; b += kReduceThreads / 32) acc += partials[(size_t)b * n + p];
   s[w][lane] = acc;
   __syncthreads();
-  if (w == 0 && p < n) {
-    double t = s[0][lane];
+  double t = 0.0;
+  if (w == 0) {
+    t = s[0][lane];
     for (int k = 1; k < kReduceThreads / 32; ++k) t += s[k][lane];
-    if (p < n1)
-      o1[p] = t;
-    else if (p < 2 * n1)
-      o2[p - n1] = t;
-    else if (o3)
-      o3[p - 2 * n1] = t;
   }
   __syncthreads();
+  return t;
 }
 
 __global__ void __launch_bounds__(kReduceThreads)
-    reduce_split_kernel(const double* __restrict__ partials, int nblocks, int n1, int n, double* __restrict__ o1,
-                        double* __restrict__ o2, double* __restrict__ o3) {
-  reduce_split_body(partials, nblocks, n1, n, o1, o2, o3, blockIdx.x);
+    reduce_partials_kernel(const double* __restrict__ partials, int nblocks, int n, double* __restrict__ out) {
+  const int p = blockIdx.x * 32 + (threadIdx.x & 31);
+  const double t = reduce_column(partials, nblocks, n, p);
+  if (threadIdx.x < 32 && p < n) out[p] = t;
+}
+
+// Reduction block `block` of a Gram pass: its outputs back in row-major order
+// (G mirrored from the tiles on and above the diagonal).
+template <bool CROSS>
+__device__ __forceinline__ void gram_reduce_body(const double* __restrict__ partials, int nblocks, int R,
+                                                 double* __restrict__ G, double* __restrict__ C,
+                                                 double* __restrict__ stats3, uint32_t block) {
+  const int n = gram_partial_len(R, CROSS), T = gram_tiles(R), NG = T * (T + 1) / 2, NT = gram_out_tiles(T, CROSS);
+  const int p = block * 32 + (threadIdx.x & 31);
+  const double t = reduce_column(partials, nblocks, n, p);
+  if (threadIdx.x >= 32 || p >= n) return;
+  if (p >= NT * 64) {
+    if (stats3) stats3[p - NT * 64] = t;
+    return;
+  }
+  int tile = p / 64;
+  const int l = (p % 64) / 2, i = l >> 2, j = 2 * (l & 3) + (p & 1);
+  if (tile < NG) {
+    int a = 0;
+    while (tile >= T - a) tile -= T - a++;
+    const int row = a * 8 + i, col = (a + tile) * 8 + j;
+    if (row >= R || col >= R) return;
+    G[row * R + col] = t;
+    if (tile) G[col * R + row] = t;
+  } else {
+    const int row = (tile - NG) / T * 8 + i, col = (tile - NG) % T * 8 + j;
+    if (row < R && col < R) C[row * R + col] = t;
+  }
+}
+
+template <bool CROSS>
+__global__ void __launch_bounds__(kReduceThreads)
+    gram_reduce_kernel(const double* __restrict__ partials, int nblocks, int R, double* __restrict__ G,
+                       double* __restrict__ C, double* __restrict__ stats3) {
+  gram_reduce_body<CROSS>(partials, nblocks, R, G, C, stats3, blockIdx.x);
 }
 
 // Grouped gram_cross_stats: partial blocks over all items (block_off
 // prefix sums of the items' nb), then reduction blocks (red_off).
-template <int PPT>
-__global__ void __launch_bounds__(kGramThreads)
+template <int TT>
+__global__ void __launch_bounds__(GramLaunch<TT>::kThreads, GramLaunch<TT>::kMinBlocks)
     gram_group_partial_kernel(Strided<GramItem> items, const uint32_t* __restrict__ block_off, int R) {
   const int K = *items.count;
   const uint32_t total = K > 0 ? block_off[K] : 0;
@@ -328,7 +355,7 @@ __global__ void __launch_bounds__(kGramThreads)
     }
     const GramItem& it = items[lo];
     if (it.active && !*it.active) continue;
-    gram_cross_partial_body<PPT>(it.P, it.U, it.I, R, it.rpb, it.part, v - block_off[lo]);
+    gram_block<TT, true>(it.P, it.U, it.I, R, it.rpb, it.part, v - block_off[lo]);
   }
 }
 
@@ -336,7 +363,6 @@ __global__ void __launch_bounds__(kReduceThreads)
     gram_group_reduce_kernel(Strided<GramItem> items, const uint32_t* __restrict__ red_off, int R) {
   const int K = *items.count;
   const uint32_t total = K > 0 ? red_off[K] : 0;
-  const int RR = R * R, n = 2 * RR + 3;
   for (uint32_t v = blockIdx.x; v < total; v += gridDim.x) {
     int lo = 0, hi = K;
     while (hi - lo > 1) {
@@ -348,13 +374,13 @@ __global__ void __launch_bounds__(kReduceThreads)
     }
     const GramItem& it = items[lo];
     if (it.active && !*it.active) continue;
-    reduce_split_body(it.part, (int)it.nb, RR, n, it.G, it.C, it.stats3, v - red_off[lo]);
+    gram_reduce_body<true>(it.part, (int)it.nb, R, it.G, it.C, it.stats3, v - red_off[lo]);
   }
 }
 
-// At least 64 rows per block, at most 4 blocks per SM.
+// At least 64 rows per block, at most kGramBlocksPerSm blocks per SM.
 void gram_split(uint64_t I, uint32_t* nb_out, uint64_t* rpb_out) {
-  uint64_t nb = std::min<uint64_t>((I + 63) / 64, (uint64_t)sms() * 4);
+  uint64_t nb = std::min<uint64_t>((I + 63) / 64, (uint64_t)sms() * kGramBlocksPerSm);
   if (nb < 1) nb = 1;
   const uint64_t rpb = (I + nb - 1) / nb;
   nb = I ? (I + rpb - 1) / rpb : 1;
@@ -362,51 +388,33 @@ void gram_split(uint64_t I, uint32_t* nb_out, uint64_t* rpb_out) {
   *rpb_out = rpb;
 }
 
-uint32_t gram_reduce_blocks(int R) { return reduce_grid(2 * R * R + 3); }
-
-// The grouped Gram's shared-memory limit for rank R raised ahead of a
-// capture (gram_group_launch raises it too; this keeps the call out of the
-// captured sequence).
-alto_status gram_group_ready(int R) {
-  const int ppt = (R * R + kGramThreads - 1) / kGramThreads;
-  const int smem = 4 * kGramRows * R * (int)sizeof(double);
-  if (smem <= 48 * 1024) return ALTO_OK;
-  const void* fn = ppt <= 1 ? (const void*)gram_group_partial_kernel<1>
-                   : ppt <= 2 ? (const void*)gram_group_partial_kernel<2>
-                   : ppt <= 4 ? (const void*)gram_group_partial_kernel<4>
-                   : ppt <= 16 ? (const void*)gram_group_partial_kernel<16>
-                               : (const void*)gram_group_partial_kernel<64>;
-  ALTO_TRY_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  return ALTO_OK;
+uint64_t gram_partial_doubles(uint64_t I, int R, bool cross) {
+  uint32_t nb = 1;
+  uint64_t rpb = 1;
+  gram_split(I, &nb, &rpb);
+  return (uint64_t)nb * gram_partial_len(R, cross);
 }
+
+uint32_t gram_reduce_blocks(int R) { return reduce_grid(gram_partial_len(R, true)); }
+
+// Launch `kernel<TT, ...>` for rank R.
+#define GRAM_DISPATCH(R, LAUNCH) \
+  switch (gram_tiles(R)) {       \
+    case 1: LAUNCH(1); break;    \
+    case 2: LAUNCH(2); break;    \
+    case 3: LAUNCH(3); break;    \
+    case 4: LAUNCH(4); break;    \
+    default: LAUNCH(0); break;   \
+  }
 
 alto_status gram_group_launch(Strided<GramItem> items, const uint32_t* block_off, const uint32_t* red_off,
                               int max_items, int R, cudaStream_t st) {
-  const int RR = R * R;
-  const int ppt = (RR + kGramThreads - 1) / kGramThreads;
-  const size_t smem = 4 * kGramRows * R * sizeof(double);  // two staged chunks of P and U
-  const unsigned grid = (unsigned)sms() * 4;
-#define GG_CASE(PP)                                                                                   \
-  case PP: {                                                                                          \
-    static size_t raised = 0;                                                                         \
-    if (smem > 48 * 1024 && smem > raised) {                                                          \
-      ALTO_TRY_CUDA(cudaFuncSetAttribute(gram_group_partial_kernel<PP>,                               \
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));   \
-      raised = smem;                                                                                  \
-    }                                                                                                 \
-    gram_group_partial_kernel<PP><<<grid, kGramThreads, smem, st>>>(items, block_off, R);             \
-    break;                                                                                            \
-  }
-  switch (ppt <= 1 ? 1 : ppt <= 2 ? 2 : ppt <= 4 ? 4 : ppt <= 16 ? 16 : 64) {
-    GG_CASE(1)
-    GG_CASE(2)
-    GG_CASE(4)
-    GG_CASE(16)
-    GG_CASE(64)
-  }
-#undef GG_CASE
+  const unsigned grid = (unsigned)sms() * 3;
+#define GG(TT) gram_group_partial_kernel<TT><<<grid, GramLaunch<TT>::kThreads, 0, st>>>(items, block_off, R)
+  GRAM_DISPATCH(R, GG)
+#undef GG
   ALTO_LAUNCHED();
-  const unsigned rgrid = (unsigned)std::max(1, std::min(max_items * (int)gram_reduce_blocks(R), (int)sms() * 8));
+  const unsigned rgrid = (unsigned)std::max(1, std::min(max_items * (int)gram_reduce_blocks(R), (int)sms() * 4));
   gram_group_reduce_kernel<<<rgrid, kReduceThreads, 0, st>>>(items, red_off, R);
   ALTO_LAUNCHED();
   return ALTO_OK;
@@ -414,58 +422,52 @@ alto_status gram_group_launch(Strided<GramItem> items, const uint32_t* block_off
 
 alto_status gram_cross_stats(const float* P, const float* U, uint64_t I, int R, double* G, double* C,
                              double* stats3, DevBuf& scratch, cudaStream_t st) {
-  const int RR = R * R;
-  const int n = 2 * RR + 3;
-  const int ppt = (RR + kGramThreads - 1) / kGramThreads;
-  uint32_t nb32 = 1;
+  uint32_t nb = 1;
   uint64_t rpb = 1;
-  gram_split(I, &nb32, &rpb);
-  uint64_t nb = nb32;
-  ALTO_TRY(scratch.ensure(nb * n * sizeof(double)));
+  gram_split(I, &nb, &rpb);
+  ALTO_TRY(scratch.ensure(gram_partial_doubles(I, R, true) * sizeof(double)));
   double* part = scratch.as<double>();
-  const size_t smem = 4 * kGramRows * R * sizeof(double);  // two staged chunks of P and U
   if (I == 0) {
-    ALTO_TRY_CUDA(cudaMemsetAsync(part, 0, n * sizeof(double), st));
-    nb = 1;
+    ALTO_TRY_CUDA(cudaMemsetAsync(part, 0, gram_partial_len(R, true) * sizeof(double), st));
   } else {
-#define GC_CASE(PP)                                                                                  \
-  case PP: {                                                                                         \
-    static size_t raised = 0;                                                                        \
-    if (smem > 48 * 1024 && smem > raised) {                                                         \
-      ALTO_TRY_CUDA(cudaFuncSetAttribute(gram_cross_partial_kernel<PP>,                             \
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));  \
-      raised = smem;                                                                                 \
-    }                                                                                                \
-    gram_cross_partial_kernel<PP><<<(unsigned)nb, kGramThreads, smem, st>>>(P, U, I, R, rpb, part); \
-    break;                                                                                           \
-  }
-    switch (ppt <= 1 ? 1 : ppt <= 2 ? 2 : ppt <= 4 ? 4 : ppt <= 16 ? 16 : 64) {
-      GC_CASE(1)
-      GC_CASE(2)
-      GC_CASE(4)
-      GC_CASE(16)
-      GC_CASE(64)
-    }
-#undef GC_CASE
+#define GC(TT) gram_kernel<TT, true><<<nb, GramLaunch<TT>::kThreads, 0, st>>>(P, U, I, R, rpb, part)
+    GRAM_DISPATCH(R, GC)
+#undef GC
     ALTO_LAUNCHED();
   }
-  reduce_split_kernel<<<reduce_grid(n), kReduceThreads, 0, st>>>(part, (int)nb, RR, n, G, C, stats3);
+  gram_reduce_kernel<true><<<gram_reduce_blocks(R), kReduceThreads, 0, st>>>(part, (int)nb, R, G, C, stats3);
+  ALTO_LAUNCHED();
+  return ALTO_OK;
+}
+
+// G = A^T A with nb partial results of rpb rows in `part`.
+static alto_status gram_into(const float* A, uint64_t I, int R, uint32_t nb, uint64_t rpb, double* part, double* out,
+                             cudaStream_t st) {
+#define GP(TT) gram_kernel<TT, false><<<nb, GramLaunch<TT>::kThreads, 0, st>>>(nullptr, A, I, R, rpb, part)
+  GRAM_DISPATCH(R, GP)
+#undef GP
+  ALTO_LAUNCHED();
+  gram_reduce_kernel<false><<<reduce_grid(gram_partial_len(R, false)), kReduceThreads, 0, st>>>(part, (int)nb, R, out,
+                                                                                              nullptr, nullptr);
   ALTO_LAUNCHED();
   return ALTO_OK;
 }
 
 alto_status gram(const float* A, uint64_t I, int R, double* out, DevBuf& scratch, cudaStream_t st) {
-  return gram_launch<float, float>(A, A, I, R, out, scratch, st);
-}
-
-alto_status cross_gram(const float* A, const float* B, uint64_t I, int R, double* out,
-                       DevBuf& scratch, cudaStream_t st) {
-  return gram_launch<float, float>(A, B, I, R, out, scratch, st);
+  if (I == 0) {
+    ALTO_TRY_CUDA(cudaMemsetAsync(out, 0, (size_t)R * R * sizeof(double), st));
+    return ALTO_OK;
+  }
+  uint32_t nb = 1;
+  uint64_t rpb = 1;
+  gram_split(I, &nb, &rpb);
+  ALTO_TRY(scratch.ensure(gram_partial_doubles(I, R, false) * sizeof(double)));
+  return gram_into(A, I, R, nb, rpb, scratch.as<double>(), out, st);
 }
 
 // ------------------------------------------------------- R x R solve setup
 
-// One CTA: V = prod_{m in mask} G_m (elementwise), then per `kind`:
+// One CTA (ranks above 64): V = prod_{m in mask} G_m (elementwise), then per `kind`:
 //   SOLVE_RIDGE: V += ridge * I;  ADMM: rho = tr(V)/R, V += rho * I.
 // Cholesky of V (upper triangle read, as dpotrf 'L' on the column-major
 // view); on success W = V^{-1}.  On failure: kind SOLVE_RIDGE_DIAG_FALLBACK
@@ -574,91 +576,211 @@ __global__ void solve_setup_kernel(const double* __restrict__ grams, int nmodes,
   }
 }
 
-// The same set-up with one thread per element of the R x R matrix (R <= 32,
-// blockDim = R * R): a right-looking Cholesky (column j scaled by its
-// diagonal, then the trailing lower triangle updated by the rank-one term),
-// the inverse of L by a right-looking forward substitution of all columns
-// at once, and W = L^-T L^-1.  Every element sees the operations of the
-// column-by-column form in the same order (its subtractions in k order,
-// then its division), as fused multiply-adds; R barriers per phase instead
-// of R^2 dependent steps in one warp.
+// The same set-up for R <= RMAX = 8, 16, 32 or 64, bound by the chain of R
+// dependent pivots.  One warp factors a 32 x 32 block (RMAX x RMAX below 32)
+// with lane i holding row i of the matrix and column i of L^-1 in registers: a
+// column of L goes through shared memory once and updates both, and the next
+// pivot's reciprocal square root is started before the rest of the update, so a
+// step costs one rsqrt and one shared-memory round trip, with no block barrier.
+// At RMAX 64 the two 32 x 32 diagonal blocks are factored so, and the rest of
+// L^-1 and W = L^-T L^-1 are float64 tensor-core products of the block.  One
+// thread per element with three to five barriers per column took 10.4 us at
+// rank 16, 40 us at rank 32 and (one column at a time) 192 us at rank 64.
+// Matrices smaller than RMAX are extended by the identity.
+
+// d += A B of one 8 x 8 tile over K (a multiple of 4): fa(i, k), fb(k, j) the
+// operands, i and j in [0, 8); lane l gets (l / 4, 2 (l % 4)) and its right
+// neighbour.
+template <typename FA, typename FB>
+__device__ __forceinline__ void dmma_tile(int K, int lane, FA fa, FB fb, double (&d)[2]) {
+  for (int k = 0; k < K; k += 4) dmma_8x8x4(d, fa(lane >> 2, k + (lane & 3)), fb(k + (lane & 3), lane >> 2));
+}
+
+// One warp: the Cholesky factor L of the N x N block at A (leading dimension
+// LD, shift added to the first `live` diagonal entries) and X = L^-1 (zero
+// above the diagonal), N <= 32.  Returns the 1-based index of the first pivot
+// that is not positive (0: none); col: 2 x 32 doubles of shared memory.
+template <int N>
+__device__ __forceinline__ int warp_chol_inverse(const double* A, int LD, double shift, int live, double* X, int LDX,
+                                                 double* col, int lane) {
+  double a[N], x[N];
+  const int row = lane < N ? lane : N - 1;
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    a[k] = A[row * LD + k] + (k == row && k < live ? shift : 0.0);
+    x[k] = k == row ? 1.0 : 0.0;
+  }
+  int info = 0;
+  double d = __shfl_sync(0xffffffffu, a[0], 0);
+  if (!(d > 0.0)) {
+    info = 1;
+    d = 1.0;
+  }
+  double rs = rsqrt(d);
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const double l = a[j] * rs;  // L[lane][j]
+    double* c = col + (j & 1) * 32;
+    c[lane] = l;
+    __syncwarp();
+    x[j] *= rs;
+    double rs_next = 0.0;
+    if (j + 1 < N) {
+      const double l1 = c[j + 1];
+      a[j + 1] = __fma_rn(-l, l1, a[j + 1]);
+      x[j + 1] = __fma_rn(-l1, x[j], x[j + 1]);
+      d = __shfl_sync(0xffffffffu, a[j + 1], j + 1);
+      if (!(d > 0.0)) {
+        if (!info) info = j + 2;
+        d = 1.0;
+      }
+      rs_next = rsqrt(d);
+    }
+#pragma unroll
+    for (int k = j + 2; k < N; ++k) {
+      const double lk = c[k];
+      a[k] = __fma_rn(-l, lk, a[k]);
+      x[k] = __fma_rn(-lk, x[j], x[k]);
+    }
+    rs = rs_next;
+  }
+  if (lane < N)
+#pragma unroll
+    for (int k = 0; k < N; ++k) X[k * LDX + lane] = k >= lane ? x[k] : 0.0;
+  return info;
+}
+
+template <int RMAX>
+struct SetupCfg {
+  static constexpr int LD = RMAX + (RMAX >= 32 ? 4 : 0);  // (tensor-core operand reads in fewer conflicts)
+  static constexpr int kThreads = RMAX <= 16 ? 128 : 256;
+  static constexpr size_t smem_bytes() { return 2 * (size_t)RMAX * LD * sizeof(double); }
+};
+
 template <int RMAX>
 __device__ __forceinline__ void solve_setup_block_body(const double* __restrict__ grams, int nmodes, unsigned mask,
                                                        int R, int kind, double ridge, double* __restrict__ W,
                                                        int* __restrict__ status, double* __restrict__ rho_out) {
-  __shared__ double A[RMAX * RMAX];
-  __shared__ double X[RMAX * RMAX];
+  constexpr int LD = SetupCfg<RMAX>::LD;
+  constexpr int N = RMAX < 32 ? RMAX : 32;
+  extern __shared__ __align__(16) double setup_smem[];
+  double* A = setup_smem;
+  double* X = A + RMAX * LD;
+  __shared__ double s_col[64];
   __shared__ double s_rho;
-  __shared__ int s_info;
+  __shared__ int s_info[2];
   const int RR = R * R;
-  const int tid = threadIdx.x;
-  const bool mine = tid < RR;
-  const int a = mine ? tid / R : 0, b = mine ? tid % R : 0;  // row, column
-  if (mine) {
-    double v = 1.0;
-    for (int m = 0; m < nmodes; ++m)
-      if (mask & (1u << m)) v *= grams[(size_t)m * RR + tid];
-    A[tid] = v;
-    X[tid] = a == b ? 1.0 : 0.0;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
+  for (int p = tid; p < RMAX * RMAX; p += blockDim.x) {
+    const int a = p / RMAX, b = p % RMAX;
+    double v = a == b ? 1.0 : 0.0;
+    if (a < R && b < R) {
+      v = 1.0;
+      for (int m = 0; m < nmodes; ++m)
+        if (mask & (1u << m)) v *= grams[(size_t)m * RR + a * R + b];
+      if (kind == kSolveRidgeDiagFallback && a == b) W[a * R + a] = v;  // the unridged diagonal, for the fallback
+    }
+    A[a * LD + b] = v;
   }
   __syncthreads();
-  if (tid == 0) {
+  if (warp == 0) {
     double add = ridge;
-    if (kind == kSolveAdmm) {
+    if (kind == kSolveAdmm) {  // rho = tr(V) / R
       double tr = 0.0;
-      for (int r = 0; r < R; ++r) tr += A[r * R + r];
+      for (int r = lane; r < R; r += 32) tr += A[r * LD + r];
+      for (int o = 16; o; o >>= 1) tr += __shfl_xor_sync(0xffffffffu, tr, o);
       add = tr / (double)R;
     }
-    s_rho = add;
-    s_info = 0;
+    const int info = warp_chol_inverse<N>(A, LD, add, min(R, N), X, LD, s_col, lane);
+    if (lane == 0) {
+      s_rho = add;
+      s_info[0] = info;
+      s_info[1] = 0;
+    }
   }
   __syncthreads();
-  if (kind == kSolveRidgeDiagFallback && mine && a == b) W[tid] = A[tid];
-  if (mine && a == b) A[tid] += s_rho;
-  __syncthreads();
-  for (int j = 0; j < R; ++j) {
-    if (tid == 0) {
-      double d = A[j * R + j];
-      if (!(d > 0.0)) {
-        if (!s_info) s_info = j + 1;
-        d = 1.0;
-      }
-      A[j * R + j] = sqrt(d);
+  if constexpr (RMAX == 64) {
+    // L21 = A21 X11^T over A21 (each warp its tiles; A12, the mirror, is free
+    // and holds the product until every tile is done), A22 -= L21 L21^T
+    constexpr int H = 32;
+    double* A21 = A + H * LD;
+    double* A12 = A + H;
+    double* A22 = A + H * LD + H;
+    double* X21 = X + H * LD;
+    double* X22 = X + H * LD + H;
+    const int i0 = lane >> 2, j0 = 2 * (lane & 3);
+    for (int q = warp; q < 16; q += nw) {
+      const int ti = (q >> 2) * 8, tj = (q & 3) * 8;
+      double d[2] = {0.0, 0.0};
+      dmma_tile(H, lane, [&](int i, int k) { return A21[(ti + i) * LD + k]; },
+                [&](int k, int j) { return X[(tj + j) * LD + k]; }, d);
+      A12[(ti + i0) * LD + tj + j0] = d[0];
+      A12[(ti + i0) * LD + tj + j0 + 1] = d[1];
     }
     __syncthreads();
-    if (mine && b == j && a > j) A[tid] = A[tid] / A[j * R + j];
+    const double* L21 = A12;
+    for (int q = warp; q < 16; q += nw) {
+      const int ti = (q >> 2) * 8, tj = (q & 3) * 8;
+      double d[2] = {0.0, 0.0};
+      dmma_tile(H, lane, [&](int i, int k) { return L21[(ti + i) * LD + k]; },
+                [&](int k, int j) { return L21[(tj + j) * LD + k]; }, d);
+      A22[(ti + i0) * LD + tj + j0] -= d[0];
+      A22[(ti + i0) * LD + tj + j0 + 1] -= d[1];
+      // T = L21 X11 over A21
+      double t[2] = {0.0, 0.0};
+      dmma_tile(H, lane, [&](int i, int k) { return L21[(ti + i) * LD + k]; },
+                [&](int k, int j) { return X[k * LD + tj + j]; }, t);
+      A21[(ti + i0) * LD + tj + j0] = t[0];
+      A21[(ti + i0) * LD + tj + j0 + 1] = t[1];
+      X[(ti + i0) * LD + H + tj + j0] = 0.0;  // above the diagonal
+      X[(ti + i0) * LD + H + tj + j0 + 1] = 0.0;
+    }
     __syncthreads();
-    if (mine && b > j && a >= b) A[tid] = __fma_rn(-A[a * R + j], A[b * R + j], A[tid]);
+    if (warp == 0) {
+      const int info = warp_chol_inverse<H>(A22, LD, s_rho, max(R - H, 0), X22, LD, s_col, lane);
+      if (lane == 0 && info) s_info[1] = H + info;
+    }
+    __syncthreads();
+    for (int q = warp; q < 16; q += nw) {  // X21 = -X22 T
+      const int ti = (q >> 2) * 8, tj = (q & 3) * 8;
+      double d[2] = {0.0, 0.0};
+      dmma_tile(H, lane, [&](int i, int k) { return X22[(ti + i) * LD + k]; },
+                [&](int k, int j) { return A21[k * LD + tj + j]; }, d);
+      X21[(ti + i0) * LD + tj + j0] = -d[0];
+      X21[(ti + i0) * LD + tj + j0 + 1] = -d[1];
+    }
     __syncthreads();
   }
-  const int info = s_info;
+  const int info = s_info[0] ? s_info[0] : s_info[1];
   if (info) {
-    if (mine) {
+    for (int p = tid; p < RR; p += blockDim.x) {
+      const int a = p / R, b = p % R;
       if (kind == kSolveRidgeDiagFallback) {
-        if (a != b) W[tid] = 0.0;
+        const double dv = a == b ? W[p] : 0.0;
+        W[p] = dv != 0.0 ? 1.0 / dv : 0.0;
       } else {
-        W[tid] = (kind == kSolveRidgeKeep && a == b) ? 1.0 : 0.0;
+        W[p] = (kind == kSolveRidgeKeep && a == b) ? 1.0 : 0.0;
       }
-    }
-    __syncthreads();
-    if (kind == kSolveRidgeDiagFallback && mine && a == b) {
-      const double d = W[tid];
-      W[tid] = d != 0.0 ? 1.0 / d : 0.0;
     }
   } else {
-    // X = L^-1 (lower): row k divided by L_kk once every earlier row has
-    // been subtracted from it, then subtracted from the rows below
-    for (int k = 0; k < R; ++k) {
-      if (mine && a == k && b <= k) X[tid] = X[tid] / A[k * R + k];
-      __syncthreads();
-      if (mine && a > k && b <= k) X[tid] = __fma_rn(-A[a * R + k], X[k * R + b], X[tid]);
-      __syncthreads();
-    }
-    if (mine) {
-      const int k0 = a > b ? a : b;
-      double sv = 0.0;
-      for (int k = k0; k < R; ++k) sv = __fma_rn(X[k * R + a], X[k * R + b], sv);
-      W[tid] = sv;
+    // W = X^T X (X is zero above its diagonal): 8 x 8 tiles on and above the
+    // diagonal, mirrored
+    constexpr int T = RMAX / 8;
+    for (int q = warp; q < T * T; q += nw) {
+      const int ti = (q / T) * 8, tj = (q % T) * 8;
+      if (tj < ti) continue;
+      double d[2] = {0.0, 0.0};
+      dmma_tile(RMAX - tj, lane, [&](int i, int k) { return X[(tj + k) * LD + ti + i]; },
+                [&](int k, int j) { return X[(tj + k) * LD + tj + j]; }, d);
+      const int a = ti + (lane >> 2);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int b = tj + 2 * (lane & 3) + e;
+        if (a < R && b < R) {
+          W[a * R + b] = d[e];
+          if (ti != tj) W[b * R + a] = d[e];
+        }
+      }
     }
   }
   if (tid == 0) {
@@ -669,16 +791,16 @@ __device__ __forceinline__ void solve_setup_block_body(const double* __restrict_
 }
 
 template <int RMAX>
-__global__ void __launch_bounds__(RMAX * RMAX)
+__global__ void __launch_bounds__(SetupCfg<RMAX>::kThreads)
     solve_setup_block_kernel(const double* __restrict__ grams, int nmodes, unsigned mask, int R, int kind,
                              double ridge, double* __restrict__ W, int* __restrict__ status,
                              double* __restrict__ rho_out) {
   solve_setup_block_body<RMAX>(grams, nmodes, mask, R, kind, ridge, W, status, rho_out);
 }
 
-// One CTA of R * R threads per item in turn (R <= 32).
+// One CTA per item in turn (R <= 32).
 template <int RMAX>
-__global__ void __launch_bounds__(RMAX * RMAX) setup_group_kernel(Strided<SetupItem> items, int R) {
+__global__ void __launch_bounds__(SetupCfg<RMAX>::kThreads) setup_group_kernel(Strided<SetupItem> items, int R) {
   const int K = *items.count;
   for (int s = blockIdx.x; s < K; s += gridDim.x) {
     const SetupItem& it = items[s];
@@ -690,11 +812,11 @@ __global__ void __launch_bounds__(RMAX * RMAX) setup_group_kernel(Strided<SetupI
 alto_status setup_group_launch(Strided<SetupItem> items, int max_items, int R, cudaStream_t st) {
   const unsigned grid = (unsigned)std::max(1, std::min(max_items, 1024));
   if (R <= 8)
-    setup_group_kernel<8><<<grid, R * R, 0, st>>>(items, R);
+    setup_group_kernel<8><<<grid, SetupCfg<8>::kThreads, SetupCfg<8>::smem_bytes(), st>>>(items, R);
   else if (R <= 16)
-    setup_group_kernel<16><<<grid, R * R, 0, st>>>(items, R);
+    setup_group_kernel<16><<<grid, SetupCfg<16>::kThreads, SetupCfg<16>::smem_bytes(), st>>>(items, R);
   else if (R <= 32)
-    setup_group_kernel<32><<<grid, R * R, 0, st>>>(items, R);
+    setup_group_kernel<32><<<grid, SetupCfg<32>::kThreads, SetupCfg<32>::smem_bytes(), st>>>(items, R);
   else {
     set_error("grouped solve set-up takes rank <= 32 (got %d)", R);
     return ALTO_ERR_UNSUPPORTED;
@@ -705,16 +827,28 @@ alto_status setup_group_launch(Strided<SetupItem> items, int max_items, int R, c
 
 alto_status solve_setup(const double* grams, int nmodes, unsigned mask, int R, int kind,
                         double ridge, double* W, int* status, double* rho, cudaStream_t st) {
-  if (R <= 32) {
-    if (R <= 8)
-      solve_setup_block_kernel<8><<<1, R * R, 0, st>>>(grams, nmodes, mask, R, kind, ridge, W, status, rho);
-    else if (R <= 16)
-      solve_setup_block_kernel<16><<<1, R * R, 0, st>>>(grams, nmodes, mask, R, kind, ridge, W, status, rho);
-    else
-      solve_setup_block_kernel<32><<<1, R * R, 0, st>>>(grams, nmodes, mask, R, kind, ridge, W, status, rho);
-    ALTO_LAUNCHED();
-    return ALTO_OK;
+#define SETUP_CASE(RM)                                                                                        \
+  if (R <= RM) {                                                                                              \
+    solve_setup_block_kernel<RM><<<1, SetupCfg<RM>::kThreads, SetupCfg<RM>::smem_bytes(), st>>>(              \
+        grams, nmodes, mask, R, kind, ridge, W, status, rho);                                                 \
+    ALTO_LAUNCHED();                                                                                          \
+    return ALTO_OK;                                                                                           \
   }
+  SETUP_CASE(8)
+  SETUP_CASE(16)
+  SETUP_CASE(32)
+  if (R <= 64) {  // (the shared-memory limit is raised once per device, outside any capture)
+    static std::atomic<bool> raised64[64];
+    int dev = 0;
+    ALTO_TRY_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || !raised64[dev].load()) {
+      ALTO_TRY_CUDA(cudaFuncSetAttribute(solve_setup_block_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)SetupCfg<64>::smem_bytes()));
+      if (dev >= 0 && dev < 64) raised64[dev] = true;
+    }
+  }
+  SETUP_CASE(64)
+#undef SETUP_CASE
   const size_t smem = (size_t)R * R * sizeof(double);
   static size_t raised = 0;
   if (smem > 48 * 1024 && smem > raised) {
@@ -1067,7 +1201,7 @@ extern "C" alto_status alto_gram(const float* U, uint64_t rows, int rank, double
 namespace {
 
 constexpr int kNoAllocBlocks = 64;    // partial sums, one R x R block each
-constexpr int kNoAllocMaxRank = 64;   // 64 blocks x 64 x 64 doubles = 2 MiB
+constexpr int kNoAllocMaxRank = 64;   // 64 blocks x 64 x 64 doubles = 2 MiB (a partial result is 36 of its 64 tiles)
 static __device__ __align__(256) double g_gram_noalloc_scratch[kNoAllocBlocks * kNoAllocMaxRank *
                                                                kNoAllocMaxRank];
 
@@ -1113,33 +1247,13 @@ extern "C" alto_status alto_gram_noalloc(const float* U, uint64_t rows, int rank
   double* part = nullptr;
   ALTO_TRY(noalloc_scratch(&part));
   cudaStream_t st = (cudaStream_t)stream;
-  const int RR = rank * rank;
   if (rows == 0) {
-    ALTO_TRY_CUDA(cudaMemsetAsync(G, 0, RR * sizeof(double), st));
+    ALTO_TRY_CUDA(cudaMemsetAsync(G, 0, (size_t)rank * rank * sizeof(double), st));
     return ALTO_OK;
   }
-  uint64_t nb = std::min<uint64_t>((rows + 255) / 256, (uint64_t)kNoAllocBlocks);
+  uint64_t nb = std::min<uint64_t>((rows + 63) / 64, (uint64_t)kNoAllocBlocks);
   const uint64_t rpb = (rows + nb - 1) / nb;
   nb = (rows + rpb - 1) / rpb;
-  // every block writes all RR entries of its partial, so no clearing is needed
-  const size_t smem = 2 * alto::kGramRows * rank * sizeof(double);  // <= 32 KiB at rank 64
-  const int ppt = (RR + alto::kGramThreads - 1) / alto::kGramThreads;
-  switch (ppt <= 1 ? 1 : ppt <= 2 ? 2 : ppt <= 4 ? 4 : 16) {
-    case 1:
-      alto::gram_partial_kernel<1, float, float><<<(unsigned)nb, alto::kGramThreads, smem, st>>>(U, U, rows, rank, rpb, part);
-      break;
-    case 2:
-      alto::gram_partial_kernel<2, float, float><<<(unsigned)nb, alto::kGramThreads, smem, st>>>(U, U, rows, rank, rpb, part);
-      break;
-    case 4:
-      alto::gram_partial_kernel<4, float, float><<<(unsigned)nb, alto::kGramThreads, smem, st>>>(U, U, rows, rank, rpb, part);
-      break;
-    default:
-      alto::gram_partial_kernel<16, float, float><<<(unsigned)nb, alto::kGramThreads, smem, st>>>(U, U, rows, rank, rpb, part);
-      break;
-  }
-  ALTO_LAUNCHED();
-  alto::reduce_partials_kernel<<<alto::reduce_grid(RR), alto::kReduceThreads, 0, st>>>(part, (int)nb, RR, G);
-  ALTO_LAUNCHED();
-  return ALTO_OK;
+  // every block writes its whole partial result, so no clearing is needed
+  return alto::gram_into(U, rows, rank, (uint32_t)nb, rpb, part, G, st);
 }

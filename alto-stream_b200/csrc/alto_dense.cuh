@@ -13,9 +13,6 @@ enum { kSolveRidge = 0, kSolveRidgeDiagFallback = 1, kSolveAdmm = 2, kSolveRidge
 
 // G = A^T A (R x R float64) of a float32 I x R matrix.
 alto_status gram(const float* A, uint64_t I, int R, double* out, DevBuf& scratch, cudaStream_t st);
-// G = A^T B.
-alto_status cross_gram(const float* A, const float* B, uint64_t I, int R, double* out,
-                       DevBuf& scratch, cudaStream_t st);
 // One pass over P and U: G = U^T U, C = P^T U and stats3 = {sum p u,
 // sum (p - u)^2, sum u^2} (stats3 may be NULL).
 alto_status gram_cross_stats(const float* P, const float* U, uint64_t I, int R, double* G, double* C,

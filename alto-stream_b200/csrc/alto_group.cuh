@@ -117,12 +117,13 @@ struct GramItem {
 // Blocks and rows per block gram_cross_stats uses for I rows (so a grouped
 // pass splits each session exactly as its own call does).
 void gram_split(uint64_t I, uint32_t* nb, uint64_t* rpb);
+// Doubles of partial sums a pass over I rows needs (G alone, or with C and the statistics).
+uint64_t gram_partial_doubles(uint64_t I, int R, bool cross);
 
 // Grouped solve set-up (one CTA per item, R <= 64).
 alto_status setup_group_launch(Strided<SetupItem> items, int max_items, int R, cudaStream_t st);
 // Grouped gram_cross_stats: block_off (device, [count + 1]) holds the prefix
 // sums of the items' nb; red_off likewise for their reduction blocks.
-alto_status gram_group_ready(int R);  // before capturing gram_group_launch at rank R
 alto_status gram_group_launch(Strided<GramItem> items, const uint32_t* block_off, const uint32_t* red_off,
                               int max_items, int R, cudaStream_t st);
 // Reduction blocks of one GramItem's pass at rank R.

@@ -1909,10 +1909,7 @@ alto_status group_prepare_session(alto_stream_session* s) {
     ALTO_TRY(det_prepare(s->at, m, fac, R, s->buf32.as<float>(), &s->det[m], st));
     if (m == s->t) continue;
     admm_part = std::max<uint64_t>(admm_part, (uint64_t)admm_blocks(R, s->dims[m]) * kAdmmSums);
-    uint32_t nb = 1;
-    uint64_t rpb = 1;
-    gram_split(s->dims[m], &nb, &rpb);
-    gram_part = std::max<uint64_t>(gram_part, (uint64_t)nb * (2 * R * R + 3));
+    gram_part = std::max<uint64_t>(gram_part, gram_partial_doubles(s->dims[m], R, true));
   }
   ALTO_TRY(s->admm_part.ensure(admm_part * sizeof(double)));
   ALTO_TRY(s->gscr.ensure(gram_part * sizeof(double)));
@@ -1962,7 +1959,7 @@ alto_status group_create(const alto_stream_session* like, int capacity, cudaStre
   ALTO_TRY_CUDA(cudaMemsetAsync(g->tab.p, 0, sizeof(SlotDesc) * capacity, st));
   ALTO_TRY_CUDA(cudaMemsetAsync(g->offs.p, 0, offs_n * 4, st));
   ALTO_TRY_CUDA(cudaMemsetAsync(g->ctl.p, 0, sizeof(GroupCtl), st));
-  if ((r = gram_group_ready(g->R)) || (r = build_group_graph(g))) {
+  if ((r = build_group_graph(g))) {
     group_destroy(g);
     return r;
   }
