@@ -19,21 +19,10 @@
 #include <mutex>
 
 #include "alto_dense.cuh"
+#include "alto_dmma.cuh"
 #include "alto_group.cuh"
 
 namespace alto {
-
-// d += a b on the float64 tensor cores, one 8 x 8 x 4 step of a warp: lane l
-// gives a = A[l / 4][l % 4] and b = B[l % 4][l / 4] and holds D[l / 4][2 (l % 4)]
-// and the element to its right.  Float64 products and sums, as __fma_rn; the
-// tensor cores' float64 rate is that of the FMA units (37 TFLOP/s measured for
-// both), but an instruction is 256 multiply-adds for two operand registers a
-// lane, where the FMA form reads shared memory for every few.
-__device__ __forceinline__ void dmma_8x8x4(double (&d)[2], double a, double b) {
-  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
-               : "+d"(d[0]), "+d"(d[1])
-               : "d"(a), "d"(b));
-}
 
 static int g_sms = 0;
 static int sms() {

@@ -39,6 +39,7 @@
 #include <vector>
 
 #include "alto_dense.cuh"
+#include "alto_dmma.cuh"
 #include "alto_group.cuh"
 
 namespace alto {
@@ -380,97 +381,53 @@ __global__ void __launch_bounds__(kAdmmThreads)
 
 // ------------------------------------------------ tiled row solves
 //
-// The row solves of a mode as small matrix products (ranks 8, 16, 32, 64):
-// a block takes a tile of T = 2048 / R rows; thread (rg, cg) holds rows
-// 2rg, 2rg + 1 and columns 4cg .. 4cg + 3 of every per-row quantity in
-// registers, and each row-times-matrix product stages the tile's input rows
-// in shared memory (row stride R + 1 doubles: conflict-free) and forms each
-// output with fused multiply-adds in k order -- the sequence of row_solve,
-// so every row's result is the one row_solve gives, without its shuffles.
+// The row solves of a mode at ranks 8, 16, 32 and 64: a warp takes eight rows
+// with every per-row quantity in registers, and each row-times-matrix product
+// is tensor-core products in float64 (alto_dmma.cuh).  Bound by the float64 rate
+// at rank 32 and above (solve of 120,000 rows at rank 32: two products, 0.25 G
+// multiply-adds, 13 us) and by HBM below.  The FMA form it replaces staged each
+// product's input rows in shared memory between barriers (76 us there; an
+// ADMM pass over 100,000 rows at rank 16 50 us).
 template <int R>
 struct TileMap {
-  static constexpr int CG = R / 4;                 // column groups
-  static constexpr int RGS = kAdmmThreads / CG;    // row groups
-  static constexpr int T = 2 * RGS;                // rows per tile
-  static constexpr int LD = R + 1;                 // padded row stride
-  static constexpr size_t smem_bytes() { return (2 * R * R + (size_t)T * LD) * sizeof(double); }
+  static constexpr int T = R / 8;                             // column tiles
+  static constexpr int kRows = 8 * (kAdmmThreads / 32);       // rows of a block's step
+  static constexpr int kMinBlocks = R <= 32 ? 2 : 1;
+  static constexpr size_t smem_bytes() { return 2 * (size_t)R * R * sizeof(double); }
 };
+
+// Blocks of a tiled pass: one wave at two blocks an SM.
+constexpr uint32_t kTileGrid = 148 * 2;
 
 template <int R>
 uint64_t tile_blocks(uint64_t I, uint64_t cap) {
-  const uint64_t b = std::min<uint64_t>((I + TileMap<R>::T - 1) / TileMap<R>::T, cap);
+  const uint64_t b = std::min<uint64_t>((I + TileMap<R>::kRows - 1) / TileMap<R>::kRows, cap);
   return std::max<uint64_t>(b, 1);
 }
 
-// x[i][j] = sum_k in[r0 + i][k] M[k][c0 + j], k ascending.
-template <int R>
-__device__ __forceinline__ void tile_product(const double* __restrict__ in, const double* __restrict__ M, int r0,
-                                             int c0, double (&x)[2][4]) {
-  constexpr int LD = TileMap<R>::LD;
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) x[i][j] = 0.0;
-#pragma unroll 8
-  for (int k = 0; k < R; ++k) {
-    const double a0 = in[r0 * LD + k], a1 = in[(r0 + 1) * LD + k];
-    const double2 w01 = *reinterpret_cast<const double2*>(M + k * R + c0);
-    const double2 w23 = *reinterpret_cast<const double2*>(M + k * R + c0 + 2);
-    x[0][0] = __fma_rn(a0, w01.x, x[0][0]);
-    x[0][1] = __fma_rn(a0, w01.y, x[0][1]);
-    x[0][2] = __fma_rn(a0, w23.x, x[0][2]);
-    x[0][3] = __fma_rn(a0, w23.y, x[0][3]);
-    x[1][0] = __fma_rn(a1, w01.x, x[1][0]);
-    x[1][1] = __fma_rn(a1, w01.y, x[1][1]);
-    x[1][2] = __fma_rn(a1, w23.x, x[1][2]);
-    x[1][3] = __fma_rn(a1, w23.y, x[1][3]);
-  }
-}
-
-// Stage v (this thread's 2 x 4 block) into the tile's rows, multiply by M,
-// and return the product in x (barriers on both sides).
-template <int R>
-__device__ __forceinline__ void tile_stage_product(double* in, const double* M, int r0, int c0,
-                                                   const double (&v)[2][4], double (&x)[2][4]) {
-  constexpr int LD = TileMap<R>::LD;
-#pragma unroll
-  for (int i = 0; i < 2; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) in[(r0 + i) * LD + c0 + j] = v[i][j];
-  __syncthreads();
-  tile_product<R>(in, M, r0, c0, x);
-  __syncthreads();
-}
-
-// Right-hand sides of a tile's rows: h = prev_U_j[i] A + mttkrp[i] (row_rhs).
-template <int R>
-__device__ __forceinline__ void tile_rhs(const float* __restrict__ P32, const float* __restrict__ B32, double* in,
-                                         const double* sA, uint64_t t0, uint64_t I, int r0, int c0,
-                                         double (&h)[2][4]) {
-  double p[2][4];
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const uint64_t row = t0 + r0 + i;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) p[i][j] = row < I ? (double)P32[row * R + c0 + j] : 0.0;
-  }
-  tile_stage_product<R>(in, sA, r0, c0, p, h);
-#pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const uint64_t row = t0 + r0 + i;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) h[i][j] = __dadd_rn(h[i][j], row < I ? (double)B32[row * R + c0 + j] : 0.0);
-  }
-}
-
+// W, then A, in fragment order.
 template <int R>
 __device__ __forceinline__ void tile_load_mats(double* smem, const double* __restrict__ A,
                                                const double* __restrict__ W) {
-  for (int p = threadIdx.x; p < R * R; p += blockDim.x) {
-    smem[p] = W[p];
-    smem[R * R + p] = A[p];
-  }
+  load_fragments(smem, W, R, R / 8);
+  load_fragments(smem + R * R, A, R, R / 8);
   __syncthreads();
+}
+
+// Right-hand sides of eight rows: h = prev_U_j[i] A + mttkrp[i] (row_rhs).
+template <int R>
+__device__ __forceinline__ void tile_rhs(const float* __restrict__ P32, const float* __restrict__ B32,
+                                         const double* sA, uint64_t row, bool in, int lane, double (&h)[R / 8][2]) {
+  constexpr int T = R / 8;
+  double p[T][2], b[T][2];
+  load_pairs<T>(P32, row, in, lane & 3, p);
+  load_pairs<T>(B32, row, in, lane & 3, b);
+  rows_product<T>(p, sA, lane, h);
+#pragma unroll
+  for (int c = 0; c < T; ++c) {
+    h[c][0] = __dadd_rn(h[c][0], b[c][0]);
+    h[c][1] = __dadd_rn(h[c][1], b[c][1]);
+  }
 }
 
 // Unconstrained solve of mode j, tiled: U_j[i] = (prev_U_j[i] A + mttkrp[i]) W.
@@ -481,29 +438,20 @@ __device__ __forceinline__ void solve_tile_body(const float* __restrict__ P32, c
                                                 uint32_t nblocks) {
   using TM = TileMap<R>;
   extern __shared__ double smem[];
-  double* sW = smem;
-  double* sA = smem + R * R;
-  double* in = smem + 2 * R * R;
   tile_load_mats<R>(smem, A, W);
-  const int cg = threadIdx.x % TM::CG, rg = threadIdx.x / TM::CG;
-  const int r0 = 2 * rg, c0 = 4 * cg;
-  for (uint64_t t0 = (uint64_t)block * TM::T; t0 < I; t0 += (uint64_t)nblocks * TM::T) {
-    double h[2][4], x[2][4];
-    tile_rhs<R>(P32, B32, in, sA, t0, I, r0, c0, h);
-    tile_stage_product<R>(in, sW, r0, c0, h, x);
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const uint64_t row = t0 + r0 + i;
-      if (row < I)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) U32[row * R + c0 + j] = (float)x[i][j];
-    }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (uint64_t r0 = (uint64_t)block * TM::kRows + 8 * warp; r0 < I; r0 += (uint64_t)nblocks * TM::kRows) {
+    const uint64_t row = r0 + (lane >> 2);
+    double h[TM::T][2], x[TM::T][2];
+    tile_rhs<R>(P32, B32, smem + R * R, row, row < I, lane, h);
+    rows_product<TM::T>(h, smem, lane, x);
+    if (row < I) store_pairs<TM::T>(U32, row, lane & 3, x);
   }
   __syncthreads();
 }
 
 template <int R>
-__global__ void __launch_bounds__(kAdmmThreads)
+__global__ void __launch_bounds__(kAdmmThreads, TileMap<R>::kMinBlocks)
     solve_tile_kernel(const float* __restrict__ P32, const float* __restrict__ B32, const double* __restrict__ A,
                       const double* __restrict__ W, uint64_t I, float* __restrict__ U32) {
   solve_tile_body<R>(P32, B32, A, W, I, U32, blockIdx.x, gridDim.x);
@@ -521,6 +469,7 @@ __device__ __forceinline__ void admm_tile_body(const float* __restrict__ P32, co
                                                double tol, cudaGraphConditionalHandle h, int in_graph,
                                                uint32_t block, uint32_t nblocks) {
   using TM = TileMap<R>;
+  constexpr int T = TM::T;
   constexpr int NW = kAdmmThreads / 32;
   if (PASS1 && state->stop) {  // a chunk after the stop (launched directly): nothing stands
     if (block == 0 && threadIdx.x == 0) state->chunk_sweeps = 0;
@@ -531,118 +480,104 @@ __device__ __forceinline__ void admm_tile_body(const float* __restrict__ P32, co
   const int nsweeps = PASS1 ? min(kAdmmChunk, kAdmmMaxIters - start) : state->chunk_sweeps;
   const bool first = start == 0;
   extern __shared__ double smem[];
-  double* sW = smem;
-  double* sA = smem + R * R;
-  double* in = smem + 2 * R * R;
-  __shared__ double wsum[kAdmmSums];
-  __shared__ double red[NW][4];
+  const double* sW = smem;
+  const double* sA = smem + R * R;
+  // each thread's sums of every sweep (registers are the row state's)
+  __shared__ double tsum[PASS1 ? kAdmmSums : 1][PASS1 ? kAdmmThreads : 1];
   if (PASS1)
-    for (int p = threadIdx.x; p < kAdmmSums; p += blockDim.x) wsum[p] = 0.0;
+#pragma unroll
+    for (int p = 0; p < kAdmmSums; ++p) tsum[p][threadIdx.x] = 0.0;
   tile_load_mats<R>(smem, A, W);
   const double rho = *rho_p;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int cg = threadIdx.x % TM::CG, rg = threadIdx.x / TM::CG;
-  const int r0 = 2 * rg, c0 = 4 * cg;
-  for (uint64_t t0 = (uint64_t)block * TM::T; t0 < I; t0 += (uint64_t)nblocks * TM::T) {
-    double H[2][4], X[2][4], Z[2][4], U[2][4], X0[2][4], a[2][4], z[2][4];
-    tile_rhs<R>(P32, B32, in, sA, t0, I, r0, c0, H);
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const uint64_t row = t0 + r0 + i;
-      const bool ok = row < I;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const uint64_t e = row * R + c0 + j;
-        X[i][j] = ok ? (first ? (double)U32[e] : primal[e]) : 0.0;
-        U[i][j] = ok ? dual[e] : 0.0;
-        Z[i][j] = ok && !first ? aux[e] : 0.0;
-        X0[i][j] = X[i][j];
-        // first update (src/admm.cpp:288-327): z = (rhs + rho (x + u)) W
-        a[i][j] = __fma_rn(rho, __dadd_rn(X[i][j], U[i][j]), H[i][j]);
-      }
-    }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, quad = lane & 3;
+  for (uint64_t r0 = (uint64_t)block * TM::kRows + 8 * warp; r0 < I; r0 += (uint64_t)nblocks * TM::kRows) {
+    const uint64_t row = r0 + (lane >> 2);
+    const bool in = row < I;
+    double H[T][2], X[T][2], Z[T][2], U[T][2], a[T][2];
+    tile_rhs<R>(P32, B32, sA, row, in, lane, H);
+    load_pairs<T>(dual, row, in, quad, U);
     if (first) {
-      tile_stage_product<R>(in, sW, r0, c0, a, z);
+      load_pairs<T>(U32, row, in, quad, X);
+    } else {
+      load_pairs<T>(primal, row, in, quad, X);
+      load_pairs<T>(aux, row, in, quad, Z);
+    }
+    if (first) {  // first update (src/admm.cpp:288-327): z = (rhs + rho (x + u)) W
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
+      for (int c = 0; c < T; ++c)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          Z[i][j] = z[i][j];
-          const double v = __dsub_rn(z[i][j], U[i][j]);
-          X[i][j] = v < 0.0 ? 0.0 : v;
+        for (int e = 0; e < 2; ++e) a[c][e] = __fma_rn(rho, __dadd_rn(X[c][e], U[c][e]), H[c][e]);
+      rows_product<T>(a, sW, lane, Z);
+#pragma unroll
+      for (int c = 0; c < T; ++c)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const double v = __dsub_rn(Z[c][e], U[c][e]);
+          X[c][e] = v < 0.0 ? 0.0 : v;
         }
     }
     for (int k = 0; k < nsweeps; ++k) {
       double p_res = 0, d_res = 0, p_norm = 0, d_norm = 0;
+      if (PASS1 && first && k == 0) {  // the change from the primal before the first update
+        double x0[T][2];
+        load_pairs<T>(U32, row, in, quad, x0);
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
+        for (int c = 0; c < T; ++c)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const double xv = X[i][j];
-          if (PASS1) {
-            if (first && k == 0) {
-              const double dd = __dsub_rn(xv, X0[i][j]);
-              d_res = __fma_rn(dd, dd, d_res);
-            }
-            p_norm = __fma_rn(xv, xv, p_norm);
+          for (int e = 0; e < 2; ++e) {
+            const double dd = __dsub_rn(X[c][e], x0[c][e]);
+            d_res = __fma_rn(dd, dd, d_res);
           }
-          const double y = __dsub_rn(xv, Z[i][j]);
-          const double di = __dadd_rn(U[i][j], y);
-          U[i][j] = di;
+      }
+#pragma unroll
+      for (int c = 0; c < T; ++c)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const double xv = X[c][e];
+          const double y = __dsub_rn(xv, Z[c][e]);
+          const double di = __dadd_rn(U[c][e], y);
+          U[c][e] = di;
           if (PASS1) {
+            p_norm = __fma_rn(xv, xv, p_norm);
             d_norm = __fma_rn(di, di, d_norm);
             p_res = __fma_rn(y, y, p_res);
           }
-          a[i][j] = __fma_rn(rho, __dadd_rn(xv, di), H[i][j]);
+          a[c][e] = __fma_rn(rho, __dadd_rn(xv, di), H[c][e]);
         }
-      tile_stage_product<R>(in, sW, r0, c0, a, z);
+      rows_product<T>(a, sW, lane, Z);
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
+      for (int c = 0; c < T; ++c)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          Z[i][j] = z[i][j];
-          const double v = __dsub_rn(z[i][j], U[i][j]);
-          X[i][j] = v < 0.0 ? 0.0 : v;
+        for (int e = 0; e < 2; ++e) {
+          const double v = __dsub_rn(Z[c][e], U[c][e]);
+          X[c][e] = v < 0.0 ? 0.0 : v;
         }
-      if (PASS1) {  // the tile's four sums: lanes, then warps in order, added per tile
-        double v4[4] = {p_res, d_res, p_norm, d_norm};
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          for (int o = 16; o; o >>= 1) v4[q] += __shfl_xor_sync(0xffffffffu, v4[q], o);
-          if (lane == 0) red[warp][q] = v4[q];
-        }
-        __syncthreads();
-        if (threadIdx.x < 4) {
-          double t = 0.0;
-          for (int w = 0; w < NW; ++w) t += red[w][threadIdx.x];
-          wsum[k * 4 + threadIdx.x] += t;
-        }
-        __syncthreads();
+      if (PASS1) {  // (rows past I are zero throughout: their rhs, primal and dual are)
+        tsum[k * 4 + 0][threadIdx.x] += p_res;
+        tsum[k * 4 + 1][threadIdx.x] += d_res;
+        tsum[k * 4 + 2][threadIdx.x] += p_norm;
+        tsum[k * 4 + 3][threadIdx.x] += d_norm;
       }
     }
-    if (!PASS1) {
-      const bool final_chunk = state->stop != 0;
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const uint64_t row = t0 + r0 + i;
-        if (row >= I) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const uint64_t e = row * R + c0 + j;
-          dual[e] = U[i][j];
-          if (final_chunk) {
-            U32[e] = (float)X[i][j];
-          } else {
-            primal[e] = X[i][j];
-            aux[e] = Z[i][j];
-          }
-        }
+    if (!PASS1 && in) {
+      store_pairs<T>(dual, row, quad, U);
+      if (state->stop != 0) {
+        store_pairs<T>(U32, row, quad, X);
+      } else {
+        store_pairs<T>(primal, row, quad, X);
+        store_pairs<T>(aux, row, quad, Z);
       }
     }
   }
   if (PASS1) {
     __syncthreads();
-    for (int p = threadIdx.x; p < kAdmmSums; p += blockDim.x) partials[(size_t)block * kAdmmSums + p] = wsum[p];
+    // the block's sums: per sum a warp, its lanes over the threads in order
+    for (int p = warp; p < kAdmmSums; p += NW) {
+      double t = 0.0;
+      for (int q = lane; q < kAdmmThreads; q += 32) t += tsum[p][q];
+      for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+      if (lane == 0) partials[(size_t)block * kAdmmSums + p] = t;
+    }
     // the last block to finish adds the blocks' sums (warp per sum, lanes
     // over blocks in order, fixed butterfly) and takes the chunk's sweep
     // count: the first sweep whose sums pass the test, else the whole chunk
@@ -683,7 +618,7 @@ __device__ __forceinline__ void admm_tile_body(const float* __restrict__ P32, co
 }
 
 template <int R, bool PASS1>
-__global__ void __launch_bounds__(kAdmmThreads)
+__global__ void __launch_bounds__(kAdmmThreads, TileMap<R>::kMinBlocks)
     admm_tile_kernel(const float* __restrict__ P32, const float* __restrict__ B32, const double* __restrict__ A,
                      float* __restrict__ U32, double* __restrict__ primal, double* __restrict__ aux,
                      double* __restrict__ dual, const double* __restrict__ W, const double* __restrict__ rho_p,
@@ -1042,7 +977,7 @@ __global__ void __launch_bounds__(256) group_mode_prep_kernel(SlotDesc* __restri
 }
 
 template <int R>
-__global__ void __launch_bounds__(kAdmmThreads)
+__global__ void __launch_bounds__(kAdmmThreads, TileMap<R>::kMinBlocks)
     group_solve_kernel(const SlotDesc* __restrict__ tab, const GroupCtl* __restrict__ ctl,
                        const uint32_t* __restrict__ off, int j) {
   const int K = ctl->count;
@@ -1075,7 +1010,7 @@ __global__ void group_admm_cond_kernel(SlotDesc* __restrict__ tab, GroupCtl* __r
 }
 
 template <int R, bool PASS1>
-__global__ void __launch_bounds__(kAdmmThreads)
+__global__ void __launch_bounds__(kAdmmThreads, TileMap<R>::kMinBlocks)
     group_admm_kernel(const SlotDesc* __restrict__ tab, const GroupCtl* __restrict__ ctl,
                       const uint32_t* __restrict__ off, int j, double tol) {
   const int K = ctl->count;
@@ -1296,7 +1231,7 @@ alto_status admm_run(alto_stream_session* s, uint64_t I, int mode, cudaStream_t 
 template <int R>
 alto_status admm_tile_run(alto_stream_session* s, uint64_t I, int mode, cudaStream_t st, const IterLaunch& L) {
   const size_t smem = TileMap<R>::smem_bytes();
-  const uint64_t blocks = tile_blocks<R>(I, 148ull * 4);
+  const uint64_t blocks = tile_blocks<R>(I, kTileGrid);
   ALTO_TRY(s->admm_part.ensure(blocks * kAdmmSums * sizeof(double)));
   static bool raised = false;  // raised once per kernel, outside any capture
   if (smem > 48 * 1024 && !raised) {
@@ -1387,7 +1322,7 @@ alto_status solve_tile_run(const float* P32, const float* B32, const double* A, 
     ALTO_TRY_CUDA(cudaFuncSetAttribute(solve_tile_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     raised = true;
   }
-  solve_tile_kernel<R><<<(unsigned)tile_blocks<R>(I, 148ull * 8), kAdmmThreads, smem, st>>>(P32, B32, A, W, I, U32);
+  solve_tile_kernel<R><<<(unsigned)tile_blocks<R>(I, kTileGrid), kAdmmThreads, smem, st>>>(P32, B32, A, W, I, U32);
   ALTO_LAUNCHED();
   return ALTO_OK;
 }
@@ -1753,8 +1688,8 @@ struct StreamGroup {
 
 namespace grp {
 
-constexpr uint32_t kSolveGrid = 148 * 8;
-constexpr uint32_t kAdmmGrid = 148 * 4;
+constexpr uint32_t kSolveGrid = kTileGrid;
+constexpr uint32_t kAdmmGrid = kTileGrid;
 
 // (as admm() and rows_solve() launch the tiled kernels, ranks 8, 16, 32)
 uint32_t admm_blocks(int R, uint64_t I) {
