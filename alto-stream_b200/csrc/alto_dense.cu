@@ -35,11 +35,6 @@ static int sms() {
   return g_sms;
 }
 
-template <typename T>
-__device__ __forceinline__ double ld(const T* p, size_t i) {
-  return (double)p[i];
-}
-
 // ------------------------------------------------------------ Grams
 //
 // G = U^T U and, in the same pass, C = P^T U with the change statistics, as
@@ -98,10 +93,19 @@ __device__ __forceinline__ void store_stats(double (&q)[3], double* __restrict__
   __syncthreads();
 }
 
+// A Gram pass that first divides column c of U by lambda[c] (CP-ALS's
+// normalisation): the scaled factor goes to Y, and in bfloat16 to shadow (may
+// be NULL); U is left as it is.
+struct GramScale {
+  const double* lambda;
+  float* Y;
+  __nv_bfloat16* shadow;
+};
+
 // Partial sums over rows [r0, r1), T <= 4 column tiles.
-template <int T, bool CROSS>
+template <int T, bool CROSS, bool SCALE>
 __device__ __forceinline__ void gram_narrow(const float* __restrict__ P, const float* __restrict__ U, uint64_t r0,
-                                            uint64_t r1, int R, double* __restrict__ out) {
+                                            uint64_t r1, int R, double* __restrict__ out, const GramScale& sc) {
   constexpr int NG = T * (T + 1) / 2, NT = gram_out_tiles(T, CROSS), NW = kGramThreads / 32;
   constexpr int S = T == 1 ? 8 : T == 2 ? 4 : 2;  // steps of four rows whose loads are issued together
   __shared__ double red[NT * 64];
@@ -111,6 +115,10 @@ __device__ __forceinline__ void gram_narrow(const float* __restrict__ P, const f
 #pragma unroll
   for (int t = 0; t < NT; ++t) acc[t][0] = acc[t][1] = 0.0;
   double q[3] = {0.0, 0.0, 0.0};
+  double inv[SCALE ? T : 1];
+  if constexpr (SCALE)
+#pragma unroll
+    for (int c = 0; c < T; ++c) inv[c] = c * 8 + kc < R ? 1.0 / sc.lambda[c * 8 + kc] : 0.0;
   float fu[S][T], fp[CROSS ? S : 1][T];
   auto fetch = [&](uint64_t k0) {
 #pragma unroll
@@ -142,6 +150,15 @@ __device__ __forceinline__ void gram_narrow(const float* __restrict__ P, const f
       double u[T], p[T];
 #pragma unroll
       for (int c = 0; c < T; ++c) {
+        if constexpr (SCALE) {
+          cu[s][c] = (float)((double)cu[s][c] * inv[c]);
+          const uint64_t row = k0 + (uint64_t)s * 4 * NW + kr;
+          const int col = c * 8 + kc;
+          if (row < r1 && col < R) {
+            sc.Y[row * R + col] = cu[s][c];
+            if (sc.shadow) sc.shadow[row * R + col] = __float2bfloat16(cu[s][c]);
+          }
+        }
         u[c] = (double)cu[s][c];
         if (CROSS) {
           p[c] = (double)cp[s][c];
@@ -177,9 +194,9 @@ __device__ __forceinline__ void gram_narrow(const float* __restrict__ P, const f
 }
 
 // The same for more than four column tiles (T at run time).
-template <bool CROSS>
+template <bool CROSS, bool SCALE>
 __device__ __forceinline__ void gram_wide(const float* __restrict__ P, const float* __restrict__ U, uint64_t r0,
-                                          uint64_t r1, int R, double* __restrict__ out) {
+                                          uint64_t r1, int R, double* __restrict__ out, const GramScale& sc) {
   const int T = gram_tiles(R), NG = T * (T + 1) / 2;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int kr = lane & 3, kc = lane >> 2;
@@ -192,6 +209,13 @@ __device__ __forceinline__ void gram_wide(const float* __restrict__ P, const flo
         g[b][0] = g[b][1] = 0.0;
         if (CROSS) c[b][0] = c[b][1] = 0.0;
       }
+      double inv[SCALE ? 9 : 1];
+      if constexpr (SCALE)
+#pragma unroll
+        for (int b = 0; b < 9; ++b) {
+          const int col = (b < 8 ? cb + b : a) * 8 + kc;
+          inv[b] = col < R ? 1.0 / sc.lambda[col] : 0.0;
+        }
       float fb[8], fa = 0.f, pa = 0.f;
       auto fetch = [&](uint64_t k0) {
         const uint64_t row = k0 + kr;
@@ -208,6 +232,17 @@ __device__ __forceinline__ void gram_wide(const float* __restrict__ P, const flo
       if (r0 < r1) fetch(r0);
       for (uint64_t k0 = r0; k0 < r1; k0 += 4) {
         double ub[8];
+        if constexpr (SCALE) {
+#pragma unroll
+          for (int b = 0; b < 8; ++b) fb[b] = (float)((double)fb[b] * inv[b]);
+          fa = (float)((double)fa * inv[8]);
+          const uint64_t row = k0 + kr;
+          const int col = a * 8 + kc;
+          if (cb == 0 && row < r1 && col < R) {
+            sc.Y[row * R + col] = fa;
+            if (sc.shadow) sc.shadow[row * R + col] = __float2bfloat16(fa);
+          }
+        }
 #pragma unroll
         for (int b = 0; b < 8; ++b) ub[b] = (double)fb[b];
         const double ua = (double)fa, pv = (double)pa;
@@ -234,16 +269,17 @@ __device__ __forceinline__ void gram_wide(const float* __restrict__ P, const flo
 }
 
 // TT: 1 to 4 column tiles, or 0 for more.
-template <int TT, bool CROSS>
+template <int TT, bool CROSS, bool SCALE = false>
 __device__ __forceinline__ void gram_block(const float* __restrict__ P, const float* __restrict__ U, uint64_t I, int R,
-                                           uint64_t rows_per_block, double* __restrict__ partials, uint32_t block) {
+                                           uint64_t rows_per_block, double* __restrict__ partials, uint32_t block,
+                                           const GramScale& sc = GramScale{}) {
   const uint64_t r0 = (uint64_t)block * rows_per_block;
   const uint64_t r1 = min(r0 + rows_per_block, I);
   double* out = partials + (size_t)block * gram_partial_len(R, CROSS);
   if constexpr (TT == 0)
-    gram_wide<CROSS>(P, U, r0, r1, R, out);
+    gram_wide<CROSS, SCALE>(P, U, r0, r1, R, out, sc);
   else
-    gram_narrow<TT, CROSS>(P, U, r0, r1, R, out);
+    gram_narrow<TT, CROSS, SCALE>(P, U, r0, r1, R, out, sc);
 }
 
 template <int TT>
@@ -257,6 +293,13 @@ __global__ void __launch_bounds__(GramLaunch<TT>::kThreads, GramLaunch<TT>::kMin
     gram_kernel(const float* __restrict__ P, const float* __restrict__ U, uint64_t I, int R, uint64_t rows_per_block,
                 double* __restrict__ partials) {
   gram_block<TT, CROSS>(P, U, I, R, rows_per_block, partials, blockIdx.x);
+}
+
+template <int TT>
+__global__ void __launch_bounds__(GramLaunch<TT>::kThreads, GramLaunch<TT>::kMinBlocks)
+    scale_gram_kernel(const float* __restrict__ U, uint64_t I, int R, uint64_t rows_per_block,
+                      double* __restrict__ partials, GramScale sc) {
+  gram_block<TT, false, true>(nullptr, U, I, R, rows_per_block, partials, blockIdx.x, sc);
 }
 
 // sum over blocks b of partials[b][p] for 32 consecutive p (one per lane), in a
@@ -435,6 +478,28 @@ static alto_status gram_into(const float* A, uint64_t I, int R, uint32_t nb, uin
 #define GP(TT) gram_kernel<TT, false><<<nb, GramLaunch<TT>::kThreads, 0, st>>>(nullptr, A, I, R, rpb, part)
   GRAM_DISPATCH(R, GP)
 #undef GP
+  ALTO_LAUNCHED();
+  gram_reduce_kernel<false><<<reduce_grid(gram_partial_len(R, false)), kReduceThreads, 0, st>>>(part, (int)nb, R, out,
+                                                                                              nullptr, nullptr);
+  ALTO_LAUNCHED();
+  return ALTO_OK;
+}
+
+alto_status scale_gram(const float* X, uint64_t I, int R, const double* lambda, float* Y, __nv_bfloat16* shadow,
+                       double* out, DevBuf& scratch, cudaStream_t st) {
+  if (I == 0) {
+    ALTO_TRY_CUDA(cudaMemsetAsync(out, 0, (size_t)R * R * sizeof(double), st));
+    return ALTO_OK;
+  }
+  uint32_t nb = 1;
+  uint64_t rpb = 1;
+  gram_split(I, &nb, &rpb);
+  ALTO_TRY(scratch.ensure(gram_partial_doubles(I, R, false) * sizeof(double)));
+  double* part = scratch.as<double>();
+  const GramScale sc{lambda, Y, shadow};
+#define SG_LAUNCH(TT) scale_gram_kernel<TT><<<nb, GramLaunch<TT>::kThreads, 0, st>>>(X, I, R, rpb, part, sc)
+  GRAM_DISPATCH(R, SG_LAUNCH)
+#undef SG_LAUNCH
   ALTO_LAUNCHED();
   gram_reduce_kernel<false><<<reduce_grid(gram_partial_len(R, false)), kReduceThreads, 0, st>>>(part, (int)nb, R, out,
                                                                                               nullptr, nullptr);
@@ -851,128 +916,180 @@ alto_status solve_setup(const double* grams, int nmodes, unsigned mask, int R, i
 }
 
 // ------------------------------------------------------------ row apply
+//
+// X = B W (float32 in and out, float64 products) and the column scales of
+// CP-ALS's normalisation, lambda[c] = sqrt(max(sum x^2, 1e-12)) (which 0) or
+// max(1, max x) (which 1) over the float32 results.  Rows in registers as in
+// alto_dmma.cuh (8 T columns; the columns past R are zero); each block leaves
+// its columns' partial statistics and the last block to finish combines them in
+// block order, so no launch of its own waits for them.  Bound by latency at
+// CP-ALS's sizes: a shuffle per term and a one-block pass over every block's
+// statistics took 50 + 17 us for up to 20,000 rows at rank 64, 10 + 3 us for
+// 1000 rows at rank 16.
+constexpr int kApplyThreads = 256;
 
-// X[i, :] = B[i, :] W (+ C[i, :] when C is given), float64 arithmetic.
-// Column statistics of the result go to per-block partials:
-// stats[b][0][r] = sum x^2, stats[b][1][r] = max x.
-template <typename TB, typename TC, typename TX>
-__global__ void __launch_bounds__(256)
-    apply_kernel(const TB* __restrict__ B, const TC* __restrict__ C,
-                 const double* __restrict__ W, uint64_t I, int R, TX* __restrict__ X,
-                 double* __restrict__ stats, uint64_t rows_per_block) {
-  extern __shared__ double sw[];  // W (R x R), then column stats (2 x R per warp)
-  const int RR = R * R;
-  for (int p = threadIdx.x; p < RR; p += blockDim.x) sw[p] = W[p];
-  const int nwarps = blockDim.x >> 5;
-  double* wsq = sw + RR;            // [nwarps][R]
-  double* wmx = wsq + nwarps * R;   // [nwarps][R]
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int r = lane; r < R; r += 32) {
-    wsq[warp * R + r] = 0.0;
-    wmx[warp * R + r] = -INFINITY;
-  }
-  __syncthreads();
-  const uint64_t r0 = (uint64_t)blockIdx.x * rows_per_block;
-  const uint64_t r1 = min(r0 + rows_per_block, I);
-  for (uint64_t i = r0 + warp; i < r1; i += nwarps) {
-    for (int c0 = 0; c0 < R; c0 += 32) {
-      const int c = c0 + lane;
-      double x = 0.0;
-      for (int k0 = 0; k0 < R; k0 += 32) {
-        const int kk = k0 + lane;
-        const double bk = kk < R ? ld(B, i * R + kk) : 0.0;
-        const int kmax = min(32, R - k0);
-        for (int k = 0; k < kmax; ++k) {
-          const double b = __shfl_sync(0xffffffffu, bk, k);
-          if (c < R) x += b * sw[(k0 + k) * R + c];
-        }
-      }
-      if (c < R) {
-        if (C) x += (double)C[i * R + c];
-        const TX xs = (TX)x;
-        X[i * R + c] = xs;
-        const double xv = (double)xs;
-        wsq[warp * R + c] += xv * xv;
-        wmx[warp * R + c] = fmax(wmx[warp * R + c], xv);
-      }
-    }
-  }
-  __syncthreads();
-  if (stats) {
-    for (int r = threadIdx.x; r < R; r += blockDim.x) {
-      double s = 0.0, m = -INFINITY;
-      for (int w = 0; w < nwarps; ++w) {
-        s += wsq[w * R + r];
-        m = fmax(m, wmx[w * R + r]);
-      }
-      stats[((size_t)blockIdx.x * 2 + 0) * R + r] = s;
-      stats[((size_t)blockIdx.x * 2 + 1) * R + r] = m;
+template <int T>
+__device__ __forceinline__ void apply_rows(const float* __restrict__ B, uint64_t row, bool in, int quad, int R,
+                                           float (&b)[T][2]) {
+#pragma unroll
+  for (int c = 0; c < T; ++c) {
+    const int col = 8 * c + 2 * quad;
+    if ((R & 1) == 0) {
+      float2 v = make_float2(0.f, 0.f);
+      if (in && col < R) v = *reinterpret_cast<const float2*>(B + row * R + col);
+      b[c][0] = v.x;
+      b[c][1] = v.y;
+    } else {
+      b[c][0] = in && col < R ? B[row * R + col] : 0.f;
+      b[c][1] = in && col + 1 < R ? B[row * R + col + 1] : 0.f;
     }
   }
 }
 
-template <typename TB, typename TC, typename TX>
-static alto_status apply_launch(const TB* B, const TC* C, const double* W, uint64_t I, int R,
-                                TX* X, DevBuf* stats, int* nblocks_out, cudaStream_t st) {
-  uint64_t nb = std::min<uint64_t>((I + 63) / 64, (uint64_t)sms() * 4);
-  if (nb < 1) nb = 1;
-  const uint64_t rpb = (I + nb - 1) / nb;
-  nb = I ? (I + rpb - 1) / rpb : 1;
-  double* sp = nullptr;
-  if (stats) {
-    ALTO_TRY(stats->ensure(nb * 2 * R * sizeof(double)));
-    sp = stats->as<double>();
+template <int T>
+__global__ void __launch_bounds__(kApplyThreads)
+    apply_kernel(const float* __restrict__ B, const double* __restrict__ W, uint64_t I, int R, float* __restrict__ X,
+                 int which, double* __restrict__ partials, unsigned* __restrict__ ticket,
+                 double* __restrict__ lambda) {
+  constexpr int NW = kApplyThreads / 32;
+  constexpr int NC = T < 4 ? T : 4;  // column tiles of a product at once
+  extern __shared__ double sfrag[];
+  __shared__ double sred[NW][8 * T];
+  __shared__ bool last;
+  load_fragments(sfrag, W, R, T);
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, quad = lane & 3;
+  double acc[T][2];
+#pragma unroll
+  for (int c = 0; c < T; ++c) acc[c][0] = acc[c][1] = which ? -INFINITY : 0.0;
+  for (uint64_t r0 = (uint64_t)blockIdx.x * 8 * NW + 8 * warp; r0 < I; r0 += (uint64_t)gridDim.x * 8 * NW) {
+    const uint64_t row = r0 + (lane >> 2);
+    const bool in = row < I;
+    float b[T][2];
+    apply_rows<T>(B, row, in, quad, R, b);
+#pragma unroll
+    for (int n0 = 0; n0 < T; n0 += NC) {
+      double x[NC][2];
+#pragma unroll
+      for (int n = 0; n < NC; ++n) x[n][0] = x[n][1] = 0.0;
+#pragma unroll
+      for (int c = 0; c < T; ++c)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const double a = (double)b[c][e];
+#pragma unroll
+          for (int n = 0; n < NC; ++n)
+            if (n0 + n < T) dmma_8x8x4(x[n], a, sfrag[((c * 2 + e) * T + n0 + n) * 32 + lane]);
+        }
+#pragma unroll
+      for (int n = 0; n < NC; ++n) {
+        if (n0 + n >= T) continue;
+        const int col = 8 * (n0 + n) + 2 * quad;
+        const float f[2] = {(float)x[n][0], (float)x[n][1]};
+        if (!in) continue;
+        if ((R & 1) == 0) {
+          if (col < R) *reinterpret_cast<float2*>(X + row * R + col) = make_float2(f[0], f[1]);
+        } else {
+          if (col < R) X[row * R + col] = f[0];
+          if (col + 1 < R) X[row * R + col + 1] = f[1];
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const double v = (double)f[e];
+          acc[n0 + n][e] = which ? fmax(acc[n0 + n][e], v) : __fma_rn(v, v, acc[n0 + n][e]);
+        }
+      }
+    }
   }
-  if (nblocks_out) *nblocks_out = (int)nb;
-  const size_t smem = ((size_t)R * R + 2 * 8 * R) * sizeof(double);
-  static size_t raised = 0;  // raised once per kernel, outside any capture
-  if (smem > 48 * 1024 && smem > raised) {
-    ALTO_TRY_CUDA(cudaFuncSetAttribute(apply_kernel<TB, TC, TX>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    raised = smem;
+  // columns: the eight rows of a warp, the warps, the blocks, each in order
+#pragma unroll
+  for (int c = 0; c < T; ++c)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      double v = acc[c][e];
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) {
+        const double y = __shfl_xor_sync(0xffffffffu, v, o);
+        v = which ? fmax(v, y) : v + y;
+      }
+      if (lane < 4) sred[warp][8 * c + 2 * lane + e] = v;
+    }
+  __syncthreads();
+  for (int r = threadIdx.x; r < 8 * T; r += kApplyThreads) {
+    double v = sred[0][r];
+    for (int w = 1; w < NW; ++w) v = which ? fmax(v, sred[w][r]) : v + sred[w][r];
+    partials[(size_t)blockIdx.x * 8 * T + r] = v;
   }
-  apply_kernel<TB, TC, TX><<<(unsigned)nb, 256, smem, st>>>(B, C, W, I, R, X, sp, rpb);
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  constexpr int kGroups = kApplyThreads / (8 * T) < NW ? kApplyThreads / (8 * T) : NW;  // threads per column
+  const int r = threadIdx.x % (8 * T), g = threadIdx.x / (8 * T);
+  if (g < kGroups) {
+    double v = which ? -INFINITY : 0.0;
+#pragma unroll 8
+    for (unsigned b = g; b < gridDim.x; b += kGroups) {
+      const double y = __ldcg(partials + (size_t)b * 8 * T + r);
+      v = which ? fmax(v, y) : v + y;
+    }
+    sred[g][r] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x < R) {
+    double v = sred[0][threadIdx.x];
+    for (int k = 1; k < kGroups; ++k) v = which ? fmax(v, sred[k][threadIdx.x]) : v + sred[k][threadIdx.x];
+    lambda[threadIdx.x] = which ? fmax(1.0, v) : sqrt(v > 1e-12 ? v : 1e-12);
+  }
+  if (threadIdx.x == 0) *ticket = 0;
+}
+
+// One block per SM at most: the last block reads every block's statistics.
+static unsigned apply_blocks(uint64_t I) {
+  return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((I + 63) / 64, (uint64_t)sms()));
+}
+
+template <int T>
+static alto_status apply_launch(const float* B, const double* W, uint64_t I, int R, float* X, int which,
+                                double* partials, unsigned* ticket, double* lambda, cudaStream_t st) {
+  const size_t smem = (size_t)64 * T * T * sizeof(double);
+  if (smem > 40 * 1024) {
+    static std::atomic<bool> raised[64];  // per device
+    int dev = 0;
+    ALTO_TRY_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || !raised[dev].load()) {
+      ALTO_TRY_CUDA(cudaFuncSetAttribute(apply_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      if (dev >= 0 && dev < 64) raised[dev] = true;
+    }
+  }
+  apply_kernel<T><<<apply_blocks(I), kApplyThreads, smem, st>>>(B, W, I, R, X, which, partials, ticket, lambda);
   ALTO_LAUNCHED();
   return ALTO_OK;
 }
 
-alto_status apply_f32(const float* B, const double* W, uint64_t I, int R, float* X,
-                      DevBuf* stats, int* nblocks, cudaStream_t st) {
-  return apply_launch<float, double, float>(B, nullptr, W, I, R, X, stats, nblocks, st);
-}
+size_t apply_scratch_bytes(uint64_t I, int R) { return 256 + (size_t)apply_blocks(I) * 8 * 16 * sizeof(double); }
 
-alto_status apply_f64_to_f32(const double* B, const double* W, uint64_t I, int R, float* X,
-                             cudaStream_t st) {
-  return apply_launch<double, double, float>(B, nullptr, W, I, R, X, nullptr, nullptr, st);
-}
-
-alto_status apply_f32_to_f64(const float* B, const float* C, const double* W, uint64_t I, int R,
-                             double* X, cudaStream_t st) {
-  return apply_launch<float, float, double>(B, C, W, I, R, X, nullptr, nullptr, st);
+alto_status apply_lambda(const float* B, const double* W, uint64_t I, int R, float* X, int which, void* scratch,
+                         double* lambda, cudaStream_t st) {
+  unsigned* ticket = static_cast<unsigned*>(scratch);
+  double* part = reinterpret_cast<double*>(static_cast<char*>(scratch) + 256);
+  const int T = gram_tiles(R);
+#define APPLY_CASE(TT) \
+  if (T <= TT) return apply_launch<TT>(B, W, I, R, X, which, part, ticket, lambda, st);
+  APPLY_CASE(1)
+  APPLY_CASE(2)
+  APPLY_CASE(3)
+  APPLY_CASE(4)
+  APPLY_CASE(8)
+  APPLY_CASE(16)
+#undef APPLY_CASE
+  set_error("rank %d is not supported", R);
+  return ALTO_ERR_UNSUPPORTED;
 }
 
 // ----------------------------------------------------------- normalisation
-
-// lambda from per-block column statistics (block order): which 0 ->
-// sqrt(max(sum x^2, 1e-12)); which 1 -> max(1, max x).
-__global__ void lambda_kernel(const double* __restrict__ stats, int nblocks, int R, int which,
-                              double* __restrict__ lambda) {
-  for (int r = threadIdx.x; r < R; r += blockDim.x) {
-    double s = 0.0, m = 1.0;
-    for (int b = 0; b < nblocks; ++b) {
-      s += stats[((size_t)b * 2 + 0) * R + r];
-      m = fmax(m, stats[((size_t)b * 2 + 1) * R + r]);
-    }
-    lambda[r] = which == 0 ? sqrt(s > 1e-12 ? s : 1e-12) : m;
-  }
-}
-
-alto_status column_lambda(const double* stats, int nblocks, int R, int which, double* lambda,
-                          cudaStream_t st) {
-  lambda_kernel<<<1, 128, 0, st>>>(stats, nblocks, R, which, lambda);
-  ALTO_LAUNCHED();
-  return ALTO_OK;
-}
 
 // X[i][r] /= lambda[r]; optional bfloat16 shadow copy.
 __global__ void scale_kernel(float* __restrict__ X, uint64_t n, int R,
@@ -1058,16 +1175,6 @@ alto_status dot_stats(const float* a, const float* b, uint64_t n, const double* 
   return ALTO_OK;
 }
 
-alto_status dot_stats_f64(const double* a, const float* b, uint64_t n, double* out3, DevBuf& scratch,
-                          cudaStream_t st) {
-  ALTO_TRY(scratch.ensure(kDotBlocks * 3 * sizeof(double)));
-  dot_partial_kernel<double, float><<<kDotBlocks, 256, 0, st>>>(a, b, n, nullptr, 1, scratch.as<double>());
-  ALTO_LAUNCHED();
-  reduce_partials_kernel<<<reduce_grid(3), kReduceThreads, 0, st>>>(scratch.as<double>(), kDotBlocks, 3, out3);
-  ALTO_LAUNCHED();
-  return ALTO_OK;
-}
-
 // Sum of squares of n float values (||X||^2 of the tensor values).
 __global__ void sumsq_partial_kernel(const float* __restrict__ v, uint64_t n, double* __restrict__ part) {
   double s = 0;
@@ -1099,7 +1206,7 @@ alto_status sum_squares(const float* v, uint64_t n, double* out, DevBuf& scratch
 __global__ void model_norm_kernel(const double* __restrict__ grams, int nmodes, int R,
                                   const double* __restrict__ lambda, int exact,
                                   double* __restrict__ out) {
-  __shared__ double part[256];
+  __shared__ double part[8];
   double s = 0.0;
   const int RR = R * R;
   for (int p = threadIdx.x; p < RR; p += blockDim.x) {
@@ -1110,11 +1217,12 @@ __global__ void model_norm_kernel(const double* __restrict__ grams, int nmodes, 
     for (int m = 0; m < nmodes; ++m) t *= grams[(size_t)m * RR + p];
     s += (a == b) ? t : 2.0 * t;
   }
-  part[threadIdx.x] = s;
+  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
   __syncthreads();
   if (threadIdx.x == 0) {
     double t = 0;
-    for (int k = 0; k < (int)blockDim.x; ++k) t += part[k];
+    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) t += part[k];
     out[0] = fabs(t);
   }
 }

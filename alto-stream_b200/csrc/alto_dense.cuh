@@ -20,24 +20,21 @@ alto_status gram_cross_stats(const float* P, const float* U, uint64_t I, int R, 
 // W = (prod_{m in mask} grams[m] + shift I)^{-1}; see the kernel comment.
 alto_status solve_setup(const double* grams, int nmodes, unsigned mask, int R, int kind,
                         double ridge, double* W, int* status, double* rho, cudaStream_t st);
-// X = B W (+ C); apply_f32 also writes per-block column statistics
-// (sum x^2, max x) when stats is given.
-alto_status apply_f32(const float* B, const double* W, uint64_t I, int R, float* X,
-                      DevBuf* stats, int* nblocks, cudaStream_t st);
-alto_status apply_f64_to_f32(const double* B, const double* W, uint64_t I, int R, float* X,
-                             cudaStream_t st);
-alto_status apply_f32_to_f64(const float* B, const float* C, const double* W, uint64_t I, int R,
-                             double* X, cudaStream_t st);
-alto_status column_lambda(const double* stats, int nblocks, int R, int which, double* lambda,
-                          cudaStream_t st);
+// X = B W and the scales of CP-ALS's normalisation of X's columns: lambda[c] =
+// sqrt(max(sum x^2, 1e-12)) (which 0) or max(1, max x) (which 1).  scratch:
+// apply_scratch_bytes(I, R) bytes whose first 4 were zeroed when it was allocated.
+alto_status apply_lambda(const float* B, const double* W, uint64_t I, int R, float* X, int which, void* scratch,
+                         double* lambda, cudaStream_t st);
+size_t apply_scratch_bytes(uint64_t I, int R);
+// Y = X / lambda by columns (with a bfloat16 copy, may be NULL) and its Gram, one pass.
+alto_status scale_gram(const float* X, uint64_t I, int R, const double* lambda, float* Y, __nv_bfloat16* shadow,
+                       double* out, DevBuf& scratch, cudaStream_t st);
 alto_status scale_columns(float* X, uint64_t I, int R, const double* lambda, __nv_bfloat16* shadow,
                           cudaStream_t st);
 alto_status to_bf16(const float* X, uint64_t n, __nv_bfloat16* Y, cudaStream_t st);
 // out3 = {sum a*b*colw, sum (a-b)^2, sum b^2}.
 alto_status dot_stats(const float* a, const float* b, uint64_t n, const double* colw, int R,
                       double* out3, DevBuf& scratch, cudaStream_t st);
-alto_status dot_stats_f64(const double* a, const float* b, uint64_t n, double* out3,
-                          DevBuf& scratch, cudaStream_t st);
 alto_status sum_squares(const float* v, uint64_t n, double* out, DevBuf& scratch, cudaStream_t st);
 alto_status model_norm(const double* grams, int nmodes, int R, const double* lambda, int exact,
                        double* out, cudaStream_t st);

@@ -352,6 +352,8 @@ alto_status run_mttkrp_feed(alto_tensor* t, int mode, const void* const* factors
                             int rank, float* out, int accumulate, alto_mttkrp_variant variant, int feed,
                             cudaStream_t st);
 alto_mttkrp_variant choose_variant(const alto_tensor* t, int mode, int rank, alto_dtype fdtype);
+// Whether alto_mttkrp_autotune has measured this mode, rank and factor type.
+bool mttkrp_tuned(const alto_tensor* t, int mode, int rank, alto_dtype fdtype);
 // Whether ALTO_MTTKRP_DETERMINISTIC runs for this rank and factor type.
 bool deterministic_supported(int rank, alto_dtype fdtype);
 // Build the per-mode row-sorted copy of the line.

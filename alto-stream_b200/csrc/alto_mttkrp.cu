@@ -1617,6 +1617,10 @@ static const TuneEntry* tuned_entry(const alto_tensor* t, int mode, int rank, al
   return nullptr;
 }
 
+bool mttkrp_tuned(const alto_tensor* t, int mode, int rank, alto_dtype fdtype) {
+  return tuned_entry(t, mode, rank, fdtype) != nullptr;
+}
+
 alto_mttkrp_variant choose_variant(const alto_tensor* t, int mode, int rank, alto_dtype fdtype) {
   if (const TuneEntry* e = tuned_entry(t, mode, rank, fdtype)) return e->variant;
   // The reference's rule (include/alto.hpp:835-846) picks atomics for long
