@@ -101,16 +101,21 @@ def kernel_launches():
     return int(lib().alto_kernel_launches())
 
 
-def _stream_handle(stream):
-    if stream is None:
-        try:
-            import torch
+_cuda = None  # torch.cuda once it is known to be usable
 
-            if torch.cuda.is_available():
-                return c_void_p(torch.cuda.current_stream().cuda_stream)
-        except ImportError:
-            pass
-        return c_void_p(0)
+
+def _stream_handle(stream):
+    global _cuda
+    if stream is None:
+        if _cuda is None:
+            try:
+                import torch
+
+                if torch.cuda.is_available():
+                    _cuda = torch.cuda
+            except ImportError:
+                pass
+        return c_void_p(_cuda.current_stream().cuda_stream if _cuda is not None else 0)
     if isinstance(stream, int):
         return c_void_p(stream)
     return c_void_p(stream.cuda_stream)

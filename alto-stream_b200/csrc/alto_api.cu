@@ -14,6 +14,74 @@ std::atomic<uint64_t> g_kernel_launches{0};
 thread_local cudaStream_t tls_alloc_stream = nullptr;
 static thread_local char g_err[512] = "";
 
+// The handles' pool of a device, and the stream its allocations and frees are
+// ordered on (nothing else runs there).
+namespace {
+struct HandlePool {
+  cudaMemPool_t pool = nullptr;
+  cudaStream_t st = nullptr;
+};
+HandlePool* handle_pool(int dev) {
+  static std::mutex mu;
+  static HandlePool pools[64];
+  if (dev < 0 || dev >= 64) return nullptr;
+  std::lock_guard<std::mutex> g(mu);
+  HandlePool& h = pools[dev];
+  if (!h.pool) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaStream_t st = nullptr;
+    cudaMemPool_t p = nullptr;
+    if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return nullptr;
+    if (cudaMemPoolCreate(&p, &props) != cudaSuccess) {
+      cudaStreamDestroy(st);
+      return nullptr;
+    }
+    uint64_t keep = kPoolKeep;
+    cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+    h.st = st;
+    h.pool = p;
+  }
+  return &h;
+}
+}  // namespace
+
+cudaError_t pool_alloc(void** p, size_t bytes, int* dev) {
+  *p = nullptr;
+  cudaError_t e = cudaGetDevice(dev);
+  if (e != cudaSuccess) return e;
+  HandlePool* h = handle_pool(*dev);
+  if (!h) return cudaErrorMemoryAllocation;
+  e = cudaMallocFromPoolAsync(p, bytes, h->pool, h->st);
+  if (e == cudaErrorMemoryAllocation) {  // what the pool keeps may be in the way, in other sizes
+    cudaGetLastError();
+    cudaDeviceSynchronize();
+    cudaMemPoolTrimTo(h->pool, 0);
+    e = cudaMallocFromPoolAsync(p, bytes, h->pool, h->st);
+    if (e != cudaSuccess) cudaGetLastError();
+  }
+  if (e != cudaSuccess) return e;
+  e = cudaStreamSynchronize(h->st);  // usable on every stream from here on
+  if (e != cudaSuccess) {
+    cudaFreeAsync(*p, h->st);
+    *p = nullptr;
+  }
+  return e;
+}
+
+void pool_free(void* p, int dev) {
+  HandlePool* h = handle_pool(dev);
+  if (!h) return;
+  int cur = dev;
+  cudaGetDevice(&cur);
+  if (cur != dev) cudaSetDevice(dev);
+  cudaDeviceSynchronize();
+  cudaFreeAsync(p, h->st);
+  if (cur != dev) cudaSetDevice(cur);
+}
+
 cudaMemPool_t transient_pool() {
   static std::mutex mu;
   static cudaMemPool_t pools[64] = {};

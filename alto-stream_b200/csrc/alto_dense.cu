@@ -1206,7 +1206,7 @@ alto_status sum_squares(const float* v, uint64_t n, double* out, DevBuf& scratch
 __global__ void model_norm_kernel(const double* __restrict__ grams, int nmodes, int R,
                                   const double* __restrict__ lambda, int exact,
                                   double* __restrict__ out) {
-  __shared__ double part[8];
+  __shared__ double part[32];
   double s = 0.0;
   const int RR = R * R;
   for (int p = threadIdx.x; p < RR; p += blockDim.x) {
@@ -1229,7 +1229,7 @@ __global__ void model_norm_kernel(const double* __restrict__ grams, int nmodes, 
 
 alto_status model_norm(const double* grams, int nmodes, int R, const double* lambda, int exact,
                        double* out, cudaStream_t st) {
-  model_norm_kernel<<<1, 256, 0, st>>>(grams, nmodes, R, lambda, exact, out);
+  model_norm_kernel<<<1, R > 16 ? 1024 : 256, 0, st>>>(grams, nmodes, R, lambda, exact, out);
   ALTO_LAUNCHED();
   return ALTO_OK;
 }
