@@ -15,8 +15,9 @@ struct FactorSet {
 struct MttkrpArgs {
   const void* line;   // line records (LineRec16 / LineRec32, or kDecoded's first array)
   const void* extra;  // kDecoded: the records' second array
-  // DETERMINISTIC: per lane-group sub-range, its first and last run (slots
-  // 2s and 2s+1: output row and R partial sums)
+  // DETERMINISTIC: per chunk of a decoded copy (per lane-group sub-range of
+  // another line), its first and last run (slots 2s and 2s+1: output row and R
+  // partial sums)
   uint32_t* det_rows;
   float* det_vals;
   const uint32_t* tile_iv;
@@ -25,9 +26,11 @@ struct MttkrpArgs {
   uint32_t ntiles;
   int target;
   int stage_rows;  // rows of the shared staging buffer (0: never stage)
-  // walks updating the output with atomics: consecutive tiles per block
-  // chunk, the open run of each lane group carried from tile to tile
+  // consecutive tiles of a block's chunk: walks updating the output with
+  // atomics carry the open run of each lane group through them, the
+  // deterministic walk of a decoded copy the block's open run
   uint32_t chunk_tiles;
+  int det_add;  // deterministic walk: add to the output's rows (0: write them)
   LineDecode dec;
   FactorSet fac;
   FactorSet in;  // the input modes' factors in mode order (kDecoded walks)
@@ -65,6 +68,7 @@ struct DetItem {
   MttkrpArgs a;
   DetLong dl;
   uint32_t nslots;
+  uint32_t nblocks;  // chunks of a decoded copy (blocks of its walk)
   int hw;
   uint64_t out_floats;
   const int* active;
@@ -76,7 +80,7 @@ alto_status det_prepare(alto_tensor* t, int mode, const void* const* factors, in
                         cudaStream_t st);
 
 // The deterministic MTTKRPs of a table of items at once; tile_off (device,
-// [count + 1]) holds the prefix sums of the items' tile counts.  Every item
+// [count + 1]) holds the prefix sums of the items' nblocks.  Every item
 // has rank `rank`, record format `hw` and `nmodes` modes.  Each live item's
 // output is zeroed and then gets exactly the sums, in the same order, that
 // a launch of that item alone gives.  Fixed grids, everything read on the

@@ -205,7 +205,34 @@ template <int V>
 struct OpenRun {
   uint32_t row;
   float acc[V];
+  // the deterministic walk's sum of the run so far, in pieces of kFoldSteps
+  // steps: a run of n nonzeros is then a chain of n / kFoldSteps additions of
+  // chains of kFoldSteps instead of one of n (5 modes, 5M nonzeros, rank 64: error
+  // 1.4e-7 instead of 3.2e-7 for 2% of the time; the walk with atomics, whose
+  // registers are all taken, lost 25% on the power-law 3-mode tensor)
+  float sum[V];
+  __device__ __forceinline__ void open() {
+    row = 0xffffffffu;
+#pragma unroll
+    for (int q = 0; q < V; ++q) acc[q] = sum[q] = 0.f;
+  }
+  __device__ __forceinline__ void fold() {
+#pragma unroll
+    for (int q = 0; q < V; ++q) {
+      sum[q] += acc[q];
+      acc[q] = 0.f;
+    }
+  }
+  // acc: the whole run
+  __device__ __forceinline__ void close() {
+#pragma unroll
+    for (int q = 0; q < V; ++q) {
+      acc[q] += sum[q];
+      sum[q] = 0.f;
+    }
+  }
 };
+constexpr uint32_t kFoldSteps = 16;
 
 template <int R, typename FT, int HW, int NM, bool SMEM, bool DET = false, bool CARRY = false>
 __device__ __forceinline__ void warp_range(const MttkrpArgs& a, const void* line, uint32_t ws, uint32_t we,
@@ -541,14 +568,52 @@ struct WalkStage {
   float v[U];
 };
 
+// The deterministic walk's meeting place (shared memory): per lane group its
+// first and last run (entries 2 g and 2 g + 1; row kNoRow: none), per warp
+// whether it is one run (then summed into its first entry), and the block's
+// open run from tile to tile.
+template <int R, int NPW>
+struct DetTile {
+  static constexpr int E = 2 * kMttkrpWarps * NPW;
+  static constexpr int Q = R / 4;
+  float4 val[E][Q];
+  float4 carry[2][Q];
+  uint32_t row[E];
+  uint32_t carry_row[2];
+  int one[kMttkrpWarps];
+};
+
+template <int R, int V, int G, int NPW>
+__device__ __forceinline__ void det_entry(DetTile<R, NPW>& d, int e, uint32_t row, int sub, const float (&acc)[V]) {
+  if (sub == 0) d.row[e] = row;
+#pragma unroll
+  for (int q = 0; q < V / 4; ++q)
+    d.val[e][q * G + sub] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
+}
+
+// A finished run of the deterministic walk that is its row's only one.
+__device__ __forceinline__ void det_put(const MttkrpArgs& a, float4* o, float4 x) {
+  if (a.det_add) {
+    const float4 y = *o;
+    x.x += y.x;
+    x.y += y.y;
+    x.z += y.z;
+    x.w += y.w;
+  }
+  *o = x;
+}
+
 // Sub-range [gs, ge) of a lane group, `steps` steps of U nonzeros (the same
 // for every group of the warp).  D steps are in the air: the rows of step
 // k + D - 1 are requested, and the records of step k + 2 D - 1, before step k
-// is summed.  DET: as warp_range's, slots of sub-range `slot0 / 2`; else the
-// open run is taken from and left in `run`.
+// is summed.  The open run is taken from and left in `run`.  det (the
+// deterministic walk): the first run to end goes to entry `ent` of it, the others
+// straight to the output, whose rows they have to themselves; returns how many
+// ended.
 template <int R, typename FT, int NIN, int V, int U, int D, bool DET>
-__device__ __forceinline__ void walk_range(const MttkrpArgs& a, uint32_t gs, uint32_t ge, uint32_t steps, int sub,
-                                           OpenRun<V>& run, uint32_t slot0) {
+__device__ __forceinline__ uint32_t walk_range(const MttkrpArgs& a, uint32_t gs, uint32_t ge, uint32_t steps, int sub,
+                                               OpenRun<V>& run,
+                                               DetTile<R, WalkMap<R, FT, V>::NPW>* det = nullptr, int ent = 0) {
   const void* base[NIN];
 #pragma unroll
   for (int j = 0; j < NIN; ++j) base[j] = a.in.f[j];
@@ -585,13 +650,19 @@ __device__ __forceinline__ void walk_range(const MttkrpArgs& a, uint32_t gs, uin
       }
       if (s.row[u] != run.row) {
         if (run.row != kNoRow) {
+          if constexpr (DET) run.close();
           if constexpr (!DET) {
             walk_flush<R, FT, V>(a.out, run.row, sub, run.acc);
           } else {
-            if (nrun++ == 0)
-              det_slot<R, V, WalkMap<R, FT, V>::G>(a, slot0, run.row, sub, run.acc, false);
-            else
-              det_plain<R, V, WalkMap<R, FT, V>::G>(a.out, run.row, sub, run.acc);
+            constexpr int G = WalkMap<R, FT, V>::G;
+            if (nrun++ == 0) {
+              det_entry<R, V, G>(*det, ent, run.row, sub, run.acc);
+            } else {
+#pragma unroll
+              for (int q = 0; q < V / 4; ++q)
+                det_put(a, reinterpret_cast<float4*>(a.out + (size_t)run.row * R + WalkMap<R, FT, V>::col(q, sub)),
+                        make_float4(run.acc[4 * q], run.acc[4 * q + 1], run.acc[4 * q + 2], run.acc[4 * q + 3]));
+            }
           }
         }
         run.row = s.row[u];
@@ -628,22 +699,9 @@ __device__ __forceinline__ void walk_range(const MttkrpArgs& a, uint32_t gs, uin
       fetch(rec[(d + kAhead) % D], i + (d + kAhead + D) * U);
       sum(st[d], i + d * U);
     }
+    if (DET && (k & (kFoldSteps - 1)) == kFoldSteps - D) run.fold();
   }
-  if constexpr (DET) {
-    constexpr int G = WalkMap<R, FT, V>::G;
-    if (run.row == kNoRow) {
-      // empty sub-range: both slots carry the row of the entry before it (the
-      // last run of an earlier sub-range) with zeros, keeping slot rows sorted
-      const uint32_t r0 = load_dec<NIN>(line, extra, gs > 0 ? min(gs - 1, last) : 0).row;
-      det_slot<R, V, G>(a, slot0, r0, sub, run.acc, true);
-      det_slot<R, V, G>(a, slot0 + 1, r0, sub, run.acc, true);
-    } else if (nrun == 0) {
-      det_slot<R, V, G>(a, slot0, run.row, sub, run.acc, false);
-      det_slot<R, V, G>(a, slot0 + 1, run.row, sub, run.acc, true);
-    } else {
-      det_slot<R, V, G>(a, slot0 + 1, run.row, sub, run.acc, false);
-    }
-  }
+  return nrun;
 }
 
 // The widths of the walk: V floats a lane, U nonzeros a step, D steps in the
@@ -662,7 +720,7 @@ __device__ __forceinline__ void walk_range(const MttkrpArgs& a, uint32_t gs, uin
 template <int R, typename FT, int NIN, bool DET, bool DEEP = false>
 struct WalkCfg {
   static constexpr int V = R >= 64 ? 8 : 4;
-  static constexpr int U = NIN == 2 && V == 4 ? 2 : 1;
+  static constexpr int U = V == 4 && (NIN == 2 || (NIN == 3 && DET)) ? 2 : 1;
   static constexpr int D = DEEP ? 2 : 1;
   static constexpr int MINB = DEEP ? 3 : NIN == 2 && V == 4 && !DET ? 5 : 4;
 };
@@ -719,44 +777,176 @@ __global__ void __launch_bounds__(kMttkrpThreads, WalkCfg<R, FT, NIN, false, DEE
   const uint32_t nchunks = (a.ntiles + ct - 1) / ct;
   for (uint32_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
     OpenRun<C::V> run;
-    run.row = kNoRow;
-#pragma unroll
-    for (int q = 0; q < C::V; ++q) run.acc[q] = 0.f;
+    run.open();
     const uint32_t t_end = min(c * ct + ct, a.ntiles);
     for (uint32_t tile = c * ct; tile < t_end; ++tile) {
       const TilePart<WM::NPW, WM::G, C::U> p(a, tile, warp, grp);
-      walk_range<R, FT, NIN, C::V, C::U, C::D, false>(a, p.gs, p.ge, p.steps, sub, run, 0);
+      walk_range<R, FT, NIN, C::V, C::U, C::D, false>(a, p.gs, p.ge, p.steps, sub, run);
     }
     const bool one = WM::NPW > 1 && merge_groups<C::V>(run.row, run.acc, WM::G, WM::NPW, lane);
     if (run.row != kNoRow && !(one && grp)) walk_flush<R, FT, C::V>(a.out, run.row, sub, run.acc);
   }
 }
 
-// One tile of the deterministic walk.
+// Chunk `chunk` of the deterministic walk (one block): consecutive tiles, each
+// cut among the lane groups as any walk's.  What a group starts and ends with
+// meets in shared memory, where runs that cross groups are summed in record
+// order; the block's open run is carried from tile to tile, its first and last
+// run go to the chunk's two slots (det_fix_kernel), and every other run is its
+// row's only one and is written without atomics.  So the slots are two per
+// block, however short the groups' sub-ranges are cut for latency: with two per
+// sub-range, the slots of a 200,000-nonzero slice were half its nonzeros and their
+// fix-up (three launches, 24 us) took longer than the walk (9 us).
 template <int R, int NIN>
-__device__ __forceinline__ void det_walk_tile(const MttkrpArgs& a, uint32_t tile) {
+__device__ __forceinline__ void det_walk_chunk(const MttkrpArgs& a, uint32_t chunk) {
   using C = WalkCfg<R, float, NIN, true>;
   using WM = WalkMap<R, float, C::V>;
+  using DT = DetTile<R, WM::NPW>;
+  constexpr int E = DT::E, Q = DT::Q, kPerWarp = 2 * WM::NPW;
+  __shared__ DT d;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int grp = lane / WM::G, sub = lane % WM::G;
-  const TilePart<WM::NPW, WM::G, C::U> p(a, tile, warp, grp);
-  OpenRun<C::V> run;
-  run.row = kNoRow;
-#pragma unroll
-  for (int q = 0; q < C::V; ++q) run.acc[q] = 0.f;
-  walk_range<R, float, NIN, C::V, C::U, C::D, true>(a, p.gs, p.ge, p.steps, sub, run,
-                                              2 * ((tile * kMttkrpWarps + warp) * WM::NPW + grp));
+  const uint32_t t0 = chunk * a.chunk_tiles, t1 = min(t0 + a.chunk_tiles, a.ntiles);
+  const uint32_t first_row = load_dec<NIN>(a.line, a.extra, t0 * a.tile_nnz).row;
+  const uint32_t slot = 2 * chunk;
+  auto put = [&](uint32_t row, int q, float4 x) {  // a finished run of the block
+    if (row == first_row)
+      *reinterpret_cast<float4*>(a.det_vals + (size_t)slot * R + q * 4) = x;
+    else
+      det_put(a, reinterpret_cast<float4*>(a.out + (size_t)row * R + q * 4), x);
+  };
+  if (threadIdx.x == 0) d.carry_row[0] = kNoRow;
+  int cur = 0;
+  for (uint32_t tile = t0; tile < t1; ++tile) {
+    const TilePart<WM::NPW, WM::G, C::U> p(a, tile, warp, grp);
+    const int ent = 2 * (warp * WM::NPW + grp);
+    OpenRun<C::V> run;
+    run.open();
+    const uint32_t ended = walk_range<R, float, NIN, C::V, C::U, C::D, true>(a, p.gs, p.ge, p.steps, sub, run, &d, ent);
+    run.close();
+    const bool one = __all_sync(0xffffffffu, ended == 0 && run.row != kNoRow) &&
+                     merge_groups<C::V>(run.row, run.acc, WM::G, WM::NPW, lane);
+    if (lane == 0) d.one[warp] = one;
+    if (run.row == kNoRow || (one && grp)) {
+      if (sub == 0) d.row[ent] = d.row[ent + 1] = kNoRow;
+    } else if (ended == 0) {
+      det_entry<R, C::V, WM::G>(d, ent, run.row, sub, run.acc);
+      if (sub == 0) d.row[ent + 1] = kNoRow;
+    } else {
+      det_entry<R, C::V, WM::G>(d, ent + 1, run.row, sub, run.acc);
+    }
+    __syncthreads();
+    const uint32_t open = d.carry_row[cur];
+    if (threadIdx.x < Q && open != kNoRow && open != d.row[0]) put(open, threadIdx.x, d.carry[cur][threadIdx.x]);
+    for (int w = threadIdx.x; w < E * Q; w += kMttkrpThreads) {
+      const int e = w / Q, q = w % Q;
+      const uint32_t r = d.row[e];
+      if (r == kNoRow) continue;
+      int prev = e - 1;
+      while (prev >= 0 && d.row[prev] == kNoRow) --prev;
+      if (prev >= 0 && d.row[prev] == r) continue;  // not the first entry of its run
+      float4 x = prev < 0 && open == r ? d.carry[cur][q] : make_float4(0.f, 0.f, 0.f, 0.f);
+      bool ends = false;
+      for (int k = e; k < E; ++k) {
+        const uint32_t rk = d.row[k];
+        if (rk == kNoRow) continue;
+        if (rk != r) {
+          ends = true;
+          break;
+        }
+        const float4 y = d.val[k][q];
+        x.x += y.x;
+        x.y += y.y;
+        x.z += y.z;
+        x.w += y.w;
+        if (k % kPerWarp == 0 && d.one[k / kPerWarp]) k += kPerWarp - 1;
+      }
+      if (ends) {
+        put(r, q, x);
+      } else {
+        d.carry[cur ^ 1][q] = x;
+        if (q == 0) d.carry_row[cur ^ 1] = r;
+      }
+    }
+    __syncthreads();
+    cur ^= 1;
+  }
+  // the open run: the chunk's last slot, or its first if that is still the same run
+  const uint32_t row = d.carry_row[cur];
+  if (threadIdx.x < Q) {
+    const float4 x = d.carry[cur][threadIdx.x];
+    const bool single = row == first_row;
+    float4* s = reinterpret_cast<float4*>(a.det_vals + (size_t)slot * R) + threadIdx.x;
+    if (single) s[0] = x;
+    s[Q] = single ? make_float4(0.f, 0.f, 0.f, 0.f) : x;
+    if (threadIdx.x == 0) {
+      a.det_rows[slot] = first_row;
+      a.det_rows[slot + 1] = row;
+    }
+  }
+  __syncthreads();
 }
 
 template <int R, int NIN>
-__global__ void __launch_bounds__(kMttkrpThreads, WalkCfg<R, float, NIN, true>::MINB)
-    det_walk_kernel(const MttkrpArgs a) {
-  for (uint32_t tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x) det_walk_tile<R, NIN>(a, tile);
+__global__ void __launch_bounds__(kMttkrpThreads, 3) det_walk_kernel(const MttkrpArgs a) {
+  det_walk_chunk<R, NIN>(a, blockIdx.x);
+}
+
+// The chunks' slots (rows non-decreasing; a row in them is in no other run):
+// a block per run of equal rows, its slots summed with a fixed split and a fixed
+// tree, then written or added to the row.
+__device__ __forceinline__ void det_fix_slots(const MttkrpArgs& a, uint32_t nslots, int R, float4* part) {
+  const uint32_t* rows = a.det_rows;
+  const float4* vals = reinterpret_cast<const float4*>(a.det_vals);
+  const int Q = R / 4, S = 256 / Q;
+  const int s = threadIdx.x / Q, q = threadIdx.x % Q;
+  for (uint32_t i = blockIdx.x; i < nslots; i += gridDim.x) {
+    const uint32_t row = rows[i];
+    if (i > 0 && rows[i - 1] == row) continue;
+    uint32_t end = i + 1;
+    for (;;) {  // (the rows are sorted: the equal ones of a window come first)
+      const uint32_t k = end + threadIdx.x;
+      const int same = __syncthreads_count(k < nslots && rows[k] == row);
+      end += same;
+      if (same < 256) break;
+    }
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+    for (uint32_t k = i + s; k < end; k += S) {
+      const float4 y = vals[(size_t)k * Q + q];
+      x.x += y.x;
+      x.y += y.y;
+      x.z += y.z;
+      x.w += y.w;
+    }
+    part[threadIdx.x] = x;
+    __syncthreads();
+    int live = S;
+    while (live > 1 && live / 2 >= (int)(end - i)) live /= 2;  // (the rest are zeros)
+    for (int stride = live / 2; stride >= 1; stride >>= 1) {
+      if (s < stride) {
+        const float4 y = part[(s + stride) * Q + q];
+        float4& m = part[s * Q + q];
+        m.x += y.x;
+        m.y += y.y;
+        m.z += y.z;
+        m.w += y.w;
+      }
+      __syncthreads();
+    }
+    if (s == 0) det_put(a, reinterpret_cast<float4*>(a.out + (size_t)row * R) + q, part[q]);
+    __syncthreads();
+  }
+}
+
+__global__ void __launch_bounds__(256) det_fix_kernel(const MttkrpArgs a, uint32_t nslots, int R) {
+  __shared__ float4 part[256];
+  det_fix_slots(a, nslots, R, part);
 }
 
 // ------------------------------------------------ deterministic fix-up
 //
-// The slots of DET hold, in line order, the first and last run of every
+// (Lines that are not decoded: 2 modes, or more than 5.)  The slots of DET hold, in line order, the first and last run of every
 // sub-range; their rows are non-decreasing, and a row appears in the slots
 // only if it is in none of the interior runs.  A chain (maximal stretch of
 // slots with one row) is summed in slot order, by one warp when it is short
@@ -974,7 +1164,7 @@ __global__ void __launch_bounds__(256) det_zero_group_kernel(Strided<DetItem> it
 }
 
 template <int R, int NIN>
-__global__ void __launch_bounds__(kMttkrpThreads, WalkCfg<R, float, NIN, true>::MINB)
+__global__ void __launch_bounds__(kMttkrpThreads, 3)
     det_tile_group_kernel(Strided<DetItem> items, const uint32_t* __restrict__ tile_off) {
   // the item's arguments staged in shared memory: the walk reads them per
   // nonzero (as a launch of its own reads them from the parameter bank)
@@ -997,43 +1187,17 @@ __global__ void __launch_bounds__(kMttkrpThreads, WalkCfg<R, float, NIN, true>::
       if (threadIdx.x == 0) s_item = s;
     }
     __syncthreads();
-    det_walk_tile<R, NIN>(sa, v - tile_off[s]);
+    det_walk_chunk<R, NIN>(sa, v - tile_off[s]);
   }
 }
 
-__global__ void __launch_bounds__(256) det_short_group_kernel(Strided<DetItem> items, int R) {
-  const int K = *items.count;
-  const int lane = threadIdx.x & 31;
-  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-  for (int s = 0; s < K; ++s) {
-    const DetItem& it = items[s];
-    if (!item_live(it.active)) continue;
-    for (uint32_t i = gw; i < it.nslots; i += nw)
-      det_short_chain(it.a.det_rows, it.a.det_vals, it.nslots, R, it.a.out, it.dl, i, lane);
-  }
-}
-
-__global__ void __launch_bounds__(256) det_seg_group_kernel(Strided<DetItem> items, int R) {
+__global__ void __launch_bounds__(256) det_fix_group_kernel(Strided<DetItem> items, int R) {
   __shared__ float4 part[256];
   const int K = *items.count;
   for (int s = 0; s < K; ++s) {
     const DetItem& it = items[s];
     if (!item_live(it.active)) continue;
-    const uint32_t nseg = it.dl.counters[1];
-    for (uint32_t g = blockIdx.x; g < nseg; g += gridDim.x) det_segment(it.a.det_vals, R, it.dl, g, part);
-  }
-}
-
-__global__ void __launch_bounds__(256) det_final_group_kernel(Strided<DetItem> items, int R) {
-  __shared__ float4 part[256];
-  __shared__ uint32_t s_nlong;
-  const int K = *items.count;
-  for (int s = 0; s < K; ++s) {
-    const DetItem& it = items[s];
-    if (!item_live(it.active)) continue;
-    const uint32_t nlong = det_take_chains(it.dl, &s_nlong);
-    for (uint32_t c = blockIdx.x; c < nlong; c += gridDim.x) det_chain_final(it.a.det_rows, R, it.a.out, it.dl, c, part);
+    det_fix_slots(it.a, it.nslots, R, part);
   }
 }
 
@@ -1337,11 +1501,18 @@ static uint32_t chunk_tiles_for(uint32_t ntiles, unsigned grid) {
 // The tiles of a walk that has no use for their intervals: sized so that
 // `grid` blocks get the same number of equal tiles (the tensor's own tiles leave
 // a last wave that is nearly empty: 489 tiles of 2048 on 444 blocks at 1M
-// nonzeros), at most kWalkTile nonzeros each, in multiples of `unit` (one step
+// nonzeros), at most `most` nonzeros each, in multiples of `unit` (one step
 // of every lane group of a block).
 constexpr uint32_t kWalkTile = 4096;
-static void even_tiles(MttkrpArgs* a, unsigned grid, uint32_t unit) {
-  const uint64_t rounds = std::max<uint64_t>(((uint64_t)a->nnz + (uint64_t)grid * kWalkTile - 1) / ((uint64_t)grid * kWalkTile), 1);
+constexpr uint32_t kDetTile = 16384;  // (a deterministic tile ends in a barrier)
+constexpr unsigned kDetSms = 148;     // (a constant: the cut must not depend on the device)
+static void even_tiles(MttkrpArgs* a, unsigned grid, uint32_t unit, uint32_t most = kWalkTile) {
+  if (!a->nnz) {
+    a->ntiles = 0;
+    return;
+  }
+  const uint64_t wave = (uint64_t)grid * most;
+  const uint64_t rounds = std::max<uint64_t>(((uint64_t)a->nnz + wave - 1) / wave, 1);
   const uint64_t per = (a->nnz + grid * rounds - 1) / (grid * rounds);
   a->tile_nnz = (uint32_t)std::max<uint64_t>((per + unit - 1) / unit * unit, unit);
   a->ntiles = (uint32_t)(((uint64_t)a->nnz + a->tile_nnz - 1) / a->tile_nnz);
@@ -1464,20 +1635,15 @@ static alto_status launch_det_fix(const MttkrpArgs& a, uint32_t nslots, int R, c
 }
 
 // Deterministic MTTKRP (float32 factors, the specialised ranks): the walk of
-// the row-sorted copy, then the fix-up kernels.
+// the row-sorted copy, then the fix-up of its chunks' slots.
 template <int R, int NIN>
 static alto_status launch_det_walk(const DetItem& it, cudaStream_t st) {
-  static int blocks_per_sm = 0;
-  if (!blocks_per_sm) {
-    ALTO_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, det_walk_kernel<R, NIN>,
-                                                                kMttkrpThreads, 0));
-    if (blocks_per_sm < 1) blocks_per_sm = 1;
-  }
-  const unsigned grid = std::min<unsigned>(it.a.ntiles, (unsigned)(num_sms() * blocks_per_sm));
-  if (!grid) return ALTO_OK;
-  det_walk_kernel<R, NIN><<<grid, kMttkrpThreads, 0, st>>>(it.a);
+  if (!it.nblocks) return ALTO_OK;
+  det_walk_kernel<R, NIN><<<it.nblocks, kMttkrpThreads, 0, st>>>(it.a);
   ALTO_LAUNCHED();
-  return launch_det_fix(it.a, it.nslots, R, it.dl, st);
+  det_fix_kernel<<<std::min<unsigned>(it.nslots, (unsigned)num_sms() * 8), 256, 0, st>>>(it.a, it.nslots, R);
+  ALTO_LAUNCHED();
+  return ALTO_OK;
 }
 
 // As launch_det_walk on lines that are not decoded (2 modes, or more than 5).
@@ -1523,24 +1689,34 @@ static alto_status launch_det_rank(const DetItem& it, int rank, cudaStream_t st)
   return ALTO_ERR_UNSUPPORTED;
 }
 
+template <int R, int NIN>
+static uint32_t det_unit_nm() {
+  using C = WalkCfg<R, float, NIN, true>;
+  return kMttkrpWarps * WalkMap<R, float, C::V>::NPW * C::U;
+}
+// Nonzeros of one step of every lane group of a deterministic walk's block.
 template <int R>
-static uint32_t det_groups(int nmodes, int hw) {
-  if (hw != kDecoded) return LaneWidth<R>::NPW;
-  switch (nmodes) {
-    case 3: return WalkMap<R, float, WalkCfg<R, float, 2, true>::V>::NPW;
-    case 4: return WalkMap<R, float, WalkCfg<R, float, 3, true>::V>::NPW;
-    default: return WalkMap<R, float, WalkCfg<R, float, 4, true>::V>::NPW;
+static uint32_t det_unit(int nmodes) {
+  return nmodes == 3 ? det_unit_nm<R, 2>() : nmodes == 4 ? det_unit_nm<R, 3>() : det_unit_nm<R, 4>();
+}
+static uint32_t det_unit_of(int rank, int nmodes) {
+  switch (rank) {
+    case 8: return det_unit<8>(nmodes);
+    case 16: return det_unit<16>(nmodes);
+    case 32: return det_unit<32>(nmodes);
+    case 64: return det_unit<64>(nmodes);
+    default: return det_unit<128>(nmodes);
   }
 }
 
-// Lane groups per warp of the deterministic walk.
-static uint32_t groups_per_warp(int rank, int nmodes, int hw) {
+// Lane groups per warp of the deterministic walk of a line that is not decoded.
+static uint32_t groups_per_warp(int rank) {
   switch (rank) {
-    case 8: return det_groups<8>(nmodes, hw);
-    case 16: return det_groups<16>(nmodes, hw);
-    case 32: return det_groups<32>(nmodes, hw);
-    case 64: return det_groups<64>(nmodes, hw);
-    default: return det_groups<128>(nmodes, hw);
+    case 8: return LaneWidth<8>::NPW;
+    case 16: return LaneWidth<16>::NPW;
+    case 32: return LaneWidth<32>::NPW;
+    case 64: return LaneWidth<64>::NPW;
+    default: return LaneWidth<128>::NPW;
   }
 }
 
@@ -1696,6 +1872,7 @@ alto_status run_mttkrp_feed(alto_tensor* t, int mode, const void* const* factors
   if (det) {
     DetItem it;
     ALTO_TRY(det_prepare(t, mode, factors, rank, out, &it, st));
+    it.a.det_add = accumulate ? 1 : 0;
     return launch_det_rank(it, rank, st);
   }
   MttkrpArgs a{};
@@ -1734,7 +1911,18 @@ alto_status det_prepare(alto_tensor* t, int mode, const void* const* factors, in
     set_error("the deterministic MTTKRP needs 16-byte aligned factors and output");
     return ALTO_ERR_UNSUPPORTED;
   }
-  const uint64_t nslots = (uint64_t)a.ntiles * kMttkrpWarps * groups_per_warp(rank, t->nmodes, hw) * 2;
+  uint64_t nslots = (uint64_t)a.ntiles * kMttkrpWarps * groups_per_warp(rank) * 2;
+  item->nblocks = 0;
+  if (hw == kDecoded) {
+    // a chunk per block, cut by nnz and rank alone (the order of the sums is a
+    // function of them); small tiles for a small tensor, whose groups' chains of
+    // dependent loads are what it waits for
+    even_tiles(&a, 3 * kDetSms, det_unit_of(rank, t->nmodes), kDetTile);
+    a.chunk_tiles = (a.ntiles + 3 * kDetSms - 1) / (3 * kDetSms);
+    if (!a.chunk_tiles) a.chunk_tiles = 1;
+    item->nblocks = (a.ntiles + a.chunk_tiles - 1) / a.chunk_tiles;
+    nslots = 2 * (uint64_t)item->nblocks;
+  }
   ALTO_TRY(tensor_ensure(t, t->det_rows, std::max<uint64_t>(nslots, 1) * 4));
   ALTO_TRY(tensor_ensure(t, t->det_vals, std::max<uint64_t>(nslots, 1) * rank * 4));
   // long chains: each has more than kShortChain slots; segments:
@@ -1773,11 +1961,7 @@ static alto_status det_group_nm(Strided<DetItem> items, const uint32_t* tile_off
   ALTO_LAUNCHED();
   det_tile_group_kernel<R, NIN><<<sm * blocks_per_sm, kMttkrpThreads, 0, st>>>(items, tile_off);
   ALTO_LAUNCHED();
-  det_short_group_kernel<<<sm * 16, 256, 0, st>>>(items, R);
-  ALTO_LAUNCHED();
-  det_seg_group_kernel<<<sm * 4, 256, 0, st>>>(items, R);
-  ALTO_LAUNCHED();
-  det_final_group_kernel<<<sm, 256, 0, st>>>(items, R);
+  det_fix_group_kernel<<<sm * 8, 256, 0, st>>>(items, R);
   ALTO_LAUNCHED();
   return ALTO_OK;
 }

@@ -1977,7 +1977,7 @@ alto_status group_set(StreamGroup* g, alto_stream_session* const* members, int k
     d.con = s->con != ALTO_UNCONSTRAINED ? 1 : 0;
     d.max_inner = s->max_inner;
     for (int m = 0; m < N; ++m) {
-      const uint32_t counts[kGroupOffKinds] = {d.det[m].a.ntiles, m == s->t ? 0u : d.gram[m].nb,
+      const uint32_t counts[kGroupOffKinds] = {d.det[m].nblocks, m == s->t ? 0u : d.gram[m].nb,
                                                m == s->t ? 0u : gram_reduce_blocks(R),
                                                m == s->t ? 0u : d.admm_blocks[m], m == s->t ? 0u : d.solve_blocks[m]};
       for (int kind = 0; kind < kGroupOffKinds; ++kind) {

@@ -302,6 +302,28 @@ def test_deterministic_five_modes_and_stream_row():
     check_deterministic(dims, cidx, vals, 16, stream_mode=0)
 
 
+@pytest.mark.parametrize("R", [8, 32, 64, 128])
+@pytest.mark.parametrize("nnz", [1, 63, 1000, 70001])
+@pytest.mark.parametrize("dims", [[1, 40, 50], [1, 3, 2000, 9], [7, 90, 20, 11, 5]])
+def test_deterministic_chunks(dims, nnz, R):
+    """Chunk edges of the deterministic walk: a mode of one row (every slot one
+    run), runs longer and shorter than a lane group's share, fewer nonzeros than
+    lane groups, partial steps; the slots' rows are written once per call, also
+    over an output that holds other values."""
+    import torch
+
+    dims = np.array(dims, np.uint64)
+    nnz = int(min(nnz, np.prod(dims.astype(np.float64)) // 2))
+    cidx, vals = synth.uniform_coo(dims, nnz, seed=R)
+    check_deterministic(dims, cidx, vals, R, seed=R)
+    t = A.create_alto(dims, cidx, vals)
+    Fd = to_dev([np.ones((int(d), R)) for d in dims], torch.float32)
+    out = torch.full((int(dims[1]), R), 3.0, device="cuda")
+    t.mttkrp(1, Fd, R, out=out, accumulate=True, variant=A.DETERMINISTIC)
+    fresh = t.mttkrp(1, Fd, R, variant=A.DETERMINISTIC)
+    np.testing.assert_allclose(out.cpu().numpy(), 3.0 + fresh.cpu().numpy(), rtol=1e-6)
+
+
 def test_deterministic_accumulates_and_rejects_unsupported():
     import torch
 
