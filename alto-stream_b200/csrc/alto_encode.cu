@@ -93,47 +93,82 @@ __device__ __forceinline__ void deposit(uint64_t x, uint64_t mlo, uint64_t mhi, 
   }
 }
 
-// PEXT: gather the bits of (klo, khi) selected by (mlo, mhi) into the low bits.
-__device__ __forceinline__ uint64_t extract(uint64_t klo, uint64_t khi, uint64_t mlo,
-                                            uint64_t mhi) {
-  uint64_t r = 0;
-  int k = 0;
-  while (mlo) {
-    int b = __ffsll((long long)mlo) - 1;
-    r |= ((klo >> b) & 1ull) << k;
-    ++k;
-    mlo &= mlo - 1;
-  }
-  while (mhi) {
-    int b = __ffsll((long long)mhi) - 1;
-    r |= ((khi >> b) & 1ull) << k;
-    ++k;
-    mhi &= mhi - 1;
-  }
-  return r;
-}
-
 struct CooPtrs {
   const void* cidx[ALTO_MAX_MODES];
 };
 
+// Encoding moves bits: a mode's index bits into the key (the masks), and the
+// sorted key's bits into the line key (mode-contiguous).  Both go a byte at a
+// time through tables in shared memory, one per source byte, that hold where
+// each of its 256 values puts its bits; every block fills them once and walks
+// its share of the nonzeros (a bit at a time, 8M nonzeros of 59 key bits took
+// 545 us each way).  to[k] is the target of source bit k, 255 for none; mode
+// m's index bits are source bits src[m] .. src[m + 1] - 1, from a byte boundary.
+constexpr int kMaxSrcBits = 192;  // 128 key bits, each of up to 8 modes' padded to whole bytes
+struct BitMap {
+  unsigned char to[kMaxSrcBits];
+  int src[ALTO_MAX_MODES + 1];  // linearisation: the modes' first source bits
+  int bytes;                    // source bytes
+};
+
+// The table of source byte t, value v.
+template <bool WIDE>
+__device__ __forceinline__ void fill_tables(const BitMap& bm, uint64_t* tab) {
+  for (int p = threadIdx.x; p < bm.bytes * 256; p += blockDim.x) {
+    const int t = p >> 8, v = p & 255;
+    uint64_t lo = 0, hi = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int to = bm.to[t * 8 + k];
+      if (!((v >> k) & 1) || to == 255) continue;
+      if (to < 64)
+        lo |= 1ull << to;
+      else
+        hi |= 1ull << (to - 64);
+    }
+    if (WIDE) {
+      tab[2 * p] = lo;
+      tab[2 * p + 1] = hi;
+    } else {
+      tab[p] = lo;
+    }
+  }
+  __syncthreads();
+}
+
+template <bool WIDE>
+__device__ __forceinline__ void or_table(const uint64_t* tab, int t, uint32_t v, uint64_t& lo, uint64_t& hi) {
+  if (WIDE) {
+    const ulonglong2 e = reinterpret_cast<const ulonglong2*>(tab)[t * 256 + v];
+    lo |= e.x;
+    hi |= e.y;
+  } else {
+    lo |= tab[t * 256 + v];
+  }
+}
+
+template <bool WIDE>
+size_t table_bytes(const BitMap& bm) {
+  return (size_t)bm.bytes * 256 * (WIDE ? 16 : 8);
+}
+
 // Key of nonzero i = OR over modes of PDEP(cidx[m][i], mask[m]).
-template <int IB>
-__global__ void linearize_kernel(CooPtrs coo, MaskSet ms, uint32_t nnz, uint64_t* __restrict__ klo,
-                                 uint64_t* __restrict__ khi, uint32_t* __restrict__ perm) {
+template <int IB, bool WIDE>
+__global__ void __launch_bounds__(256) linearize_kernel(CooPtrs coo, int nmodes, const BitMap bm, uint32_t nnz,
+                                                        uint64_t* __restrict__ klo, uint64_t* __restrict__ khi) {
+  extern __shared__ __align__(16) uint64_t tab[];
+  fill_tables<WIDE>(bm, tab);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += gridDim.x * blockDim.x) {
     uint64_t lo = 0, hi = 0;
 #pragma unroll
     for (int m = 0; m < ALTO_MAX_MODES; ++m) {
-      if (m < ms.nmodes) {
-        uint64_t x = IB == 8 ? ((const uint64_t*)coo.cidx[m])[i]
-                             : (uint64_t)((const uint32_t*)coo.cidx[m])[i];
-        deposit(x, ms.lo[m], ms.hi[m], lo, hi);
+      if (m < nmodes) {
+        uint32_t x = IB == 8 ? (uint32_t)((const uint64_t*)coo.cidx[m])[i] : ((const uint32_t*)coo.cidx[m])[i];
+        for (int t = bm.src[m] >> 3; t < bm.src[m + 1] >> 3; ++t, x >>= 8) or_table<WIDE>(tab, t, x & 255, lo, hi);
       }
     }
     klo[i] = lo;
-    if (khi) khi[i] = hi;
-    perm[i] = i;
+    if (WIDE) khi[i] = hi;
   }
 }
 
@@ -143,10 +178,44 @@ constexpr int kSortTile = kSortThreads * kSortItems;
 constexpr int kRadixBits = 8;
 constexpr int kRadix = 1 << kRadixBits;
 
-__device__ __forceinline__ uint32_t digit_of(const uint64_t* klo, const uint64_t* khi, uint32_t i,
-                                             int shift) {
-  uint64_t w = shift >= 64 ? khi[i] : klo[i];
-  return (uint32_t)(w >> (shift & 63)) & (kRadix - 1);
+// Keys of W 32-bit words: 1 (uint32 array in lo), 2 (uint64 array in lo) or 4
+// (uint64 arrays lo and hi).
+struct KeyArrays {
+  void* lo;
+  uint64_t* hi;
+};
+template <int W>
+struct SortKey {
+  uint64_t lo, hi;
+  __device__ __forceinline__ void load(const KeyArrays& k, uint32_t i) {
+    lo = W == 1 ? static_cast<const uint32_t*>(k.lo)[i] : static_cast<const uint64_t*>(k.lo)[i];
+    hi = W == 4 ? k.hi[i] : 0;
+  }
+  __device__ __forceinline__ void store(const KeyArrays& k, uint32_t i) const {
+    if (W == 1)
+      static_cast<uint32_t*>(k.lo)[i] = (uint32_t)lo;
+    else
+      static_cast<uint64_t*>(k.lo)[i] = lo;
+    if (W == 4) k.hi[i] = hi;
+  }
+  __device__ __forceinline__ uint32_t digit(int shift) const {
+    if (W == 1) return ((uint32_t)lo >> shift) & (kRadix - 1);
+    return (uint32_t)((W == 4 && shift >= 64 ? hi : lo) >> (shift & 63)) & (kRadix - 1);
+  }
+};
+
+// The lanes of `among` whose digit is d (a lane of `among` asks).  Eight ballots:
+// match.any takes a round per distinct value, up to 32 for the low digits of
+// spread keys, and was the sort's longest stall.
+__device__ __forceinline__ unsigned digit_peers(unsigned among, uint32_t d) {
+  unsigned peers = among;
+#pragma unroll
+  for (int b = 0; b < kRadixBits; ++b) {
+    const bool bit = (d >> b) & 1;
+    const unsigned m = __ballot_sync(among, bit);
+    peers &= bit ? m : ~m;
+  }
+  return peers;
 }
 
 // One-sweep LSD radix sort.  The digit counts of every pass come from one
@@ -168,9 +237,9 @@ constexpr int kLookbackBatch = 8;               // look-back words loaded togeth
 // accumulated; zeroed by the caller), in shared memory first.  A warp whose
 // lanes all hold one digit (the high digits of keys take few values) adds
 // it once.
+template <int W>
 __global__ void __launch_bounds__(kSortThreads)
-    radix_all_hist_kernel(const uint64_t* __restrict__ klo, const uint64_t* __restrict__ khi, uint32_t n,
-                          int npass, uint32_t* __restrict__ ghist) {
+    radix_all_hist_kernel(const KeyArrays keys, uint32_t n, int npass, uint32_t* __restrict__ ghist) {
   __shared__ uint32_t h[kMaxSortPasses * kRadix];
   for (int q = threadIdx.x; q < npass * kRadix; q += kSortThreads) h[q] = 0;
   __syncthreads();
@@ -179,12 +248,12 @@ __global__ void __launch_bounds__(kSortThreads)
     const uint32_t i = base + threadIdx.x;
     const bool valid = i < n;
     const unsigned vmask = __ballot_sync(0xffffffffu, valid);
-    const uint64_t lo = valid ? klo[i] : 0, hi = (valid && khi) ? khi[i] : 0;
     if (valid) {
+      SortKey<W> k;
+      k.load(keys, i);
       const int leader = __ffs(vmask) - 1;
       for (int p = 0; p < npass; ++p) {
-        const int shift = p * kRadixBits;
-        const uint32_t d = (uint32_t)((shift >= 64 ? hi : lo) >> (shift & 63)) & (kRadix - 1);
+        const uint32_t d = k.digit(p * kRadixBits);
         const uint32_t d0 = __shfl_sync(vmask, d, leader);
         if (__all_sync(vmask, d == d0)) {
           if (lane == leader) atomicAdd(&h[p * kRadix + d], (uint32_t)__popc(vmask));
@@ -222,10 +291,10 @@ __global__ void __launch_bounds__(kSortThreads) radix_offsets_kernel(uint32_t* _
   }
 }
 
-// One pass over the digit at `shift`.  Warp w of the block owns the tile's
-// elements [w*256, w*256 + 256) and ranks them in index order, 32 at a time,
-// with its own per-digit counters (the lanes of one digit found with
-// match_any; no block barrier while ranking).  The tile's digit counts are
+// One pass over the digit at `shift` (pin NULL: element i's payload is i).  Warp w
+// of the block owns the tile's elements [w*256, w*256 + 256) and ranks them in
+// index order, 32 at a time, with its own per-digit counters (digit_peers; no
+// block barrier while ranking).  The tile's digit counts are
 // published and looked back on (thread d for digit d), the tile is
 // reordered by digit in shared memory and written out in that order, so
 // consecutive threads write consecutive addresses of a digit's run.
@@ -236,12 +305,12 @@ __global__ void __launch_bounds__(kSortThreads) radix_offsets_kernel(uint32_t* _
 // so every write stays inside the array).
 // Dynamic shared memory: the tile's keys (one or two words) and payloads.
 static_assert(kSortTile / (kSortThreads / 32) == kSortItems * 32, "each warp ranks kSortItems rounds of 32");
+template <int W>
 __global__ void __launch_bounds__(kSortThreads)
-    radix_onesweep_kernel(const uint64_t* __restrict__ klo, const uint64_t* __restrict__ khi,
-                          const uint32_t* __restrict__ pin, uint32_t n, int shift, uint32_t tag,
+    radix_onesweep_kernel(const KeyArrays kin, const uint32_t* __restrict__ pin, uint32_t n, int shift, uint32_t tag,
                           const uint32_t* __restrict__ goff, uint32_t* __restrict__ ticket,
-                          unsigned long long* __restrict__ status, int* __restrict__ err,
-                          uint64_t* __restrict__ olo, uint64_t* __restrict__ ohi, uint32_t* __restrict__ pout) {
+                          unsigned long long* __restrict__ status, int* __restrict__ err, const KeyArrays kout,
+                          uint32_t* __restrict__ pout) {
   constexpr int kWarps = kSortThreads / 32;
   constexpr int kPerWarp = kSortTile / kWarps;  // 256 elements, kPerWarp / 32 = kSortItems rounds
   __shared__ uint32_t wrun[kWarps][kRadix];      // per warp: digit counts, then the warp's start in the digit
@@ -250,9 +319,8 @@ __global__ void __launch_bounds__(kSortThreads)
   __shared__ uint32_t wsum[kWarps];
   __shared__ uint32_t s_tile;
   extern __shared__ __align__(16) unsigned char dsm[];
-  uint64_t* s_lo = reinterpret_cast<uint64_t*>(dsm);
-  uint64_t* s_hi = s_lo + kSortTile;
-  uint32_t* s_p = reinterpret_cast<uint32_t*>(khi ? s_hi + kSortTile : s_lo + kSortTile);
+  const KeyArrays s_key{dsm, reinterpret_cast<uint64_t*>(dsm) + kSortTile};
+  uint32_t* s_p = reinterpret_cast<uint32_t*>(dsm + (size_t)kSortTile * 4 * W);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
 #pragma unroll
   for (int w = 0; w < kWarps; ++w) wrun[w][tid] = 0;
@@ -260,18 +328,16 @@ __global__ void __launch_bounds__(kSortThreads)
   __syncthreads();
   const uint32_t tile = s_tile;
   const uint32_t base = tile * kSortTile;
-  uint64_t vlo[kSortItems], vhi[kSortItems];
+  SortKey<W> v[kSortItems];
   uint32_t vp[kSortItems], dg[kSortItems], rk[kSortItems];
 #pragma unroll
   for (int r = 0; r < kSortItems; ++r) {  // every round's loads first, all in flight together
     const uint32_t i = base + warp * kPerWarp + r * 32 + lane;
-    vlo[r] = 0;
-    vhi[r] = 0;
-    vp[r] = 0;
+    v[r].lo = v[r].hi = 0;
+    vp[r] = i;
     if (i < n) {
-      vlo[r] = klo[i];
-      if (khi) vhi[r] = khi[i];
-      vp[r] = pin[i];
+      v[r].load(kin, i);
+      if (pin) vp[r] = pin[i];
     }
   }
 #pragma unroll
@@ -282,8 +348,8 @@ __global__ void __launch_bounds__(kSortThreads)
     rk[r] = 0;
     const unsigned vmask = __ballot_sync(0xffffffffu, valid);
     if (valid) {
-      dg[r] = (uint32_t)((shift >= 64 ? vhi[r] : vlo[r]) >> (shift & 63)) & (kRadix - 1);
-      const unsigned peers = __match_any_sync(vmask, dg[r]);
+      dg[r] = v[r].digit(shift);
+      const unsigned peers = digit_peers(vmask, dg[r]);
       const int leader = __ffs(peers) - 1;
       uint32_t before = 0;
       if (lane == leader) {
@@ -333,8 +399,7 @@ __global__ void __launch_bounds__(kSortThreads)
   for (int r = 0; r < kSortItems; ++r) {
     if (base + warp * kPerWarp + r * 32 + lane < n) {
       const uint32_t at = lstart[dg[r]] + wrun[warp][dg[r]] + rk[r];
-      s_lo[at] = vlo[r];
-      if (khi) s_hi[at] = vhi[r];
+      v[r].store(s_key, at);
       s_p[at] = vp[r];
     }
   }
@@ -380,43 +445,39 @@ __global__ void __launch_bounds__(kSortThreads)
   __syncthreads();
   const uint32_t tile_n = min((uint32_t)kSortTile, n - base);
   for (uint32_t j = tid; j < tile_n; j += kSortThreads) {
-    const uint64_t lo = s_lo[j], hi = khi ? s_hi[j] : 0;
-    const uint32_t d = (uint32_t)((shift >= 64 ? hi : lo) >> (shift & 63)) & (kRadix - 1);
+    SortKey<W> k;
+    k.load(s_key, j);
+    const uint32_t d = k.digit(shift);
     const uint32_t dst = gbase[d] + (j - lstart[d]);
-    olo[dst] = lo;
-    if (ohi) ohi[dst] = hi;
+    k.store(kout, dst);
     pout[dst] = s_p[j];
   }
 }
 
-// Dynamic shared memory of radix_onesweep_kernel for one- or two-word keys.
-size_t scatter_smem(bool two_words) { return (size_t)kSortTile * ((two_words ? 16 : 8) + 4); }
+// Dynamic shared memory of radix_onesweep_kernel for keys of W words.
+template <int W>
+constexpr size_t scatter_smem() {
+  return (size_t)kSortTile * (4 * W + 4);
+}
 
 // Sorted interleaved keys -> line records (mode-contiguous key + value), the
 // value gathered by input position (float64 or float32 input, stored float32).
-template <typename VT>
-__global__ void layout_kernel(const uint64_t* __restrict__ slo, const uint64_t* __restrict__ shi,
-                              const uint32_t* __restrict__ sperm, const VT* __restrict__ vin,
-                              MaskSet ms, LineDecode dec, uint32_t nnz, void* __restrict__ line,
-                              uint32_t* __restrict__ perm_out) {
+template <typename VT, bool WIDE>
+__global__ void __launch_bounds__(256)
+    layout_kernel(const uint64_t* __restrict__ slo, const uint64_t* __restrict__ shi,
+                  const uint32_t* __restrict__ sperm, const VT* __restrict__ vin, const BitMap bm, int hi_words,
+                  uint32_t nnz, void* __restrict__ line, uint32_t* __restrict__ perm_out) {
+  extern __shared__ __align__(16) uint64_t tab[];
+  fill_tables<WIDE>(bm, tab);
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += gridDim.x * blockDim.x) {
-    uint64_t klo = slo[i], khi = shi ? shi[i] : 0;
+    uint64_t klo = slo[i], khi = WIDE ? shi[i] : 0;
+    const uint32_t p = sperm[i];
+    const float v = (float)vin[p];
     uint64_t lo = 0, hi = 0;
 #pragma unroll
-    for (int m = 0; m < ALTO_MAX_MODES; ++m) {
-      if (m < ms.nmodes) {
-        uint64_t x = extract(klo, khi, ms.lo[m], ms.hi[m]);
-        int p = dec.pos[m];
-        if (p >= 64) {
-          hi |= x << (p - 64);
-        } else {
-          lo |= x << p;
-          if (p > 0) hi |= x >> (64 - p);
-        }
-      }
-    }
-    const uint32_t p = sperm[i];
-    rec_write(line, dec.hi_words, i, lo, hi, (float)vin[p]);
+    for (int t = 0; t < (WIDE ? 16 : 8); ++t)
+      if (t < bm.bytes) or_table<WIDE>(tab, t, (uint32_t)((t < 8 ? klo : khi) >> (8 * (t & 7))) & 255, lo, hi);
+    rec_write(line, hi_words, i, lo, hi, v);
     perm_out[i] = p;
   }
 }
@@ -750,6 +811,37 @@ static alto_status finish_layout(alto_tensor* t, int nprtn, cudaStream_t st) {
   return ALTO_OK;
 }
 
+// Blocks of a table kernel: a few per SM, each with many nonzeros per table fill.
+static unsigned table_grid(uint64_t n) {
+  return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + 1023) / 1024, 148ull * 6));
+}
+
+template <int IB, bool WIDE>
+static alto_status launch_linearize(const CooPtrs& cp, int nmodes, const BitMap& bm, uint32_t nnz, uint64_t* klo,
+                                    uint64_t* khi, cudaStream_t st) {
+  const size_t smem = table_bytes<WIDE>(bm);
+  if (smem > 48 * 1024) {  // (wide keys of many modes: set on every such call, once per tensor)
+    ALTO_TRY_CUDA(cudaFuncSetAttribute(linearize_kernel<IB, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(kMaxSrcBits / 8 * 256 * 16)));
+  }
+  linearize_kernel<IB, WIDE><<<table_grid(nnz), 256, smem, st>>>(cp, nmodes, bm, nnz, klo, khi);
+  ALTO_LAUNCHED();
+  return ALTO_OK;
+}
+
+template <typename VT, bool WIDE>
+static alto_status launch_layout(const uint64_t* klo, const uint64_t* khi, const uint32_t* perm, const void* vin,
+                                 const BitMap& bm, alto_tensor* t, uint32_t nnz, cudaStream_t st) {
+  const size_t smem = table_bytes<WIDE>(bm);
+  if (smem > 48 * 1024)
+    ALTO_TRY_CUDA(cudaFuncSetAttribute(layout_kernel<VT, WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(kMaxSrcBits / 8 * 256 * 16)));
+  layout_kernel<VT, WIDE><<<table_grid(nnz), 256, smem, st>>>(klo, khi, perm, static_cast<const VT*>(vin), bm,
+                                                              t->dec.hi_words, nnz, t->line.p, t->perm.as<uint32_t>());
+  ALTO_LAUNCHED();
+  return ALTO_OK;
+}
+
 alto_status encode_tensor(alto_tensor* t, const alto_coo* coo, int nprtn, cudaStream_t st) {
   const int N = coo->nmodes;
   const uint64_t nnz = coo->nnz;
@@ -825,33 +917,48 @@ alto_status encode_tensor(alto_tensor* t, const alto_coo* coo, int nprtn, cudaSt
     vin = sb + o_vals;
   }
 
-  MaskSet ms{};
-  ms.nmodes = N;
+  // the bits' ways: index -> key, and key -> line key
+  BitMap in_map{}, out_map{};
+  std::memset(in_map.to, 255, sizeof(in_map.to));
+  std::memset(out_map.to, 255, sizeof(out_map.to));
+  int src = 0;
   for (int m = 0; m < N; ++m) {
-    ms.lo[m] = t->masks[m].lo;
-    ms.hi[m] = t->masks[m].hi;
+    in_map.src[m] = src;
+    int k = 0;  // bit of the index
+    for (int b = 0; b < 128; ++b) {
+      const uint64_t word = b < 64 ? t->masks[m].lo : t->masks[m].hi;
+      if (!((word >> (b & 63)) & 1)) continue;
+      in_map.to[src + k] = (unsigned char)b;
+      out_map.to[b] = (unsigned char)(dec.pos[m] + k);
+      ++k;
+    }
+    src += (k + 7) / 8 * 8;
   }
+  for (int m = N; m <= ALTO_MAX_MODES; ++m) in_map.src[m] = src;
+  in_map.bytes = src / 8;
+  out_map.bytes = (total + 7) / 8;
 
   const uint32_t n32 = (uint32_t)nnz;
   if (nnz) {
     if (coo->index_bytes == 8)
-      linearize_kernel<8><<<grid_for(nnz, 256), 256, 0, st>>>(cp, ms, n32, klo[0], khi[0], pm[0]);
+      ALTO_TRY((two_words ? launch_linearize<8, true>(cp, N, in_map, n32, klo[0], khi[0], st)
+                          : launch_linearize<8, false>(cp, N, in_map, n32, klo[0], khi[0], st)));
     else
-      linearize_kernel<4><<<grid_for(nnz, 256), 256, 0, st>>>(cp, ms, n32, klo[0], khi[0], pm[0]);
-    ALTO_LAUNCHED();
+      ALTO_TRY((two_words ? launch_linearize<4, true>(cp, N, in_map, n32, klo[0], khi[0], st)
+                          : launch_linearize<4, false>(cp, N, in_map, n32, klo[0], khi[0], st)));
 
     // LSD radix sort over the used bits
     int cur = 0;
     ALTO_TRY(ensure_error_words(t, st));
-    ALTO_TRY(radix_sort_pairs(klo, khi, pm, n32, total, sort_scratch, t->err.as<int>() + kSortErrorWord, st, &cur));
+    ALTO_TRY(radix_sort_pairs(klo, khi, pm, n32, total, true, sort_scratch, t->err.as<int>() + kSortErrorWord, st,
+                              &cur));
 
     if (coo->val_dtype == ALTO_F64)
-      layout_kernel<double><<<grid_for(nnz, 256), 256, 0, st>>>(
-          klo[cur], khi[cur], pm[cur], (const double*)vin, ms, dec, n32, t->line.p, t->perm.as<uint32_t>());
+      ALTO_TRY((two_words ? launch_layout<double, true>(klo[cur], khi[cur], pm[cur], vin, out_map, t, n32, st)
+                          : launch_layout<double, false>(klo[cur], khi[cur], pm[cur], vin, out_map, t, n32, st)));
     else
-      layout_kernel<float><<<grid_for(nnz, 256), 256, 0, st>>>(
-          klo[cur], khi[cur], pm[cur], (const float*)vin, ms, dec, n32, t->line.p, t->perm.as<uint32_t>());
-    ALTO_LAUNCHED();
+      ALTO_TRY((two_words ? launch_layout<float, true>(klo[cur], khi[cur], pm[cur], vin, out_map, t, n32, st)
+                          : launch_layout<float, false>(klo[cur], khi[cur], pm[cur], vin, out_map, t, n32, st)));
   }
 
   ALTO_TRY(finish_layout(t, nprtn, st));
@@ -878,15 +985,14 @@ alto_status restrict_line(alto_tensor* t, uint64_t begin, uint64_t end, cudaStre
 
 // ------------------------------------------------ per-mode row-sorted lines
 
-// Row index of every line entry for one mode, and the identity payload.
+// Row index of every line entry for one mode.
 __global__ void mode_rows_kernel(const void* __restrict__ line, LineDecode dec, int mode, uint32_t nnz,
-                                 uint64_t* __restrict__ rows, uint32_t* __restrict__ pos) {
+                                 uint32_t* __restrict__ rows) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += gridDim.x * blockDim.x) {
     uint64_t lo, hi;
     float v;
     rec_read(line, dec.hi_words, i, lo, hi, v);
-    rows[i] = line_field(lo, hi, dec.pos[mode], dec.mask[mode]);
-    pos[i] = i;
+    rows[i] = (uint32_t)line_field(lo, hi, dec.pos[mode], dec.mask[mode]);
   }
 }
 
@@ -895,7 +1001,7 @@ __global__ void gather_line_kernel(const uint4* __restrict__ line, int words,
                                    const uint32_t* __restrict__ order, uint32_t nnz,
                                    uint4* __restrict__ out) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += gridDim.x * blockDim.x) {
-    const uint32_t p = order[i];
+    const uint32_t p = order ? order[i] : i;
     for (int w = 0; w < words; ++w) out[(size_t)i * words + w] = line[(size_t)p * words + w];
   }
 }
@@ -933,17 +1039,29 @@ size_t radix_scratch_bytes(uint64_t n) {
   return lookback_bytes(n) + align_up((size_t)kMaxSortPasses * kRadix * 4 + kMaxSortPasses * 4, 256);
 }
 
-// Stable LSD radix sort of (key, payload) pairs over the low `bits` bits of a
-// 64- or 128-bit key (khi[0] NULL for 64-bit keys), ping-ponging between
-// the two buffers of each array; *cur receives the buffer holding the
-// result.  scratch: radix_scratch_bytes(n) bytes; *err (device) is set if a
-// look-back gave up.
-alto_status radix_sort_pairs(uint64_t* klo[2], uint64_t* khi[2], uint32_t* pm[2], uint32_t n, int bits,
-                             void* scratch, int* err, cudaStream_t st, int* cur_out) {
+// Stable LSD radix sort of (key, payload) pairs over the low `bits` bits of keys
+// of W words, ping-ponging between the two buffers of each array; *cur receives
+// the buffer holding the result.  identity: element i's payload is i, and pm[0]
+// need not hold it (unless no pass runs: then it is filled in).  scratch:
+// radix_scratch_bytes(n) bytes; *err (device) is set if a look-back gave up.
+__global__ void iota_kernel(uint32_t* __restrict__ p, uint32_t n) {
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) p[i] = i;
+}
+
+template <int W>
+static alto_status radix_sort(KeyArrays (&k)[2], uint32_t* pm[2], uint32_t n, int bits, bool identity, void* scratch,
+                              int* err, cudaStream_t st, int* cur_out) {
   int cur = 0;
   *cur_out = 0;
   const int npass = (bits + kRadixBits - 1) / kRadixBits;
-  if (!n || npass <= 0) return ALTO_OK;
+  if (!n) return ALTO_OK;
+  if (npass <= 0) {
+    if (identity) {
+      iota_kernel<<<grid_for(n, 256), 256, 0, st>>>(pm[0], n);
+      ALTO_LAUNCHED();
+    }
+    return ALTO_OK;
+  }
   if (npass > kMaxSortPasses) {
     set_error("sort key of %d bits (at most %d)", bits, kMaxSortPasses * kRadixBits);
     return ALTO_ERR_UNSUPPORTED;
@@ -953,8 +1071,8 @@ alto_status radix_sort_pairs(uint64_t* klo[2], uint64_t* khi[2], uint32_t* pm[2]
   int dev = 0;
   ALTO_TRY_CUDA(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64 || !raised[dev].load()) {
-    ALTO_TRY_CUDA(cudaFuncSetAttribute(radix_onesweep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)scatter_smem(true)));
+    ALTO_TRY_CUDA(cudaFuncSetAttribute(radix_onesweep_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)scatter_smem<W>()));
     if (dev >= 0 && dev < 64) raised[dev] = true;
   }
   char* sb = static_cast<char*>(scratch);
@@ -966,14 +1084,14 @@ alto_status radix_sort_pairs(uint64_t* klo[2], uint64_t* khi[2], uint32_t* pm[2]
   ALTO_TRY_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const unsigned hist_grid =
       std::min<unsigned>((n + kSortThreads - 1) / kSortThreads, (unsigned)std::max(sms, 1) * 4);
-  radix_all_hist_kernel<<<hist_grid, kSortThreads, 0, st>>>(klo[0], khi[0], n, npass, ghist);
+  radix_all_hist_kernel<W><<<hist_grid, kSortThreads, 0, st>>>(k[0], n, npass, ghist);
   ALTO_LAUNCHED();
   radix_offsets_kernel<<<1, kSortThreads, 0, st>>>(ghist, npass);
   ALTO_LAUNCHED();
   for (int p = 0; p < npass; ++p) {
-    radix_onesweep_kernel<<<ntiles, kSortThreads, scatter_smem(khi[cur] != nullptr), st>>>(
-        klo[cur], khi[cur], pm[cur], n, p * kRadixBits, (uint32_t)p + 1, ghist + p * kRadix, tickets + p, status,
-        err, klo[cur ^ 1], khi[cur ^ 1], pm[cur ^ 1]);
+    radix_onesweep_kernel<W><<<ntiles, kSortThreads, scatter_smem<W>(), st>>>(
+        k[cur], p == 0 && identity ? nullptr : pm[cur], n, p * kRadixBits, (uint32_t)p + 1, ghist + p * kRadix,
+        tickets + p, status, err, k[cur ^ 1], pm[cur ^ 1]);
     ALTO_LAUNCHED();
     cur ^= 1;
   }
@@ -981,6 +1099,18 @@ alto_status radix_sort_pairs(uint64_t* klo[2], uint64_t* khi[2], uint32_t* pm[2]
   return ALTO_OK;
 }
 
+alto_status radix_sort_pairs(uint64_t* klo[2], uint64_t* khi[2], uint32_t* pm[2], uint32_t n, int bits, bool identity,
+                             void* scratch, int* err, cudaStream_t st, int* cur_out) {
+  KeyArrays k[2] = {{klo[0], khi[0]}, {klo[1], khi[1]}};
+  if (khi[0]) return radix_sort<4>(k, pm, n, bits, identity, scratch, err, st, cur_out);
+  return radix_sort<2>(k, pm, n, bits, identity, scratch, err, st, cur_out);
+}
+
+alto_status radix_sort_pairs32(uint32_t* key[2], uint32_t* pm[2], uint32_t n, int bits, bool identity, void* scratch,
+                               int* err, cudaStream_t st, int* cur_out) {
+  KeyArrays k[2] = {{key[0], nullptr}, {key[1], nullptr}};
+  return radix_sort<1>(k, pm, n, bits, identity, scratch, err, st, cur_out);
+}
 
 // A copy of the line ordered by the row of `mode`, ALTO order kept among
 // equal rows (stable LSD sort over the mode's bits).  This is the device
@@ -997,35 +1127,38 @@ alto_status build_sorted_line(alto_tensor* t, int mode, cudaStream_t st) {
     ALTO_TRY(tensor_ensure(t, s.extra, (nnz + kLinePad) * decoded_extra_bytes(t->nmodes)));
   const size_t cap = std::max<uint64_t>(nnz, 1);
   size_t off = 0;
-  size_t o_r0 = off; off = align_up(off + cap * 8, 256);
-  size_t o_r1 = off; off = align_up(off + cap * 8, 256);
+  size_t o_r0 = off; off = align_up(off + cap * 4, 256);
+  size_t o_r1 = off; off = align_up(off + cap * 4, 256);
   size_t o_p0 = off; off = align_up(off + cap * 4, 256);
   size_t o_p1 = off; off = align_up(off + cap * 4, 256);
   size_t o_cnt = off; off = align_up(off + radix_scratch_bytes(nnz), 256);
   ALTO_TRY(tensor_ensure(t, t->scratch, off));
   char* sb = t->scratch.as<char>();
-  uint64_t* rk[2] = {(uint64_t*)(sb + o_r0), (uint64_t*)(sb + o_r1)};
+  uint32_t* rk[2] = {(uint32_t*)(sb + o_r0), (uint32_t*)(sb + o_r1)};
   uint32_t* pm[2] = {(uint32_t*)(sb + o_p0), (uint32_t*)(sb + o_p1)};
   void* sort_scratch = sb + o_cnt;
   const uint32_t n32 = (uint32_t)nnz;
   if (nnz) {
     ALTO_TRY(ensure_error_words(t, st));
-    mode_rows_kernel<<<grid_for(nnz, 256), 256, 0, st>>>(t->line.p, t->dec, mode, n32, rk[0], pm[0]);
-    ALTO_LAUNCHED();
-    int cur = 0;
-    uint64_t* nohi[2] = {nullptr, nullptr};
-    ALTO_TRY(radix_sort_pairs(rk, nohi, pm, n32, t->mode_bits[mode], sort_scratch,
-                              t->err.as<int>() + kSortErrorWord, st, &cur));
+    const uint32_t* order = nullptr;  // (a mode of one row is in row order already)
+    if (t->mode_bits[mode]) {
+      mode_rows_kernel<<<grid_for(nnz, 256), 256, 0, st>>>(t->line.p, t->dec, mode, n32, rk[0]);
+      ALTO_LAUNCHED();
+      int cur = 0;
+      ALTO_TRY(radix_sort_pairs32(rk, pm, n32, t->mode_bits[mode], true, sort_scratch,
+                                  t->err.as<int>() + kSortErrorWord, st, &cur));
+      order = pm[cur];
+    }
     const unsigned gg = grid_for(nnz, 256);
     if (s.hw == kDecoded && t->nmodes == 3)
-      gather_decode_kernel<3><<<gg, 256, 0, st>>>(t->line.p, t->dec, mode, pm[cur], n32, s.line.as<uint4>(), s.extra.p);
+      gather_decode_kernel<3><<<gg, 256, 0, st>>>(t->line.p, t->dec, mode, order, n32, s.line.as<uint4>(), s.extra.p);
     else if (s.hw == kDecoded && t->nmodes == 4)
-      gather_decode_kernel<4><<<gg, 256, 0, st>>>(t->line.p, t->dec, mode, pm[cur], n32, s.line.as<uint4>(), s.extra.p);
+      gather_decode_kernel<4><<<gg, 256, 0, st>>>(t->line.p, t->dec, mode, order, n32, s.line.as<uint4>(), s.extra.p);
     else if (s.hw == kDecoded)
-      gather_decode_kernel<5><<<gg, 256, 0, st>>>(t->line.p, t->dec, mode, pm[cur], n32, s.line.as<uint4>(), s.extra.p);
+      gather_decode_kernel<5><<<gg, 256, 0, st>>>(t->line.p, t->dec, mode, order, n32, s.line.as<uint4>(), s.extra.p);
     else
       gather_line_kernel<<<grid_for(nnz, 256), 256, 0, st>>>(t->line.as<uint4>(), rec_bytes(hw) / 16,
-                                                             pm[cur], n32, s.line.as<uint4>());
+                                                             order, n32, s.line.as<uint4>());
     ALTO_LAUNCHED();
   }
   s.ntiles = t->ntiles;

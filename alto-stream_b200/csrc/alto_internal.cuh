@@ -349,10 +349,13 @@ inline alto_status tensor_ensure(const alto_tensor* t, DevBuf& b, size_t n) {
 // Encode (linearise, sort, lay out, partition) a COO tensor into t.
 alto_status encode_tensor(alto_tensor* t, const alto_coo* coo, int nprtn, cudaStream_t st);
 // Stable one-sweep LSD radix sort of (key, uint32 payload) pairs
-// (alto_encode.cu); scratch of radix_scratch_bytes(n) bytes; *err (device)
-// is set if a look-back gave up.
-alto_status radix_sort_pairs(uint64_t* klo[2], uint64_t* khi[2], uint32_t* pm[2], uint32_t n, int bits,
+// (alto_encode.cu) with 64-bit, 128-bit (khi not NULL) or 32-bit keys; identity:
+// element i's payload is i (pm[0] is not read); scratch of
+// radix_scratch_bytes(n) bytes; *err (device) is set if a look-back gave up.
+alto_status radix_sort_pairs(uint64_t* klo[2], uint64_t* khi[2], uint32_t* pm[2], uint32_t n, int bits, bool identity,
                              void* scratch, int* err, cudaStream_t st, int* cur_out);
+alto_status radix_sort_pairs32(uint32_t* key[2], uint32_t* pm[2], uint32_t n, int bits, bool identity, void* scratch,
+                               int* err, cudaStream_t st, int* cur_out);
 size_t radix_scratch_bytes(uint64_t n);
 // Device error words of a tensor (t->err, four ints): [0] a bulk-feed
 // MTTKRP wait gave up, [kSortErrorWord] a radix-sort look-back gave up.

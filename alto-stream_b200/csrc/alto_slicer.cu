@@ -72,11 +72,11 @@ __device__ __forceinline__ uint32_t get_field(uint64_t lo, uint64_t hi, int shif
   return (uint32_t)(v & ((1ull << bits) - 1));
 }
 
-// Sort keys and the identity payload; an index outside its mode sets *err
+// Sort keys; an index outside its mode sets *err
 // (and is clamped to 0, so nothing downstream leaves its table).
 template <int IB>
 __global__ void slice_key_kernel(InPtrs in, SortFields f, uint32_t nnz, uint64_t* __restrict__ klo,
-                                 uint64_t* __restrict__ khi, uint32_t* __restrict__ perm, int* __restrict__ err) {
+                                 uint64_t* __restrict__ khi, int* __restrict__ err) {
   for (uint64_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += gridDim.x * blockDim.x) {
     uint64_t lo = 0, hi = 0;
     for (int m = 0; m < f.nmodes; ++m) {
@@ -89,26 +89,22 @@ __global__ void slice_key_kernel(InPtrs in, SortFields f, uint32_t nnz, uint64_t
     }
     klo[i] = lo;
     if (khi) khi[i] = hi;
-    perm[i] = (uint32_t)i;
   }
 }
 
 // Sorted order: the stream mode's time step, the original index of every
 // other mode (relabelled in place later), the values gathered, and per
-// index value its first sorted position (lowest lane of each run of equal
-// values in a warp takes the atomic minimum).
+// index value its first sorted position: an atomic minimum, only where the
+// position is below what is there (a stale read costs an atomic, no more; the
+// lanes of one value found with match.any first took a round per distinct value,
+// and most positions come after their value's first).
 template <typename VT>
 __global__ void slice_decode_kernel(const uint64_t* __restrict__ klo, const uint64_t* __restrict__ khi,
                                     const uint32_t* __restrict__ perm, SortFields f, int t, uint32_t nnz,
                                     const VT* __restrict__ vin, VT* __restrict__ vout, uint32_t* __restrict__ gtime,
                                     uint32_t* __restrict__ idx, uint32_t* __restrict__ first) {
   const uint64_t stride = gridDim.x * blockDim.x;
-  const int lane = threadIdx.x & 31;
-  for (uint64_t base = blockIdx.x * blockDim.x; base < nnz; base += stride) {
-    const uint64_t i = base + threadIdx.x;
-    const bool valid = i < nnz;
-    const unsigned vmask = __ballot_sync(0xffffffffu, valid);
-    if (!valid) continue;
+  for (uint64_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += stride) {
     const uint64_t lo = klo[i], hi = khi ? khi[i] : 0;
     vout[i] = vin[perm[i]];
     for (int m = 0; m < f.nmodes; ++m) {
@@ -118,8 +114,8 @@ __global__ void slice_decode_kernel(const uint64_t* __restrict__ klo, const uint
         continue;
       }
       idx[(size_t)m * nnz + i] = v;
-      const unsigned peers = __match_any_sync(vmask, v);
-      if (lane == __ffs(peers) - 1) atomicMin(first + f.first_off[m] + v, (uint32_t)i);
+      uint32_t* at = first + f.first_off[m] + v;
+      if (__ldcg(at) > (uint32_t)i) atomicMin(at, (uint32_t)i);
     }
   }
 }
@@ -339,12 +335,12 @@ alto_status slicer_build(alto_slicer* s, const alto_coo* coo) {
   const dim3 gm(grid_n(nnz, 256), N);
   if (nnz) {
     if (coo->index_bytes == 8)
-      slice_key_kernel<8><<<grid_n(nnz, 256), 256, 0, st>>>(in, f, n32, klo[0], khi[0], pm[0], d_err);
+      slice_key_kernel<8><<<grid_n(nnz, 256), 256, 0, st>>>(in, f, n32, klo[0], khi[0], d_err);
     else
-      slice_key_kernel<4><<<grid_n(nnz, 256), 256, 0, st>>>(in, f, n32, klo[0], khi[0], pm[0], d_err);
+      slice_key_kernel<4><<<grid_n(nnz, 256), 256, 0, st>>>(in, f, n32, klo[0], khi[0], d_err);
     ALTO_LAUNCHED();
     int cur = 0;
-    ALTO_TRY(radix_sort_pairs(klo, khi, pm, n32, total, sb + o_cnt, d_err + 1, st, &cur));
+    ALTO_TRY(radix_sort_pairs(klo, khi, pm, n32, total, true, sb + o_cnt, d_err + 1, st, &cur));
     if (coo->val_dtype == ALTO_F64)
       slice_decode_kernel<double><<<grid_n(nnz, 256), 256, 0, st>>>(
           klo[cur], khi[cur], pm[cur], f, t, n32, (const double*)vin, s->vals.as<double>(), s->gtime.as<uint32_t>(),
@@ -363,7 +359,7 @@ alto_status slicer_build(alto_slicer* s, const alto_coo* coo) {
     uint64_t* nohi[2] = {nullptr, nullptr};
     int pc = 0;
     const int pair_bits = 32 + (N > 1 ? 32 - __builtin_clz((unsigned)(N - 1)) : 0);
-    ALTO_TRY(radix_sort_pairs(klo, nohi, pm, (uint32_t)nfirst, pair_bits, sb + o_cnt, d_err + 1, st, &pc));
+    ALTO_TRY(radix_sort_pairs(klo, nohi, pm, (uint32_t)nfirst, pair_bits, false, sb + o_cnt, d_err + 1, st, &pc));
     slice_label_table_kernel<<<grid_n(nfirst, 256), 256, 0, st>>>(klo[pc], pm[pc], f, nfirst, first,
                                                                   s->iperm.as<uint32_t>());
     ALTO_LAUNCHED();
