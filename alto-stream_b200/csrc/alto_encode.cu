@@ -172,9 +172,10 @@ __global__ void __launch_bounds__(256) linearize_kernel(CooPtrs coo, int nmodes,
   }
 }
 
-constexpr int kSortThreads = 256;
+constexpr int kSortThreads = 256;   // histogram blocks; digits
+constexpr int kSweepThreads = 512;  // a pass's blocks
 constexpr int kSortItems = 8;
-constexpr int kSortTile = kSortThreads * kSortItems;
+constexpr int kSortTile = kSweepThreads * kSortItems;
 constexpr int kRadixBits = 8;
 constexpr int kRadix = 1 << kRadixBits;
 
@@ -204,15 +205,15 @@ struct SortKey {
   }
 };
 
-// The lanes of `among` whose digit is d (a lane of `among` asks).  Eight ballots:
-// match.any takes a round per distinct value, up to 32 for the low digits of
-// spread keys, and was the sort's longest stall.
+// The lanes of `among` whose digit is this lane's d (every lane of the warp
+// calls).  Eight ballots: match.any takes a round per distinct value, up to 32 for
+// the low digits of spread keys, and was the sort's longest stall.
 __device__ __forceinline__ unsigned digit_peers(unsigned among, uint32_t d) {
   unsigned peers = among;
 #pragma unroll
   for (int b = 0; b < kRadixBits; ++b) {
     const bool bit = (d >> b) & 1;
-    const unsigned m = __ballot_sync(among, bit);
+    const unsigned m = __ballot_sync(0xffffffffu, bit);
     peers &= bit ? m : ~m;
   }
   return peers;
@@ -304,26 +305,27 @@ __global__ void __launch_bounds__(kSortThreads) radix_offsets_kernel(uint32_t* _
 // kLookbackSpins times sets *err and takes the count so far (a lower start,
 // so every write stays inside the array).
 // Dynamic shared memory: the tile's keys (one or two words) and payloads.
-static_assert(kSortTile / (kSortThreads / 32) == kSortItems * 32, "each warp ranks kSortItems rounds of 32");
+static_assert(kSortTile / (kSweepThreads / 32) == kSortItems * 32, "each warp ranks kSortItems rounds of 32");
 template <int W>
-__global__ void __launch_bounds__(kSortThreads)
+__global__ void __launch_bounds__(kSweepThreads)
     radix_onesweep_kernel(const KeyArrays kin, const uint32_t* __restrict__ pin, uint32_t n, int shift, uint32_t tag,
                           const uint32_t* __restrict__ goff, uint32_t* __restrict__ ticket,
                           unsigned long long* __restrict__ status, int* __restrict__ err, const KeyArrays kout,
                           uint32_t* __restrict__ pout) {
-  constexpr int kWarps = kSortThreads / 32;
+  constexpr int kWarps = kSweepThreads / 32;
   constexpr int kPerWarp = kSortTile / kWarps;  // 256 elements, kPerWarp / 32 = kSortItems rounds
   __shared__ uint32_t wrun[kWarps][kRadix];      // per warp: digit counts, then the warp's start in the digit
   __shared__ uint32_t gbase[kRadix];
   __shared__ uint32_t lstart[kRadix];
-  __shared__ uint32_t wsum[kWarps];
+  __shared__ uint32_t wsum[kRadix / 32];
   __shared__ uint32_t s_tile;
   extern __shared__ __align__(16) unsigned char dsm[];
   const KeyArrays s_key{dsm, reinterpret_cast<uint64_t*>(dsm) + kSortTile};
   uint32_t* s_p = reinterpret_cast<uint32_t*>(dsm + (size_t)kSortTile * 4 * W);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool dig = tid < kRadix;  // thread d also works for digit d
 #pragma unroll
-  for (int w = 0; w < kWarps; ++w) wrun[w][tid] = 0;
+  for (int q = 0; q < kWarps * kRadix / kSweepThreads; ++q) (&wrun[0][0])[q * kSweepThreads + tid] = 0;
   if (tid == 0) s_tile = atomicAdd(ticket, 1u);
   __syncthreads();
   const uint32_t tile = s_tile;
@@ -344,26 +346,25 @@ __global__ void __launch_bounds__(kSortThreads)
   for (int r = 0; r < kSortItems; ++r) {
     const uint32_t i = base + warp * kPerWarp + r * 32 + lane;
     const bool valid = i < n;
-    dg[r] = 0;
-    rk[r] = 0;
     const unsigned vmask = __ballot_sync(0xffffffffu, valid);
-    if (valid) {
-      dg[r] = v[r].digit(shift);
-      const unsigned peers = digit_peers(vmask, dg[r]);
-      const int leader = __ffs(peers) - 1;
-      uint32_t before = 0;
-      if (lane == leader) {
-        before = wrun[warp][dg[r]];
-        wrun[warp][dg[r]] = before + __popc(peers);
-      }
-      before = __shfl_sync(peers, before, leader);
-      rk[r] = before + __popc(peers & ((1u << lane) - 1));  // rank among the warp's digit-d elements
+    dg[r] = v[r].digit(shift);
+    const unsigned peers = digit_peers(vmask, dg[r]);
+    const int leader = valid ? __ffs(peers) - 1 : lane;
+    uint32_t before = 0;
+    if (valid && lane == leader) {
+      before = wrun[warp][dg[r]];
+      wrun[warp][dg[r]] = before + __popc(peers);
     }
+    before = __shfl_sync(0xffffffffu, before, leader);
+    rk[r] = before + __popc(peers & ((1u << lane) - 1));  // rank among the warp's digit-d elements
     __syncwarp();
   }
   __syncthreads();
-  uint32_t cnt;
-  {  // digit tid: each warp's start within the digit, in warp order; the tile's count
+  uint32_t cnt = 0;
+  const unsigned long long tg = (unsigned long long)tag << 32;
+  volatile unsigned long long* mine = status + (size_t)tile * kRadix + tid;
+  uint32_t x = 0;
+  if (dig) {  // digit tid: each warp's start within the digit, in warp order; the tile's count
     uint32_t run = 0;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) {
@@ -372,23 +373,22 @@ __global__ void __launch_bounds__(kSortThreads)
       run += c;
     }
     cnt = run;
-  }
-  // the tile's count of digit tid, published for the tiles after it
-  const unsigned long long tg = (unsigned long long)tag << 32;
-  volatile unsigned long long* mine = status + (size_t)tile * kRadix + tid;
-  *mine = (tile == 0 ? kLbPrefix : kLbAggregate) | tg | cnt;
-  {  // the tile's digit starts: exclusive scan of its digit counts
-    uint32_t x = cnt;
+    // the tile's count of digit tid, published for the tiles after it
+    *mine = (tile == 0 ? kLbPrefix : kLbAggregate) | tg | cnt;
+    // the tile's digit starts: exclusive scan of its digit counts
+    x = cnt;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
       if (lane >= o) x += y;
     }
     if (lane == 31) wsum[warp] = x;
-    __syncthreads();
+  }
+  __syncthreads();
+  if (dig) {
     uint32_t pre = 0;
 #pragma unroll
-    for (int w = 0; w < kWarps; ++w)
+    for (int w = 0; w < kRadix / 32; ++w)
       if (w < warp) pre += wsum[w];
     lstart[tid] = pre + x - cnt;
   }
@@ -403,7 +403,7 @@ __global__ void __launch_bounds__(kSortThreads)
       s_p[at] = vp[r];
     }
   }
-  {  // digit tid's start among the preceding tiles (decoupled look-back)
+  if (dig) {  // digit tid's start among the preceding tiles (decoupled look-back)
     uint32_t excl = 0;
     if (tile > 0) {
       // the preceding tiles' words, kLookbackBatch at a time (independent
@@ -444,7 +444,7 @@ __global__ void __launch_bounds__(kSortThreads)
   }
   __syncthreads();
   const uint32_t tile_n = min((uint32_t)kSortTile, n - base);
-  for (uint32_t j = tid; j < tile_n; j += kSortThreads) {
+  for (uint32_t j = tid; j < tile_n; j += kSweepThreads) {
     SortKey<W> k;
     k.load(s_key, j);
     const uint32_t d = k.digit(shift);
@@ -1089,7 +1089,7 @@ static alto_status radix_sort(KeyArrays (&k)[2], uint32_t* pm[2], uint32_t n, in
   radix_offsets_kernel<<<1, kSortThreads, 0, st>>>(ghist, npass);
   ALTO_LAUNCHED();
   for (int p = 0; p < npass; ++p) {
-    radix_onesweep_kernel<W><<<ntiles, kSortThreads, scatter_smem<W>(), st>>>(
+    radix_onesweep_kernel<W><<<ntiles, kSweepThreads, scatter_smem<W>(), st>>>(
         k[cur], p == 0 && identity ? nullptr : pm[cur], n, p * kRadixBits, (uint32_t)p + 1, ghist + p * kRadix,
         tickets + p, status, err, k[cur ^ 1], pm[cur ^ 1]);
     ALTO_LAUNCHED();
