@@ -82,9 +82,10 @@ alto_status det_prepare(alto_tensor* t, int mode, const void* const* factors, in
 // The deterministic MTTKRPs of a table of items at once; tile_off (device,
 // [count + 1]) holds the prefix sums of the items' nblocks.  Every item
 // has rank `rank`, record format `hw` and `nmodes` modes.  Each live item's
-// output is zeroed and then gets exactly the sums, in the same order, that
-// a launch of that item alone gives.  Fixed grids, everything read on the
+// output, zeroed by det_group_zero, gets exactly the sums, in the same order,
+// that a launch of that item alone gives.  Fixed grids, everything read on the
 // device: capturable once and relaunched with other items.
+alto_status det_group_zero(Strided<DetItem> items, cudaStream_t st);
 alto_status det_group_launch(Strided<DetItem> items, const uint32_t* tile_off, int rank, int hw, int nmodes,
                              cudaStream_t st);
 

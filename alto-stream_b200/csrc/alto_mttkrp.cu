@@ -1505,7 +1505,8 @@ static uint32_t chunk_tiles_for(uint32_t ntiles, unsigned grid) {
 // of every lane group of a block).
 constexpr uint32_t kWalkTile = 4096;
 constexpr uint32_t kDetTile = 16384;  // (a deterministic tile ends in a barrier)
-constexpr unsigned kDetSms = 148;     // (a constant: the cut must not depend on the device)
+constexpr unsigned kDetSms = 144;     // (a constant: the cut must not depend on the device; a few SMs left
+                                      // for what runs beside the walk in a stream group)
 static void even_tiles(MttkrpArgs* a, unsigned grid, uint32_t unit, uint32_t most = kWalkTile) {
   if (!a->nnz) {
     a->ntiles = 0;
@@ -1957,11 +1958,15 @@ static alto_status det_group_nm(Strided<DetItem> items, const uint32_t* tile_off
     if (blocks_per_sm < 1) blocks_per_sm = 1;
   }
   const unsigned sm = (unsigned)num_sms();
-  det_zero_group_kernel<<<sm * 4, 256, 0, st>>>(items);
-  ALTO_LAUNCHED();
   det_tile_group_kernel<R, NIN><<<sm * blocks_per_sm, kMttkrpThreads, 0, st>>>(items, tile_off);
   ALTO_LAUNCHED();
   det_fix_group_kernel<<<sm * 8, 256, 0, st>>>(items, R);
+  ALTO_LAUNCHED();
+  return ALTO_OK;
+}
+
+alto_status det_group_zero(Strided<DetItem> items, cudaStream_t st) {
+  det_zero_group_kernel<<<(unsigned)num_sms() * 4, 256, 0, st>>>(items);
   ALTO_LAUNCHED();
   return ALTO_OK;
 }

@@ -899,7 +899,7 @@ struct SlotDesc {
   double eps;
   int con;        // 1: non-negative ADMM solves
   int max_inner;
-  int act;        // runs the current step (set on the device)
+  int act;        // runs the current step (set on the device, before the loop and at each step's end)
   int admm_act;   // its ADMM of the current mode still sweeps (set on the device)
 };
 
@@ -946,13 +946,13 @@ __global__ void group_begin_kernel(SlotDesc* __restrict__ tab, GroupCtl* __restr
                                    cudaGraphConditionalHandle h) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   bool any = false;
-  for (int s = 0; s < ctl->count; ++s) any = any || slot_runnable(tab[s]);
+  for (int s = 0; s < ctl->count; ++s) {
+    const bool run = slot_runnable(tab[s]);
+    tab[s].act = run ? 1 : 0;
+    any = any || run;
+  }
   ctl->steps = 0;
   cudaGraphSetConditional(h, (any && ctl->limit > 0) ? 1u : 0u);
-}
-
-__global__ void group_step_begin_kernel(SlotDesc* __restrict__ tab, const GroupCtl* __restrict__ ctl) {
-  for (int s = threadIdx.x; s < ctl->count; s += blockDim.x) tab[s].act = slot_runnable(tab[s]) ? 1 : 0;
 }
 
 __global__ void __launch_bounds__(256) group_time_update_kernel(const SlotDesc* __restrict__ tab,
@@ -992,8 +992,8 @@ __global__ void __launch_bounds__(kAdmmThreads, TileMap<R>::kMinBlocks)
   }
 }
 
-// The ADMM chunk loop goes on while some slot's ADMM of mode j sweeps
-// (first: before the loop, which resets the chunk count).
+// After a chunk of ADMM sweeps (first: the one every mode starts with): the
+// chunk loop goes on while some slot's ADMM of mode j sweeps.
 __global__ void group_admm_cond_kernel(SlotDesc* __restrict__ tab, GroupCtl* __restrict__ ctl,
                                        cudaGraphConditionalHandle h, int first) {
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
@@ -1003,7 +1003,7 @@ __global__ void group_admm_cond_kernel(SlotDesc* __restrict__ tab, GroupCtl* __r
     if (d.act && d.admm_act && d.admm->stop) d.admm_act = 0;
     any = any || (d.act && d.admm_act);
   }
-  ctl->chunks = first ? 0 : ctl->chunks + 1;
+  ctl->chunks = first ? 1 : ctl->chunks + 1;
   if (any && ctl->chunks >= kAdmmChunkBound) {
     ctl->error = 1;
     any = false;
@@ -1038,6 +1038,7 @@ __global__ void group_converge_kernel(SlotDesc* __restrict__ tab, GroupCtl* __re
     SlotDesc& d = tab[s];
     if (d.act) converge_step(d.dstat, N, t, d.status, d.con, d.eps, d.max_inner, d.iter, 0);
     const bool run = slot_runnable(d);
+    d.act = run ? 1 : 0;  // in the next step
     out[s] = SlotState{run ? 1 : 0, d.iter->done, d.iter->stop, d.iter->info};
     any = any || run;
   }
@@ -1678,8 +1679,11 @@ namespace alto {
 struct StreamGroup {
   int R = 0, N = 0, t = 0, cap = 0, count = 0;
   int hw[ALTO_MAX_MODES] = {0};
+  // the members' solves: a group of one session has its kind, others take both
+  bool solves = true, admm = true;
   cudaStream_t st = nullptr;
-  cudaStream_t capst[2] = {nullptr, nullptr};
+  cudaStream_t capst[3] = {nullptr, nullptr, nullptr};  // the step, loop bodies, what runs beside the step
+  cudaEvent_t fork = nullptr, join = nullptr;
   DevBuf tab, offs, ctl, states;
   SlotDesc* h_tab = nullptr;  // pinned staging of the table and the offsets
   uint32_t* h_offs = nullptr;
@@ -1717,20 +1721,28 @@ alto_status capture_mode_solves(StreamGroup* g, cudaStream_t cs, int j, cudaGrap
   SlotDesc* tab = g->tab.as<SlotDesc>();
   GroupCtl* ctl = g->ctl.as<GroupCtl>();
   uint32_t* offs = g->offs.as<uint32_t>();
-  group_solve_kernel<R><<<kSolveGrid, kAdmmThreads, smem, cs>>>(tab, ctl, off_of(offs, g->cap, kOffSolve, j), j);
-  ALTO_LAUNCHED();
-  // while some slot's ADMM of mode j sweeps: one chunk (pass 1, pass 2)
-  group_admm_cond_kernel<<<1, 32, 0, cs>>>(tab, ctl, h, 1);
+  if (g->solves) {
+    group_solve_kernel<R><<<kSolveGrid, kAdmmThreads, smem, cs>>>(tab, ctl, off_of(offs, g->cap, kOffSolve, j), j);
+    ALTO_LAUNCHED();
+  }
+  if (!g->admm) return ALTO_OK;
+  const double tol = (double)1e-6f;
+  const uint32_t* ao = off_of(offs, g->cap, kOffAdmm, j);
+  // the first chunk in line (most solves stop within it, and entering a loop
+  // body costs 12 us), then while some slot's ADMM of mode j sweeps: one chunk
+  // (pass 1, pass 2)
+  auto chunk = [&](cudaStream_t st, int first) {
+    group_admm_kernel<R, true><<<kAdmmGrid, kAdmmThreads, smem, st>>>(tab, ctl, ao, j, tol);
+    group_admm_kernel<R, false><<<kAdmmGrid, kAdmmThreads, smem, st>>>(tab, ctl, ao, j, tol);
+    group_admm_cond_kernel<<<1, 32, 0, st>>>(tab, ctl, h, first);
+  };
+  chunk(cs, 1);
   ALTO_LAUNCHED();
   cudaGraph_t body;
   ALTO_TRY(capture_while(cs, h, &body));
   ALTO_TRY_CUDA(cudaStreamBeginCaptureToGraph(g->capst[1], body, nullptr, nullptr, 0,
                                               cudaStreamCaptureModeThreadLocal));
-  const double tol = (double)1e-6f;
-  const uint32_t* ao = off_of(offs, g->cap, kOffAdmm, j);
-  group_admm_kernel<R, true><<<kAdmmGrid, kAdmmThreads, smem, g->capst[1]>>>(tab, ctl, ao, j, tol);
-  group_admm_kernel<R, false><<<kAdmmGrid, kAdmmThreads, smem, g->capst[1]>>>(tab, ctl, ao, j, tol);
-  group_admm_cond_kernel<<<1, 32, 0, g->capst[1]>>>(tab, ctl, h, 0);
+  chunk(g->capst[1], 0);
   const cudaError_t le = cudaGetLastError();
   cudaGraph_t done = nullptr;
   const cudaError_t ee = cudaStreamEndCapture(g->capst[1], &done);
@@ -1745,7 +1757,11 @@ alto_status capture_solves(StreamGroup* g, cudaStream_t cs, int j, cudaGraphCond
   return capture_mode_solves<32>(g, cs, j, h);
 }
 
-// One inner iteration of every acting slot (the body of the step loop).
+// One inner iteration of every acting slot (the body of the step loop).  The
+// one-block set-up of a mode's solve needs the other modes' Grams only, and the
+// MTTKRP output is free again once a mode's solves have read it, so the set-ups run
+// beside the MTTKRPs and the clearing of the output beside the Gram passes
+// (10 us of 55 per mode at rank 32).
 alto_status capture_step(StreamGroup* g, cudaStream_t cs, cudaGraphConditionalHandle outer,
                          const cudaGraphConditionalHandle* admm_h) {
   const int N = g->N, t = g->t, R = g->R;
@@ -1753,27 +1769,52 @@ alto_status capture_step(StreamGroup* g, cudaStream_t cs, cudaGraphConditionalHa
   GroupCtl* ctl = g->ctl.as<GroupCtl>();
   uint32_t* offs = g->offs.as<uint32_t>();
   const unsigned per_slot = (unsigned)std::min(g->cap, 148);
-  group_step_begin_kernel<<<1, 256, 0, cs>>>(tab, ctl);
-  ALTO_LAUNCHED();
+  cudaStream_t beside = g->capst[2];
+  auto fork = [&]() -> alto_status {
+    ALTO_TRY_CUDA(cudaEventRecord(g->fork, cs));
+    ALTO_TRY_CUDA(cudaStreamWaitEvent(beside, g->fork, 0));
+    return ALTO_OK;
+  };
+  auto join = [&]() -> alto_status {
+    ALTO_TRY_CUDA(cudaEventRecord(g->join, beside));
+    ALTO_TRY_CUDA(cudaStreamWaitEvent(cs, g->join, 0));
+    return ALTO_OK;
+  };
+  auto items = [&](int m) { return strided<DetItem>(g, offsetof(SlotDesc, det) + m * sizeof(DetItem)); };
+  auto setup = [&](int m) {
+    return setup_group_launch(strided<SetupItem>(g, offsetof(SlotDesc, setup) + m * sizeof(SetupItem)), g->cap, R,
+                              beside);
+  };
   // time rows: MTTKRP of the stream mode, solve with the other Grams
-  ALTO_TRY(det_group_launch(strided<DetItem>(g, offsetof(SlotDesc, det) + t * sizeof(DetItem)),
-                            off_of(offs, g->cap, kOffTile, t), R, g->hw[t], N, cs));
-  ALTO_TRY(setup_group_launch(strided<SetupItem>(g, offsetof(SlotDesc, setup) + t * sizeof(SetupItem)), g->cap, R,
-                              cs));
+  ALTO_TRY(det_group_zero(items(t), cs));
+  ALTO_TRY(fork());
+  ALTO_TRY(setup(t));
+  ALTO_TRY(det_group_launch(items(t), off_of(offs, g->cap, kOffTile, t), R, g->hw[t], N, cs));
+  ALTO_TRY(join());
   group_time_update_kernel<<<per_slot, 256, 0, cs>>>(tab, ctl, t, R);
   ALTO_LAUNCHED();
+  bool cleared = false;  // the next mode's output is clear
   for (int j = 0; j < N; ++j) {
     if (j == t) continue;
-    ALTO_TRY(det_group_launch(strided<DetItem>(g, offsetof(SlotDesc, det) + j * sizeof(DetItem)),
-                              off_of(offs, g->cap, kOffTile, j), R, g->hw[j], N, cs));
-    group_mode_prep_kernel<<<per_slot, 256, 0, cs>>>(tab, ctl, j, t, N, R);
+    if (!cleared) ALTO_TRY(det_group_zero(items(j), cs));
+    ALTO_TRY(fork());
+    ALTO_TRY(setup(j));
+    group_mode_prep_kernel<<<per_slot, 256, 0, beside>>>(tab, ctl, j, t, N, R);
     ALTO_LAUNCHED();
-    ALTO_TRY(setup_group_launch(strided<SetupItem>(g, offsetof(SlotDesc, setup) + j * sizeof(SetupItem)), g->cap,
-                                R, cs));
+    ALTO_TRY(det_group_launch(items(j), off_of(offs, g->cap, kOffTile, j), R, g->hw[j], N, cs));
+    ALTO_TRY(join());
     ALTO_TRY(capture_solves(g, cs, j, admm_h[j]));
+    int next = j + 1;
+    if (next == t) ++next;
+    cleared = next < N;
+    if (cleared) {
+      ALTO_TRY(fork());
+      ALTO_TRY(det_group_zero(items(next), beside));
+    }
     ALTO_TRY(gram_group_launch(strided<GramItem>(g, offsetof(SlotDesc, gram) + j * sizeof(GramItem)),
                                off_of(offs, g->cap, kOffGram, j), off_of(offs, g->cap, kOffGramRed, j), g->cap, R,
                                cs));
+    if (cleared) ALTO_TRY(join());
   }
   group_converge_kernel<<<1, 32, 0, cs>>>(tab, ctl, g->states.as<SlotState>(), N, t, outer);
   ALTO_LAUNCHED();
@@ -1792,7 +1833,7 @@ alto_status build_group_graph(StreamGroup* g) {
                           __LINE__)))
       break;
     for (int j = 0; j < g->N && st == ALTO_OK; ++j)
-      if (j != g->t)
+      if (j != g->t && g->admm)
         st = cuda_status(cudaGraphConditionalHandleCreate(&admm_h[j], graph, 0, 0), "conditional handle", __FILE__,
                          __LINE__);
     if (st) break;
@@ -1856,6 +1897,7 @@ alto_status group_prepare_session(alto_stream_session* s) {
 
 bool group_fits(const StreamGroup* g, const alto_stream_session* s) {
   if (g->R != s->R || g->N != s->N || g->t != s->t) return false;
+  if (!(s->con == ALTO_UNCONSTRAINED ? g->solves : g->admm)) return false;
   for (int m = 0; m < s->N; ++m)
     if (g->hw[m] != s->det[m].hw) return false;
   return true;
@@ -1872,6 +1914,10 @@ alto_status group_create(const alto_stream_session* like, int capacity, cudaStre
   g->t = like->t;
   g->cap = capacity;
   g->st = st;
+  if (capacity == 1) {
+    g->solves = like->con == ALTO_UNCONSTRAINED;
+    g->admm = !g->solves;
+  }
   for (int m = 0; m < like->N; ++m) g->hw[m] = like->det[m].hw;
   const size_t offs_n = (size_t)kGroupOffKinds * ALTO_MAX_MODES * (capacity + 1);
   alto_status r = ALTO_OK;
@@ -1884,7 +1930,10 @@ alto_status group_create(const alto_stream_session* like, int capacity, cudaStre
       cudaMallocHost((void**)&g->h_offs, offs_n * 4) != cudaSuccess ||
       cudaMallocHost((void**)&g->h_ctl, sizeof(GroupCtl)) != cudaSuccess ||
       cudaStreamCreateWithFlags(&g->capst[0], cudaStreamNonBlocking) != cudaSuccess ||
-      cudaStreamCreateWithFlags(&g->capst[1], cudaStreamNonBlocking) != cudaSuccess) {
+      cudaStreamCreateWithFlags(&g->capst[1], cudaStreamNonBlocking) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&g->capst[2], cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&g->fork, cudaEventDisableTiming) != cudaSuccess ||
+      cudaEventCreateWithFlags(&g->join, cudaEventDisableTiming) != cudaSuccess) {
     group_destroy(g);
     set_error("group set-up failed: %s", cudaGetErrorString(cudaGetLastError()));
     return ALTO_ERR_CUDA;
@@ -1909,6 +1958,8 @@ void group_destroy(StreamGroup* g) {
   if (g->exec) cudaGraphExecDestroy(g->exec);
   for (cudaStream_t c : g->capst)
     if (c) cudaStreamDestroy(c);
+  if (g->fork) cudaEventDestroy(g->fork);
+  if (g->join) cudaEventDestroy(g->join);
   if (g->h_tab) cudaFreeHost(g->h_tab);
   if (g->h_offs) cudaFreeHost(g->h_offs);
   if (g->h_ctl) cudaFreeHost(g->h_ctl);
