@@ -750,11 +750,12 @@ struct TilePart {
 // The lane groups' open runs at the end of a chunk: when a whole warp ends on
 // one row (a hot row, or a mode of few rows) its groups are summed first, in
 // group order, and the row is updated once instead of once per group.  Groups
-// of G lanes; lanes past the last group hold zeros.
+// of G lanes; lanes past the last group, and groups without records (the ragged
+// end of a tile), hold zeros.
 template <int V>
 __device__ __forceinline__ bool merge_groups(uint32_t row, float (&acc)[V], int G, int npw, int lane) {
   const uint32_t row0 = __shfl_sync(0xffffffffu, row, 0);
-  if (!__all_sync(0xffffffffu, row == row0 || lane >= G * npw)) return false;
+  if (!__all_sync(0xffffffffu, row == row0 || row == kNoRow || lane >= G * npw)) return false;
   for (int g = 1; g < npw; ++g)
 #pragma unroll
     for (int q = 0; q < V; ++q) {
@@ -802,7 +803,7 @@ __device__ __forceinline__ void det_walk_chunk(const MttkrpArgs& a, uint32_t chu
   using C = WalkCfg<R, float, NIN, true>;
   using WM = WalkMap<R, float, C::V>;
   using DT = DetTile<R, WM::NPW>;
-  constexpr int E = DT::E, Q = DT::Q, kPerWarp = 2 * WM::NPW;
+  constexpr int E = DT::E, Q = DT::Q, kPerWarp = 2 * WM::NPW, kAhead = 4;
   __shared__ DT d;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int grp = lane / WM::G, sub = lane % WM::G;
@@ -824,7 +825,7 @@ __device__ __forceinline__ void det_walk_chunk(const MttkrpArgs& a, uint32_t chu
     run.open();
     const uint32_t ended = walk_range<R, float, NIN, C::V, C::U, C::D, true>(a, p.gs, p.ge, p.steps, sub, run, &d, ent);
     run.close();
-    const bool one = __all_sync(0xffffffffu, ended == 0 && run.row != kNoRow) &&
+    const bool one = __all_sync(0xffffffffu, ended == 0) &&
                      merge_groups<C::V>(run.row, run.acc, WM::G, WM::NPW, lane);
     if (lane == 0) d.one[warp] = one;
     if (run.row == kNoRow || (one && grp)) {
@@ -843,23 +844,38 @@ __device__ __forceinline__ void det_walk_chunk(const MttkrpArgs& a, uint32_t chu
       const uint32_t r = d.row[e];
       if (r == kNoRow) continue;
       int prev = e - 1;
+      if (prev >= 0 && d.one[prev / kPerWarp]) prev -= prev % kPerWarp;  // (a merged warp's one entry is its first)
       while (prev >= 0 && d.row[prev] == kNoRow) --prev;
       if (prev >= 0 && d.row[prev] == r) continue;  // not the first entry of its run
       float4 x = prev < 0 && open == r ? d.carry[cur][q] : make_float4(0.f, 0.f, 0.f, 0.f);
       bool ends = false;
-      for (int k = e; k < E; ++k) {
-        const uint32_t rk = d.row[k];
-        if (rk == kNoRow) continue;
-        if (rk != r) {
-          ends = true;
-          break;
+      // (a merged warp has one entry; of the others four are loaded at a time, or
+      // each would wait for the one before it: 90 cycles an entry, 12 us for a
+      // chunk of one row at rank 8)
+      for (int k = e; k < E && !ends;) {
+        const bool merged = d.one[k / kPerWarp];
+        const int stop = k - k % kPerWarp + kPerWarp;
+        uint32_t rk[kAhead];
+        float4 y[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+          const bool in = k + u < stop && (u == 0 || !merged);
+          rk[u] = in ? d.row[k + u] : kNoRow;
+          y[u] = d.val[min(k + u, E - 1)][q];
         }
-        const float4 y = d.val[k][q];
-        x.x += y.x;
-        x.y += y.y;
-        x.z += y.z;
-        x.w += y.w;
-        if (k % kPerWarp == 0 && d.one[k / kPerWarp]) k += kPerWarp - 1;
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+          if (ends || rk[u] == kNoRow) continue;
+          if (rk[u] != r) {
+            ends = true;
+            continue;
+          }
+          x.x += y[u].x;
+          x.y += y[u].y;
+          x.z += y[u].z;
+          x.w += y[u].w;
+        }
+        k = merged ? stop : min(k + kAhead, stop);
       }
       if (ends) {
         put(r, q, x);
@@ -894,30 +910,46 @@ __global__ void __launch_bounds__(kMttkrpThreads, 3) det_walk_kernel(const Mttkr
 
 // The chunks' slots (rows non-decreasing; a row in them is in no other run):
 // a block per run of equal rows, its slots summed with a fixed split and a fixed
-// tree, then written or added to the row.
-__device__ __forceinline__ void det_fix_slots(const MttkrpArgs& a, uint32_t nslots, int R, float4* part) {
+// tree, then written or added to the row.  What it waits for is one SM's loads
+// of a single row's slots (780 at rank 64: 15 us with the loads one after the
+// other, 8.9 us with eight in the air); 3 us when every row has a few slots.
+// Block `first` of `step` that share the item.
+__device__ __forceinline__ void det_fix_slots(const MttkrpArgs& a, uint32_t nslots, int R, float4* part,
+                                              uint32_t first, uint32_t step) {
   const uint32_t* rows = a.det_rows;
   const float4* vals = reinterpret_cast<const float4*>(a.det_vals);
   const int Q = R / 4, S = 256 / Q;
   const int s = threadIdx.x / Q, q = threadIdx.x % Q;
-  for (uint32_t i = blockIdx.x; i < nslots; i += gridDim.x) {
+  for (uint32_t i = first; i < nslots; i += step) {
     const uint32_t row = rows[i];
     if (i > 0 && rows[i - 1] == row) continue;
     uint32_t end = i + 1;
-    for (;;) {  // (the rows are sorted: the equal ones of a window come first)
-      const uint32_t k = end + threadIdx.x;
-      const int same = __syncthreads_count(k < nslots && rows[k] == row);
+    for (;;) {  // (the rows are sorted: the equal ones of a window of 1024 come first)
+      uint32_t next[4];
+#pragma unroll
+      for (uint32_t u = 0; u < 4; ++u) {
+        const uint32_t k = end + u * 256 + threadIdx.x;
+        next[u] = k < nslots ? rows[k] : ~row;
+      }
+      int same = 0;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) same += __syncthreads_count(next[u] == row);
       end += same;
-      if (same < 256) break;
+      if (same < 1024) break;
     }
     float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-    for (uint32_t k = i + s; k < end; k += S) {
-      const float4 y = vals[(size_t)k * Q + q];
-      x.x += y.x;
-      x.y += y.y;
-      x.z += y.z;
-      x.w += y.w;
+    for (uint32_t k = i + s; k < end; k += 8 * S) {  // (eight loads in the air)
+      float4 y[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        y[u] = k + u * S < end ? vals[(size_t)(k + u * S) * Q + q] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        x.x += y[u].x;
+        x.y += y[u].y;
+        x.z += y[u].z;
+        x.w += y[u].w;
+      }
     }
     part[threadIdx.x] = x;
     __syncthreads();
@@ -941,7 +973,7 @@ __device__ __forceinline__ void det_fix_slots(const MttkrpArgs& a, uint32_t nslo
 
 __global__ void __launch_bounds__(256) det_fix_kernel(const MttkrpArgs a, uint32_t nslots, int R) {
   __shared__ float4 part[256];
-  det_fix_slots(a, nslots, R, part);
+  det_fix_slots(a, nslots, R, part, blockIdx.x, gridDim.x);
 }
 
 // ------------------------------------------------ deterministic fix-up
@@ -1150,11 +1182,28 @@ __device__ __forceinline__ int item_of(const uint32_t* __restrict__ off, int K, 
   return lo;
 }
 
+// A grid's blocks split evenly among the items (several items per block when
+// there are more items than blocks): every block going through all the items is
+// a chain of dependent loads per item (the fix-up of four served slices of
+// 50,000 nonzeros: 11.4 us so, 7.1 us split).
+struct ItemShare {
+  uint32_t items, blocks;        // items; blocks per item
+  uint32_t item, block, stride;  // this block's first item, its place there, items between its items
+  __device__ __forceinline__ explicit ItemShare(int count) {
+    items = count > 0 ? (uint32_t)count : 0;
+    blocks = items ? max(gridDim.x / items, 1u) : 1;
+    stride = max(gridDim.x / blocks, 1u);
+    item = blockIdx.x / blocks;
+    block = blockIdx.x % blocks;
+    if (item >= stride) item = items;  // (the remainder of the split)
+  }
+};
+
 __global__ void __launch_bounds__(256) det_zero_group_kernel(Strided<DetItem> items) {
-  const int K = *items.count;
-  const uint64_t tid = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
-  const uint64_t nth = (uint64_t)gridDim.x * blockDim.x;
-  for (int s = 0; s < K; ++s) {
+  const ItemShare sh(*items.count);
+  const uint64_t tid = sh.block * (uint64_t)blockDim.x + threadIdx.x;
+  const uint64_t nth = (uint64_t)sh.blocks * blockDim.x;
+  for (uint32_t s = sh.item; s < sh.items; s += sh.stride) {
     const DetItem& it = items[s];
     if (!item_live(it.active)) continue;
     float4* o = reinterpret_cast<float4*>(it.a.out);
@@ -1193,11 +1242,11 @@ __global__ void __launch_bounds__(kMttkrpThreads, 3)
 
 __global__ void __launch_bounds__(256) det_fix_group_kernel(Strided<DetItem> items, int R) {
   __shared__ float4 part[256];
-  const int K = *items.count;
-  for (int s = 0; s < K; ++s) {
+  const ItemShare sh(*items.count);
+  for (uint32_t s = sh.item; s < sh.items; s += sh.stride) {
     const DetItem& it = items[s];
     if (!item_live(it.active)) continue;
-    det_fix_slots(it.a, it.nslots, R, part);
+    det_fix_slots(it.a, it.nslots, R, part, sh.block, sh.blocks);
   }
 }
 

@@ -679,6 +679,7 @@ __device__ __forceinline__ void time_update_body(const float* __restrict__ B32, 
     const uint64_t i = q / R;
     const int c = (int)(q % R);
     double x = 0.0;
+#pragma unroll 8
     for (int k = 0; k < R; ++k) x = __fma_rn((double)B32[i * R + k], W[k * R + c], x);
     time64[q] = x;
     U32[q] = (float)x;
@@ -992,17 +993,18 @@ __global__ void __launch_bounds__(kAdmmThreads, TileMap<R>::kMinBlocks)
   }
 }
 
-// After a chunk of ADMM sweeps (first: the one every mode starts with): the
+// (One warp, a lane per slot, as group_converge_kernel.)  After a chunk of ADMM sweeps (first: the one every mode starts with): the
 // chunk loop goes on while some slot's ADMM of mode j sweeps.
 __global__ void group_admm_cond_kernel(SlotDesc* __restrict__ tab, GroupCtl* __restrict__ ctl,
                                        cudaGraphConditionalHandle h, int first) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
   bool any = false;
-  for (int s = 0; s < ctl->count; ++s) {
+  for (int s = threadIdx.x; s < ctl->count; s += 32) {
     SlotDesc& d = tab[s];
     if (d.act && d.admm_act && d.admm->stop) d.admm_act = 0;
     any = any || (d.act && d.admm_act);
   }
+  any = __any_sync(0xffffffffu, any);
+  if (threadIdx.x != 0) return;
   ctl->chunks = first ? 1 : ctl->chunks + 1;
   if (any && ctl->chunks >= kAdmmChunkBound) {
     ctl->error = 1;
@@ -1032,9 +1034,8 @@ __global__ void __launch_bounds__(kAdmmThreads, TileMap<R>::kMinBlocks)
 // while a slot can run and the launch's step allowance lasts.
 __global__ void group_converge_kernel(SlotDesc* __restrict__ tab, GroupCtl* __restrict__ ctl,
                                       SlotState* __restrict__ out, int N, int t, cudaGraphConditionalHandle h) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
   bool any = false;
-  for (int s = 0; s < ctl->count; ++s) {
+  for (int s = threadIdx.x; s < ctl->count; s += 32) {
     SlotDesc& d = tab[s];
     if (d.act) converge_step(d.dstat, N, t, d.status, d.con, d.eps, d.max_inner, d.iter, 0);
     const bool run = slot_runnable(d);
@@ -1042,6 +1043,8 @@ __global__ void group_converge_kernel(SlotDesc* __restrict__ tab, GroupCtl* __re
     out[s] = SlotState{run ? 1 : 0, d.iter->done, d.iter->stop, d.iter->info};
     any = any || run;
   }
+  any = __any_sync(0xffffffffu, any);
+  if (threadIdx.x != 0) return;
   ctl->steps += 1;
   ctl->any = any ? 1 : 0;
   cudaGraphSetConditional(h, (any && ctl->steps < ctl->limit) ? 1u : 0u);
