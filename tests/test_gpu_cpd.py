@@ -75,3 +75,36 @@ def test_early_stop_matches_epsilon():
     _, _, fits, it = A.cpd_alto(t, U0, np.ones(R), R, 50, 1e-3)
     _, _, fo, ito = O.cpd_als(O.build(dims, cidx, vals), U0, np.ones(R), R, 50, 1e-3)
     assert it == ito
+
+
+@pytest.mark.parametrize("R", [1, 7, 9, 15, 17, 31, 33, 48, 63, 64, 65, 100])
+def test_ranks_around_the_column_tiles(R):
+    """Every width of the row solves, the set-up and the Grams; the module's
+    bound on fits is relative, so the data have a fit of about one half."""
+    rng = np.random.default_rng(R)
+    dims = np.array([150, 131, 160], np.uint64)
+    cidx = np.stack([rng.integers(0, int(d), 30000) for d in dims])
+    cidx = np.unique(cidx, axis=1).astype(np.uint64)
+    vals = (1.0 + rng.uniform(0, 1, cidx.shape[1])).astype(np.float32).astype(np.float64)
+    U0 = [u.astype(np.float32).astype(np.float64) for u in init_model(dims, R, R)]
+    t = A.create_alto(dims, cidx, vals)
+    U, lam, fits, it = A.cpd_alto(t, U0, np.ones(R), R, 4, 1e-12)
+    _, lo, fo, ito = O.cpd_als(O.build(dims, cidx, vals), U0, np.ones(R), R, 4, 1e-12)
+    assert it == ito
+    # a float32 MTTKRP is right to 1e-6; the fit is 1 - sqrt(y) with an error of y below 4e-6
+    np.testing.assert_allclose(fits, fo, rtol=0, atol=1e-5)
+
+
+def test_more_iterations_than_a_window_of_fits():
+    """Without a stopping test the fits are read back 64 at a time."""
+    dims = np.array([40, 50, 60], np.uint64)
+    cidx, vals = synth.uniform_coo(dims, 8000, seed=6)
+    vals = vals.astype(np.float32).astype(np.float64)
+    R = 2
+    U0 = [u.astype(np.float32).astype(np.float64) for u in init_model(dims, R, 3)]
+    t = A.create_alto(dims, cidx, vals)
+    _, _, fits, it = A.cpd_alto(t, U0, np.ones(R), R, 131, 0.0)
+    _, _, fo, ito = O.cpd_als(O.build(dims, cidx, vals), U0, np.ones(R), R, 131, 0.0)
+    assert it == ito == 131 and len(fits) == 131
+    # the bound of a single fit, in absolute terms, over the two factors' whole descent
+    np.testing.assert_allclose(fits, fo, rtol=0, atol=1e-4)

@@ -90,3 +90,25 @@ def test_large_one_million_nonzeros():
     cidx, vals = synth.uniform_coo(dims, 1000000, seed=55)
     t = A.create_alto(dims, cidx, vals, nprtn=8)
     check_same(t, dims, cidx, vals, 8)
+
+
+@pytest.mark.parametrize("dims", [[70001, 300, 1], [5000, 4000, 3000, 2000], [4097] * 8])
+@pytest.mark.parametrize("nnz", [1, 31, 33, 4095, 4096, 4097, 8193, 12289])
+def test_encoding_at_sort_tile_edges(dims, nnz):
+    """Sort tiles of 4096 elements, warps of 32, keys of one and two words, byte
+    tables with padding bits in every mode; then the row-sorted copies' 32-bit sorts
+    through an MTTKRP of integers, which is exact in any order."""
+    import torch
+
+    dims = np.array(dims, np.uint64)
+    rng = np.random.default_rng(nnz + len(dims))
+    cidx = np.stack([rng.integers(0, int(d), nnz) for d in dims]).astype(np.uint64)
+    vals = rng.integers(1, 4, nnz).astype(np.float64)
+    t = A.create_alto(dims, cidx, vals, nprtn=3)
+    check_same(t, dims, cidx, vals, 3)
+    for m in range(len(dims)):
+        F = [torch.ones((int(d), 8), device="cuda") for d in dims]
+        out = t.mttkrp(m, F, 8, variant=A.SORTED).cpu().numpy()
+        ref = np.zeros(int(dims[m]))
+        np.add.at(ref, cidx[m].astype(np.int64), vals)
+        assert np.array_equal(out, np.repeat(ref[:, None], 8, 1).astype(np.float32))

@@ -203,3 +203,27 @@ def test_cpd64_streaming_models(tmp_path, model, label):
     assert r.returncode == 0, r.stderr[-2000:]
     assert f"{label} (ALTO) on the GPU: 5 batches" in r.stdout
     assert "final fit error: " in r.stdout
+
+
+@pytest.mark.parametrize("R", [8, 12, 16, 32, 64])
+@pytest.mark.parametrize("nonneg", [0, 1])
+def test_ranks_of_the_tiled_solves(R, nonneg):
+    """Row solves and ADMM passes at every tile width and at a rank without
+    one, on rows that end inside a tile; 20011 rows of rank 8 and more are read
+    back in parallel.  Slices of R communities, so that the solves are well
+    conditioned and the module's bound holds."""
+    rng = np.random.default_rng(R)
+    dims = np.array([2, 20011, 301], np.uint64)
+    batches = []
+    for _ in range(3):
+        nnz = 60000
+        i = rng.integers(0, 20011, nnz)
+        k = rng.integers(0, 301 // R, nnz) * R + i % R
+        c = np.unique(np.stack([rng.integers(0, 2, nnz), i, k]), axis=1).astype(np.uint64)
+        v = rng.uniform(0.5, 1.5, c.shape[1]).astype(np.float32).astype(np.float64)
+        batches.append(dict(dims=dims, cidx=c, vals=v))
+    iv = synth.init_values(int(np.sum(dims)) * R + 8 * R, seed=R).astype(np.float32).astype(np.float64)
+    outs, _, _ = run_gpu(batches, R, 4, 0.0, nonneg, iv)
+    oo, _, _ = O.cpstream(batches, 0, R, 4, 0.0, nonneg, iv)
+    for a, c in zip(outs, oo):
+        assert normwise(a, c) <= 1e-4, normwise(a, c)
