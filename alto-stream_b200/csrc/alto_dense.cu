@@ -10,8 +10,8 @@
 //   cpd_fit_alto                             include/cpd.hpp:193-275
 //
 // Reductions are deterministic: every kernel that reduces over rows writes
-// per-block partials and a second, single-block kernel sums them in block
-// order.  The normal-equation solve forms the inverse of the Cholesky-
+// per-block partials and a second kernel, or the last block to finish, sums
+// them in block order.  The normal-equation solve forms the inverse of the Cholesky-
 // factored R x R matrix once (one CTA) and applies it to all I rows as a
 // float64 row-times-matrix product; the reference runs dpotrs over the rows.
 #include <algorithm>
@@ -45,9 +45,9 @@ static int sms() {
 // a warp reads each element once, with no shared memory, and a step of four
 // rows is T (T + 1) / 2 + T^2 products for 2 T loads (T = ceil(R / 8); G only
 // on and above the diagonal tiles).  Bound by the float64 rate from rank 32
-// (120,000 rows at rank 32: 11 us), by HBM below.  The form before staged the
-// rows in shared memory and read two doubles for every multiply-add (73 us
-// there; 93 us for 20,000 rows at rank 64).
+// (120,000 rows at rank 32: 12.5 us), by HBM below.  The form before staged the
+// rows in shared memory and read two doubles for every multiply-add (61 us
+// there; 109 us for 20,000 rows at rank 64, now 15).
 //
 // Up to rank 32 every warp of a block holds all tiles and takes its own rows;
 // above, the block's eight warps share the rows and warp w holds the tiles of
@@ -639,7 +639,8 @@ __global__ void solve_setup_kernel(const double* __restrict__ grams, int nmodes,
 // At RMAX 64 the two 32 x 32 diagonal blocks are factored so, and the rest of
 // L^-1 and W = L^-T L^-1 are float64 tensor-core products of the block.  One
 // thread per element with three to five barriers per column took 10.4 us at
-// rank 16, 40 us at rank 32 and (one column at a time) 192 us at rank 64.
+// rank 16, 40 us at rank 32 and (one column at a time) 192 us at rank 64; now 6, 10 and
+// 50 us.
 // Matrices smaller than RMAX are extended by the identity.
 
 // d += A B of one 8 x 8 tile over K (a multiple of 4): fa(i, k), fb(k, j) the
@@ -924,8 +925,8 @@ alto_status solve_setup(const double* grams, int nmodes, unsigned mask, int R, i
 // its columns' partial statistics and the last block to finish combines them in
 // block order, so no launch of its own waits for them.  Bound by latency at
 // CP-ALS's sizes: a shuffle per term and a one-block pass over every block's
-// statistics took 50 + 17 us for up to 20,000 rows at rank 64, 10 + 3 us for
-// 1000 rows at rank 16.
+// statistics took 50 + 17 us for up to 20,000 rows at rank 64 (now 14), 10 + 3 us
+// for 1000 rows at rank 16.
 constexpr int kApplyThreads = 256;
 
 template <int T>

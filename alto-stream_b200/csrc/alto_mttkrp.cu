@@ -8,8 +8,8 @@
 // Device design.  The line is cut into tiles of tile_nnz nonzeros (the
 // reference's partitions, sized for the GPU); a persistent grid, sized by
 // occupancy, walks the tiles, and each warp takes an equal chunk of a tile.
-// Inside a warp, G = R/8 lanes own one nonzero (each lane 8 consecutive rank
-// elements, two 16-byte loads per factor row), and the warp's chunk is split
+// Inside a warp, G lanes own one nonzero (each lane 4 rank elements, one 16-byte
+// load per factor row, or 8 in two loads: LaneWidth, WalkCfg), and the warp's chunk is split
 // into 32/G contiguous sub-ranges, one per lane group.  A group walks its
 // sub-range in line order, two nonzeros per iteration with all their keys,
 // values and factor rows loaded before any product is formed, and keeps the

@@ -20,19 +20,21 @@
 // |delta - prev_delta| < epsilon.  After the batch: G_t *= forgetting,
 // prev_U <- U, time rows appended.
 //
-// ADMM of a mode runs as three launches: a pass over the rows that runs all
-// 25 sweeps in registers and records every sweep's stopping-test sums, a
-// one-block kernel that picks the sweep count from them, and a second pass
-// that reruns that many sweeps and writes the result (admm_rows_kernel).
+// ADMM of a mode runs in chunks of up to three sweeps, each two passes over the
+// rows: the first runs the chunk's sweeps in registers and records every
+// sweep's stopping-test sums, its last block to finish picks the sweep count,
+// and the second reruns that many sweeps and writes the result (admm_tile_kernel;
+// admm_rows_kernel at ranks without column tiles).
 //
-// Launch structure.  The first inner iteration of a batch is issued
-// directly (it sizes every buffer and builds the row-sorted lines); the
-// remaining iterations run as one CUDA graph: a while node whose body is one
-// inner iteration, ending in a kernel that computes delta and decides on the
-// device whether to go on.  A batch costs one eager iteration, one capture
-// and one graph launch, with no host synchronisation between inner
-// iterations.  alto_stream_set_graph(s, 0) issues every iteration directly
-// instead (the same kernels in the same order: identical results).
+// Launch structure.  At ranks 8, 16 and 32 a batch's inner iterations are one
+// launch of a graph that a stream group keeps (StreamGroup, capture_step): a
+// while node whose body is one inner iteration of every member.  Otherwise the
+// first inner iteration of a batch is issued directly (it sizes every buffer and
+// builds the row-sorted lines) and the remaining ones run as a graph of the batch
+// (run_graph).  Both end an iteration in a kernel that computes delta and decides
+// on the device whether to go on, so there is no host synchronisation between
+// inner iterations.  alto_stream_set_graph(s, 0) issues every iteration directly
+// instead (the same arithmetic in the same order: identical results).
 #include <chrono>
 #include <cmath>
 #include <cstring>
@@ -387,9 +389,9 @@ __global__ void __launch_bounds__(kAdmmThreads)
 // with every per-row quantity in registers, and each row-times-matrix product
 // is tensor-core products in float64 (alto_dmma.cuh).  Bound by the float64 rate
 // at rank 32 and above (solve of 120,000 rows at rank 32: two products, 0.25 G
-// multiply-adds, 13 us) and by HBM below.  The FMA form it replaces staged each
-// product's input rows in shared memory between barriers (76 us there; an
-// ADMM pass over 100,000 rows at rank 16 50 us).
+// multiply-adds, 12 us) and by HBM below.  The FMA form before staged each
+// product's input rows in shared memory between barriers (38 us there; the two
+// ADMM passes over 100,000 rows at rank 16 44 and 34 us, now 21 and 11).
 template <int R>
 struct TileMap {
   static constexpr int T = R / 8;                             // column tiles
