@@ -20,6 +20,7 @@ namespace {
 struct HandlePool {
   cudaMemPool_t pool = nullptr;
   cudaStream_t st = nullptr;
+  void* hold = nullptr;  // keeps the slab that device_idle allocates from
 };
 HandlePool* handle_pool(int dev) {
   static std::mutex mu;
@@ -41,6 +42,7 @@ HandlePool* handle_pool(int dev) {
     }
     uint64_t keep = kPoolKeep;
     cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+    if (cudaMalloc(&h.hold, 256) != cudaSuccess) cudaGetLastError();  // (device_idle works without)
     h.st = st;
     h.pool = p;
   }
@@ -48,21 +50,34 @@ HandlePool* handle_pool(int dev) {
 }
 }  // namespace
 
+// Waits for everything on the device, as freeing a buffer of its own does:
+// cudaFree of a small allocation (3 us, its slab being held by h.hold; 0.65 ms
+// otherwise).  cudaDeviceSynchronize would end another thread's stream capture,
+// whatever its mode; cudaMalloc and cudaFree only concern captures in global mode.
+static bool device_idle() {
+  void* d = nullptr;
+  if (cudaMalloc(&d, 256) == cudaSuccess) return cudaFree(d) == cudaSuccess;
+  cudaGetLastError();
+  return cudaDeviceSynchronize() == cudaSuccess;
+}
+
 cudaError_t pool_alloc(void** p, size_t bytes, int* dev) {
   *p = nullptr;
   cudaError_t e = cudaGetDevice(dev);
   if (e != cudaSuccess) return e;
   HandlePool* h = handle_pool(*dev);
   if (!h) return cudaErrorMemoryAllocation;
-  e = cudaMallocFromPoolAsync(p, bytes, h->pool, h->st);
+  const bool pooled = bytes <= kPoolMost;
+  if (!pooled) *dev = -1;
+  e = pooled ? cudaMallocFromPoolAsync(p, bytes, h->pool, h->st) : cudaMalloc(p, bytes);
   if (e == cudaErrorMemoryAllocation) {  // what the pool keeps may be in the way, in other sizes
     cudaGetLastError();
-    cudaDeviceSynchronize();
+    device_idle();
     cudaMemPoolTrimTo(h->pool, 0);
-    e = cudaMallocFromPoolAsync(p, bytes, h->pool, h->st);
+    e = pooled ? cudaMallocFromPoolAsync(p, bytes, h->pool, h->st) : cudaMalloc(p, bytes);
     if (e != cudaSuccess) cudaGetLastError();
   }
-  if (e != cudaSuccess) return e;
+  if (e != cudaSuccess || !pooled) return e;
   e = cudaStreamSynchronize(h->st);  // usable on every stream from here on
   if (e != cudaSuccess) {
     cudaFreeAsync(*p, h->st);
@@ -77,8 +92,7 @@ void pool_free(void* p, int dev) {
   int cur = dev;
   cudaGetDevice(&cur);
   if (cur != dev) cudaSetDevice(dev);
-  cudaDeviceSynchronize();
-  cudaFreeAsync(p, h->st);
+  if (device_idle()) cudaFreeAsync(p, h->st);  // (else this thread captures: kept, as cudaFree would refuse it)
   if (cur != dev) cudaSetDevice(cur);
 }
 

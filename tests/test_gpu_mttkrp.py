@@ -373,3 +373,30 @@ def test_shards_sum_to_the_whole(nparts):
         ref = whole.mttkrp(m, Fd, R).cpu().numpy()
         tot = sum(p.mttkrp(m, Fd, R, variant=v).cpu().numpy() for p in parts for v in (A.AUTO,))
         assert rel_err(tot, ref) <= 1e-5
+
+
+def test_freeing_a_tensor_leaves_another_threads_capture():
+    """Destroying a handle waits for the device; a capture that another thread
+    has under way (not in global mode) goes on."""
+    import threading
+
+    import torch
+
+    dims = np.array([50, 60, 70], np.uint64)
+    cidx, vals = synth.uniform_coo(dims, 5000, seed=1)
+    t = A.create_alto(dims, cidx, vals)
+    x = torch.zeros(1000, device="cuda")
+    x.add_(1.0)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, capture_error_mode="thread_local"):
+        x.add_(1.0)
+        held = [t]
+        del t
+        th = threading.Thread(target=held.clear)
+        th.start()
+        th.join()
+        x.add_(1.0)
+    g.replay()
+    torch.cuda.synchronize()
+    assert float(x.sum()) == 3000.0
