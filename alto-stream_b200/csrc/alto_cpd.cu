@@ -167,11 +167,19 @@ static alto_status als_variant(alto_tensor* t, int mode, int rank, alto_dtype fd
     }
     ALTO_TRY(s);
   }
-  // (with long runs the deterministic walk: its sums are split in short chains
-  // and fixed trees, error 1.4e-7 against 3.3e-7 with atomics there, for 5% of the
-  // walk; a short walk would take half as long again for its fix-up)
-  *variant = deterministic_supported(rank, fdtype) && t->nnz >= (2u << 20) ? ALTO_MTTKRP_DETERMINISTIC
-                                                                             : ALTO_MTTKRP_SORTED;
+  // Where a row's run is long the atomics' partial sums make the walk's error, and
+  // the deterministic walk splits it in short chains and fixed trees (power law,
+  // three modes of 5000: 394,950 nonzeros at rank 64, worst factor's error 3.6e-6
+  // with atomics against 7.2e-7, six iterations 4.34 ms against 4.46; 1,578,155 at
+  // rank 8 6.1e-6 against 1.4e-6, 2.01 ms against 2.31).  Without long runs both
+  // are equal (uniform, 3.5e-7 and 3.7e-7), and its fix-up costs a short walk more
+  // (1000^3, 1M nonzeros, 20 iterations at rank 16: 2.90 ms against 3.42) than a long
+  // one (5%), whose error it still lowers.
+  *variant = ALTO_MTTKRP_SORTED;
+  if (!deterministic_supported(rank, fdtype)) return ALTO_OK;
+  bool det = t->nnz >= (2u << 20);
+  if (!det) ALTO_TRY(sorted_long_runs(t, mode, &det, st));
+  if (det) *variant = ALTO_MTTKRP_DETERMINISTIC;
   return ALTO_OK;
 }
 

@@ -1172,6 +1172,7 @@ alto_status build_sorted_line(alto_tensor* t, int mode, cudaStream_t st) {
   }
   s.ready = true;
   s.for_nnz = nnz;
+  s.long_runs = -1;
   return ALTO_OK;
 }
 

@@ -60,9 +60,14 @@ extern thread_local cudaStream_t tls_alloc_stream;
 // never handed out again while work on any stream may still touch it.  The pool
 // keeps up to kPoolKeep bytes of freed memory for later allocations and gives
 // the rest back to the driver (cudaMalloc and cudaFree cost 0.40 and 0.35 ms
-// each here whatever the size, pool_alloc and pool_free 4 us: encoding a tensor
+// each here whatever the size, pool_alloc and pool_free 4 and 7 us: encoding a tensor
 // of 8M nonzeros and three row-sorted copies of it spent half its time in them).
+// Buffers above kPoolMost are cudaMalloc's own: past kPoolKeep the pool unmaps and
+// maps memory again, which costs more than cudaMalloc does (creating a tensor of 40M
+// nonzeros 23 ms all pooled, 14.5 with cudaMalloc alone, 10 so; destroying it 13, 5.4
+// and 4.5 ms; of 8M 2.0 and 0.1 ms pooled, 4.2 and 2.3 with cudaMalloc).
 constexpr uint64_t kPoolKeep = 2ull << 30;
+constexpr uint64_t kPoolMost = 512ull << 20;
 cudaError_t pool_alloc(void** p, size_t bytes, int* dev);
 void pool_free(void* p, int dev);
 
@@ -70,7 +75,7 @@ void pool_free(void* p, int dev);
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
-  int pool_dev = -1;  // device of the library's pool it came from (-1: cudaMallocAsync)
+  int pool_dev = -1;  // device of the library's pool it came from (-1: cudaMallocAsync or cudaMalloc)
   DevBuf() = default;
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
@@ -270,6 +275,7 @@ struct SortedLine {
   uint32_t ntiles = 0;
   uint64_t for_nnz = 0;
   bool ready = false;
+  int long_runs = -1;  // sorted_long_runs of this copy (-1: not looked for)
 };
 
 // Tuned MTTKRP choice per (mode, rank, factor dtype).
@@ -381,6 +387,11 @@ bool mttkrp_tuned(const alto_tensor* t, int mode, int rank, alto_dtype fdtype);
 // Whether ALTO_MTTKRP_DETERMINISTIC runs for this rank and factor type.
 bool deterministic_supported(int rank, alto_dtype fdtype);
 // Build the per-mode row-sorted copy of the line.
+// Whether some row of mode `mode`'s decoded copy holds more than kLongRun
+// nonzeros (every row of 2 kLongRun or more is found, none below kLongRun + 1).
+// Waits for the stream the first time.
+constexpr uint32_t kLongRun = 4096;
+alto_status sorted_long_runs(alto_tensor* t, int mode, bool* found, cudaStream_t st);
 alto_status build_sorted_line(alto_tensor* t, int mode, cudaStream_t st);
 // Measure the variants per mode and record the fastest (synchronous).
 alto_status autotune(alto_tensor* t, const void* const* factors, alto_dtype fdtype, int rank,

@@ -2043,6 +2043,37 @@ alto_status det_group_launch(Strided<DetItem> items, const uint32_t* tile_off, i
   return ALTO_ERR_UNSUPPORTED;
 }
 
+// One block: whether two records kLongRun apart, kLongRun * k and the next, have
+// one row (nnz / kLongRun reads).
+template <int NIN>
+__global__ void __launch_bounds__(256)
+    long_run_kernel(const void* __restrict__ line, const void* __restrict__ extra, uint64_t nnz, int* __restrict__ found) {
+  int any = 0;
+  for (uint64_t i = (uint64_t)threadIdx.x * kLongRun; i + kLongRun < nnz; i += 256ull * kLongRun)
+    any |= load_dec<NIN>(line, extra, (uint32_t)i).row == load_dec<NIN>(line, extra, (uint32_t)(i + kLongRun)).row;
+  any = __syncthreads_or(any);
+  if (threadIdx.x == 0) *found = any;
+}
+
+alto_status sorted_long_runs(alto_tensor* t, int mode, bool* found, cudaStream_t st) {
+  SortedLine& s = t->sorted[mode];
+  if (s.long_runs < 0) {
+    DevBuf flag;
+    ALTO_TRY(flag.ensure(sizeof(int)));
+    const void *line = s.line.p, *extra = s.extra.p;
+    if (t->nmodes == 3) long_run_kernel<2><<<1, 256, 0, st>>>(line, extra, t->nnz, flag.as<int>());
+    if (t->nmodes == 4) long_run_kernel<3><<<1, 256, 0, st>>>(line, extra, t->nnz, flag.as<int>());
+    if (t->nmodes == 5) long_run_kernel<4><<<1, 256, 0, st>>>(line, extra, t->nnz, flag.as<int>());
+    ALTO_LAUNCHED();
+    int any = 0;
+    ALTO_TRY_CUDA(cudaMemcpyAsync(&any, flag.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    ALTO_TRY_CUDA(cudaStreamSynchronize(st));
+    s.long_runs = any;
+  }
+  *found = s.long_runs != 0;
+  return ALTO_OK;
+}
+
 // Time every applicable variant once per mode (after one warm run) into a
 // scratch output and record the fastest for ALTO_MTTKRP_AUTO.  Synchronous;
 // not for use inside stream capture.

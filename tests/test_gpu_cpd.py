@@ -108,3 +108,25 @@ def test_more_iterations_than_a_window_of_fits():
     assert it == ito == 131 and len(fits) == 131
     # the bound of a single fit, in absolute terms, over the two factors' whole descent
     np.testing.assert_allclose(fits, fo, rtol=0, atol=1e-4)
+
+
+@pytest.mark.parametrize("heavy", [4000, 4096, 4097, 8191, 8192, 8193, 20000])
+@pytest.mark.parametrize("nmodes", [3, 4, 5])
+def test_a_row_with_a_long_run(nmodes, heavy):
+    """One row of mode 0 holds `heavy` nonzeros: found for certain from 8192 on
+    (then that mode's walk is reproducible), right on either side."""
+    rng = np.random.default_rng(heavy + nmodes)
+    dims = np.array([60, 170, 150, 20, 10][:nmodes], np.uint64)
+    flat = rng.choice(170 * 150, heavy, replace=False)
+    rest = np.arange(170 * 59)
+    c = np.concatenate([np.stack([np.zeros(heavy, np.int64), flat % 170, flat // 170]),
+                        np.stack([1 + rest // 170, rest % 170, rng.integers(0, 150, rest.size)])], axis=1)
+    c = np.concatenate([c, np.stack([rng.integers(0, int(d), c.shape[1]) for d in dims[3:]])]) if nmodes > 3 else c
+    c = c.astype(np.uint64)
+    vals = (1.0 + rng.uniform(0, 1, c.shape[1])).astype(np.float32).astype(np.float64)
+    R = 8
+    U0 = [u.astype(np.float32).astype(np.float64) for u in init_model(dims, R, 3)]
+    t = A.create_alto(dims, c, vals)
+    U, lam, fits, it = A.cpd_alto(t, U0, np.ones(R), R, 4, 0.0)
+    _, _, fo, _ = O.cpd_als(O.build(dims, c, vals), U0, np.ones(R), R, 4, 0.0)
+    np.testing.assert_allclose(fits, fo, rtol=0, atol=1e-5)
