@@ -39,6 +39,7 @@
 #include <cmath>
 #include <cstring>
 #include <exception>
+#include <mutex>
 #include <thread>
 #include <vector>
 
@@ -1091,8 +1092,10 @@ struct alto_stream_session {
   uint64_t pushes = 0, inner_total = 0;
   cudaEvent_t inner_ev[2] = {nullptr, nullptr};
   // pinned staging of the new model rows (grown geometrically; the
-  // previous push's copies out of it are complete when a push starts)
+  // previous push's copies out of it are complete when a push starts), and
+  // the lock of the threads that read factors through it
   float* pin_rows = nullptr;
+  std::mutex pin_mu;
   size_t pin_cap = 0;
   ~alto_stream_session() {
     alto::group_destroy(own_group);
@@ -2539,6 +2542,7 @@ bool stream_group_key_equal(const alto_stream_session* a, const alto_stream_sess
 // eight), so a large factor is widened by several threads.
 static alto_status factor_to_host(alto_stream_session* s, int mode, uint64_t n, double* host_out) {
   constexpr uint64_t kParallel = 1u << 17;  // values below which one thread is as fast
+  std::lock_guard<std::mutex> lk(s->pin_mu);  // (factors of one session may be read by several threads)
   std::vector<float> own;
   float* stage = s->pin_rows;
   uint64_t cap = s->pin_cap;

@@ -227,3 +227,34 @@ def test_ranks_of_the_tiled_solves(R, nonneg):
     oo, _, _ = O.cpstream(batches, 0, R, 4, 0.0, nonneg, iv)
     for a, c in zip(outs, oo):
         assert normwise(a, c) <= 1e-4, normwise(a, c)
+
+
+def test_factors_read_by_several_threads():
+    """Threads that read factors of one session at once each get their mode's
+    values (they share the session's pinned staging): the values that reading
+    one mode after the other gives, at sizes read back by one thread and by
+    several."""
+    import threading
+
+    R = 16
+    dims = np.array([1, 30011, 20011, 301], np.uint64)
+    rng = np.random.default_rng(2)
+    c = np.stack([np.zeros(20000, np.int64)] + [rng.integers(0, int(d), 20000) for d in dims[1:]]).astype(np.uint64)
+    c = np.unique(c, axis=1)
+    v = rng.uniform(0.5, 1.5, c.shape[1])
+    s = A.CPStream(4, 0, R, max_inner=2, epsilon=0.0)
+    s.push(dims, c, v, synth.init_values(int(dims.sum()) * R, seed=4))
+    want = {m: s.factor(m, int(dims[m])) for m in (1, 2, 3)}
+    bad = []
+
+    def reader(m):
+        for _ in range(30):
+            if not np.array_equal(s.factor(m, int(dims[m])), want[m]):
+                bad.append(m)
+
+    threads = [threading.Thread(target=reader, args=(m,)) for m in (1, 2, 3, 1)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
