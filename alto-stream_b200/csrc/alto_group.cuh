@@ -34,6 +34,7 @@ struct MttkrpArgs {
   LineDecode dec;
   FactorSet fac;
   FactorSet in;  // the input modes' factors in mode order (kDecoded walks)
+  uint64_t in_rows;  // their rows
   float* out;
 };
 

@@ -712,11 +712,16 @@ __device__ __forceinline__ uint32_t walk_range(const MttkrpArgs& a, uint32_t gs,
 // 12M nonzeros: float32 631 us against 645, bfloat16 494 against 541) and worse
 // at rank 16 and 32 (power-law 3-mode, 40M nonzeros, rank 32: 936 us against
 // 809; uniform 1000^3, 1M nonzeros, rank 16: 27.6 against 21.5).  3 modes in
-// float32 wait for their rows (two loads a nonzero, the longest stall by far),
-// so a long walk keeps two steps in the air at three blocks an SM (40M
-// nonzeros: 769 us; one step at five blocks 802); a short one has its rows in
-// L2 and wants the blocks (5M: 124 us against 119; 20,000: 2.9 against 2.4),
-// and with more rows per nonzero two steps spill (2.1 ms against 0.63).
+// float32 wait for their rows (two loads a nonzero, the longest stall by far).
+// Rows from L2 want the blocks: one step in the air at five blocks an SM took
+// 3 to 15% less than two at three from 9M to 40M nonzeros at ranks 8, 16 and 32
+// (uniform, rows of 15 to 32 MB, 25M: 264 us against 288 at rank 16, 443 against
+// 474 at rank 32; 1000 rows, 40M, rank 16: 350 against 394; by at most 3% more,
+// 15M at rank 8).  Rows from memory are better asked for two steps ahead, or
+// as fast (40M distinct nonzeros over 4.8M x 1.8M x 1.8M, rank 32, three modes:
+// 2433 us against 2508 at the same error; power law, 15M, rank 16: 201 against
+// 223 and 213, but rank 8 121 against 118); with more rows per nonzero two steps
+// spill (2.1 ms against 0.63).
 template <int R, typename FT, int NIN, bool DET, bool DEEP = false>
 struct WalkCfg {
   static constexpr int V = R >= 64 ? 8 : 4;
@@ -724,8 +729,9 @@ struct WalkCfg {
   static constexpr int D = DEEP ? 2 : 1;
   static constexpr int MINB = DEEP ? 3 : NIN == 2 && V == 4 && !DET ? 5 : 4;
 };
-// Whether two steps in the air pay: 3 modes in float32 whose walk is long and
-// gathers from more than the L2 holds.
+// Whether two steps in the air pay: 3 modes in float32 whose walk is long
+// (kDeepNnz: 5M nonzeros 124 us against 119) and whose input factors are more
+// than the L2 holds (launch_walk).
 template <int R, typename FT, int NIN>
 constexpr bool kCanBeDeep = NIN == 2 && R < 64 && sizeof(FT) == 4;
 constexpr uint32_t kDeepNnz = 8u << 20;
@@ -1536,6 +1542,17 @@ static int num_sms() {
   return g_num_sms;
 }
 
+static uint64_t l2_bytes() {
+  static int bytes = 0;
+  if (!bytes) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&bytes, cudaDevAttrL2CacheSize, dev);
+    if (bytes <= 0) bytes = 126 << 20;
+  }
+  return (uint64_t)bytes;
+}
+
 // Tiles per chunk of the direct walks: up to kChunkTilesMax, keeping at
 // least kChunksPerBlock chunks per block so the round robin still balances
 // the blocks.
@@ -1556,16 +1573,32 @@ constexpr uint32_t kWalkTile = 4096;
 constexpr uint32_t kDetTile = 16384;  // (a deterministic tile ends in a barrier)
 constexpr unsigned kDetSms = 144;     // (a constant: the cut must not depend on the device; a few SMs left
                                       // for what runs beside the walk in a stream group)
-static void even_tiles(MttkrpArgs* a, unsigned grid, uint32_t unit, uint32_t most = kWalkTile) {
-  if (!a->nnz) {
-    a->ntiles = 0;
-    return;
-  }
+static uint64_t tile_rounds(const MttkrpArgs& a, unsigned grid, uint32_t most) {  // tiles of a block
   const uint64_t wave = (uint64_t)grid * most;
-  const uint64_t rounds = std::max<uint64_t>(((uint64_t)a->nnz + wave - 1) / wave, 1);
+  return std::max<uint64_t>(((uint64_t)a.nnz + wave - 1) / wave, 1);
+}
+static void cut_tiles(MttkrpArgs* a, unsigned grid, uint32_t unit, uint64_t rounds) {
   const uint64_t per = (a->nnz + grid * rounds - 1) / (grid * rounds);
   a->tile_nnz = (uint32_t)std::max<uint64_t>((per + unit - 1) / unit * unit, unit);
   a->ntiles = (uint32_t)(((uint64_t)a->nnz + a->tile_nnz - 1) / a->tile_nnz);
+}
+static void even_tiles(MttkrpArgs* a, unsigned grid, uint32_t unit, uint32_t most = kWalkTile) {
+  cut_tiles(a, grid, unit, tile_rounds(*a, grid, most));
+}
+// The same with the blocks' tiles in equal chunks of up to kChunkTilesMax, at
+// least `chunks` of them a block; returns the tiles of a chunk.  A hot row is
+// updated once per warp and chunk, so short chunks lengthen the chain of its
+// atomics, long ones the chains in registers.  Five of the walk with five blocks
+// an SM are as long as eight of the walk with three, whose error they keep; two
+// measured up to a sixth faster (4 modes, rank 16, 40M nonzeros: 495 us against
+// 584) with up to a fifth more error (1000 rows of 20,000: 2.7e-7 against 2.4e-7).
+static uint32_t even_chunks(MttkrpArgs* a, unsigned grid, uint32_t unit, uint32_t chunks) {
+  uint64_t rounds = tile_rounds(*a, grid, kWalkTile);
+  uint32_t c = kChunkTilesMax;
+  while (c > 1 && rounds < (uint64_t)c * chunks) c >>= 1;
+  rounds = (rounds + c - 1) / c * c;
+  cut_tiles(a, grid, unit, rounds);
+  return c;
 }
 
 template <int R, typename FT, int HW, bool STAGE, int NM>
@@ -1615,7 +1648,7 @@ static alto_status launch_tma(const MttkrpArgs& a, int* err, cudaStream_t st) {
 template <int R, typename FT, int NIN, bool DEEP = false>
 static alto_status launch_walk(const MttkrpArgs& a, cudaStream_t st) {
   if constexpr (kCanBeDeep<R, FT, NIN> && !DEEP)
-    if (a.nnz >= kDeepNnz) return launch_walk<R, FT, NIN, true>(a, st);
+    if (a.nnz >= kDeepNnz && a.in_rows * (R * sizeof(FT)) > l2_bytes()) return launch_walk<R, FT, NIN, true>(a, st);
   static int blocks_per_sm = 0;
   if (!blocks_per_sm) {
     // no shared memory: all of the unified L1 / shared storage as L1 (factor rows hit it)
@@ -1629,9 +1662,8 @@ static alto_status launch_walk(const MttkrpArgs& a, cudaStream_t st) {
   MttkrpArgs b = a;
   using C = WalkCfg<R, FT, NIN, false, DEEP>;
   const unsigned full = (unsigned)(num_sms() * blocks_per_sm);
-  even_tiles(&b, full, kMttkrpWarps * WalkMap<R, FT, C::V>::NPW * C::U);
+  b.chunk_tiles = even_chunks(&b, full, kMttkrpWarps * WalkMap<R, FT, C::V>::NPW * C::U, DEEP ? kChunksPerBlock : 5);
   const unsigned grid = std::min<unsigned>(b.ntiles, full);
-  b.chunk_tiles = chunk_tiles_for(b.ntiles, grid);
   walk_kernel<R, FT, NIN, DEEP><<<grid, kMttkrpThreads, 0, st>>>(b);
   ALTO_LAUNCHED();
   return ALTO_OK;
@@ -1887,9 +1919,12 @@ static alto_status fill_args(alto_tensor* t, int mode, const void* const* factor
   a.dec = t->dec;
   a.out = out;
   int j = 0;
+  a.in_rows = 0;
   for (int m = 0; m < t->nmodes; ++m) {
     a.fac.f[m] = factors[m];
-    if (m != mode) a.in.f[j++] = factors[m];
+    if (m == mode) continue;
+    a.in.f[j++] = factors[m];
+    a.in_rows += t->dims[m];
   }
   return ALTO_OK;
 }

@@ -345,6 +345,43 @@ def test_deterministic_accumulates_and_rejects_unsupported():
         t.mttkrp(0, [f.to(torch.bfloat16) for f in Fd], R, variant=A.DETERMINISTIC)
 
 
+# ------------------------------------------------------------ long walks
+
+def check_long(dims, nnz, R, variant, seed):
+    """Every mode's MTTKRP of nnz random nonzeros with positive values and
+    factors against float64 sums, element by element.  An output element is a
+    sum of positive products, so its relative error is at most the number of
+    float32 roundings on the way of a product to it: a few products, and fewer
+    than 1000 additions (a lane group's run, its meeting with the others', and
+    the block's or the atomics' chain), 2^-24 each."""
+    import torch
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    idx = [torch.randint(0, d, (nnz,), generator=g, device="cuda") for d in dims]
+    vals = torch.rand(nnz, generator=g, device="cuda") + 0.5
+    F = [torch.rand((d, R), generator=g, device="cuda") + 0.5 for d in dims]
+    t = A.create_alto(np.array(dims, np.uint64), idx, vals)
+    for m in range(len(dims)):
+        want = torch.zeros((dims[m], R), dtype=torch.float64, device="cuda")
+        for a in range(0, nnz, 1 << 21):
+            p = vals[a:a + (1 << 21)].double()[:, None].expand(-1, R)
+            for j in range(len(dims)):
+                if j != m:
+                    p = p * F[j][idx[j][a:a + (1 << 21)]].double()
+            want.index_add_(0, idx[m][a:a + (1 << 21)], p)
+        got = t.mttkrp(m, F, R, variant=variant).double()
+        assert bool(((got - want).abs() <= 1000 * 2.0 ** -24 * want).all()), m
+
+
+@pytest.mark.parametrize("nnz", [(8 << 20) - 1, 8 << 20, (8 << 20) + 1237])
+@pytest.mark.parametrize("dims,R", [([1200000, 40, 1100000], 32), ([3000, 40, 2000], 32), ([4200000, 7, 4300000], 8)])
+def test_long_sorted_walks(dims, R, nnz):
+    """Around the length from which a walk over input factors larger than L2
+    (first and last dims, every mode) has two steps of rows in the air."""
+    check_long(dims, nnz, R, A.SORTED, seed=nnz % 97)
+
+
 # ------------------------------------------------------------ shards
 
 @pytest.mark.parametrize("nparts", [1, 3, 8])
