@@ -382,6 +382,15 @@ def test_long_sorted_walks(dims, R, nnz):
     check_long(dims, nnz, R, A.SORTED, seed=nnz % 97)
 
 
+@pytest.mark.parametrize("dims,nnz", [([1, 5, 200000], 7100003), ([1, 5, 200000], 14200001),
+                                      ([9, 1, 300, 2000, 30000], 7100003)])
+def test_deterministic_chunks_of_several_tiles(dims, nnz):
+    """The deterministic walk's blocks have one tile each up to 7.08M nonzeros;
+    above, a block carries its open run from tile to tile: through all of them (a
+    mode of one row), through some (a few rows), and not at all (a long mode)."""
+    check_long(dims, nnz, 8, A.DETERMINISTIC, seed=len(dims))
+
+
 # ------------------------------------------------------------ shards
 
 @pytest.mark.parametrize("nparts", [1, 3, 8])
