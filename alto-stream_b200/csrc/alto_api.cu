@@ -17,10 +17,11 @@ static thread_local char g_err[512] = "";
 // The handles' pool of a device, and the stream its allocations and frees are
 // ordered on (nothing else runs there).
 namespace {
+constexpr size_t kGuardBytes = 256;
 struct HandlePool {
   cudaMemPool_t pool = nullptr;
   cudaStream_t st = nullptr;
-  void* hold = nullptr;  // keeps the slab that device_idle allocates from
+  void* hold = nullptr;  // keeps the slab that the guards are allocated from (0.65 ms a free otherwise, 3 us so)
 };
 HandlePool* handle_pool(int dev) {
   static std::mutex mu;
@@ -42,7 +43,7 @@ HandlePool* handle_pool(int dev) {
     }
     uint64_t keep = kPoolKeep;
     cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
-    if (cudaMalloc(&h.hold, 256) != cudaSuccess) cudaGetLastError();  // (device_idle works without)
+    if (cudaMalloc(&h.hold, kGuardBytes) != cudaSuccess) cudaGetLastError();  // (the guards work without)
     h.st = st;
     h.pool = p;
   }
@@ -50,50 +51,53 @@ HandlePool* handle_pool(int dev) {
 }
 }  // namespace
 
-// Waits for everything on the device, as freeing a buffer of its own does:
-// cudaFree of a small allocation (3 us, its slab being held by h.hold; 0.65 ms
-// otherwise).  cudaDeviceSynchronize would end another thread's stream capture,
-// whatever its mode; cudaMalloc and cudaFree only concern captures in global mode.
-static bool device_idle() {
-  void* d = nullptr;
-  if (cudaMalloc(&d, 256) == cudaSuccess) return cudaFree(d) == cudaSuccess;
-  cudaGetLastError();
-  return cudaDeviceSynchronize() == cudaSuccess;
-}
-
-cudaError_t pool_alloc(void** p, size_t bytes, int* dev) {
+cudaError_t pool_alloc(void** p, size_t bytes, PoolMem* m) {
   *p = nullptr;
-  cudaError_t e = cudaGetDevice(dev);
+  *m = PoolMem{};
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  HandlePool* h = handle_pool(*dev);
+  HandlePool* h = handle_pool(dev);
   if (!h) return cudaErrorMemoryAllocation;
   const bool pooled = bytes <= kPoolMost;
-  if (!pooled) *dev = -1;
-  e = pooled ? cudaMallocFromPoolAsync(p, bytes, h->pool, h->st) : cudaMalloc(p, bytes);
+  auto take = [&]() -> cudaError_t {
+    if (!pooled) return cudaMalloc(p, bytes);
+    if (!m->guard) {
+      const cudaError_t g = cudaMalloc(&m->guard, kGuardBytes);
+      if (g != cudaSuccess) return g;
+    }
+    return cudaMallocFromPoolAsync(p, bytes, h->pool, h->st);
+  };
+  e = take();
   if (e == cudaErrorMemoryAllocation) {  // what the pool keeps may be in the way, in other sizes
     cudaGetLastError();
-    device_idle();
+    cudaStreamSynchronize(h->st);
     cudaMemPoolTrimTo(h->pool, 0);
-    e = pooled ? cudaMallocFromPoolAsync(p, bytes, h->pool, h->st) : cudaMalloc(p, bytes);
-    if (e != cudaSuccess) cudaGetLastError();
+    e = take();
   }
-  if (e != cudaSuccess || !pooled) return e;
-  e = cudaStreamSynchronize(h->st);  // usable on every stream from here on
-  if (e != cudaSuccess) {
-    cudaFreeAsync(*p, h->st);
-    *p = nullptr;
+  if (e == cudaSuccess && pooled) {
+    e = cudaStreamSynchronize(h->st);  // usable on every stream from here on
+    if (e != cudaSuccess) cudaFreeAsync(*p, h->st);
   }
+  if (e == cudaSuccess) {
+    if (pooled) m->dev = dev;
+    return e;
+  }
+  if (m->guard) cudaFree(m->guard);
+  cudaGetLastError();  // (the error is the caller's status, not the next launch's)
+  *p = nullptr;
+  *m = PoolMem{};
   return e;
 }
 
-void pool_free(void* p, int dev) {
-  HandlePool* h = handle_pool(dev);
+void pool_free(void* p, const PoolMem& m) {
+  HandlePool* h = handle_pool(m.dev);
   if (!h) return;
-  int cur = dev;
+  int cur = m.dev;
   cudaGetDevice(&cur);
-  if (cur != dev) cudaSetDevice(dev);
-  if (device_idle()) cudaFreeAsync(p, h->st);  // (else this thread captures: kept, as cudaFree would refuse it)
-  if (cur != dev) cudaSetDevice(cur);
+  if (cur != m.dev) cudaSetDevice(m.dev);
+  if (cudaFree(m.guard) == cudaSuccess) cudaFreeAsync(p, h->st);  // (else this thread captures: kept)
+  if (cur != m.dev) cudaSetDevice(cur);
 }
 
 cudaMemPool_t transient_pool() {

@@ -56,26 +56,37 @@ extern thread_local cudaStream_t tls_alloc_stream;
 
 // Device memory for the handles' buffers, one pool per device, with the
 // semantics of cudaMalloc / cudaFree: what pool_alloc returns may be used on
-// any stream at once, and pool_free first waits for the device, so memory is
-// never handed out again while work on any stream may still touch it.  The pool
-// keeps up to kPoolKeep bytes of freed memory for later allocations and gives
-// the rest back to the driver (cudaMalloc and cudaFree cost 0.40 and 0.35 ms
-// each here whatever the size, pool_alloc and pool_free 4 and 7 us: encoding a tensor
-// of 8M nonzeros and three row-sorted copies of it spent half its time in them).
+// any stream at once, pool_free first waits for the device, so memory is never
+// handed out again while work on any stream may still touch it, and both are
+// refused where cudaMalloc and cudaFree are (a thread that captures a stream).
+// Each buffer has a guard for that, a small cudaMalloc allocation made with it:
+// whatever was launched while the buffer lived was launched while the guard did,
+// and freeing the guard synchronises the GPU with all of it, as cudaFree of the
+// buffer itself would.  (cudaDeviceSynchronize would end another thread's
+// capture, whatever its mode; cudaMalloc and cudaFree only concern captures in
+// global mode.)  The pool keeps up to kPoolKeep bytes of freed memory for later
+// allocations and gives the rest back to the driver (cudaMalloc and cudaFree cost
+// 0.40 and 0.35 ms each here whatever the size, pool_alloc and pool_free 5 and
+// 5 us: encoding a tensor of 8M nonzeros and three row-sorted copies of it spent
+// half its time in them).
 // Buffers above kPoolMost are cudaMalloc's own: past kPoolKeep the pool unmaps and
 // maps memory again, which costs more than cudaMalloc does (creating a tensor of 40M
 // nonzeros 23 ms all pooled, 14.5 with cudaMalloc alone, 10 so; destroying it 13, 5.4
 // and 4.5 ms; of 8M 2.0 and 0.1 ms pooled, 4.2 and 2.3 with cudaMalloc).
 constexpr uint64_t kPoolKeep = 2ull << 30;
 constexpr uint64_t kPoolMost = 512ull << 20;
-cudaError_t pool_alloc(void** p, size_t bytes, int* dev);
-void pool_free(void* p, int dev);
+struct PoolMem {
+  void* guard = nullptr;
+  int dev = -1;  // device of the pool (-1: cudaMalloc's own, no guard)
+};
+cudaError_t pool_alloc(void** p, size_t bytes, PoolMem* m);
+void pool_free(void* p, const PoolMem& m);
 
 // A growable device allocation owned by a handle.
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
-  int pool_dev = -1;  // device of the library's pool it came from (-1: cudaMallocAsync or cudaMalloc)
+  PoolMem pool;  // of the library's pool (dev -1: cudaMallocAsync or cudaMalloc)
   DevBuf() = default;
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
@@ -83,27 +94,27 @@ struct DevBuf {
   void swap(DevBuf& o) {
     std::swap(p, o.p);
     std::swap(bytes, o.bytes);
-    std::swap(pool_dev, o.pool_dev);
+    std::swap(pool, o.pool);
   }
   void release() {
     if (p) {
-      if (tls_alloc_stream)
+      if (pool.dev >= 0)
+        pool_free(p, pool);
+      else if (tls_alloc_stream)
         cudaFreeAsync(p, tls_alloc_stream);
-      else if (pool_dev >= 0)
-        pool_free(p, pool_dev);
       else
         cudaFree(p);
     }
     p = nullptr;
     bytes = 0;
+    pool = PoolMem{};
   }
   // Ensure at least n bytes; contents are not preserved on growth.
   alto_status ensure(size_t n) {
     if (n <= bytes && p) return ALTO_OK;
     release();
     size_t want = n < 256 ? 256 : n;
-    pool_dev = -1;
-    cudaError_t e = tls_alloc_stream ? cudaMallocAsync(&p, want, tls_alloc_stream) : pool_alloc(&p, want, &pool_dev);
+    cudaError_t e = tls_alloc_stream ? cudaMallocAsync(&p, want, tls_alloc_stream) : pool_alloc(&p, want, &pool);
     if (e != cudaSuccess) {
       p = nullptr;
       return cuda_status(e, "device allocation", __FILE__, __LINE__);

@@ -446,3 +446,73 @@ def test_freeing_a_tensor_leaves_another_threads_capture():
     g.replay()
     torch.cuda.synchronize()
     assert float(x.sum()) == 3000.0
+
+
+def long_tensor(seed):
+    """A tensor of 2M nonzeros and factors, the inputs of the tests below."""
+    import torch
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    dims = [3000, 2000, 1000]
+    idx = [torch.randint(0, d, (2000000,), generator=g, device="cuda") for d in dims]
+    vals = torch.rand(2000000, generator=g, device="cuda")
+    F = [torch.rand((d, 16), generator=g, device="cuda") for d in dims]
+    return np.array(dims, np.uint64), idx, vals, F
+
+
+def test_freeing_a_tensor_waits_for_work_on_other_streams():
+    """A tensor destroyed while another stream still walks it: the walks end
+    first, and what is then made in its memory does not reach them."""
+    import torch
+
+    dims, idx, vals, F = long_tensor(3)
+    _, other, vals2, _ = long_tensor(4)
+    side, third = torch.cuda.Stream(), torch.cuda.Stream()
+    results, ended = [], []
+    for early in (False, True):
+        t = A.create_alto(dims, idx, vals)
+        out = torch.zeros((int(dims[0]), 16), device="cuda")
+        t.mttkrp(0, F, 16, out=out, variant=A.DETERMINISTIC)  # (builds the row-sorted copy)
+        done = torch.cuda.Event()
+        torch.cuda.synchronize()
+        for _ in range(1500):  # about 0.1 s of device time, 0.02 s to queue
+            t.mttkrp(0, F, 16, out=out, accumulate=True, variant=A.DETERMINISTIC, stream=side)
+        done.record(side)
+        if not early:
+            torch.cuda.synchronize()
+        t.close()
+        ended.append(done.query())
+        u = A.create_alto(dims, other, vals2, stream=third)  # same sizes, other contents
+        torch.cuda.synchronize()
+        results.append(out)
+        u.close()
+    assert all(ended)
+    assert torch.equal(*results)
+
+
+def test_first_use_inside_a_capture_is_refused():
+    """A call that has to allocate is refused under a stream capture (the copy it
+    would build there would only be captured, not made), and works after it."""
+    import torch
+
+    rt = pytest.importorskip("cuda.bindings.runtime")
+    dims, idx, vals, F = long_tensor(5)
+    t = A.create_alto(dims, idx, vals)
+    out = torch.zeros((int(dims[1]), 16), device="cuda")
+    torch.cuda.synchronize()
+    s = torch.cuda.Stream()
+    for mode in (rt.cudaStreamCaptureMode.cudaStreamCaptureModeGlobal,
+                 rt.cudaStreamCaptureMode.cudaStreamCaptureModeThreadLocal):
+        rt.cudaStreamBeginCapture(s.cuda_stream, mode)
+        try:
+            with pytest.raises(A.AltoError):
+                t.mttkrp(1, F, 16, out=out, variant=A.SORTED, stream=s)
+        finally:
+            err, graph = rt.cudaStreamEndCapture(s.cuda_stream)
+        assert err != rt.cudaError_t.cudaSuccess
+        rt.cudaGetLastError()
+    t.mttkrp(1, F, 16, out=out, variant=A.SORTED, stream=s)
+    s.synchronize()
+    want = A.create_alto(dims, idx, vals).mttkrp(1, F, 16, variant=A.ATOMIC)
+    assert float((out - want).abs().max() / want.abs().max()) <= TOL
