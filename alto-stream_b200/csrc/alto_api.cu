@@ -36,17 +36,17 @@ HandlePool* handle_pool(int dev) {
     props.location.id = dev;
     cudaStream_t st = nullptr;
     cudaMemPool_t p = nullptr;
-    if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess) return nullptr;
-    if (cudaMemPoolCreate(&p, &props) != cudaSuccess) {
-      cudaStreamDestroy(st);
+    if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess || cudaMemPoolCreate(&p, &props) != cudaSuccess) {
+      if (st) cudaStreamDestroy(st);
+      cudaGetLastError();  // (pool_alloc does without)
       return nullptr;
     }
     uint64_t keep = kPoolKeep;
     cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
-    if (cudaMalloc(&h.hold, kGuardBytes) != cudaSuccess) cudaGetLastError();  // (the guards work without)
     h.st = st;
     h.pool = p;
   }
+  if (!h.hold && cudaMalloc(&h.hold, kGuardBytes) != cudaSuccess) cudaGetLastError();  // (the guards work without)
   return &h;
 }
 }  // namespace
@@ -57,9 +57,8 @@ cudaError_t pool_alloc(void** p, size_t bytes, PoolMem* m) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  HandlePool* h = handle_pool(dev);
-  if (!h) return cudaErrorMemoryAllocation;
-  const bool pooled = bytes <= kPoolMost;
+  HandlePool* h = handle_pool(dev);  // (NULL: no pool to be had, all from cudaMalloc)
+  const bool pooled = h && bytes <= kPoolMost;
   auto take = [&]() -> cudaError_t {
     if (!pooled) return cudaMalloc(p, bytes);
     if (!m->guard) {
@@ -69,7 +68,7 @@ cudaError_t pool_alloc(void** p, size_t bytes, PoolMem* m) {
     return cudaMallocFromPoolAsync(p, bytes, h->pool, h->st);
   };
   e = take();
-  if (e == cudaErrorMemoryAllocation) {  // what the pool keeps may be in the way, in other sizes
+  if (e == cudaErrorMemoryAllocation && h) {  // what the pool keeps may be in the way, in other sizes
     cudaGetLastError();
     cudaStreamSynchronize(h->st);
     cudaMemPoolTrimTo(h->pool, 0);
