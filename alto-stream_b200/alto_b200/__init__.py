@@ -44,7 +44,7 @@ CPSTREAM, SPCPSTREAM = range(2)  # streaming models (alto_stream_set_model)
 FIT_REFERENCE, FIT_EXACT = 0, 1
 
 EXPORTED = [
-    "alto_status_string", "alto_last_error", "alto_version", "alto_kernel_launches",
+    "alto_status_string", "alto_last_error", "alto_version", "alto_kernel_launches", "alto_release_memory",
     "alto_compute_masks", "alto_tensor_create", "alto_tensor_update", "alto_tensor_export", "alto_tensor_info",
     "alto_tensor_device_bytes", "alto_tensor_restrict", "alto_tensor_destroy", "alto_mttkrp", "alto_mttkrp_variant_run",
     "alto_mttkrp_choose", "alto_mttkrp_autotune", "alto_mttkrp_host", "alto_mttkrp_host_changed", "alto_gram",
@@ -99,6 +99,11 @@ def check(status):
 
 def kernel_launches():
     return int(lib().alto_kernel_launches())
+
+
+def release_memory():
+    """Give back the device memory the library keeps and nothing uses (alto_release_memory)."""
+    check(lib().alto_release_memory())
 
 
 _cuda = None  # torch.cuda once it is known to be usable

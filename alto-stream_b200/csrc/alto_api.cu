@@ -68,10 +68,9 @@ cudaError_t pool_alloc(void** p, size_t bytes, PoolMem* m) {
     return cudaMallocFromPoolAsync(p, bytes, h->pool, h->st);
   };
   e = take();
-  if (e == cudaErrorMemoryAllocation && h) {  // what the pool keeps may be in the way, in other sizes
+  if (e == cudaErrorMemoryAllocation) {  // what the pools keep may be in the way, in other sizes
     cudaGetLastError();
-    cudaStreamSynchronize(h->st);
-    cudaMemPoolTrimTo(h->pool, 0);
+    trim_pools();
     e = take();
   }
   if (e == cudaSuccess && pooled) {
@@ -99,13 +98,17 @@ void pool_free(void* p, const PoolMem& m) {
   if (cur != m.dev) cudaSetDevice(cur);
 }
 
+namespace {
+std::mutex g_transient_mu;
+cudaMemPool_t g_transient[64] = {};
+}  // namespace
+
 cudaMemPool_t transient_pool() {
-  static std::mutex mu;
-  static cudaMemPool_t pools[64] = {};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  std::lock_guard<std::mutex> g(mu);
-  if (!pools[dev]) {
+  std::lock_guard<std::mutex> g(g_transient_mu);
+  cudaMemPool_t& pool = g_transient[dev];
+  if (!pool) {
     cudaMemPoolProps props{};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -114,9 +117,20 @@ cudaMemPool_t transient_pool() {
     if (cudaMemPoolCreate(&p, &props) != cudaSuccess) return nullptr;
     uint64_t keep = ~0ull;  // keep freed memory for the next call
     cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
-    pools[dev] = p;
+    pool = p;
   }
-  return pools[dev];
+  return pool;
+}
+
+void trim_pools() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
+  if (HandlePool* h = handle_pool(dev)) {
+    cudaStreamSynchronize(h->st);
+    cudaMemPoolTrimTo(h->pool, 0);
+  }
+  std::lock_guard<std::mutex> g(g_transient_mu);
+  if (g_transient[dev]) cudaMemPoolTrimTo(g_transient[dev], 0);
 }
 
 void set_error(const char* fmt, ...) {
@@ -214,6 +228,11 @@ const char* alto_status_string(alto_status s) {
 const char* alto_last_error(void) { return g_err; }
 int alto_version(void) { return ALTO_VERSION; }
 uint64_t alto_kernel_launches(void) { return g_kernel_launches.load(); }
+
+alto_status alto_release_memory(void) {
+  trim_pools();
+  return ALTO_OK;
+}
 
 alto_status alto_compute_masks(int nmodes, const uint64_t* dims, int key_bits, uint64_t* masks,
                                uint64_t* alto_mask, int* alto_bits) {

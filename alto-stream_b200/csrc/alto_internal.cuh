@@ -54,6 +54,11 @@ inline alto_status cuda_status(cudaError_t e, const char* what, const char* file
 // serving workers) do not stall one another when buffers grow.
 extern thread_local cudaStream_t tls_alloc_stream;
 
+// Gives back what the library's two pools (the handles', below, and
+// transient_pool) keep of the current device's memory and nothing uses: when an
+// allocation fails, and on request.
+void trim_pools();
+
 // Device memory for the handles' buffers, one pool per device, with the
 // semantics of cudaMalloc / cudaFree: what pool_alloc returns may be used on
 // any stream at once, pool_free first waits for the device, so memory is never
@@ -115,6 +120,11 @@ struct DevBuf {
     release();
     size_t want = n < 256 ? 256 : n;
     cudaError_t e = tls_alloc_stream ? cudaMallocAsync(&p, want, tls_alloc_stream) : pool_alloc(&p, want, &pool);
+    if (e == cudaErrorMemoryAllocation && tls_alloc_stream) {
+      cudaGetLastError();
+      trim_pools();
+      e = cudaMallocAsync(&p, want, tls_alloc_stream);
+    }
     if (e != cudaSuccess) {
       p = nullptr;
       return cuda_status(e, "device allocation", __FILE__, __LINE__);
@@ -158,6 +168,11 @@ struct PoolBuf {
     st = s;
     const size_t want = n < 256 ? 256 : n;
     cudaError_t e = cudaMallocFromPoolAsync(&p, want, pool, s);
+    if (e == cudaErrorMemoryAllocation) {
+      cudaGetLastError();
+      trim_pools();
+      e = cudaMallocFromPoolAsync(&p, want, pool, s);
+    }
     if (e != cudaSuccess) {
       p = nullptr;
       return cuda_status(e, "cudaMallocFromPoolAsync", __FILE__, __LINE__);

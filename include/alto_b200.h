@@ -103,6 +103,13 @@ const char* alto_last_error(void);
 int alto_version(void);
 /* Number of kernels this library launched since load (for launch audits). */
 uint64_t alto_kernel_launches(void);
+/* Give back the device memory that the library keeps on the current device
+ * and nothing uses: up to 2 GiB freed by tensors, sessions, servers and
+ * alto_cpd_als (kept for later buffers until the process exits) and what
+ * file reads and slicers left (see alto_read_tensor).  An allocation of the
+ * library that fails does so by itself and tries again; call it to make room
+ * for other allocators. */
+alto_status alto_release_memory(void);
 
 /* ------------------------------------------------------ the ALTO tensor */
 
@@ -328,7 +335,7 @@ typedef struct alto_dcoo alto_dcoo;
  * nonzeros or a short binary file is ALTO_ERR_INVALID.  The read's working
  * buffers (about the file's size plus 8 bytes per line) come from a device
  * memory pool the library keeps for later reads and slicers until the
- * process exits.  Synchronous. */
+ * process exits or alto_release_memory.  Synchronous. */
 alto_status alto_read_tensor(const char* path, alto_file_format format, int zero_based,
                              alto_cuda_stream stream, alto_dcoo** out);
 /* A device view of the tensor (on_device 1, index_bytes 8, ALTO_F64), valid

@@ -112,3 +112,62 @@ def test_encoding_at_sort_tile_edges(dims, nnz):
         ref = np.zeros(int(dims[m]))
         np.add.at(ref, cidx[m].astype(np.int64), vals)
         assert np.array_equal(out, np.repeat(ref[:, None], 8, 1).astype(np.float32))
+
+
+def held():
+    """Device memory in use, in MiB."""
+    import torch
+
+    torch.cuda.synchronize()
+    free, total = torch.cuda.mem_get_info()
+    return (total - free) >> 20
+
+
+def test_kept_memory_is_bounded_and_given_back():
+    """What destroyed tensors leave in the library's pool is at most 2 GiB, and
+    release_memory gives it back."""
+    import torch
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    dims = np.array([3000, 2000, 1000], np.uint64)
+    idx = [torch.randint(0, int(d), (8000000,), generator=g, device="cuda") for d in dims]
+    vals = torch.rand(8000000, generator=g, device="cuda")
+    A.create_alto(dims, idx[:3], vals).close()
+    A.release_memory()
+    before = held()
+    tensors = [A.create_alto(dims, idx, vals) for _ in range(8)]  # about 0.5 GB each, buffers below 512 MiB
+    assert held() - before > 2500
+    for t in tensors:
+        t.close()
+    assert 500 <= held() - before <= 2048 + 64  # (64: other allocations' slabs)
+    A.release_memory()
+    assert held() - before <= 64
+
+
+def test_kept_memory_makes_way_for_the_library():
+    """With the device all but full, an allocation from one pool gets what the
+    other one keeps."""
+    import torch
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(2)
+    dims = np.array([100, 2000, 1000], np.uint64)
+    idx = [torch.randint(0, int(d), (8000000,), generator=g, device="cuda") for d in dims]
+    vals = torch.rand(8000000, generator=g, device="cuda")
+    A.Slicer(dims, [i[:1000].contiguous() for i in idx], vals[:1000].contiguous(), 0).close()  # (kernels loaded)
+    A.release_memory()
+    tensors = [A.create_alto(dims, idx, vals) for _ in range(4)]
+    for t in tensors:
+        t.close()
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    filler = torch.empty(free - (256 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        s = A.Slicer(dims, idx, vals, 0)  # 60 bytes a nonzero: 480 MB
+        assert s.next(1, 1) is not None
+        s.close()
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+        A.release_memory()
