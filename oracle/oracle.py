@@ -18,6 +18,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import unittest
 from ctypes import POINTER, c_double, c_int, c_uint64, c_void_p
 
 import numpy as np
@@ -63,12 +64,17 @@ def ref_available(bits=64):
     return os.path.exists(os.path.join(HERE, "_ref", f"libaltoref{bits}.so"))
 
 
+class ReferenceMissing(unittest.SkipTest, FileNotFoundError):
+    """The compiled reference is not built on this machine (its sources are not
+    here): a check against it is skipped, not failed."""
+
+
 def ref_lib(bits=64):
     """Load the compiled reference (64- or 128-bit ALTO keys)."""
     if bits not in _REF:
         path = os.path.join(HERE, "_ref", f"libaltoref{bits}.so")
         if not os.path.exists(path):
-            raise FileNotFoundError(f"{path} missing: run `make -C oracle ref REF=<reference dir>` where the reference sources exist")
+            raise ReferenceMissing(f"{path} missing: run `make -C oracle ref REF=<reference dir>` where the reference sources exist")
         L = ctypes.CDLL(path)
         L.ref_alto_create.restype = c_void_p
         L.ref_alto_destroy.argtypes = [c_void_p]

@@ -236,3 +236,31 @@ def test_cut_all_equals_repeated_next():
         p = sl.stream_prev(5)
         assert p is not None and p.dims[0] == 5
         sl.close()
+
+
+@pytest.mark.parametrize("model", [A.CPSTREAM, A.SPCPSTREAM])
+def test_stream_error_of_the_last_steps(model):
+    """cpd_error against stream_prev's tensor and the time rows of its steps,
+    where the compiled reference is not there to compare with."""
+    dims = np.array([12, 40, 30, 20], np.uint64)
+    cidx, vals = synth.uniform_coo(dims, 2500, seed=5)
+    R = 8
+    iv = np.random.default_rng(6).random(4096 * R)
+    s = A.CPStream(4, 0, R, constraint=A.NONNEG, max_inner=10, epsilon=1e-5)
+    s.set_model(model)
+    sl = A.Slicer(dims, cidx, vals, 0)
+    prev, used = np.zeros(4, np.int64), 0
+    while (b := sl.next(300, 3)) is not None:
+        d = b.dims.astype(np.int64)
+        need = int(np.sum(np.maximum(d - prev, 0))) * R
+        s.push_batch(b, iv[used:used + need])
+        used += need
+        prev = np.maximum(prev, d)
+    F = [s.factor(0, 12)] + [np.vstack([s.factor(m, int(prev[m])), np.zeros((int(dims[m] - prev[m]), R))])
+                             for m in (1, 2, 3)]
+    P = sl.stream_prev(3)
+    c, v = P.to_host()
+    want = O.cpd_error(c, v, [F[0][-3:]] + F[1:])
+    assert abs(s.error(P) - want) <= 1e-10 * max(1.0, want)
+    s.close()
+    sl.close()
