@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "alto_dense.cuh"
+#include "alto_group.cuh"
 
 namespace alto {
 
@@ -147,39 +148,51 @@ static alto_status mttkrp_host_impl(alto_tensor* t, int mode, double* const* fac
 // Iterations whose fits are kept on the device between copies to the host.
 constexpr int kFitWindow = 64;
 
+// What the walk of mode `mode`'s row-sorted copy needs, made now: the copy, and
+// where the deterministic walk is chosen the slots of its runs' ends.
+// Where a row's run is long the atomics' partial sums make the walk's error, and
+// the deterministic walk splits it in short chains and fixed trees (power law,
+// three modes of 5000: 394,950 nonzeros at rank 64, worst factor's error 3.6e-6
+// with atomics against 7.2e-7, six iterations 4.34 ms against 4.46; 1,578,155 at
+// rank 8 6.1e-6 against 1.4e-6, 2.01 ms against 2.31).  Without long runs both
+// are equal (uniform, 3.5e-7 and 3.7e-7), and its fix-up costs a short walk more
+// (1000^3, 1M nonzeros, 20 iterations at rank 16: 2.90 ms against 3.42) than a long
+// one (5%), whose error it still lowers.
+static alto_status prepare_sorted(alto_tensor* t, int mode, const void* const* fac, alto_dtype fdtype, int rank,
+                                  float* out, alto_mttkrp_variant* variant, cudaStream_t st) {
+  if (!t->sorted[mode].ready || t->sorted[mode].for_nnz != t->nnz) ALTO_TRY(build_sorted_line(t, mode, st));
+  *variant = ALTO_MTTKRP_SORTED;
+  if (!deterministic_supported(rank, fdtype)) return ALTO_OK;
+  bool det = t->nnz >= (2u << 20);
+  if (!det) ALTO_TRY(sorted_long_runs(t, mode, &det, st));
+  if (!det) return ALTO_OK;
+  DetItem item;
+  ALTO_TRY(det_prepare(t, mode, fac, rank, out, &item, st));
+  *variant = ALTO_MTTKRP_DETERMINISTIC;
+  return ALTO_OK;
+}
+
 // The MTTKRP of mode `mode` in a CP-ALS of max_iters iterations: the tuned
 // variant where the tensor has one.  Else, from the second walk of a mode on, a
 // row-sorted copy pays wherever rows repeat -- staging in shared memory and
 // atomics along the line measured 2 to 4 times slower (1000^3, 1M nonzeros, rank
 // 16: 55 us staged against 12.5; 5 modes, 5M nonzeros, rank 64: 1178 us against
 // 280), and building the copy costs two to three walks -- so the copy is built
-// now, and where its memory cannot be had the line is walked as AUTO chooses.
-static alto_status als_variant(alto_tensor* t, int mode, int rank, alto_dtype fdtype, int max_iters,
-                               alto_mttkrp_variant* variant, cudaStream_t st) {
+// now, and where its memory cannot be had the line is walked without one.
+static alto_status als_variant(alto_tensor* t, int mode, const void* const* fac, alto_dtype fdtype, int rank,
+                               float* out, int max_iters, alto_mttkrp_variant* variant, cudaStream_t st) {
   *variant = ALTO_MTTKRP_AUTO;
   if (max_iters < 4 || !decoded_modes(t->nmodes) || t->nnz < 2 * t->dims[mode] || mttkrp_tuned(t, mode, rank, fdtype))
     return ALTO_OK;
-  if (!t->sorted[mode].ready || t->sorted[mode].for_nnz != t->nnz) {
-    const alto_status s = build_sorted_line(t, mode, st);
-    if (s == ALTO_ERR_NOMEM) {
-      cudaGetLastError();  // (the failed allocation is handled here)
-      return ALTO_OK;
-    }
-    ALTO_TRY(s);
-  }
-  // Where a row's run is long the atomics' partial sums make the walk's error, and
-  // the deterministic walk splits it in short chains and fixed trees (power law,
-  // three modes of 5000: 394,950 nonzeros at rank 64, worst factor's error 3.6e-6
-  // with atomics against 7.2e-7, six iterations 4.34 ms against 4.46; 1,578,155 at
-  // rank 8 6.1e-6 against 1.4e-6, 2.01 ms against 2.31).  Without long runs both
-  // are equal (uniform, 3.5e-7 and 3.7e-7), and its fix-up costs a short walk more
-  // (1000^3, 1M nonzeros, 20 iterations at rank 16: 2.90 ms against 3.42) than a long
-  // one (5%), whose error it still lowers.
-  *variant = ALTO_MTTKRP_SORTED;
-  if (!deterministic_supported(rank, fdtype)) return ALTO_OK;
-  bool det = t->nnz >= (2u << 20);
-  if (!det) ALTO_TRY(sorted_long_runs(t, mode, &det, st));
-  if (det) *variant = ALTO_MTTKRP_DETERMINISTIC;
+  const alto_status s = prepare_sorted(t, mode, fac, fdtype, rank, out, variant, st);
+  if (s != ALTO_ERR_NOMEM || *variant == ALTO_MTTKRP_SORTED)  // (the copy without its slots: with atomics)
+    return s == ALTO_ERR_NOMEM ? ALTO_OK : s;
+  SortedLine& c = t->sorted[mode];  // what there is of the copy makes room again
+  c.ready = false;
+  c.line.release();
+  c.extra.release();
+  c.tile_iv.release();
+  *variant = unsorted_variant(t, mode, rank);
   return ALTO_OK;
 }
 
@@ -241,13 +254,18 @@ extern "C" alto_status alto_cpd_als(alto_tensor* t, int rank, double* const* U_h
     ALTO_TRY_CUDA(cudaStreamSynchronize(st));
   }
 
+  // (everything the iterations need but the row-sorted copies, which may fail)
+  ALTO_TRY(dscr.ensure(dot_scratch_bytes()));
+  ALTO_TRY(ensure_error_words(t, st));
+
   const void* fac[ALTO_MAX_MODES];
   for (int m = 0; m < N; ++m) fac[m] = bf16 ? Ub[m].p : U[m].p;
   const alto_dtype fdt = bf16 ? ALTO_BF16 : ALTO_F32;
   const unsigned all = (1u << N) - 1;
 
   alto_mttkrp_variant variant[ALTO_MAX_MODES];
-  for (int m = 0; m < N; ++m) ALTO_TRY(als_variant(t, m, R, fdt, max_iters, &variant[m], st));
+  for (int m = 0; m < N; ++m)
+    ALTO_TRY(als_variant(t, m, fac, fdt, R, mbuf.as<float>(), max_iters, &variant[m], st));
 
   double prev_fit = 0.0;
   int it_run = max_iters;

@@ -1166,9 +1166,11 @@ __global__ void __launch_bounds__(256)
 
 static constexpr int kDotBlocks = 296;
 
+size_t dot_scratch_bytes() { return kDotBlocks * 3 * sizeof(double); }
+
 alto_status dot_stats(const float* a, const float* b, uint64_t n, const double* colw, int R,
                       double* out3, DevBuf& scratch, cudaStream_t st) {
-  ALTO_TRY(scratch.ensure(kDotBlocks * 3 * sizeof(double)));
+  ALTO_TRY(scratch.ensure(dot_scratch_bytes()));
   dot_partial_kernel<float, float><<<kDotBlocks, 256, 0, st>>>(a, b, n, colw, R, scratch.as<double>());
   ALTO_LAUNCHED();
   reduce_partials_kernel<<<reduce_grid(3), kReduceThreads, 0, st>>>(scratch.as<double>(), kDotBlocks, 3, out3);

@@ -35,6 +35,7 @@ alto_status to_bf16(const float* X, uint64_t n, __nv_bfloat16* Y, cudaStream_t s
 // out3 = {sum a*b*colw, sum (a-b)^2, sum b^2}.
 alto_status dot_stats(const float* a, const float* b, uint64_t n, const double* colw, int R,
                       double* out3, DevBuf& scratch, cudaStream_t st);
+size_t dot_scratch_bytes();  // the scratch dot_stats and sum_squares grow to
 alto_status sum_squares(const float* v, uint64_t n, double* out, DevBuf& scratch, cudaStream_t st);
 alto_status model_norm(const double* grams, int nmodes, int R, const double* lambda, int exact,
                        double* out, cudaStream_t st);

@@ -408,17 +408,19 @@ alto_status run_mttkrp_feed(alto_tensor* t, int mode, const void* const* factors
                             int rank, float* out, int accumulate, alto_mttkrp_variant variant, int feed,
                             cudaStream_t st);
 alto_mttkrp_variant choose_variant(const alto_tensor* t, int mode, int rank, alto_dtype fdtype);
+// The best variant that walks the line itself (no row-sorted copy).
+alto_mttkrp_variant unsorted_variant(const alto_tensor* t, int mode, int rank);
 // Whether alto_mttkrp_autotune has measured this mode, rank and factor type.
 bool mttkrp_tuned(const alto_tensor* t, int mode, int rank, alto_dtype fdtype);
 // Whether ALTO_MTTKRP_DETERMINISTIC runs for this rank and factor type.
 bool deterministic_supported(int rank, alto_dtype fdtype);
 // Build the per-mode row-sorted copy of the line.
+alto_status build_sorted_line(alto_tensor* t, int mode, cudaStream_t st);
 // Whether some row of mode `mode`'s decoded copy holds more than kLongRun
 // nonzeros (every row of 2 kLongRun or more is found, none below kLongRun + 1).
 // Waits for the stream the first time.
 constexpr uint32_t kLongRun = 4096;
 alto_status sorted_long_runs(alto_tensor* t, int mode, bool* found, cudaStream_t st);
-alto_status build_sorted_line(alto_tensor* t, int mode, cudaStream_t st);
 // Measure the variants per mode and record the fastest (synchronous).
 alto_status autotune(alto_tensor* t, const void* const* factors, alto_dtype fdtype, int rank,
                      cudaStream_t st, alto_mttkrp_variant* chosen);

@@ -1879,6 +1879,12 @@ bool mttkrp_tuned(const alto_tensor* t, int mode, int rank, alto_dtype fdtype) {
   return tuned_entry(t, mode, rank, fdtype) != nullptr;
 }
 
+alto_mttkrp_variant unsorted_variant(const alto_tensor* t, int mode, int rank) {
+  if (mode == t->stream_mode && t->dims[mode] * rank * 4 <= (uint64_t)kStageBytes) return ALTO_MTTKRP_STREAM;
+  if (stageable_fraction(t, mode, rank) >= 0.5) return ALTO_MTTKRP_STAGED;
+  return ALTO_MTTKRP_ATOMIC;
+}
+
 alto_mttkrp_variant choose_variant(const alto_tensor* t, int mode, int rank, alto_dtype fdtype) {
   if (const TuneEntry* e = tuned_entry(t, mode, rank, fdtype)) return e->variant;
   // The reference's rule (include/alto.hpp:835-846) picks atomics for long
@@ -1886,12 +1892,9 @@ alto_mttkrp_variant choose_variant(const alto_tensor* t, int mode, int rank, alt
   // otherwise.  On the device: stage where the tiles' intervals fit, walk a
   // row-sorted copy where rows are reused but the intervals are too wide,
   // else plain vector atomics.
-  const uint64_t dim = t->dims[mode];
-  const uint64_t reuse = dim ? t->nnz / dim : 0;
-  if (mode == t->stream_mode && dim * rank * 4 <= (uint64_t)kStageBytes) return ALTO_MTTKRP_STREAM;
-  if (stageable_fraction(t, mode, rank) >= 0.5) return ALTO_MTTKRP_STAGED;
-  if (reuse > 4) return ALTO_MTTKRP_SORTED;
-  return ALTO_MTTKRP_ATOMIC;
+  const alto_mttkrp_variant v = unsorted_variant(t, mode, rank);
+  const uint64_t reuse = t->dims[mode] ? t->nnz / t->dims[mode] : 0;
+  return v == ALTO_MTTKRP_ATOMIC && reuse > 4 ? ALTO_MTTKRP_SORTED : v;
 }
 
 // The arguments of a walk of mode `mode` into `out`: of the line, or of the

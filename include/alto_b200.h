@@ -243,6 +243,10 @@ alto_status alto_gram_noalloc(const float* U, uint64_t rows, int rank, double* G
  * storage (ALTO_F32 or ALTO_BF16); MTTKRP accumulates in float32; Grams,
  * Cholesky, solves and fit are float64.  fits (max_iters, may be NULL)
  * receives the per-iteration residual; *iters the iterations run.
+ * Of four iterations on, a 3- to 5-mode tensor gets a row-sorted copy of
+ * every mode whose rows repeat (16, 20 or 24 bytes per nonzero), as an
+ * untuned alto_mttkrp builds them; the copies stay with the tensor for later
+ * calls.  A mode whose copy does not fit is walked without one.
  * Synchronous. */
 alto_status alto_cpd_als(alto_tensor* t, int rank, double* const* U_host, double* lambda_host,
                          int max_iters, double epsilon, alto_fit_mode fit_mode,

@@ -130,3 +130,38 @@ def test_a_row_with_a_long_run(nmodes, heavy):
     U, lam, fits, it = A.cpd_alto(t, U0, np.ones(R), R, 4, 0.0)
     _, _, fo, _ = O.cpd_als(O.build(dims, c, vals), U0, np.ones(R), R, 4, 0.0)
     np.testing.assert_allclose(fits, fo, rtol=0, atol=1e-5)
+
+
+@pytest.mark.parametrize("spare", [256, 560])
+def test_copies_that_do_not_fit(spare):
+    """With `spare` MiB of device memory left, none or one of the modes' row-sorted
+    copies (256 MB each) fits beside the call's own 160 MB: the other modes are
+    walked without, and the fits are those of a run with every copy, to the
+    module's bound on a single fit in absolute terms."""
+    import torch
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(1)
+    dims, nnz, R = np.array([200000, 150000, 100000], np.uint64), 16000000, 16
+    idx = [torch.randint(0, int(d), (nnz,), generator=g, device="cuda") for d in dims]
+    vals = torch.rand(nnz, generator=g, device="cuda") + 0.5
+    U0 = init_model(dims, R, 4)
+    t = A.create_alto(dims, idx, vals)
+    _, _, want, _ = A.cpd_alto(t, U0, np.ones(R), R, 4, 0.0)
+    t.close()
+    t = A.create_alto(dims, idx, vals)
+    before = t.device_bytes()
+    A.release_memory()
+    torch.cuda.empty_cache()
+    filler = torch.empty(torch.cuda.mem_get_info()[0] - (spare << 20), dtype=torch.uint8, device="cuda")
+    try:
+        _, _, fits, _ = A.cpd_alto(t, U0, np.ones(R), R, 4, 0.0)
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    copies = (t.device_bytes() - before) / (16 * nnz)
+    assert 0 <= copies < (0.5 if spare == 256 else 2.5)
+    np.testing.assert_allclose(fits, want, rtol=0, atol=1e-5)
+    _, _, fits, _ = A.cpd_alto(t, U0, np.ones(R), R, 4, 0.0)  # with room again
+    np.testing.assert_allclose(fits, want, rtol=0, atol=1e-5)
+    assert (t.device_bytes() - before) / (16 * nnz) > 2.9
