@@ -143,14 +143,18 @@ void record_latency(alto_server* s, double ms) {  // caller holds s->mu
 // sort scratch and one row-sorted copy per mode.
 uint64_t reserve_estimate(const alto_stream_config& c, const uint64_t* max_dims, uint64_t max_nnz) {
   uint64_t sum_dims = 0, max_dim = 0;
+  int bits = 0;  // of the line key
   for (int m = 0; m < c.nmodes; ++m) {
     sum_dims += max_dims[m];
     max_dim = std::max(max_dim, max_dims[m]);
+    if (max_dims[m] > 1) bits += 64 - __builtin_clzll(max_dims[m] - 1);
   }
+  const uint64_t rec = rec_bytes(bits > 96 ? 2 : 0);
+  const uint64_t copy = decoded_modes(c.nmodes) ? 16 + decoded_extra_bytes(c.nmodes) : rec;
   const uint64_t R = (uint64_t)c.rank;
   const uint64_t model = (sum_dims * R * (4 + 4 + 8) * 3) / 2;
   const uint64_t solve = max_dim * R * (4 + 8 * 4);
-  const uint64_t tensor = max_nnz * (16 + 4 + 40 + 8ull * c.nmodes + 8 + 16ull * c.nmodes);
+  const uint64_t tensor = max_nnz * (rec + 4 + 40 + 8ull * c.nmodes + 8 + copy * c.nmodes);
   return model + solve + tensor + (64ull << 10) * c.nmodes + (16ull << 20);
 }
 

@@ -160,3 +160,25 @@ def test_close_of_pending_stream_wakes_its_waiters():
     srv.drain()
     srv.close(s1)
     srv.destroy()
+
+
+@pytest.mark.parametrize("space", [[100, 300, 200], [100, 300, 200, 50], [100, 300, 200, 50, 20]])
+def test_admission_counts_the_encoded_slice(space):
+    """What a stream reserves grows with its largest slice by at least what that
+    slice takes encoded, with its sort scratch and a row-sorted copy per mode."""
+    n, N = 1000000, len(space)
+    rng = np.random.default_rng(N)
+    cidx = np.stack([rng.integers(0, d, n) for d in space]).astype(np.uint64)
+    t = A.create_alto(np.array(space, np.uint64), cidx, np.ones(n))
+    import torch
+
+    F = [torch.ones((d, 8), device="cuda") for d in space]
+    for m in range(N):
+        t.mttkrp(m, F, 8, variant=A.SORTED)
+    srv = A.Server(64 << 30, workers=1)
+    srv.open(N, 0, 8, space, 0)
+    empty = srv.stats()["reserved_bytes"]
+    srv.open(N, 0, 8, space, n)
+    grown = srv.stats()["reserved_bytes"] - 2 * empty
+    srv.destroy()
+    assert grown >= t.device_bytes() - (1 << 20)  # (1 MiB: tile and partition tables, counters)
