@@ -37,6 +37,7 @@
 // instead (the same arithmetic in the same order: identical results).
 #include <chrono>
 #include <cmath>
+#include <condition_variable>
 #include <cstring>
 #include <exception>
 #include <mutex>
@@ -2539,7 +2540,9 @@ bool stream_group_key_equal(const alto_stream_session* a, const alto_stream_sess
 // staging buffer (free between pushes, and sized for all the rows the model has
 // gained at once).  A caller's array is usually fresh memory, whose pages cost
 // more to touch than the values to copy (40 MB: 14 ms on one core, 2.5 ms on
-// eight), so a large factor is widened by several threads.
+// eight), so a large factor is widened by a team of threads, started once for
+// the call: this thread copies stretch after stretch into the staging buffer,
+// and each member widens its share of every stretch.
 static alto_status factor_to_host(alto_stream_session* s, int mode, uint64_t n, double* host_out) {
   constexpr uint64_t kParallel = 1u << 17;  // values below which one thread is as fast
   std::lock_guard<std::mutex> lk(s->pin_mu);  // (factors of one session may be read by several threads)
@@ -2551,30 +2554,63 @@ static alto_status factor_to_host(alto_stream_session* s, int mode, uint64_t n, 
     stage = own.data();
     cap = own.size();
   }
-  const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-  for (uint64_t q = 0; q < n; q += cap) {
-    const uint64_t c = std::min(n - q, cap);
-    ALTO_TRY_CUDA(cudaMemcpyAsync(stage, s->U[mode].as<float>() + q, c * 4, cudaMemcpyDeviceToHost, s->st));
-    ALTO_TRY_CUDA(cudaStreamSynchronize(s->st));
-    const unsigned T = c < kParallel ? 1u : std::min(8u, hw);
-    auto widen = [&](uint64_t a, uint64_t b) {
-      for (uint64_t k = a; k < b; ++k) host_out[q + k] = stage[k];
-    };
-    const uint64_t per = (c + T - 1) / T;
-    std::vector<std::thread> threads;
-    uint64_t next = per;  // thread 0's share is this thread's
-    try {
-      for (; next < c; next += per) {
-        const uint64_t a = next, b = std::min(next + per, c);
-        threads.emplace_back([=] { widen(a, b); });
-      }
-    } catch (const std::exception&) {  // no more threads to be had: the rest here
+  std::mutex mu;
+  std::condition_variable cv;
+  uint64_t at = 0, len = 0;                // the stretch of turn `turn`
+  unsigned turn = 0, left = 0, T = 1;      // members still at it; members
+  bool done = false;
+  auto widen = [&](unsigned k) {
+    const uint64_t per = (len + T - 1) / T;
+    for (uint64_t i = k * per; i < std::min((k + 1) * per, len); ++i) host_out[at + i] = stage[i];
+  };
+  auto member = [&](unsigned k) {
+    unsigned seen = 0;
+    std::unique_lock<std::mutex> l(mu);
+    for (;;) {
+      cv.wait(l, [&] { return done || turn != seen; });
+      if (done) return;
+      seen = turn;
+      l.unlock();
+      widen(k);
+      l.lock();
+      if (--left == 0) cv.notify_all();
     }
-    widen(0, std::min(per, c));
-    if (next < c) widen(next, c);
-    for (auto& t : threads) t.join();
+  };
+  std::vector<std::thread> team;
+  if (std::min(n, cap) >= kParallel) {
+    const unsigned most = std::min(8u, std::max(1u, std::thread::hardware_concurrency()));
+    try {
+      for (unsigned k = 1; k < most; ++k) team.emplace_back(member, k);
+    } catch (const std::exception&) {  // no more threads to be had: fewer members
+    }
   }
-  return ALTO_OK;
+  T = 1 + (unsigned)team.size();  // (the members read it from their first turn on)
+  alto_status st = ALTO_OK;
+  for (uint64_t q = 0; q < n && st == ALTO_OK; q += cap) {
+    const uint64_t c = std::min(n - q, cap);
+    st = cuda_status(cudaMemcpyAsync(stage, s->U[mode].as<float>() + q, c * 4, cudaMemcpyDeviceToHost, s->st),
+                     "cudaMemcpyAsync", __FILE__, __LINE__);
+    if (st == ALTO_OK) st = cuda_status(cudaStreamSynchronize(s->st), "cudaStreamSynchronize", __FILE__, __LINE__);
+    if (st != ALTO_OK) break;
+    {
+      std::lock_guard<std::mutex> l(mu);
+      at = q;
+      len = c;
+      left = T - 1;
+      ++turn;
+    }
+    cv.notify_all();
+    widen(0);
+    std::unique_lock<std::mutex> l(mu);
+    cv.wait(l, [&] { return left == 0; });
+  }
+  {
+    std::lock_guard<std::mutex> l(mu);
+    done = true;
+  }
+  cv.notify_all();
+  for (auto& t : team) t.join();
+  return st;
 }
 
 extern "C" {
@@ -2686,7 +2722,12 @@ alto_status alto_stream_factor(alto_stream_session* s, int mode, double* host_ou
   const uint64_t n = s->dims[mode] * (uint64_t)s->R;
   if (rows) *rows = s->dims[mode];
   if (!host_out || !n) return ALTO_OK;
-  return factor_to_host(s, mode, n, host_out);
+  try {
+    return factor_to_host(s, mode, n, host_out);
+  } catch (const std::exception& e) {  // (host memory)
+    set_error("reading a factor: %s", e.what());
+    return ALTO_ERR_NOMEM;
+  }
 }
 
 alto_status alto_stream_error(alto_stream_session* s, const alto_coo* X, double* err) {

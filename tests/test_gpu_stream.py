@@ -258,3 +258,25 @@ def test_factors_read_by_several_threads():
     for t in threads:
         t.join()
     assert not bad
+
+
+def test_factor_longer_than_its_staging():
+    """A mode that has grown by 10,007 rows a push is read back in several
+    stretches by several threads (the staging holds one push's rows), to the
+    module's bound."""
+    R = 16
+    rng = np.random.default_rng(8)
+    batches = []
+    for k in range(1, 6):
+        dims = np.array([1, 10007 * k, 48], np.uint64)
+        i = rng.integers(0, int(dims[1]), 30000)
+        c = np.stack([np.zeros(30000, np.int64), i, rng.integers(0, 3, 30000) * R + i % R])
+        c = np.unique(c, axis=1).astype(np.uint64)
+        v = rng.uniform(0.5, 1.5, c.shape[1]).astype(np.float32).astype(np.float64)
+        batches.append(dict(dims=dims, cidx=c, vals=v))
+    iv = synth.init_values(60000 * R, seed=9).astype(np.float32).astype(np.float64)
+    outs, _, _ = run_gpu(batches, R, 4, 0.0, 0, iv)
+    oo, _, _ = O.cpstream(batches, 0, R, 4, 0.0, 0, iv)
+    assert outs[1].shape == (50035, R)
+    for a, c in zip(outs, oo):
+        assert normwise(a, c) <= 1e-4, normwise(a, c)
