@@ -591,15 +591,16 @@ __device__ __forceinline__ void det_entry(DetTile<R, NPW>& d, int e, uint32_t ro
     d.val[e][q * G + sub] = make_float4(acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
 }
 
+__device__ __forceinline__ void add4(float4& x, const float4& y) {
+  x.x += y.x;
+  x.y += y.y;
+  x.z += y.z;
+  x.w += y.w;
+}
+
 // A finished run of the deterministic walk that is its row's only one.
 __device__ __forceinline__ void det_put(const MttkrpArgs& a, float4* o, float4 x) {
-  if (a.det_add) {
-    const float4 y = *o;
-    x.x += y.x;
-    x.y += y.y;
-    x.z += y.z;
-    x.w += y.w;
-  }
+  if (a.det_add) add4(x, *o);
   *o = x;
 }
 
@@ -754,20 +755,22 @@ struct TilePart {
 };
 
 // The lane groups' open runs at the end of a chunk: when a whole warp ends on
-// one row (a hot row, or a mode of few rows) its groups are summed first, in
-// group order, and the row is updated once instead of once per group.  Groups
+// one row (a hot row, or a mode of few rows) its groups are summed first, by a
+// tree, and the row is updated once instead of once per group.  Groups
 // of G lanes; lanes past the last group, and groups without records (the ragged
 // end of a tile), hold zeros.
 template <int V>
 __device__ __forceinline__ bool merge_groups(uint32_t row, float (&acc)[V], int G, int npw, int lane) {
   const uint32_t row0 = __shfl_sync(0xffffffffu, row, 0);
   if (!__all_sync(0xffffffffu, row == row0 || row == kNoRow || lane >= G * npw)) return false;
-  for (int g = 1; g < npw; ++g)
+  for (int live = npw, half; live > 1; live = half) {
+    half = (live + 1) / 2;
 #pragma unroll
     for (int q = 0; q < V; ++q) {
-      const float x = __shfl_sync(0xffffffffu, acc[q], (g * G + lane) & 31);
-      if (lane < G) acc[q] += x;
+      const float x = __shfl_sync(0xffffffffu, acc[q], (lane + half * G) & 31);
+      if (lane < (live - half) * G) acc[q] += x;
     }
+  }
   return true;
 }
 
@@ -853,11 +856,14 @@ __device__ __forceinline__ void det_walk_chunk(const MttkrpArgs& a, uint32_t chu
       if (prev >= 0 && d.one[prev / kPerWarp]) prev -= prev % kPerWarp;  // (a merged warp's one entry is its first)
       while (prev >= 0 && d.row[prev] == kNoRow) --prev;
       if (prev >= 0 && d.row[prev] == r) continue;  // not the first entry of its run
-      float4 x = prev < 0 && open == r ? d.carry[cur][q] : make_float4(0.f, 0.f, 0.f, 0.f);
+      float4 x = make_float4(0.f, 0.f, 0.f, 0.f), upper = x, part = x;
       bool ends = false;
       // (a merged warp has one entry; of the others four are loaded at a time, or
       // each would wait for the one before it: 90 cycles an entry, 12 us for a
-      // chunk of one row at rank 8)
+      // chunk of one row at rank 8.  The entries of a warp are summed in `part`, the
+      // warps of each half of the block in x and `upper`: one after the other all
+      // made the error of rows of some hundred nonzeros, 500 rows at rank 8 7.2e-8
+      // rms from 50,000 nonzeros and 6.7e-8 from 1M, now 4.5e-8 both)
       for (int k = e; k < E && !ends;) {
         const bool merged = d.one[k / kPerWarp];
         const int stop = k - k % kPerWarp + kPerWarp;
@@ -876,13 +882,19 @@ __device__ __forceinline__ void det_walk_chunk(const MttkrpArgs& a, uint32_t chu
             ends = true;
             continue;
           }
-          x.x += y[u].x;
-          x.y += y[u].y;
-          x.z += y[u].z;
-          x.w += y[u].w;
+          add4(part, y[u]);
         }
         k = merged ? stop : min(k + kAhead, stop);
+        if (k == stop || ends) {
+          if (k <= E / 2)
+            add4(x, part);
+          else
+            add4(upper, part);
+          part = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
       }
+      add4(x, upper);
+      if (prev < 0 && open == r) add4(x, d.carry[cur][q]);
       if (ends) {
         put(r, q, x);
       } else {
@@ -915,12 +927,16 @@ __global__ void __launch_bounds__(kMttkrpThreads, 3) det_walk_kernel(const Mttkr
 }
 
 // The chunks' slots (rows non-decreasing; a row in them is in no other run):
-// a block per run of equal rows, its slots summed with a fixed split and a fixed
-// tree, then written or added to the row.  What it waits for is one SM's loads
-// of a single row's slots (780 at rank 64: 15 us with the loads one after the
-// other, 8.9 us with eight in the air); 3 us when every row has a few slots.
-// Block `first` of `step` that share the item.
-__device__ __forceinline__ void det_fix_slots(const MttkrpArgs& a, uint32_t nslots, int R, float4* part,
+// a block per run of equal rows, its slots summed in float64 with a fixed split
+// and a fixed tree, then written or added to the row (60 rows at rank 8 from 1M
+// nonzeros: 4.9e-8 rms error with float32 sums, 3.1e-8 so, in the same time).
+// What it waits for is one SM's loads of a single row's slots (780 at rank 64:
+// 15 us with the loads one after the other, 8.9 us with eight in the air); 3 us when
+// every row has a few slots.  Block `first` of `step` that share the item.
+struct __align__(16) Sum4 {
+  double x, y, z, w;
+};
+__device__ __forceinline__ void det_fix_slots(const MttkrpArgs& a, uint32_t nslots, int R, Sum4* part,
                                               uint32_t first, uint32_t step) {
   const uint32_t* rows = a.det_rows;
   const float4* vals = reinterpret_cast<const float4*>(a.det_vals);
@@ -943,19 +959,20 @@ __device__ __forceinline__ void det_fix_slots(const MttkrpArgs& a, uint32_t nslo
       end += same;
       if (same < 1024) break;
     }
-    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    Sum4 x = {0.0, 0.0, 0.0, 0.0};
     for (uint32_t k = i + s; k < end; k += 8 * S) {  // (eight loads in the air)
       float4 y[8];
 #pragma unroll
       for (int u = 0; u < 8; ++u)
         y[u] = k + u * S < end ? vals[(size_t)(k + u * S) * Q + q] : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        x.x += y[u].x;
-        x.y += y[u].y;
-        x.z += y[u].z;
-        x.w += y[u].w;
-      }
+      for (int stride = 4; stride >= 1; stride >>= 1)
+#pragma unroll
+        for (int u = 0; u < stride; ++u) add4(y[u], y[u + stride]);
+      x.x += y[0].x;
+      x.y += y[0].y;
+      x.z += y[0].z;
+      x.w += y[0].w;
     }
     part[threadIdx.x] = x;
     __syncthreads();
@@ -963,8 +980,8 @@ __device__ __forceinline__ void det_fix_slots(const MttkrpArgs& a, uint32_t nslo
     while (live > 1 && live / 2 >= (int)(end - i)) live /= 2;  // (the rest are zeros)
     for (int stride = live / 2; stride >= 1; stride >>= 1) {
       if (s < stride) {
-        const float4 y = part[(s + stride) * Q + q];
-        float4& m = part[s * Q + q];
+        const Sum4 y = part[(s + stride) * Q + q];
+        Sum4& m = part[s * Q + q];
         m.x += y.x;
         m.y += y.y;
         m.z += y.z;
@@ -972,20 +989,24 @@ __device__ __forceinline__ void det_fix_slots(const MttkrpArgs& a, uint32_t nslo
       }
       __syncthreads();
     }
-    if (s == 0) det_put(a, reinterpret_cast<float4*>(a.out + (size_t)row * R) + q, part[q]);
+    if (s == 0) {
+      const Sum4 t = part[q];
+      det_put(a, reinterpret_cast<float4*>(a.out + (size_t)row * R) + q,
+              make_float4((float)t.x, (float)t.y, (float)t.z, (float)t.w));
+    }
     __syncthreads();
   }
 }
 
 __global__ void __launch_bounds__(256) det_fix_kernel(const MttkrpArgs a, uint32_t nslots, int R) {
-  __shared__ float4 part[256];
+  __shared__ Sum4 part[256];
   det_fix_slots(a, nslots, R, part, blockIdx.x, gridDim.x);
 }
 
 // ------------------------------------------------ deterministic fix-up
 //
-// (Lines that are not decoded: 2 modes, or more than 5.)  The slots of DET hold, in line order, the first and last run of every
-// sub-range; their rows are non-decreasing, and a row appears in the slots
+// (Lines that are not decoded: 2 modes, or more than 5.)  The slots of DET hold,
+// in line order, the first and last run of every sub-range; their rows are non-decreasing, and a row appears in the slots
 // only if it is in none of the interior runs.  A chain (maximal stretch of
 // slots with one row) is summed in slot order, by one warp when it is short
 // and by one block with a fixed split and a fixed tree when it is long (a
@@ -1247,7 +1268,7 @@ __global__ void __launch_bounds__(kMttkrpThreads, 3)
 }
 
 __global__ void __launch_bounds__(256) det_fix_group_kernel(Strided<DetItem> items, int R) {
-  __shared__ float4 part[256];
+  __shared__ Sum4 part[256];
   const ItemShare sh(*items.count);
   for (uint32_t s = sh.item; s < sh.items; s += sh.stride) {
     const DetItem& it = items[s];
