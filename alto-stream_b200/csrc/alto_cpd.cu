@@ -221,20 +221,20 @@ extern "C" alto_status alto_cpd_als(alto_tensor* t, int rank, double* const* U_h
   const bool bf16 = storage == ALTO_BF16;
 
   DevBuf U[ALTO_MAX_MODES], Ub[ALTO_MAX_MODES];
-  DevBuf grams, W, status, mbuf, xbuf, stats, lam, scal, gscr, dscr, stage64;
+  DevBuf grams, W, status, mbuf, stats, lam, scal, gscr, dscr, stage64;
   uint64_t max_dim = 0;
   for (int m = 0; m < N; ++m) max_dim = std::max<uint64_t>(max_dim, t->dims[m]);
   ALTO_TRY(grams.ensure((size_t)N * R * R * 8));
   ALTO_TRY(W.ensure((size_t)R * R * 8));
   ALTO_TRY(status.ensure(16));
   ALTO_TRY(mbuf.ensure(max_dim * R * 4));
-  ALTO_TRY(xbuf.ensure(max_dim * R * 4));
   ALTO_TRY(stats.ensure(apply_scratch_bytes(max_dim, R)));
   ALTO_TRY_CUDA(cudaMemsetAsync(stats.p, 0, 4, st));
   ALTO_TRY(lam.ensure(R * 8));
   // [0] normX, then per iteration of a window {dot stats (3), normU}
   ALTO_TRY(scal.ensure((1 + 4 * kFitWindow) * 8));
   ALTO_TRY(stage64.ensure(max_dim * R * 8));
+  float* xbuf = stage64.as<float>();  // the solves' rows before their normalisation (the iterations stage nothing)
   for (int m = 0; m < N; ++m) {
     const uint64_t n = t->dims[m] * (uint64_t)R;
     ALTO_TRY(U[m].ensure(n * 4));
@@ -277,9 +277,9 @@ extern "C" alto_status alto_cpd_als(alto_tensor* t, int rank, double* const* U_h
       ALTO_TRY(run_mttkrp(t, j, fac, fdt, R, mbuf.as<float>(), 0, variant[j], st));
       ALTO_TRY(solve_setup(grams.as<double>(), N, all & ~(1u << j), R, kSolveRidgeDiagFallback, 1e-3,
                            W.as<double>(), status.as<int>(), nullptr, st));
-      ALTO_TRY(apply_lambda(mbuf.as<float>(), W.as<double>(), I, R, xbuf.as<float>(), it == 0 ? 0 : 1, stats.p,
+      ALTO_TRY(apply_lambda(mbuf.as<float>(), W.as<double>(), I, R, xbuf, it == 0 ? 0 : 1, stats.p,
                             lam.as<double>(), st));
-      ALTO_TRY(scale_gram(xbuf.as<float>(), I, R, lam.as<double>(), U[j].as<float>(),
+      ALTO_TRY(scale_gram(xbuf, I, R, lam.as<double>(), U[j].as<float>(),
                           bf16 ? Ub[j].as<__nv_bfloat16>() : nullptr, grams.as<double>() + (size_t)j * R * R, gscr,
                           st));
     }

@@ -165,3 +165,26 @@ def test_copies_that_do_not_fit(spare):
     _, _, fits, _ = A.cpd_alto(t, U0, np.ones(R), R, 4, 0.0)  # with room again
     np.testing.assert_allclose(fits, want, rtol=0, atol=1e-5)
     assert (t.device_bytes() - before) / (16 * nnz) > 2.9
+
+
+def test_room_for_factors_and_staging():
+    """A call needs the factors, the MTTKRP's output and one float64 factor of device
+    memory (256 + 256 + 512 MiB here), and no fourth array of a factor's size."""
+    import torch
+
+    g = torch.Generator(device="cuda")
+    g.manual_seed(2)
+    dims, nnz, R = np.array([1 << 21, 64, 64], np.uint64), 100000, 32
+    idx = [torch.randint(0, int(d), (nnz,), generator=g, device="cuda") for d in dims]
+    t = A.create_alto(dims, idx, torch.rand(nnz, generator=g, device="cuda") + 0.5)
+    U0 = init_model(dims, R, 4)
+    _, _, want, _ = A.cpd_alto(t, U0, np.ones(R), R, 2, 0.0)
+    A.release_memory()
+    torch.cuda.empty_cache()
+    filler = torch.empty(torch.cuda.mem_get_info()[0] - (1150 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        _, _, fits, _ = A.cpd_alto(t, U0, np.ones(R), R, 2, 0.0)
+    finally:
+        del filler
+        torch.cuda.empty_cache()
+    np.testing.assert_allclose(fits, want, rtol=0, atol=1e-5)
