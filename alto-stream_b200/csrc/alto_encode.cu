@@ -1162,10 +1162,10 @@ alto_status build_sorted_line(alto_tensor* t, int mode, cudaStream_t st) {
     ALTO_LAUNCHED();
   }
   s.ntiles = t->ntiles;
-  ALTO_TRY(tensor_ensure(t, s.tile_iv, (size_t)std::max<uint32_t>(t->ntiles, 1) * t->nmodes * 2 * 4));
   // (tile intervals are read only by shared-memory staging, which never
-  // walks a sorted copy; the decoded copies carry none)
+  // walks a sorted copy; the decoded copies have none)
   if (t->ntiles && s.hw != kDecoded) {
+    ALTO_TRY(tensor_ensure(t, s.tile_iv, (size_t)t->ntiles * t->nmodes * 2 * 4));
     tile_interval_kernel<<<t->ntiles, 256, 0, st>>>(s.line.p, t->dec, n32, t->tile_nnz,
                                                     s.tile_iv.as<uint32_t>());
     ALTO_LAUNCHED();

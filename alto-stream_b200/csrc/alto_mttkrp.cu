@@ -2034,22 +2034,25 @@ alto_status det_prepare(alto_tensor* t, int mode, const void* const* factors, in
   }
   ALTO_TRY(tensor_ensure(t, t->det_rows, std::max<uint64_t>(nslots, 1) * 4));
   ALTO_TRY(tensor_ensure(t, t->det_vals, std::max<uint64_t>(nslots, 1) * rank * 4));
-  // long chains: each has more than kShortChain slots; segments:
-  // sum over chains of ceil(len / kChainSeg)
-  const uint64_t max_chains = nslots / (kShortChain + 1) + 1;
-  const uint64_t max_segs = nslots / kChainSeg + max_chains;
-  auto up = [](uint64_t x) { return (x + 255) & ~uint64_t(255); };
-  const uint64_t o_chains = 256, o_segs = o_chains + up(max_chains * sizeof(uint4)),
-                 o_part = o_segs + up(max_segs * sizeof(uint2)), bytes = o_part + max_segs * rank * 4;
-  const size_t before = t->det_long.bytes;  // a new allocation starts with zero counters
-  ALTO_TRY(tensor_ensure(t, t->det_long, bytes));
-  if (t->det_long.bytes != before) ALTO_TRY_CUDA(cudaMemsetAsync(t->det_long.p, 0, 16, st));
   a.det_rows = t->det_rows.as<uint32_t>();
   a.det_vals = t->det_vals.as<float>();
-  char* base = t->det_long.as<char>();
   item->a = a;
-  item->dl = DetLong{reinterpret_cast<uint32_t*>(base), reinterpret_cast<uint4*>(base + o_chains),
-                     reinterpret_cast<uint2*>(base + o_segs), reinterpret_cast<float*>(base + o_part)};
+  item->dl = DetLong{};
+  if (hw != kDecoded) {
+    // long chains: each has more than kShortChain slots; segments:
+    // sum over chains of ceil(len / kChainSeg)
+    const uint64_t max_chains = nslots / (kShortChain + 1) + 1;
+    const uint64_t max_segs = nslots / kChainSeg + max_chains;
+    auto up = [](uint64_t x) { return (x + 255) & ~uint64_t(255); };
+    const uint64_t o_chains = 256, o_segs = o_chains + up(max_chains * sizeof(uint4)),
+                   o_part = o_segs + up(max_segs * sizeof(uint2)), bytes = o_part + max_segs * rank * 4;
+    const size_t before = t->det_long.bytes;  // a new allocation starts with zero counters
+    ALTO_TRY(tensor_ensure(t, t->det_long, bytes));
+    if (t->det_long.bytes != before) ALTO_TRY_CUDA(cudaMemsetAsync(t->det_long.p, 0, 16, st));
+    char* base = t->det_long.as<char>();
+    item->dl = DetLong{reinterpret_cast<uint32_t*>(base), reinterpret_cast<uint4*>(base + o_chains),
+                       reinterpret_cast<uint2*>(base + o_segs), reinterpret_cast<float*>(base + o_part)};
+  }
   item->nslots = (uint32_t)nslots;
   item->hw = hw;
   item->out_floats = t->dims[mode] * (uint64_t)rank;

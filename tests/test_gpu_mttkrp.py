@@ -414,6 +414,21 @@ def test_deterministic_error_of_short_runs(rows, nnz):
     assert sq ** 0.5 <= (14 / 3) ** 0.5 * 2.53e-8, sq ** 0.5
 
 
+@pytest.mark.parametrize("dims,per", [([300, 400, 500], 16), ([30, 40, 50, 60], 20), ([30, 40, 50, 60, 7], 24)])
+def test_row_sorted_copy_bytes(dims, per):
+    """A decoded copy is its records (and 16 of padding), and nothing else."""
+    import torch
+
+    rng = np.random.default_rng(5)
+    nnz = 20000
+    t = A.create_alto(np.array(dims, np.uint64), np.stack([rng.integers(0, d, nnz) for d in dims]).astype(np.uint64),
+                      rng.random(nnz))
+    before = t.device_bytes()
+    F = [torch.rand((d, 16), device="cuda") for d in dims]
+    t.mttkrp(0, F, 16, variant=A.SORTED)
+    assert t.device_bytes() - before == (nnz + 16) * per
+
+
 # ------------------------------------------------------------ shards
 
 @pytest.mark.parametrize("nparts", [1, 3, 8])
