@@ -34,7 +34,8 @@ struct MttkrpArgs {
   LineDecode dec;
   FactorSet fac;
   FactorSet in;  // the input modes' factors in mode order (kDecoded walks)
-  uint64_t in_rows;  // their rows
+  uint64_t in_rows;   // their rows
+  uint64_t out_rows;  // the output's rows
   float* out;
 };
 

@@ -1455,7 +1455,7 @@ __device__ __forceinline__ DecRec<NIN> any_rec(const MttkrpArgs& a, uint32_t i) 
   }
 }
 
-template <typename FT, int VW, int NIN, bool DEC>
+template <typename FT, int VW, int NIN, bool DEC, bool STAGE>
 __global__ void __launch_bounds__(kMttkrpThreads, 4) any_walk_kernel(const MttkrpArgs a, int rank) {
   constexpr int V = 4, Q = V / VW;
   constexpr int U = NIN <= 3 ? 2 : 1;
@@ -1475,6 +1475,11 @@ __global__ void __launch_bounds__(kMttkrpThreads, 4) any_walk_kernel(const Mttkr
     mine[q] = c < cols && !idle;
     col[q] = c0 + min(c, cols - VW);
   }
+  extern __shared__ float any_smem[];  // STAGE: the output's rows, this window's columns
+  if constexpr (STAGE) {
+    for (int p = threadIdx.x; p < a.stage_rows * cols; p += kMttkrpThreads) any_smem[p] = 0.f;
+    __syncthreads();
+  }
   const uint32_t last = a.nnz - 1;
   const uint32_t ct = a.chunk_tiles ? a.chunk_tiles : 1;
   const uint32_t nchunks = (a.ntiles + ct - 1) / ct;
@@ -1488,10 +1493,17 @@ __global__ void __launch_bounds__(kMttkrpThreads, 4) any_walk_kernel(const Mttkr
 #pragma unroll
     for (int q = 0; q < V; ++q) acc[q] = 0.f;
     auto flush = [&]() {
-      float* o = a.out + (size_t)cur * rank;
+      if constexpr (STAGE) {
+        float* o = any_smem + (size_t)cur * cols - c0;
 #pragma unroll
-      for (int q = 0; q < Q; ++q)
-        if (mine[q]) any_flush<VW>(o + col[q], acc + q * VW);
+        for (int q = 0; q < V; ++q)
+          if (mine[q / VW]) atomicAdd(o + col[q / VW] + q % VW, acc[q]);
+      } else {
+        float* o = a.out + (size_t)cur * rank;
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+          if (mine[q]) any_flush<VW>(o + col[q], acc + q * VW);
+      }
     };
     const uint32_t t_end = min(c * ct + ct, a.ntiles);
     for (uint32_t tile = c * ct; tile < t_end; ++tile) {
@@ -1548,6 +1560,11 @@ __global__ void __launch_bounds__(kMttkrpThreads, 4) any_walk_kernel(const Mttkr
     }
     const bool one = NPW > 1 && merge_groups<V>(cur, acc, G, NPW, lane);
     if (cur != kNoRow && !(one && grp)) flush();
+  }
+  if constexpr (STAGE) {
+    __syncthreads();
+    for (int p = threadIdx.x; p < a.stage_rows * cols; p += kMttkrpThreads)
+      if (any_smem[p] != 0.f) atomicAdd(a.out + (size_t)(p / cols) * rank + c0 + p % cols, any_smem[p]);
   }
 }
 
@@ -1690,15 +1707,44 @@ static alto_status launch_walk(const MttkrpArgs& a, cudaStream_t st) {
   return ALTO_OK;
 }
 
+// A line's output mode of few rows is summed in shared memory, block by block, where
+// the rank is no multiple of four: a lane group's update is then two to four
+// atomics, and these lengthen the chain of a hot row (6 modes, 500,000 nonzeros, 70
+// rows: rank 3 391 us, a warp per nonzero 273, so 23; rank 10 165, 136 and 37).
+// Fewer blocks where each would update the rows more often than it has nonzeros for
+// them, as long as its groups have at most two steps (20,000 nonzeros, 70 rows,
+// rank 3: 24.8 us, a warp per nonzero 14.9, so 9.3; with up to four steps 300 rows at
+// rank 10 took 11.4 us instead of 8.4).
+constexpr uint64_t kAnyStageBytes = 32 << 10;
+constexpr uint64_t kAnyStageSteps = 2;
+
 template <typename FT, int VW, int NIN, bool DEC>
 static alto_status launch_any(const MttkrpArgs& a, int rank, cudaStream_t st) {
   const unsigned windows = (unsigned)((rank + 127) / 128);
   if (!a.nnz) return ALTO_OK;
   MttkrpArgs b = a;
-  even_tiles(&b, (unsigned)num_sms() * 4, 128);
-  const unsigned grid = std::min<unsigned>(b.ntiles, (unsigned)num_sms() * 4);
+  unsigned full = (unsigned)num_sms() * 4;
+  const uint64_t cols = std::min(rank, 128), groups = kMttkrpWarps * (32 / ((cols + 3) / 4));
+  b.stage_rows = 0;
+  if (!DEC && VW < 4 && a.out_rows * cols * 4 <= kAnyStageBytes) {
+    const uint64_t few = std::min<uint64_t>(std::max<uint64_t>(a.nnz / a.out_rows, 1), full);
+    if (few == full || a.nnz <= kAnyStageSteps * groups * few) {
+      full = (unsigned)few;
+      b.stage_rows = (int)a.out_rows;
+    }
+  }
+  even_tiles(&b, full, kMttkrpWarps);  // (the unit is a nonzero a warp: short walks want the blocks)
+  const unsigned grid = std::min<unsigned>(b.ntiles, full);
   b.chunk_tiles = chunk_tiles_for(b.ntiles, grid);
-  any_walk_kernel<FT, VW, NIN, DEC><<<dim3(grid, windows), kMttkrpThreads, 0, st>>>(b, rank);
+  const dim3 blocks(grid, windows);
+  if constexpr (!DEC && VW < 4) {
+    if (b.stage_rows) {
+      any_walk_kernel<FT, VW, NIN, false, true><<<blocks, kMttkrpThreads, b.stage_rows * cols * 4, st>>>(b, rank);
+      ALTO_LAUNCHED();
+      return ALTO_OK;
+    }
+  }
+  any_walk_kernel<FT, VW, NIN, DEC, false><<<blocks, kMttkrpThreads, 0, st>>>(b, rank);
   ALTO_LAUNCHED();
   return ALTO_OK;
 }
@@ -1944,6 +1990,7 @@ static alto_status fill_args(alto_tensor* t, int mode, const void* const* factor
   a.out = out;
   int j = 0;
   a.in_rows = 0;
+  a.out_rows = t->dims[mode];
   for (int m = 0; m < t->nmodes; ++m) {
     a.fac.f[m] = factors[m];
     if (m == mode) continue;

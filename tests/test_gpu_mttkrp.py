@@ -429,6 +429,22 @@ def test_row_sorted_copy_bytes(dims, per):
     assert t.device_bytes() - before == (nnz + 16) * per
 
 
+@pytest.mark.parametrize("dims,nnz,R", [
+    ([2730, 5, 30], 3001, 3),  # 32,760 bytes of rows: staged
+    ([2731, 5, 30], 3001, 3),  # 32,772: not; 5 rows: a full grid of staging blocks
+    ([7, 600, 40, 3, 50, 60], 20003, 1),
+    ([70, 300], 4099, 10),
+    ([62, 11, 40, 9], 9001, 130),  # two windows of columns, of 128 and 2
+    ([1, 3, 2, 2, 2, 2, 2, 2], 40, 5)])
+@pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
+def test_any_rank_line_of_few_rows(dims, nnz, R, dtype):
+    import torch
+
+    rng = np.random.default_rng(nnz)
+    cidx = np.stack([rng.integers(0, d, nnz) for d in dims]).astype(np.uint64)
+    check_modes(dims, cidx, rng.uniform(-1.0, 1.0, nnz), R, (A.ATOMIC, A.AUTO), getattr(torch, dtype))
+
+
 # ------------------------------------------------------------ shards
 
 @pytest.mark.parametrize("nparts", [1, 3, 8])
