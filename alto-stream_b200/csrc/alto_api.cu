@@ -36,7 +36,8 @@ HandlePool* handle_pool(int dev) {
     props.location.id = dev;
     cudaStream_t st = nullptr;
     cudaMemPool_t p = nullptr;
-    if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess || cudaMemPoolCreate(&p, &props) != cudaSuccess) {
+    if (cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaMemPoolCreate(&p, &props) != cudaSuccess) {
       if (st) cudaStreamDestroy(st);
       cudaGetLastError();  // (pool_alloc does without)
       return nullptr;
@@ -399,7 +400,8 @@ alto_status alto_tensor_device_bytes(const alto_tensor* t, uint64_t* bytes) {
   }
   uint64_t b = t->line.bytes + t->perm.bytes + t->tile_iv.bytes + t->prtn_iv.bytes + t->scratch.bytes +
                t->scan_scratch.bytes + t->err.bytes;
-  for (int m = 0; m < ALTO_MAX_MODES; ++m) b += t->sorted[m].line.bytes + t->sorted[m].extra.bytes + t->sorted[m].tile_iv.bytes;
+  for (int m = 0; m < ALTO_MAX_MODES; ++m)
+    b += t->sorted[m].line.bytes + t->sorted[m].extra.bytes + t->sorted[m].tile_iv.bytes;
   *bytes = b;
   return ALTO_OK;
 }

@@ -465,13 +465,15 @@ __global__ void __launch_bounds__(kMttkrpThreads, 3)
 // SORTED and DETERMINISTIC on 3- to 5-mode tensors: the walk over a kDecoded
 // copy.  As warp_range, a warp's range is split into NPW contiguous
 // sub-ranges, one per lane group of G = R / V lanes; each lane holds V floats
-// of every row.  The walk is bound by issue slots, not by a bandwidth (5
-// modes at rank 64: 64 warp instructions per nonzero with a decoded key and
-// four floats a lane), so a step does as little as possible besides its row
-// loads: the rows come decoded, target last (no decode, no selection among
-// the modes), the loads past the end of a sub-range are clamped to the last
-// record instead of being predicated, and V is as wide as the registers
-// allow, which divides the per-nonzero overhead by the nonzeros in flight.
+// of every row.  A walk over the line's keys with four floats a lane was bound by
+// issue slots (5 modes at rank 64: 64 warp instructions per nonzero), so a step
+// does as little as possible besides its row loads: the rows come decoded, target
+// last (no decode, no selection among the modes), the loads past the end of a
+// sub-range are clamped to the last record instead of being predicated, and V is as
+// wide as the registers allow, which divides the per-nonzero overhead by the
+// nonzeros in flight.  Now the latency of the gathers bounds it (20 to 22
+// instructions there, issue slots 33% busy in float32 and 55% in bfloat16, L1 66% and
+// 58%; long walks of 3 modes 8.5 instructions and 40%).
 
 template <int NIN>
 struct DecRec {
@@ -800,7 +802,7 @@ __global__ void __launch_bounds__(kMttkrpThreads, WalkCfg<R, FT, NIN, false, DEE
 
 // Chunk `chunk` of the deterministic walk (one block): consecutive tiles, each
 // cut among the lane groups as any walk's.  What a group starts and ends with
-// meets in shared memory, where runs that cross groups are summed in record
+// meets in shared memory, where runs that cross groups are summed in a fixed
 // order; the block's open run is carried from tile to tile, its first and last
 // run go to the chunk's two slots (det_fix_kernel), and every other run is its
 // row's only one and is written without atomics.  So the slots are two per
@@ -1394,10 +1396,12 @@ __global__ void __launch_bounds__(kMttkrpThreads, 3)
 // factors, VW the widest of 4, 2, 1 that divides the rank and that every
 // pointer is aligned for.  Sub-ranges, runs and chunks are the specialised
 // walk's (one vector atomic per run and lane); ranks above 128 take one
-// column window of 128 per blockIdx.y.  Bound by issue slots and, where runs
-// are short, by atomics.  A warp per nonzero with a scalar atomic per
-// factor, its form before, took 802 us per mode on a ragged 4-mode tensor of 3M
-// nonzeros at rank 10, at any of the line orders.
+// column window of 128 per blockIdx.y.  Bound by the L1's load path (rank 10 over a
+// row-sorted copy: 91% busy, 72 us for 3M nonzeros of a ragged 4-mode tensor) and,
+// where runs are short, by atomics.  A warp per nonzero with a scalar atomic per
+// factor, its form before, took 802 us there, at any of the line orders.
+// STAGE: the runs of a line's mode of few rows are added in shared memory first
+// (launch_any).
 
 template <typename FT, int VW>
 __device__ __forceinline__ void any_piece(const char* p, float* x) {

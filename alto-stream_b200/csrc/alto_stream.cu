@@ -997,8 +997,9 @@ __global__ void __launch_bounds__(kAdmmThreads, TileMap<R>::kMinBlocks)
   }
 }
 
-// (One warp, a lane per slot, as group_converge_kernel.)  After a chunk of ADMM sweeps (first: the one every mode starts with): the
-// chunk loop goes on while some slot's ADMM of mode j sweeps.
+// After a chunk of ADMM sweeps (first: the one every mode starts with): the
+// chunk loop goes on while some slot's ADMM of mode j sweeps.  One warp, a lane
+// per slot, as group_converge_kernel.
 __global__ void group_admm_cond_kernel(SlotDesc* __restrict__ tab, GroupCtl* __restrict__ ctl,
                                        cudaGraphConditionalHandle h, int first) {
   bool any = false;
